@@ -629,6 +629,162 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
     if (warp == 0) tc::tmem_dealloc(tmem, p.tmem_cols);
 }
 
+// ---------------------------------------------------------------------------
+// Weight gradients of a 3x3 convolution: dW[dy][dx][co][ci] += sum over pixels p of
+// dZ[p][co] * X[p + (dy - 1, dx - 1)][ci], as one tcgen05 contraction over pixels.
+//
+// Both operands are read as the NHWC tensors store them (MN-major: channels contiguous, one
+// pixel = one K row), so nothing is transposed in memory. A tile is kWgRows x bw pixels of X
+// with one halo column on each side, and the (kWgRows + 2) x bw pixels of dZ around it, both
+// by one TMA box (zero fill outside the image = zero padding). All 9 taps of 16 pixels are one
+// MMA: the operands' 32-channel groups lie a leading offset apart in shared memory, and that
+// offset is one pixel for A (M = 128: X shifted by dx = 0, 1, 2 and a fourth, unused shift) and
+// one image row for B (N = 3 x co_block: dZ rows y - 1, y, y + 1, that is dy = 2, 1, 0). The
+// shifted views start at any pixel: swizzling works on absolute shared-memory addresses.
+//
+// A CTA owns n_ci blocks of 32 input channels and one block of output channels, walks its
+// share of the tiles and adds its FP32 sums to dW by atomics (lane = input channel, so a warp's
+// add is one 128-byte line).
+//
+// Bound: operand fetch of the tensor core at full resolution, launch and first-tile latency at
+// the deep levels. On a batch of 16 crops of 128 x 128 the 19 layers of the denoiser's backward
+// pass take 0.34 ms in this form (9 to 38 us each, cold cache); as 9 shifted transposes and 9
+// GEMMs a layer, each reading its operands from HBM again, they took 12.8 ms.
+//
+// One CTA of 128 threads: warp 0 lane 0 issues TMA, warp 1 lane 0 the MMAs, warps 0-2 (one per
+// dx) drain TMEM. Every wait is bounded as in the kernels above.
+// ---------------------------------------------------------------------------
+constexpr int kWgRows = 8;     // X rows of a tile
+constexpr int kWgMaxCi = 5;    // blocks of 32 input channels per CTA (5 x 96 TMEM columns)
+constexpr int kWgMaxStages = 4;
+
+struct WgradParams {
+    int tiles_x, tiles_y, num_tiles;
+    int bw;                   // tile width: 8, 16 or 32
+    int n_ci;                 // blocks of 32 input channels per CTA
+    int co_block;             // 32 or 64 output channels
+    int stages;
+    uint32_t x_stride;        // bytes of one 32-channel X tile (1024-aligned slot)
+    uint32_t stage_stride;
+    uint32_t x_bytes, z_bytes;
+    uint32_t tmem_cols;
+    int Cin, Cout;
+    float* dw;
+};
+
+__global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtensorMap tmX,
+                                                  const __grid_constant__ CUtensorMap tmZ, const WgradParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)p.stages * p.stage_stride);
+    uint64_t* empty = full + kWgMaxStages;
+    uint64_t* done = empty + kWgMaxStages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int co0 = blockIdx.y * p.co_block;
+    const int ci0 = blockIdx.z * p.n_ci * 32;
+    const int n_ci = min(p.n_ci, p.Cin / 32 - (int)blockIdx.z * p.n_ci);
+    const uint32_t acc_cols = 3u * (uint32_t)p.co_block;
+
+    if (warp == 0) tc::tmem_alloc(tmem_slot, p.tmem_cols);
+    if (threadIdx.x == 32) {
+        for (int s = 0; s < p.stages; ++s) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        tc::mbar_init(done, 1);
+        tc::fence_barrier_init();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0 && lane == 0) {
+        uint32_t it = 0, s = 0;
+        for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
+            if (it >= (uint32_t)p.stages && !tc::mbar_wait(&empty[s], ((it / p.stages) - 1) & 1, kWaitBudget)) {
+                set_error(21);
+                break;
+            }
+            const int per_img = p.tiles_x * p.tiles_y;
+            const int n_img = t / per_img, r = t % per_img;
+            const int y0 = (r / p.tiles_x) * kWgRows, x0 = (r % p.tiles_x) * p.bw;
+            uint8_t* st = smem + s * p.stage_stride;
+            tc::mbar_arrive_expect_tx(&full[s], (uint32_t)n_ci * p.x_bytes + p.z_bytes);
+            tc::tma_load_4d(st, &tmZ, &full[s], co0, x0, y0 - 1, n_img);
+            st += p.stage_stride - p.n_ci * p.x_stride;
+            for (int c = 0; c < n_ci; ++c)
+                tc::tma_load_4d(st + c * p.x_stride, &tmX, &full[s], ci0 + 32 * c, x0 - 1, y0, n_img);
+            if (++s == (uint32_t)p.stages) s = 0;
+        }
+        // drain: every issued copy must have landed before the CTA may exit
+        for (uint32_t q = 0; q < (uint32_t)p.stages && q < it; ++q) {
+            const uint32_t last = ((it - 1 - q) / p.stages) * p.stages + q;
+            if (!tc::mbar_wait(&full[q], (last / p.stages) & 1, kWaitBudget)) set_error(22);
+        }
+    } else if (warp == 1 && lane == 0) {
+        const uint32_t zrow = 2u * (uint32_t)p.co_block;     // bytes of one dZ pixel (its swizzle width)
+        const uint32_t xrow = 64u;
+        const uint32_t ximg = (uint32_t)(p.bw + 2) * xrow;   // one image row of the X tile
+        // K = 16 pixels: two groups of 8, of one image row or, for 8-wide tiles, of two
+        const uint32_t segs = p.bw >= 16 ? (uint32_t)p.bw / 16 : 1, row_step = p.bw >= 16 ? 1 : 2;
+        const uint64_t ax = tc::smem_desc_mn(0, xrow, p.bw >= 16 ? 8u * xrow : ximg, 4u);
+        const uint64_t bz = tc::smem_desc_mn(0, (uint32_t)p.bw * zrow, 8u * zrow, p.co_block == 64 ? 2u : 4u);
+        const uint32_t idesc = tc::idesc_bf16(128, 3u * (uint32_t)p.co_block) | tc::kIdescMnMajorAB;
+        uint32_t it = 0, s = 0;
+        for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
+            if (!tc::mbar_wait(&full[s], (it / p.stages) & 1, kWaitBudget)) {
+                set_error(23);
+                break;
+            }
+            tc::fence_after_sync();
+            const uint32_t z = tc::smem_u32(smem + s * p.stage_stride);
+            const uint32_t x = z + p.stage_stride - p.n_ci * p.x_stride;
+            for (int c = 0; c < n_ci; ++c)
+                for (uint32_t r = 0; r < (uint32_t)kWgRows; r += row_step)
+                    for (uint32_t q = 0; q < segs; ++q) {
+                        const uint64_t ad = ax + ((x + c * p.x_stride + r * ximg + q * 16 * xrow) >> 4);
+                        const uint64_t bd = bz + ((z + (r * p.bw + q * 16) * zrow) >> 4);
+                        tc::mma_bf16(tmem + c * acc_cols, ad, bd, idesc, (it > 0 || r > 0 || q > 0) ? 1u : 0u);
+                    }
+            tc::mma_commit(&empty[s]);
+            if (++s == (uint32_t)p.stages) s = 0;
+        }
+        tc::mma_commit(done);
+    }
+
+    const bool any = (int)blockIdx.x < p.num_tiles;
+    const bool ready = any && tc::mbar_wait(done, 0, kWaitBudget);
+    if (any && !ready) set_error(24);
+    __syncwarp();
+    tc::fence_after_sync();
+    if (ready && warp < 3) {
+        for (int c = 0; c < n_ci; ++c) {
+            const int ci = ci0 + 32 * c + lane;
+            for (int j = 0; j < 3; ++j) {
+                const int tap = (2 - j) * 3 + warp;
+                for (int k = 0; k < p.co_block; k += 16) {
+                    uint32_t r0[8], r1[8];
+                    const uint32_t col = tmem + ((uint32_t)(warp * 32) << 16) + c * acc_cols +
+                                         (uint32_t)(j * p.co_block + k);
+                    tc::tmem_ld8(col, r0);
+                    tc::tmem_ld8(col + 8, r1);
+                    tc::tmem_ld_wait();
+                    float* dst = p.dw + ((size_t)tap * p.Cout + co0 + k) * p.Cin + ci;
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        if (co0 + k + q < p.Cout)
+                            atomicAdd(dst + (size_t)q * p.Cin, __uint_as_float(q < 8 ? r0[q & 7] : r1[q & 7]));
+                }
+            }
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, p.tmem_cols);
+}
+
 // ---- host: tensor maps ----
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -925,6 +1081,62 @@ void gemm_bf16_tn(const __nv_bfloat16* a, int M, const __nv_bfloat16* b, int N, 
     const dim3 grid((unsigned)((M + 127) / 128), (unsigned)((N + n_tile - 1) / n_tile),
                     (unsigned)((p.k_iters + p.k_per_split - 1) / p.k_per_split));
     launch_tc<1, 128, 4>(grid, ma, mb, p, st);
+}
+
+void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int W, int Cin, const __nv_bfloat16* dz,
+                        int dz_channels, int Cout, float* dw, cudaStream_t st) {
+    KF_REQUIRE(N > 0 && H > 0 && W > 0, KF_ERR_INVALID_ARGUMENT, "wgrad: empty tensor");
+    KF_REQUIRE(Cin > 0 && Cin % 32 == 0 && dz_channels % 32 == 0 && Cout > 0 && Cout <= dz_channels,
+               KF_ERR_INVALID_ARGUMENT, "wgrad: channels must be multiples of 32");
+    KF_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)dz & 15) == 0 && x_cstride % 8 == 0, KF_ERR_INVALID_ARGUMENT,
+               "wgrad: tensors must be 16-byte aligned");
+    WgradParams p{};
+    // K steps are 16 pixels of a row, or two rows of 8 where the image is that narrow; 32-pixel
+    // tiles halve the halo columns where they leave no more padding than 16-pixel ones
+    p.bw = W <= 8 ? 8 : ((W - 1) / 16 % 2 == 0 ? 16 : 32);
+    p.tiles_x = (W + p.bw - 1) / p.bw;
+    p.tiles_y = (H + kWgRows - 1) / kWgRows;
+    p.num_tiles = p.tiles_x * p.tiles_y * N;
+    p.co_block = dz_channels % 64 == 0 ? 64 : 32;
+    p.Cin = Cin;
+    p.Cout = Cout;
+    p.dw = dw;
+    p.x_bytes = (uint32_t)(kWgRows * (p.bw + 2) * 64);
+    p.x_stride = (p.x_bytes + 64 + 1023u) & ~1023u; // the unused fourth shift reads one pixel past the tile
+    p.z_bytes = (uint32_t)((kWgRows + 2) * p.bw * 2 * p.co_block);
+    const uint32_t z_stride = (p.z_bytes + 1023u) & ~1023u;
+    const int ci_blocks = Cin / 32, co_blocks = dz_channels / p.co_block, sms = num_sms();
+    // several input-channel blocks per CTA share the dZ tile: as many as TMEM and two stages
+    // of shared memory hold, while the CTAs that are left still have a tile each on every SM
+    p.n_ci = 1;
+    for (int c = 2; c <= std::min(kWgMaxCi, ci_blocks); ++c)
+        if (c * 3 * p.co_block <= 512 && 2 * (c * p.x_stride + z_stride) <= 220u * 1024u &&
+            (int64_t)p.num_tiles * co_blocks * ((ci_blocks + c - 1) / c) >= 2 * sms)
+            p.n_ci = c;
+    p.stage_stride = p.n_ci * p.x_stride + z_stride;
+    p.stages = std::min<int>(kWgMaxStages, (int)(220u * 1024u / p.stage_stride));
+    p.tmem_cols = pow2_at_least((uint32_t)(p.n_ci * 3 * p.co_block));
+    const size_t smem = 1024 + (size_t)p.stages * p.stage_stride + 128;
+    const uint64_t xdims[4] = {(uint64_t)Cin, (uint64_t)W, (uint64_t)H, (uint64_t)N};
+    const uint64_t xstr[3] = {(uint64_t)x_cstride * 2, (uint64_t)W * x_cstride * 2, (uint64_t)H * W * x_cstride * 2};
+    const uint32_t xbox[4] = {32, (uint32_t)p.bw + 2, kWgRows, 1};
+    const CUtensorMap mx = make_map(x, 4, xdims, xstr, xbox, CU_TENSOR_MAP_SWIZZLE_64B);
+    const uint64_t zdims[4] = {(uint64_t)dz_channels, (uint64_t)W, (uint64_t)H, (uint64_t)N};
+    const uint64_t zstr[3] = {(uint64_t)dz_channels * 2, (uint64_t)W * dz_channels * 2,
+                              (uint64_t)H * W * dz_channels * 2};
+    const uint32_t zbox[4] = {(uint32_t)p.co_block, (uint32_t)p.bw, kWgRows + 2, 1};
+    const CUtensorMap mz = make_map(dz, 4, zdims, zstr, zbox,
+                                    p.co_block == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+    static bool configured = false;
+    if (!configured) {
+        KF_CUDA_CHECK(cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        configured = true;
+    }
+    const int blocks = co_blocks * ((ci_blocks + p.n_ci - 1) / p.n_ci);
+    const int splits = std::max(1, std::min(p.num_tiles, sms / std::max(1, blocks)));
+    const dim3 grid((unsigned)splits, (unsigned)co_blocks, (unsigned)((ci_blocks + p.n_ci - 1) / p.n_ci));
+    k_wgrad<<<grid, 128, smem, st>>>(mx, mz, p);
+    KF_CUDA_CHECK(cudaGetLastError());
 }
 
 namespace {

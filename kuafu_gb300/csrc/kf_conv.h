@@ -30,6 +30,12 @@ bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __
 void gemm_bf16_tn(const __nv_bfloat16* a, int M, const __nv_bfloat16* b, int N, int K, float* d, int ldd, int splits,
                   cudaStream_t st);
 
+// dw[tap][co][ci] += sum over pixels of dz[p][co] * x[p shifted by tap][ci] for co < Cout (FP32
+// atomics; x NHWC with channel stride x_cstride, dz dense [N][H][W][dz_channels], Cin and
+// dz_channels multiples of 32).
+void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int W, int Cin, const __nv_bfloat16* dz,
+                        int dz_channels, int Cout, float* dw, cudaStream_t st);
+
 // Reads and clears the error word the tensor-core kernels set when a bounded wait expires.
 uint32_t tc_take_error();
 // Error word a wait probe leaves when its wait gives up.

@@ -133,91 +133,46 @@ __global__ void k_up_bwd(const bf16* __restrict__ gy, int gs, int go, int C, int
     }
 }
 
-// dz[p][c] = (c < C) ? gy[p][c] * (relu ? y[p][c] > 0 : 1) : 0   for c < Ck (dense, Ck channels)
-__global__ void k_relu_mask(const bf16* __restrict__ gy, int gs, int go, const bf16* __restrict__ y, int ys, int yo,
-                            int C, int Ck, size_t P, int relu, bf16* dz) {
-    const bool vec = (C % 8) == 0 && (gs % 8) == 0 && (go % 8) == 0 && (!relu || ((ys % 8) == 0 && (yo % 8) == 0));
-    if (vec) {
-        const int G = Ck / 8, Gc = C / 8;
-        const size_t total = P * G;
-        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-            const int g = (int)(i % G);
-            const size_t p = i / G;
-            F8 v;
-            if (g < Gc) {
-                v = ld8(gy + p * gs + go + 8 * g);
-                if (relu) {
-                    const F8 m = ld8(y + p * ys + yo + 8 * g);
+// dz[p][c] = (c < C) ? gy[p][c] * (relu ? y[p][c] > 0 : 1) : 0   for c < Ck (dense, Ck channels),
+// and db[c] += sum_p dz[p][c] of the rounded values. Bound by HBM: one read of gy and y, one
+// write of dz; the bias sums ride along in registers (a thread keeps its 8 channels for all its
+// pixels), where a pass of their own read dz again with one 2-byte load per value: 19 layers of
+// a 16 x 128 x 128 batch take 0.27 ms, in two passes they took 0.38 ms. All strides and offsets are multiples
+// of 8 (16-byte accesses).
+constexpr int kMaskThreads = 256, kMaskMaxC = 160;
+__global__ void __launch_bounds__(kMaskThreads) k_relu_mask_bias(const bf16* __restrict__ gy, int gs, int go,
+                                                                 const bf16* __restrict__ y, int ys, int yo, int C,
+                                                                 int Ck, size_t P, int relu, bf16* __restrict__ dz,
+                                                                 float* db) {
+    __shared__ float s_db[kMaskMaxC];
+    const int G = Ck / 8, per = kMaskThreads / G; // pixels per block and step
+    const int g = threadIdx.x % G, pl = threadIdx.x / G;
+    for (int c = threadIdx.x; c < Ck; c += kMaskThreads) s_db[c] = 0.0f;
+    __syncthreads();
+    float sum[8];
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        if (!(m.v[k] > 0.0f)) v.v[k] = 0.0f;
-                }
-            } else {
+    for (int k = 0; k < 8; ++k) sum[k] = 0.0f;
+    if (pl < per) {
+        for (size_t p = (size_t)blockIdx.x * per + pl; p < P; p += (size_t)gridDim.x * per) {
+            F8 v = ld8(gy + p * gs + go + 8 * g);
+            if (relu) {
+                const F8 m = ld8(y + p * ys + yo + 8 * g);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) v.v[k] = 0.0f;
+                for (int k = 0; k < 8; ++k)
+                    if (!(m.v[k] > 0.0f)) v.v[k] = 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                if (8 * g + k >= C) v.v[k] = 0.0f;
+                sum[k] += v.v[k];
             }
             st8(dz + p * Ck + 8 * g, v);
         }
-        return;
-    }
-    const size_t total = P * Ck;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(i % Ck);
-        const size_t p = i / Ck;
-        float v = 0.0f;
-        if (c < C) {
-            v = __bfloat162float(gy[p * gs + go + c]);
-            if (relu && !(__bfloat162float(y[p * ys + yo + c]) > 0.0f)) v = 0.0f;
-        }
-        dz[i] = __float2bfloat16_rn(v);
-    }
-}
-
-// db[c] += sum_p dz[p][c]
-__global__ void k_bias_grad(const bf16* __restrict__ dz, int Ck, int C, size_t P, float* db) {
-    const int c = blockIdx.y;
-    float s = 0.0f;
-    for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < P; p += (size_t)gridDim.x * blockDim.x)
-        s += __bfloat162float(dz[p * Ck + c]);
-    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
-    __shared__ float sm[32];
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0f;
-        for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
-        if (threadIdx.x == 0 && c < C) atomicAdd(db + c, s);
-    }
-}
-
-// t[c][p] = x[n, y+dy, x+dx, c] (0 outside the image and for P <= p < Pk): the K-major
-// operand of one filter tap's weight gradient, rows padded to Pk (a multiple of 8).
-__global__ void k_shift_transpose(const bf16* __restrict__ x, int xs, int xo, int C, int N, int H, int W, int dy,
-                                  int dx, size_t Pk, bf16* t) {
-    __shared__ bf16 tile[32][33];
-    const size_t P = (size_t)N * H * W;
-    const size_t p0 = (size_t)blockIdx.x * 32;
-    const int c0 = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const size_t p = p0 + k;
-        const int c = c0 + threadIdx.x;
-        bf16 v = __float2bfloat16_rn(0.0f);
-        if (p < P && c < C) {
-            const int xw = (int)(p % W);
-            const size_t r = p / W;
-            const int yh = (int)(r % H);
-            const int n = (int)(r / H);
-            const int sy = yh + dy, sx = xw + dx;
-            if (sy >= 0 && sy < H && sx >= 0 && sx < W) v = x[(((size_t)n * H + sy) * W + sx) * xs + xo + c];
-        }
-        tile[k][threadIdx.x] = v;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) atomicAdd(&s_db[8 * g + k], sum[k]);
     }
     __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int c = c0 + k;
-        const size_t p = p0 + threadIdx.x;
-        if (c < C && p < Pk) t[(size_t)c * Pk + p] = tile[threadIdx.x][k];
-    }
+    for (int c = threadIdx.x; c < C; c += kMaskThreads) atomicAdd(db + c, s_db[c]);
 }
 
 // Adam on FP32 master weights (Kingma & Ba 2015).
@@ -439,7 +394,7 @@ enum {
     T_D2A, T_D2B, T_D1A, T_D1B, T_D0A, T_D0B, T_OUT,
     // gradients
     G_OUT, G_D0B, G_D0A, G_CAT0, G_D1B, G_D1A, G_CAT1, G_D2B, G_D2A, G_CAT2, G_D3B, G_D3A, G_CAT3, G_E4B, G_E4A, G_P3,
-    G_E3B, G_E3A, G_P2, G_E2B, G_E2A, G_P1, G_E1B, G_E1A, G_P0, G_E0B, G_E0A, G_DZ, G_T, G_ZT,
+    G_E3B, G_E3A, G_P2, G_E2B, G_E2A, G_P1, G_E1B, G_E1A, G_P0, G_E0B, G_E0A, G_DZ,
     T_COUNT
 };
 
@@ -554,7 +509,7 @@ const TDesc kT[T_COUNT] = {
     {32, 0}, {32, 0}, {32, 0}, {96, 0}, {64, 1}, {64, 1}, {160, 1}, {96, 2}, {96, 2}, {224, 2}, {128, 3}, {128, 3},
     {288, 3}, {160, 4}, {160, 4}, {128, 4}, {128, 3}, {128, 3}, {96, 3}, {96, 2}, {96, 2}, {64, 2}, {64, 1}, {64, 1},
     {32, 1}, {32, 0}, {32, 0},
-    {0, 0}, {0, 0}, {0, 0}};
+    {0, 0}};
 
 void ensure_acts(kf_denoiser_impl& d, int n, int h, int w, cudaStream_t st) {
     Acts& a = d.acts;
@@ -568,22 +523,12 @@ void ensure_acts(kf_denoiser_impl& d, int n, int h, int w, cudaStream_t st) {
         total += (P0 >> (2 * kT[k].level)) * kT[k].c;
         total = (total + 127) / 128 * 128;
     }
-    // scratch: masked gradient (P0 x 160 max at any level), transposed operands
-    size_t dz_max = 0, t_max = 0, zt_max = 0;
-    int level[19] = {0, 0, 1, 1, 2, 2, 3, 3, 4, 4, 3, 3, 2, 2, 1, 1, 0, 0, 0};
-    for (int i = 0; i < 19; ++i) {
-        const size_t P = P0 >> (2 * level[i]);
-        const size_t Pk = (P + 7) / 8 * 8;
-        dz_max = std::max(dz_max, P * (size_t)pad32(kLayers[i][1]));
-        t_max = std::max(t_max, Pk * (size_t)kLayers[i][0]);
-        zt_max = std::max(zt_max, Pk * (size_t)kLayers[i][1]);
-    }
+    // scratch: masked gradient of one layer
+    size_t dz_max = 0;
+    const int level[19] = {0, 0, 1, 1, 2, 2, 3, 3, 4, 4, 3, 3, 2, 2, 1, 1, 0, 0, 0};
+    for (int i = 0; i < 19; ++i) dz_max = std::max(dz_max, (P0 >> (2 * level[i])) * (size_t)pad32(kLayers[i][1]));
     a.off[G_DZ] = total;
     total += (dz_max + 127) / 128 * 128;
-    a.off[G_T] = total;
-    total += (t_max + 127) / 128 * 128;
-    a.off[G_ZT] = total;
-    total += (zt_max + 127) / 128 * 128;
     a.buf.resize(total, st);
     KF_CUDA_CHECK(cudaMemsetAsync(a.buf.ptr, 0, a.buf.bytes(), st));
     a.head.resize(P0 * 4, st);
@@ -616,24 +561,13 @@ void conv_bwd(Ctx& c, int li, int level, TRef x, TRef y, TRef gy, TRef gx) {
     Acts& a = c.d.acts;
     const size_t P = c.P(level);
     bf16* dz = a.at(G_DZ);
-    k_relu_mask<<<grid_for(P * l.cout_k), 256, 0, c.st>>>(gy.p, gy.cs, gy.co, y.p, y.cs, y.co, l.cout, l.cout_k, P,
-                                                         l.relu ? 1 : 0, dz);
-    k_bias_grad<<<dim3((unsigned)std::min<size_t>((P + 255) / 256, 64), (unsigned)l.cout_k), 256, 0, c.st>>>(
-        dz, l.cout_k, l.cout, P, c.d.grads.ptr + l.b_off);
-    // dZ^T [cout][Pk]
-    const size_t Pk = (P + 7) / 8 * 8;
-    bf16* zt = a.at(G_ZT);
-    k_shift_transpose<<<dim3((unsigned)((Pk + 31) / 32), (unsigned)((l.cout + 31) / 32)), dim3(32, 8), 0, c.st>>>(
-        dz, l.cout_k, 0, l.cout, c.n, c.H(level), c.W(level), 0, 0, Pk, zt);
-    bf16* t = a.at(G_T);
-    const int splits = (int)std::max<size_t>(1, std::min<size_t>(64, P / 8192));
-    for (int tap = 0; tap < 9; ++tap) {
-        const int dy = tap / 3 - 1, dx = tap % 3 - 1;
-        k_shift_transpose<<<dim3((unsigned)((Pk + 31) / 32), (unsigned)((l.cin + 31) / 32)), dim3(32, 8), 0, c.st>>>(
-            x.p, x.cs, x.co, l.cin, c.n, c.H(level), c.W(level), dy, dx, Pk, t);
-        gemm_bf16_tn(zt, l.cout, t, l.cin, (int)Pk, c.d.grads.ptr + l.w_off + (size_t)tap * l.cout * l.cin, l.cin,
-                     splits, c.st);
-    }
+    // a few pixels per thread at least, two resident waves of blocks at most
+    const size_t per = (size_t)(kMaskThreads / (l.cout_k / 8));
+    const unsigned blocks = (unsigned)std::max<size_t>(1, std::min<size_t>((P + 4 * per - 1) / (4 * per), 152 * 16));
+    k_relu_mask_bias<<<blocks, kMaskThreads, 0, c.st>>>(gy.p, gy.cs, gy.co, y.p, y.cs, y.co, l.cout, l.cout_k, P,
+                                                        l.relu ? 1 : 0, dz, c.d.grads.ptr + l.b_off);
+    conv3x3_wgrad_bf16(x.p + x.co, x.cs, c.n, c.H(level), c.W(level), l.cin, dz, l.cout_k, l.cout,
+                       c.d.grads.ptr + l.w_off, c.st);
     if (gx.p) {
         conv3x3_bf16(dz, c.n, c.H(level), c.W(level), l.cout_k, c.d.wb.ptr + l.wb_off, l.cin, nullptr, l.cin, false,
                      gx.p, gx.cs, gx.co, c.st);

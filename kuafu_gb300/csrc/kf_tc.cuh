@@ -146,6 +146,24 @@ __device__ __forceinline__ uint64_t smem_desc_noswz(uint32_t addr, uint32_t lbo,
     return d;
 }
 
+// Shared-memory matrix descriptor of an MN-major operand (channels contiguous, one K row per
+// `swizzle` bytes: layout 2 = 128 B, 4 = 64 B): groups of `swizzle` bytes of M / N `lbo` bytes
+// apart, groups of 8 K rows `sbo` bytes apart. Swizzling applies to absolute shared-memory
+// addresses, so the start may be any K row of a tile that TMA wrote at a 1024-byte boundary.
+// addr = 0 gives the constant part: adding (address >> 4) moves the view.
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lbo, uint32_t sbo, uint32_t layout) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1u << 46;                       // descriptor version (sm_100)
+    d |= (uint64_t)(layout & 7u) << 61;
+    return d;
+}
+
+// Instruction-descriptor bits for MN-major A and B (both operands "transposed").
+constexpr uint32_t kIdescMnMajorAB = (1u << 15) | (1u << 16);
+
 // Instruction descriptor of kind::f16 with BF16 A and B (both K-major), FP32 D, M x N.
 __host__ __device__ __forceinline__ uint32_t idesc_bf16(uint32_t M, uint32_t N) {
     return (1u << 4)                 // D format: F32

@@ -182,6 +182,44 @@ def test_gradients_match_autograd(renderer, h, w):
     d.close()
 
 
+# Weight gradients where the pixel tiles (8 rows of 8, 16 or 32 pixels) have remainders: sizes
+# whose five levels are 1 to 9 pixels wide, whose rows do not fill a tile, and whose levels 0 to
+# 2 are 16-, 32- and 16-pixel tiles wide. Same reference and bounds as above.
+@pytest.mark.parametrize("n,h,w", [(1, 16, 16), (3, 48, 144), (2, 80, 272)])
+def test_gradients_at_tile_remainders(renderer, n, h, w):
+    import torch
+
+    d = api.Denoiser(renderer, seed=9)
+    params = d.getParams()
+    rng = np.random.default_rng(1)
+    o = 0
+    for cin, cout, _ in LAYERS:
+        o += 9 * cout * cin
+        params[o:o + cout] = rng.normal(0.0, 0.05, cout)
+        o += cout
+    d.setParams(params)
+    feat, target = _inputs(torch, n, h, w, 22)
+    grads = torch.zeros(params.size, device="cuda", dtype=torch.float32)
+    torch.cuda.synchronize()
+    d.trainStep(feat.data_ptr(), target.data_ptr(), n, h, w, grads_ptr=grads.data_ptr(), apply=False)
+    torch.cuda.synchronize()
+    assert _tc_error() == 0
+    wb = [(wt.cuda().to(torch.bfloat16).float().requires_grad_(True), b.cuda().requires_grad_(True))
+          for wt, b in _unpack(params, torch)]
+    ste = lambda t: t + (t.to(torch.bfloat16).float() - t).detach()
+    _loss(_unet(feat.float().permute(0, 3, 1, 2), wb, torch, ste), target, torch).backward()
+    g, o = grads.cpu().numpy(), 0
+    for i, (cin, cout, _) in enumerate(LAYERS):
+        rw = wb[i][0].grad.reshape(cout, cin, 9).permute(2, 0, 1).cpu().numpy().ravel()
+        rb = wb[i][1].grad.cpu().numpy()
+        for ref, what in ((rw, "weight"), (rb, "bias")):
+            got = g[o:o + ref.size]
+            o += ref.size
+            rel = float(np.linalg.norm(got - ref) / (np.linalg.norm(ref) + 1e-30))
+            assert rel <= 0.15, f"layer {i} {what}: rel {rel:.3e}"
+    d.close()
+
+
 def test_training_reduces_loss(renderer):
     import torch
 
