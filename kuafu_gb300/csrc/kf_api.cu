@@ -442,6 +442,7 @@ KF_API int kf_renderer_download_aov(kf_renderer r, kf_camera cam, int kind, void
         const size_t npix = (size_t)c->target_w * c->target_h;
         const void* src = nullptr;
         size_t need = 0;
+        uint32_t path_words = 0; // per-path data: float4 per path (kept pixel-major, returned sample-major)
         switch (kind) {
             case KF_AOV_RADIANCE_F32: src = c->accum.ptr; need = npix * 16; break;
             case KF_AOV_ALBEDO_F32: src = c->albedo.ptr; need = npix * 16; break;
@@ -451,11 +452,13 @@ KF_API int kf_renderer_download_aov(kf_renderer r, kf_camera cam, int kind, void
             case KF_AOV_PATH_RADIANCE:
                 src = r->wave.radiance.ptr + c->last_path_start;
                 need = (size_t)c->last_spp * npix * 16;
+                path_words = 1;
                 break;
             case KF_AOV_PRIMARY_HITS:
                 KF_REQUIRE(r->cfg.debug_outputs, KF_ERR_STATE, "primary hits need debug_outputs = 1");
                 src = r->wave.primary.ptr + c->last_path_start;
                 need = (size_t)c->last_spp * npix * sizeof(kf_hit);
+                path_words = sizeof(kf_hit) / 16;
                 break;
             case KF_AOV_SEGMENTATION: src = c->seg.ptr; need = npix * 16; break;
             case KF_AOV_DENOISED_F32:
@@ -466,6 +469,18 @@ KF_API int kf_renderer_download_aov(kf_renderer r, kf_camera cam, int kind, void
             default: throw KfError(KF_ERR_INVALID_ARGUMENT, "unknown AOV kind");
         }
         KF_REQUIRE(bytes >= need, KF_ERR_OUT_OF_RANGE, "output buffer too small for the AOV");
+        if (path_words) {
+            DeviceBuffer<float4> slice; // one sample's image at a time
+            slice.resize(npix * path_words, r->stream);
+            for (uint32_t k = 0; k < c->last_spp; ++k) {
+                launch_sample_slice(static_cast<const float4*>(src), (uint32_t)npix, c->last_spp, k, path_words,
+                                    slice.ptr, r->stream);
+                KF_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t*>(out) + k * slice.bytes(), slice.ptr, slice.bytes(),
+                                              cudaMemcpyDeviceToHost, r->stream));
+            }
+            sync_stream(r);
+            return;
+        }
         KF_CUDA_CHECK(cudaMemcpyAsync(out, src, need, cudaMemcpyDeviceToHost, r->stream));
         sync_stream(r);
     });

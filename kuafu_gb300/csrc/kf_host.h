@@ -159,14 +159,15 @@ struct BatchState {
 
 // Wavefront buffers sized for one chunk of paths.
 struct WaveBuffers {
-    kf::DeviceBuffer<float4> q_o0, q_o1, q_d0, q_d1, hit, weight, nee_w, nee_in, contrib, sq_o, sq_d;
+    kf::DeviceBuffer<float4> q_o0, q_o1, q_d0, q_d1, hit, nee_w, nee_in, contrib, sq_o, sq_d;
+    kf::DeviceBuffer<float2> q_w0, q_w1;
     kf::DeviceBuffer<uint32_t> counters, hit_prim, sel, scount;
     kf::DeviceBuffer<uint64_t> req;
     kf::DeviceBuffer<uint8_t> vis;
     kf::DeviceBuffer<float4> radiance;      // per path of the frame
     kf::DeviceBuffer<kf_hit> primary;       // per path of the frame (debug)
     kf::DeviceBuffer<unsigned long long> stats;
-    kf::DeviceBuffer<uint16_t> path_item;   // batched launches: item of each path of a chunk
+    kf::DeviceBuffer<uint16_t> path_item, hit_item; // batched launches: item of each path / hit of a chunk
     uint32_t chunk_cap = 0, slot_cap = 0;
     uint64_t radiance_cap = 0;
 };

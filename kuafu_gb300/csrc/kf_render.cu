@@ -177,14 +177,15 @@ void ensure_targets(kf_renderer_s* r, kf_camera_s* c) {
     }
 }
 
-void ensure_wave(kf_renderer_s* r, uint32_t chunk, uint32_t slots, uint64_t npaths) {
+void ensure_wave(kf_renderer_s* r, uint32_t chunk, uint32_t slots, uint64_t npaths, uint32_t max_depth) {
     WaveBuffers& W = r->wave;
     cudaStream_t st = r->stream;
     if (W.chunk_cap < chunk) {
         W.q_o0.resize(chunk, st); W.q_o1.resize(chunk, st);
         W.q_d0.resize(chunk, st); W.q_d1.resize(chunk, st);
+        W.q_w0.resize(chunk, st); W.q_w1.resize(chunk, st);
         W.hit.resize(chunk, st); W.hit_prim.resize(chunk, st); W.sel.resize(chunk, st);
-        W.weight.resize(chunk, st); W.nee_w.resize(chunk, st); W.nee_in.resize((size_t)6 * chunk, st);
+        W.nee_w.resize(chunk, st); W.nee_in.resize((size_t)5 * chunk, st);
         W.req.resize(chunk, st);
         W.chunk_cap = chunk;
         W.slot_cap = 0;
@@ -202,26 +203,28 @@ void ensure_wave(kf_renderer_s* r, uint32_t chunk, uint32_t slots, uint64_t npat
         W.radiance_cap = npaths;
     }
     if (r->cfg.debug_outputs && W.primary.count < npaths) W.primary.resize(npaths, st);
-    if (W.counters.count == 0) W.counters.resize(8, st);
-    if (W.scount.count == 0) W.scount.resize(64, st);
+    // one row per bounce, and the row the last bounce's shading would append to
+    const size_t rows = (size_t)max_depth + 2;
+    if (W.counters.count < rows * (kCounterRow + kSlotRow)) W.counters.resize(rows * (kCounterRow + kSlotRow), st);
     if (W.stats.count == 0) {
         W.stats.resize(16, st);
         KF_CUDA_CHECK(cudaMemsetAsync(W.stats.ptr, 0, W.stats.bytes(), st));
     }
 }
 
-WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c) {
+WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, bool lit) {
     WaveBuffers& W = r->wave;
     WaveDev w{};
     w.q_o[0] = W.q_o0.ptr; w.q_o[1] = W.q_o1.ptr;
     w.q_d[0] = W.q_d0.ptr; w.q_d[1] = W.q_d1.ptr;
+    w.q_w[0] = W.q_w0.ptr; w.q_w[1] = W.q_w1.ptr;
     w.counters = W.counters.ptr;
     w.hit = W.hit.ptr;
     w.hit_prim = W.hit_prim.ptr;
     w.sel = W.sel.ptr;
-    w.scount = W.scount.ptr;
+    w.scount = W.counters.ptr + ((size_t)max_depth + 2) * kCounterRow;
+    w.lit = lit ? 1u : 0u;
     w.nslot = W.slot_cap;
-    w.weight = W.weight.ptr;
     w.nee_w = W.nee_w.ptr;
     w.nee_in = W.nee_in.ptr;
     w.req = W.req.ptr;
@@ -245,67 +248,23 @@ WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c) {
 // The bounce loop on two streams. Bounce d's shadow traversal and NEE gather (stream2)
 // overlap bounce d+1's closest-hit traversal (stream): they share no buffer — the closest-hit
 // kernel reads the next ray queue and writes hit records, the shadow kernel reads the shadow
-// queue and writes visibility, the gather reads bounce d's queue and adds to the radiance.
-// Everything bounce d+1 writes that bounce d's gather reads (its queue count, the NEE
-// requests, contributions, visibility and radiance of the paths) is written by k_miss /
-// k_shade, which wait for the gather (the join). Counters: [3] / [4] fetch cursors, [2]
-// shadow count, [5] hit count, each zeroed on the stream that uses it next.
-static void enqueue_paths_overlapped(kf_renderer_s* r, const SceneDev& sv, const FrameDev* fd, const BatchDev& b,
-                                     const WaveDev& w, uint32_t max_depth, uint64_t npaths, uint32_t chunk) {
-    cudaStream_t st = r->stream, st2 = r->stream2;
-    const bool dyn = r->cfg.traversal == 1;
-    for (uint64_t start = 0; start < npaths; start += chunk) {
-        const uint32_t n = (uint32_t)std::min<uint64_t>(chunk, npaths - start);
-        launch_raygen(fd, b, w, start, n, st);
-        int cur = 0;
-        for (uint32_t depth = 0; depth <= max_depth; ++depth) {
-            KF_CUDA_CHECK(cudaMemsetAsync(w.counters + 3, 0, sizeof(uint32_t), st));
-            if (dyn)
-                launch_trace_dyn(sv, fd, b, w, cur, depth, start, false, r->grid_dyn, r->count_traversal,
-                                 r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
-            else
-                launch_extend(sv, fd, b, w, cur, depth, start, r->grid_extend, r->count_traversal, st);
-            if (depth > 0) KF_CUDA_CHECK(cudaStreamWaitEvent(st, r->ev_join, 0)); // previous gather done
-            KF_CUDA_CHECK(cudaMemsetAsync(w.counters + (cur ^ 1), 0, sizeof(uint32_t), st));
-            KF_CUDA_CHECK(cudaMemsetAsync(w.scount, 0, w.nslot * sizeof(uint32_t), st));
-            KF_CUDA_CHECK(cudaMemsetAsync(w.counters + 5, 0, sizeof(uint32_t), st));
-            launch_miss(sv, fd, b, w, cur, depth, start, r->grid_shade, st);
-            launch_shade(sv, fd, b, w, cur, depth, start, r->grid_shade, st);
-            launch_nee(sv, fd, b, w, depth, start, r->grid_shade, st);
-            KF_CUDA_CHECK(cudaEventRecord(r->ev_fork, st));
-            KF_CUDA_CHECK(cudaStreamWaitEvent(st2, r->ev_fork, 0));
-            KF_CUDA_CHECK(cudaMemsetAsync(w.counters + 4, 0, sizeof(uint32_t), st2));
-            if (dyn)
-                launch_trace_dyn(sv, fd, b, w, cur, depth, start, true, r->grid_dyn_shadow, r->count_traversal,
-                                 r->cfg.dyn_refill_below, r->cfg.dyn_steps, st2);
-            else
-                launch_shadow(sv, b, w, r->grid_extend, r->count_traversal, st2);
-            launch_gather(sv, b, w, cur, start, r->grid_shade, st2);
-            KF_CUDA_CHECK(cudaEventRecord(r->ev_join, st2));
-            cur ^= 1;
-        }
-        KF_CUDA_CHECK(cudaStreamWaitEvent(st, r->ev_join, 0)); // last gather done
-    }
-}
-
-// Records the bounce loop over npaths paths (chunks of `chunk`) into the renderer stream.
+// queue and writes visibility, the gather reads bounce d's hit records of the NEE and adds to
+// the radiance. What bounce d+1 writes of that (the NEE records, requests, contributions and
+// the radiance of the paths) is written by k_miss / k_shade, which wait for the gather (the
+// join). Counters are per bounce and cleared once per chunk, after the last gather of the
+// chunk before it. A launch without lights has no NEE: one stream, three kernels per bounce.
+// With `profile` everything runs on one stream with events around the kernel groups.
 static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* fd, const BatchDev& b,
                           const WaveDev& w, uint32_t max_depth, uint64_t npaths, uint32_t chunk, bool profile) {
-    cudaStream_t st = r->stream;
-    if (!profile) {
-        enqueue_paths_overlapped(r, sv, fd, b, w, max_depth, npaths, chunk);
-        return;
-    }
+    cudaStream_t st = r->stream, st2 = profile ? r->stream : r->stream2;
+    const bool dyn = r->cfg.traversal == 1, lit = w.lit != 0, fork = lit && !profile;
+    const size_t clear = ((size_t)max_depth + 2) * (kCounterRow + kSlotRow) * sizeof(uint32_t);
     for (uint64_t start = 0; start < npaths; start += chunk) {
         const uint32_t n = (uint32_t)std::min<uint64_t>(chunk, npaths - start);
+        KF_CUDA_CHECK(cudaMemsetAsync(w.counters, 0, clear, st));
         launch_raygen(fd, b, w, start, n, st);
         int cur = 0;
         for (uint32_t depth = 0; depth <= max_depth; ++depth) {
-            const bool dyn = r->cfg.traversal == 1;
-            KF_CUDA_CHECK(cudaMemsetAsync(w.counters + (cur ^ 1), 0, sizeof(uint32_t), st));
-            // [2] shadow queue count, [3] / [4] dynamic-fetch cursors, [5] rays that hit
-            KF_CUDA_CHECK(cudaMemsetAsync(w.counters + 2, 0, 4 * sizeof(uint32_t), st));
-            KF_CUDA_CHECK(cudaMemsetAsync(w.scount, 0, w.nslot * sizeof(uint32_t), st));
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[0], st));
             if (dyn)
                 launch_trace_dyn(sv, fd, b, w, cur, depth, start, false, r->grid_dyn, r->count_traversal,
@@ -313,17 +272,25 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
             else
                 launch_extend(sv, fd, b, w, cur, depth, start, r->grid_extend, r->count_traversal, st);
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[1], st));
+            if (fork && depth > 0) KF_CUDA_CHECK(cudaStreamWaitEvent(st, r->ev_join, 0)); // previous gather done
             launch_miss(sv, fd, b, w, cur, depth, start, r->grid_shade, st);
             launch_shade(sv, fd, b, w, cur, depth, start, r->grid_shade, st);
-            launch_nee(sv, fd, b, w, depth, start, r->grid_shade, st);
+            if (lit) launch_nee(sv, fd, b, w, depth, start, r->grid_shade, st);
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[2], st));
-            if (dyn)
-                launch_trace_dyn(sv, fd, b, w, cur, depth, start, true, r->grid_dyn_shadow, r->count_traversal,
-                                 r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
-            else
-                launch_shadow(sv, b, w, r->grid_extend, r->count_traversal, st);
+            if (lit) {
+                if (fork) {
+                    KF_CUDA_CHECK(cudaEventRecord(r->ev_fork, st));
+                    KF_CUDA_CHECK(cudaStreamWaitEvent(st2, r->ev_fork, 0));
+                }
+                if (dyn)
+                    launch_trace_dyn(sv, fd, b, w, cur, depth, start, true, r->grid_dyn_shadow, r->count_traversal,
+                                     r->cfg.dyn_refill_below, r->cfg.dyn_steps, st2);
+                else
+                    launch_shadow(sv, b, w, depth, r->grid_extend, r->count_traversal, st2);
+            }
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[3], st));
-            launch_gather(sv, b, w, cur, start, r->grid_shade, st);
+            if (lit) launch_gather(sv, b, w, depth, start, r->grid_shade, st2);
+            if (fork) KF_CUDA_CHECK(cudaEventRecord(r->ev_join, st2));
             if (profile) {
                 KF_CUDA_CHECK(cudaEventSynchronize(r->ev[3]));
                 float a = 0, bb = 0, d = 0;
@@ -336,6 +303,7 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
             }
             cur ^= 1;
         }
+        if (fork) KF_CUDA_CHECK(cudaStreamWaitEvent(st, r->ev_join, 0)); // last gather done
     }
 }
 
@@ -344,8 +312,7 @@ static void enqueue_frame(kf_renderer_s* r, const SceneDev& sv, const WaveDev& w
                           uint32_t max_depth, uint64_t npaths, uint32_t chunk, kf_camera_s* c, bool profile) {
     const FrameDev* fd = r->frame_dev.ptr;
     enqueue_paths(r, sv, fd, BatchDev{nullptr, 0, 0}, w, max_depth, npaths, chunk, profile);
-    launch_resolve(fd, w.radiance, npix, spp, c->accum.ptr, c->sum64.ptr, r->stream);
-    launch_srgb(c->accum.ptr, npix, c->bgra.ptr, r->stream);
+    launch_resolve(fd, w.radiance, npix, spp, c->accum.ptr, c->sum64.ptr, c->bgra.ptr, r->stream);
 }
 
 // Frame constants of camera c of scene s (push constants: PushConstants.glsl:1-16, filled
@@ -424,7 +391,7 @@ void render_frame(kf_renderer_s* r, kf_scene_s* s, kf_camera_s* c, uint32_t spp)
     const uint64_t npaths = (uint64_t)npix * spp;
     const uint32_t chunk = chunk_for(r, npaths);
     const SceneDev& sv = s->gpu.view;
-    ensure_wave(r, chunk, sv.num_slots, npaths);
+    ensure_wave(r, chunk, sv.num_slots, npaths, r->cfg.path_depth);
 
     // Context::update (context.cpp:345-349): frame counter for the running mean
     if (r->cfg.accumulate_frames)
@@ -435,10 +402,7 @@ void render_frame(kf_renderer_s* r, kf_scene_s* s, kf_camera_s* c, uint32_t spp)
     const FrameDev f = make_frame(r, s, c, spp, r->frame_count);
     if (r->frame_dev.count == 0) r->frame_dev.resize(1, st);
     KF_CUDA_CHECK(cudaMemcpyAsync(r->frame_dev.ptr, &f, sizeof(f), cudaMemcpyHostToDevice, st));
-    KF_CUDA_CHECK(cudaMemsetAsync(c->albedo.ptr, 0, c->albedo.bytes(), st));
-    KF_CUDA_CHECK(cudaMemsetAsync(c->normal.ptr, 0, c->normal.bytes(), st));
-
-    const WaveDev w = wave_view(r, c);
+    const WaveDev w = wave_view(r, c, r->cfg.path_depth, sv.num_slots > 0);
     const bool profile = r->cfg.profile != 0;
     cudaEvent_t f0 = r->ev[4], f1 = r->ev[5];
     if (profile) KF_CUDA_CHECK(cudaEventRecord(f0, st));
@@ -447,11 +411,11 @@ void render_frame(kf_renderer_s* r, kf_scene_s* s, kf_camera_s* c, uint32_t spp)
         // The launch sequence depends only on buffer addresses and sizes; the
         // per-frame values live in frame_dev, so a captured graph replays as is.
         char head[512];
-        std::snprintf(head, sizeof(head), "%p|%p|%llu|%u|%u|%u|%llu|%u|%p|%p|%p|%p|%p|%u|%s|", (void*)s, (void*)c,
+        std::snprintf(head, sizeof(head), "%p|%p|%llu|%u|%u|%u|%llu|%u|%p|%p|%p|%p|%p|%p|%u|%s|", (void*)s, (void*)c,
                       (unsigned long long)s->gpu.generation, npix, spp, r->cfg.path_depth,
                       (unsigned long long)npaths, chunk, (void*)w.q_o[0], (void*)w.radiance, (void*)w.contrib,
-                      (void*)c->accum.ptr, (void*)w.primary, r->cfg.russian_roulette | (r->cfg.traversal << 1),
-                      launch_shape_key(r).c_str());
+                      (void*)w.counters, (void*)c->accum.ptr, (void*)w.primary,
+                      r->cfg.russian_roulette | (r->cfg.traversal << 1), launch_shape_key(r).c_str());
         const std::string key = std::string(head) + scene_view_key(sv);
         if (!r->graph_exec || r->graph_key != key) {
             if (r->graph_exec) {
@@ -515,7 +479,8 @@ void render_batch(kf_renderer_s* r, const kf_batch_item* items, uint32_t count) 
     BatchState& B = *r->batch;
     std::vector<ItemDev> hv(count);
     uint64_t total = 0;
-    uint32_t max_slots = 1;
+    uint64_t resolve_blocks = 0;
+    uint32_t max_slots = 0;
     std::vector<uint32_t> inst_base(scenes.size(), 0), geom_base(scenes.size(), 0);
     for (size_t k = 1; k < scenes.size(); ++k) {
         inst_base[k] = inst_base[k - 1] + (uint32_t)scenes[k - 1]->instances.size();
@@ -547,44 +512,43 @@ void render_batch(kf_renderer_s* r, const kf_batch_item* items, uint32_t count) 
         it.depth = c->depth.ptr;
         it.seg = c->seg.ptr;
         it.geom_base = geom_base[k];
+        it.spp = items[i].spp;
+        it.block_start = (uint32_t)resolve_blocks;
+        resolve_blocks += (it.f.npix + kResolvePix - 1) / kResolvePix;
+        it.accum = c->accum.ptr;
+        it.sum64 = c->sum64.ptr;
+        it.bgra = c->bgra.ptr;
         max_slots = std::max(max_slots, sv.num_slots);
     }
+    KF_REQUIRE(resolve_blocks < (1ull << 31), KF_ERR_LIMIT, "too many pixels in one batch");
     const uint32_t chunk = chunk_for(r, total);
-    ensure_wave(r, chunk, max_slots, total);
+    ensure_wave(r, chunk, max_slots, total, r->cfg.path_depth);
     if (r->wave.path_item.count < chunk) r->wave.path_item.resize(chunk, st);
+    if (r->wave.hit_item.count < chunk) r->wave.hit_item.resize(chunk, st);
     B.items.resize(count, st);
     KF_CUDA_CHECK(cudaMemcpyAsync(B.items.ptr, hv.data(), sizeof(ItemDev) * count, cudaMemcpyHostToDevice, st));
-    for (uint32_t i = 0; i < count; ++i) {
-        KF_CUDA_CHECK(cudaMemsetAsync(items[i].camera->albedo.ptr, 0, items[i].camera->albedo.bytes(), st));
-        KF_CUDA_CHECK(cudaMemsetAsync(items[i].camera->normal.ptr, 0, items[i].camera->normal.bytes(), st));
-    }
-    WaveDev w = wave_view(r, items[0].camera);
+    WaveDev w = wave_view(r, items[0].camera, r->cfg.path_depth, max_slots > 0);
     w.path_item = r->wave.path_item.ptr;
+    w.hit_item = r->wave.hit_item.ptr;
     const BatchDev bd{B.items.ptr, count, 0};
     auto enqueue = [&](bool profile) {
         enqueue_paths(r, B.view, nullptr, bd, w, r->cfg.path_depth, total, chunk, profile);
-        for (uint32_t i = 0; i < count; ++i) {
-            kf_camera_s* c = items[i].camera;
-            launch_resolve(&B.items.ptr[i].f, w.radiance + hv[i].path_start, hv[i].f.npix, items[i].spp,
-                           c->accum.ptr, c->sum64.ptr, st);
-            launch_srgb(c->accum.ptr, hv[i].f.npix, c->bgra.ptr, st);
-        }
+        launch_resolve_batch(bd, w.radiance, (uint32_t)resolve_blocks, st);
     };
     const bool profile = r->cfg.profile != 0;
     cudaEvent_t f0 = r->ev[4], f1 = r->ev[5];
     if (profile) KF_CUDA_CHECK(cudaEventRecord(f0, st));
     if (r->cfg.use_graph && !profile && !r->count_traversal) {
         std::string key;
-        char buf[160];
-        std::snprintf(buf, sizeof(buf), "%llu|%u|%llu|%u|%p|%p|%p|%u|%u|", (unsigned long long)B.generation, count,
-                      (unsigned long long)total, chunk, (void*)w.q_o[0], (void*)w.radiance, (void*)B.items.ptr,
-                      r->cfg.path_depth, r->cfg.russian_roulette | (r->cfg.traversal << 1));
-        key = buf + launch_shape_key(r) + "|" + scene_view_key(B.view) + "|";
-        for (uint32_t i = 0; i < count; ++i) {
-            std::snprintf(buf, sizeof(buf), "%p,%u,%u;", (void*)items[i].camera->accum.ptr, hv[i].f.npix,
-                          items[i].spp);
-            key += buf;
-        }
+        // the items (sizes, samples, targets, lights) live in device memory; what a graph bakes
+        // in are the wave buffers, the pools and the launch counts
+        char buf[256];
+        std::snprintf(buf, sizeof(buf), "%llu|%u|%llu|%u|%llu|%p|%p|%p|%p|%p|%p|%p|%p|%u|%u|%u|%u|",
+                      (unsigned long long)B.generation, count, (unsigned long long)total, chunk,
+                      (unsigned long long)resolve_blocks, (void*)w.q_o[0], (void*)w.radiance, (void*)w.contrib,
+                      (void*)w.counters, (void*)w.path_item, (void*)w.hit_item, (void*)w.primary, (void*)B.items.ptr,
+                      w.nslot, w.lit, r->cfg.path_depth, r->cfg.russian_roulette | (r->cfg.traversal << 1));
+        key = buf + launch_shape_key(r) + "|" + scene_view_key(B.view);
         if (!B.graph_exec || B.graph_key != key) {
             if (B.graph_exec) {
                 cudaGraphExecDestroy(B.graph_exec);

@@ -13,7 +13,8 @@
 //   gather   ordered NEE sum into the path radiance        (rchit:457-460, rgen:111)
 // then a per-pixel resolve (rgen:140-166) and the sRGB frame (PostProcessing.frag).
 // Queues are compacted in order: a block scan per tile with one atomic per tile (warp
-// ballots + one atomic per warp where the warps of a block differ).
+// ballots + one atomic per warp where the warps of a block differ). A launch whose views have
+// no lights to sample skips nee, shadow and gather.
 //
 // This file is compiled with -fmad=false: float expressions round exactly as
 // written, matching the CPU oracle operation for operation.
@@ -58,22 +59,22 @@ struct AnyHitCtx {
     Stream st;
 };
 
-// Sample and pixel of path g of a view (sample-major): a 32-bit division whenever g fits
+// Pixel and sample of path g of a view (pixel-major): a 32-bit division whenever g fits
 // in 32 bits (a view below 2^32 paths), the 64-bit one otherwise.
-__device__ __forceinline__ void split_path(uint64_t g, uint32_t npix, uint32_t& sample, uint32_t& pix) {
+__device__ __forceinline__ void split_path(uint64_t g, uint32_t spp, uint32_t& pix, uint32_t& sample) {
     if ((g >> 32) == 0) {
         const uint32_t g32 = (uint32_t)g;
-        sample = g32 / npix;
-        pix = g32 - sample * npix;
+        pix = g32 / spp;
+        sample = g32 - pix * spp;
     } else {
-        sample = (uint32_t)(g / npix);
-        pix = (uint32_t)(g % npix);
+        pix = (uint32_t)(g / spp);
+        sample = (uint32_t)(g % spp);
     }
 }
 
 __device__ __forceinline__ PathKey path_key(const FrameDev& f, uint64_t g) {
     uint32_t sample, pix;
-    split_path(g, f.npix, sample, pix);
+    split_path(g, f.pc.spp, pix, sample);
     return PathKey{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
 }
 
@@ -369,11 +370,11 @@ template <bool BATCH> __device__ __forceinline__ uint32_t root_of(const SceneDev
 // ---------------------------------------------------------------------------
 // Ray generation (PathTrace.rgen:30-75).
 // ---------------------------------------------------------------------------
-// Queue order of a sample's pixels: bands of kTileH rows, each cut into kTileW-wide column
+// Queue order of a view's pixels: bands of kTileH rows, each cut into kTileW-wide column
 // blocks (narrower at the right edge), a block's pixels row by row — a warp's 32 camera rays
 // cover a 4x8 tile instead of 32 pixels of one row, and stay coherent downstream (4x8
-// measured fastest of 2x16 .. 16x4 on the 256-icosphere frame). idx is the position within
-// the sample, the result the row-major pixel index (a bijection for any size).
+// measured fastest of 2x16 .. 16x4 on the 256-icosphere frame). idx is the position in the
+// view, the result the row-major pixel index (a bijection for any size, within each band).
 constexpr uint32_t kTileW = 4, kTileH = 8;
 __device__ __forceinline__ uint32_t tiled_pixel(uint32_t idx, uint32_t width, uint32_t height) {
     const uint32_t band = width * kTileH;
@@ -403,24 +404,21 @@ __global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
     }
     const FrameDev& f = *fsel;
     g -= view_start;
+    // a pixel's samples are queued one after the other, so a warp's camera rays start in few
+    // neighbouring pixels (+5 % over queuing each sample's pixels together); a band of kTileH
+    // rows that lies in this chunk is queued in tile order
     uint32_t sample, pix;
-    if (view_start >= chunk_start && view_start + (uint64_t)f.npix * f.pc.spp <= chunk_start + chunk_n) {
-        // the whole view in this chunk: a pixel's samples are queued one after the other,
-        // pixels in tile order, so a warp's camera rays start in 4 neighbouring pixels
-        // (+5 % over queuing each sample's pixels in tile order)
-        uint32_t t;
-        split_path(g, f.pc.spp, t, sample);
-        pix = tiled_pixel(t, f.width, f.height);
-    } else {
-        split_path(g, f.npix, sample, pix);
-        // a sample whose pixels all lie in this chunk is queued in tile order
-        const uint64_t row0 = view_start + (uint64_t)sample * f.npix;
-        if (row0 >= chunk_start && row0 + f.npix <= chunk_start + chunk_n) pix = tiled_pixel(pix, f.width, f.height);
-    }
-    // the path id p (the index of all per-path state) stays the row-major one
-    const uint64_t row = view_start + (uint64_t)sample * f.npix;
-    const uint32_t p = (uint32_t)(row + pix - chunk_start);
+    split_path(g, f.pc.spp, pix, sample);
+    const uint32_t band = f.width * kTileH, first = pix / band * band;
+    const uint64_t b0 = view_start + (uint64_t)first * f.pc.spp;
+    const uint64_t b1 = view_start + (uint64_t)min(first + band, f.npix) * f.pc.spp;
+    if (b0 >= chunk_start && b1 <= chunk_start + chunk_n) pix = tiled_pixel(pix, f.width, f.height);
+    const uint32_t p = (uint32_t)(view_start + (uint64_t)pix * f.pc.spp + sample - chunk_start);
     if (BATCH) w.path_item[p] = (uint16_t)item;
+    if (sample == 0) { // the AOVs of pixels that hit no material stay zero
+        (BATCH ? b.items[item].albedo : w.albedo)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        (BATCH ? b.items[item].normal : w.normal)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
     const uint32_t px = pix % f.width, py = pix / f.width;
     PathKey pk{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
     Stream js;
@@ -464,8 +462,7 @@ __global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
         mat4_mul(f.cam.view_inv, din, dir);
     }
     w.q_o[0][j] = make_float4(origin[0], origin[1], origin[2], __uint_as_float(p));
-    w.q_d[0][j] = make_float4(dir[0], dir[1], dir[2], 0.0f);
-    w.weight[p] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+    w.q_d[0][j] = make_float4(dir[0], dir[1], dir[2], 1.0f);
     w.radiance[chunk_start + p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
@@ -476,7 +473,7 @@ template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(128) k_extend(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
                                                 int cur, uint32_t depth, uint64_t chunk_start) {
     __shared__ uint32_t s_stack[kSmemStack * kThreadsTrace];
-    const uint32_t count = w.counters[cur];
+    const uint32_t count = w.counters[depth * kCounterRow];
     const float4* __restrict__ qo = w.q_o[cur];
     const float4* __restrict__ qd = w.q_d[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.stats[depth == 0 ? 0 : 1], (unsigned long long)count);
@@ -824,27 +821,32 @@ __device__ bool light_sample(const SceneDev& s, const LS& ls, uint32_t slot, uin
 template <bool BATCH>
 __device__ __forceinline__ void miss_path(const SceneDev& s, const FrameDev* fp, const BatchDev& b, const WaveDev& w,
                                           int cur, uint32_t depth, uint64_t chunk_start, uint32_t i) {
-    const float4 qo = w.q_o[cur][i], qd = w.q_d[cur][i];
-    const uint32_t p = __float_as_uint(qo.w);
+    const float4 qd = w.q_d[cur][i];
+    const uint32_t p = __float_as_uint(w.q_o[cur][i].w);
     const uint64_t g = chunk_start + p;
     const View<BATCH> vw = view_of<BATCH>(fp, b, w, chunk_start, p);
     const FrameDev& f = *vw.f;
     const float4* env = BATCH ? vw.it->env : s.env;
     const uint32_t env_size = BATCH ? vw.it->env_size : s.env_size;
-    const float4 w4 = w.weight[p];
-    const v3 wold = mk(w4.x, w4.y, w4.z);
-    const float4 col4 = w.radiance[g];
-    v3 color = mk(col4.x, col4.y, col4.z);
+    // camera rays carry weight 1 and find the radiance still zero
+    v3 wold = splat(1.0f), color = splat(0.0f);
+    if (depth > 0) {
+        const float2 wyz = w.q_w[cur][i];
+        wold = mk(qd.w, wyz.x, wyz.y);
+        color = xyz(w.radiance[g]);
+    }
     const v3 emission = (f.pc.use_env_map && env) ? env_lookup(env, env_size, mk(qd.x, qd.y, qd.z))
                                                    : ld3(f.pc.clear_color) * f.pc.clear_color[3];
     color = color + emission * wold;
     w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
-    w.req[p] = 0;
-    if (depth == 0 && vw.g < f.npix) { // sample 0 of the first bounce
-        const uint32_t pix = (uint32_t)vw.g;
-        (BATCH ? vw.it->depth : w.depth)[pix] = 0.0f;
-        uint4* aov_seg = BATCH ? vw.it->seg : w.seg;
-        if (aov_seg) aov_seg[pix] = make_uint4(kMiss, kMiss, kMiss, 0u);
+    if (depth == 0) { // sample 0 of the first bounce
+        uint32_t pix, sample;
+        split_path(vw.g, f.pc.spp, pix, sample);
+        if (sample == 0) {
+            (BATCH ? vw.it->depth : w.depth)[pix] = 0.0f;
+            uint4* aov_seg = BATCH ? vw.it->seg : w.seg;
+            if (aov_seg) aov_seg[pix] = make_uint4(kMiss, kMiss, kMiss, 0u);
+        }
     }
 }
 
@@ -858,7 +860,8 @@ __global__ void __launch_bounds__(kMissThreads) k_miss(SceneDev s, const FrameDe
                                                        WaveDev w, int cur, uint32_t depth, uint64_t chunk_start) {
     __shared__ uint32_t s_cnt[kMissThreads / 32];
     __shared__ uint32_t s_base;
-    const uint32_t count = w.counters[cur];
+    uint32_t* ctr = w.counters + depth * kCounterRow;
+    const uint32_t count = ctr[0];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr uint32_t tile = kMissThreads * kMissPer;
     for (uint32_t base = blockIdx.x * tile; base < count; base += gridDim.x * tile) {
@@ -886,7 +889,7 @@ __global__ void __launch_bounds__(kMissThreads) k_miss(SceneDev s, const FrameDe
         if (threadIdx.x == 0) {
             uint32_t t = 0;
             for (uint32_t k = 0; k < kMissThreads / 32; ++k) t += s_cnt[k];
-            s_base = t ? atomicAdd(&w.counters[5], t) : 0u;
+            s_base = t ? atomicAdd(ctr + 1, t) : 0u;
         }
         __syncthreads();
         uint32_t pos = s_base + x - nh;
@@ -908,7 +911,7 @@ template <bool BATCH>
 // 4 resident blocks per SM (128 registers, no spill) measured fastest; unbounded it takes 148.
 __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
                                                int cur, uint32_t depth, uint64_t chunk_start) {
-    const uint32_t count = w.counters[5]; // rays of this bounce that hit (k_miss takes the others)
+    const uint32_t count = w.counters[depth * kCounterRow + 1]; // rays that hit (k_miss takes the others)
     const int nxt = cur ^ 1;
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -936,17 +939,18 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const Fr
             vw = view_of<BATCH>(fp, b, w, chunk_start, p);
             const FrameDev& f = *vw.f;
             uint32_t sample, pix;
-            split_path(vw.g, f.npix, sample, pix);
+            split_path(vw.g, f.pc.spp, pix, sample);
             pk = PathKey{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
             float4* aov_albedo = BATCH ? vw.it->albedo : w.albedo;
             float4* aov_normal = BATCH ? vw.it->normal : w.normal;
             float* aov_depth = BATCH ? vw.it->depth : w.depth;
             const float4 hv = w.hit[i];
             const uint32_t inst = __float_as_uint(hv.w); // never kMiss here
-            const float4 w4 = w.weight[p];
-            const v3 wold = mk(w4.x, w4.y, w4.z);
-            float4 col4 = w.radiance[g];
-            v3 color = mk(col4.x, col4.y, col4.z);
+            v3 wold = splat(1.0f); // camera rays
+            if (depth > 0) {
+                const float2 wyz = w.q_w[cur][i];
+                wold = mk(qd.w, wyz.x, wyz.y);
+            }
             const v3 rayD = mk(qd.x, qd.y, qd.z);
             {
                 const uint32_t prim = w.hit_prim[i];
@@ -968,6 +972,7 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const Fr
                 const v3 emission = ld3(mat.emission) * mat.emission[3];
                 if (emission != splat(0.0f)) {
                     // emissive hit ends the path (rchit:330-335)
+                    v3 color = depth > 0 ? xyz(w.radiance[g]) : splat(0.0f);
                     color = color + (ld3(mat.emission) * mat.emission[3]) * wold;
                     w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
                 } else {
@@ -1115,16 +1120,27 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const Fr
                 }
             }
         }
-        // what the light samples of this hit need, for k_nee (hit-list order)
-        if (valid) {
-            float4* rec = w.nee_in + (size_t)6 * (base + lane);
-            rec[0] = make_float4(worldPos.x, worldPos.y, worldPos.z,
-                                 __uint_as_float(p | (is_mat ? 0x80000000u : 0u) | (sh.isInside ? 0x40000000u : 0u)));
-            rec[1] = make_float4(N.x, N.y, N.z, sh.f);
-            rec[2] = make_float4(V.x, V.y, V.z, sh.a2);
-            rec[3] = make_float4(sh.diffuseColor.x, sh.diffuseColor.y, sh.diffuseColor.z, wnew.x);
-            rec[4] = make_float4(sh.specularColor.x, sh.specularColor.y, sh.specularColor.z, wnew.y);
-            rec[5] = make_float4(sh.transmissionColor.x, sh.transmissionColor.y, sh.transmissionColor.z, wnew.z);
+        // what the light samples of this hit need, for k_nee (hit-list order, one array per
+        // field group so that a warp's stores are whole lines); of hits that take none only
+        // the flags, and nothing at all where no view of the launch has a light
+        if (w.lit && valid) {
+            const uint32_t k = base + lane;
+            if (BATCH) {
+                w.hit_item[k] = w.path_item[p];
+                is_mat = is_mat && vw.it->num_slots > 0;
+            }
+            w.nee_w[k] = make_float4(wnew.x, wnew.y, wnew.z,
+                                     __uint_as_float(p | (is_mat ? 0x80000000u : 0u) | (sh.isInside ? 0x40000000u : 0u)));
+            if (is_mat) {
+                float4* rec = w.nee_in + k;
+                const size_t n = w.chunk_cap;
+                rec[0] = make_float4(worldPos.x, worldPos.y, worldPos.z, sh.f);
+                rec[n] = make_float4(N.x, N.y, N.z, sh.a2);
+                rec[2 * n] = make_float4(V.x, V.y, V.z, sh.diffuseColor.x);
+                rec[3 * n] = make_float4(sh.diffuseColor.y, sh.diffuseColor.z, sh.specularColor.x, sh.specularColor.y);
+                rec[4 * n] = make_float4(sh.specularColor.z, sh.transmissionColor.x, sh.transmissionColor.y,
+                                         sh.transmissionColor.z);
+            }
         }
         // next rays in hit-list order: one atomic per block tile
         const uint32_t m = __ballot_sync(kFull, cont);
@@ -1133,15 +1149,15 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const Fr
         if (threadIdx.x == 0) {
             uint32_t t = 0;
             for (uint32_t k = 0; k < kShadeWarps; ++k) t += s_cnt[par][k];
-            s_base[par] = t ? atomicAdd(&w.counters[nxt], t) : 0u;
+            s_base[par] = t ? atomicAdd(w.counters + (depth + 1) * kCounterRow, t) : 0u;
         }
         __syncthreads();
         uint32_t pos = s_base[par] + __popc(m & lanemask_lt());
         for (uint32_t k = 0; k < wid; ++k) pos += s_cnt[par][k];
         if (cont) {
             w.q_o[nxt][pos] = make_float4(worldPos.x, worldPos.y, worldPos.z, __uint_as_float(p));
-            w.q_d[nxt][pos] = make_float4(L.x, L.y, L.z, 0.0f);
-            w.weight[p] = make_float4(wcont.x, wcont.y, wcont.z, 0.0f);
+            w.q_d[nxt][pos] = make_float4(L.x, L.y, L.z, wcont.x);
+            w.q_w[nxt][pos] = make_float2(wcont.y, wcont.z);
         }
     }
 }
@@ -1155,15 +1171,15 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const Fr
 template <bool BATCH>
 __global__ void __launch_bounds__(kShadeThreads) k_nee(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
                                              uint32_t depth, uint64_t chunk_start) {
-    const uint32_t count = w.counters[5];
+    const uint32_t count = w.counters[depth * kCounterRow + 1];
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t bbase = blockIdx.x * blockDim.x; bbase < count; bbase += stride) {
         const uint32_t base = bbase + (threadIdx.x & ~31u);
         const bool valid = base + lane < count;
-        uint32_t p = 0;
+        const uint32_t k = base + lane; // hit-list position
         bool is_mat = false;
-        v3 worldPos = splat(0.0f), N = splat(0.0f), V = splat(0.0f), wnew = splat(0.0f);
+        v3 worldPos = splat(0.0f), N = splat(0.0f), V = splat(0.0f);
         Shading sh;
         sh.f = 1.0f; sh.a2 = 0.0f;
         sh.diffuseColor = sh.specularColor = sh.transmissionColor = splat(0.0f);
@@ -1171,28 +1187,34 @@ __global__ void __launch_bounds__(kShadeThreads) k_nee(SceneDev s, const FrameDe
         View<BATCH> vw{fp, nullptr, 0};
         PathKey pk{make_uint2(0, 0), 0, 0};
         if (valid) {
-            const float4* rec = w.nee_in + (size_t)6 * (base + lane);
-            const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3], r4 = rec[4], r5 = rec[5];
-            const uint32_t bits = __float_as_uint(r0.w);
-            p = bits & 0x3FFFFFFFu;
+            const uint32_t bits = __float_as_uint(w.nee_w[k].w);
             is_mat = (bits & 0x80000000u) != 0;
-            sh.isInside = (bits & 0x40000000u) != 0;
-            worldPos = mk(r0.x, r0.y, r0.z);
-            N = mk(r1.x, r1.y, r1.z);
-            sh.f = r1.w;
-            V = mk(r2.x, r2.y, r2.z);
-            sh.a2 = r2.w;
-            sh.diffuseColor = mk(r3.x, r3.y, r3.z);
-            sh.specularColor = mk(r4.x, r4.y, r4.z);
-            sh.transmissionColor = mk(r5.x, r5.y, r5.z);
-            wnew = mk(r3.w, r4.w, r5.w);
-            vw = view_of<BATCH>(fp, b, w, chunk_start, p);
-            const FrameDev& f = *vw.f;
-            pk = path_key(f, vw.g);
+            if (is_mat) {
+                const float4* rec = w.nee_in + k;
+                const size_t n = w.chunk_cap;
+                const float4 r0 = rec[0], r1 = rec[n], r2 = rec[2 * n], r3 = rec[3 * n], r4 = rec[4 * n];
+                sh.isInside = (bits & 0x40000000u) != 0;
+                worldPos = mk(r0.x, r0.y, r0.z);
+                sh.f = r0.w;
+                N = mk(r1.x, r1.y, r1.z);
+                sh.a2 = r1.w;
+                V = mk(r2.x, r2.y, r2.z);
+                sh.diffuseColor = mk(r2.w, r3.x, r3.y);
+                sh.specularColor = mk(r3.z, r3.w, r4.x);
+                sh.transmissionColor = mk(r4.y, r4.z, r4.w);
+                const uint32_t p = bits & 0x3FFFFFFFu;
+                if (BATCH) {
+                    vw.it = b.items + w.hit_item[k];
+                    vw.f = &vw.it->f;
+                    vw.g = chunk_start + p - vw.it->path_start;
+                } else
+                    vw.g = chunk_start + p;
+                pk = path_key(*vw.f, vw.g);
+            }
         }
         uint64_t req = 0;
         const uint32_t nslots =
-            BATCH ? __reduce_max_sync(kFull, valid ? vw.it->num_slots : 0u) : s.num_slots;
+            BATCH ? __reduce_max_sync(kFull, is_mat ? vw.it->num_slots : 0u) : s.num_slots;
         for (uint32_t j = 0; j < nslots; ++j) {
             v3 Ls = splat(0.0f), c = splat(0.0f);
             float tmax = 0.0f;
@@ -1206,20 +1228,17 @@ __global__ void __launch_bounds__(kShadeThreads) k_nee(SceneDev s, const FrameDe
             // towards one light from neighbouring points; one atomic per warp and slot (a
             // block-wide scan instead waited at two barriers per slot for the warp with the
             // longest light sampling)
-            const uint32_t pos = warp_append(emit, &w.scount[j]);
+            const uint32_t pos = warp_append(emit, &w.scount[depth * kSlotRow + j]);
             if (emit) {
                 const size_t q = (size_t)j * w.chunk_cap + pos;
                 w.sq_o[q] = make_float4(worldPos.x, worldPos.y, worldPos.z, tmax);
-                w.sq_d[q] = make_float4(Ls.x, Ls.y, Ls.z, __uint_as_float((j << 26) | p));
-                w.contrib[(size_t)j * w.chunk_cap + p] = make_float4(c.x, c.y, c.z, 0.0f);
-                w.vis[(size_t)j * w.chunk_cap + p] = 0;
+                w.sq_d[q] = make_float4(Ls.x, Ls.y, Ls.z, __uint_as_float((j << 26) | k));
+                w.contrib[(size_t)j * w.chunk_cap + k] = make_float4(c.x, c.y, c.z, 0.0f);
+                w.vis[(size_t)j * w.chunk_cap + k] = 0;
                 req |= 1ull << j;
             }
         }
-        if (valid) {
-            w.req[p] = req;
-            if (req) w.nee_w[p] = make_float4(wnew.x, wnew.y, wnew.z, 0.0f);
-        }
+        if (valid) w.req[k] = req;
     }
 }
 
@@ -1231,12 +1250,12 @@ __global__ void __launch_bounds__(kShadeThreads) k_nee(SceneDev s, const FrameDe
 // shared memory (all threads of the block must call it) and returns the total.
 constexpr uint32_t kMaxSlots = 64;
 static_assert(1 + KF_MAX_POINT_LIGHTS + KF_MAX_ACTIVE_LIGHTS <= kMaxSlots, "light slots exceed the shadow queues");
-__device__ __forceinline__ uint32_t shadow_prefix(const WaveDev& w, uint32_t* s_pre) {
+__device__ __forceinline__ uint32_t shadow_prefix(const WaveDev& w, uint32_t depth, uint32_t* s_pre) {
     if (threadIdx.x == 0) {
         uint32_t t = 0;
         for (uint32_t j = 0; j < w.nslot; ++j) {
             s_pre[j] = t;
-            t += w.scount[j];
+            t += w.scount[depth * kSlotRow + j];
         }
         s_pre[w.nslot] = t;
     }
@@ -1251,22 +1270,22 @@ __device__ __forceinline__ uint32_t shadow_entry(const WaveDev& w, const uint32_
 }
 
 template <bool COUNT, bool BATCH>
-__global__ void __launch_bounds__(128) k_shadow(SceneDev s, BatchDev b, WaveDev w) {
+__global__ void __launch_bounds__(128) k_shadow(SceneDev s, BatchDev b, WaveDev w, uint32_t depth) {
     __shared__ uint32_t s_stack[kSmemStack * kThreadsTrace];
     __shared__ uint32_t s_pre[kMaxSlots + 1];
-    const uint32_t count = shadow_prefix(w, s_pre);
+    const uint32_t count = shadow_prefix(w, depth, s_pre);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.stats[2], (unsigned long long)count);
     TraceCounters cnt{0, 0, 0};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t e = shadow_entry(w, s_pre, i);
         const float4 o = w.sq_o[e], d = w.sq_d[e];
         const uint32_t tag = __float_as_uint(d.w);
-        const uint32_t slot = tag >> 26, p = tag & ((1u << 26) - 1u);
-        const uint32_t root = BATCH ? b.items[w.path_item[p]].root : (s.has_tlas ? 0u : kNoRoot);
+        const uint32_t slot = tag >> 26, k = tag & ((1u << 26) - 1u);
+        const uint32_t root = BATCH ? b.items[w.hit_item[k]].root : (s.has_tlas ? 0u : kNoRoot);
         HitOut h;
         const bool occluded =
             trace<true, COUNT>(s, root, s_stack, o.x, o.y, o.z, d.x, d.y, d.z, KF_T_MIN, o.w, h, cnt);
-        if (!occluded) w.vis[(size_t)slot * w.chunk_cap + p] = 1;
+        if (!occluded) w.vis[(size_t)slot * w.chunk_cap + k] = 1;
     }
     if (COUNT) {
         atomicAdd(&w.stats[6], (unsigned long long)cnt.nodes);
@@ -1292,8 +1311,9 @@ __global__ void __launch_bounds__(128, SHADOW ? 9 : 7)
                 uint64_t chunk_start, uint32_t refill_below, int steps) {
     __shared__ uint32_t s_stack[kSmemStack * kThreadsTrace];
     __shared__ uint32_t s_pre[SHADOW ? kMaxSlots + 1 : 1];
-    const uint32_t count = SHADOW ? shadow_prefix(w, s_pre) : w.counters[cur];
-    uint32_t* fetch = w.counters + (SHADOW ? 4 : 3);
+    uint32_t* ctr = w.counters + depth * kCounterRow;
+    const uint32_t count = SHADOW ? shadow_prefix(w, depth, s_pre) : ctr[0];
+    uint32_t* fetch = ctr + (SHADOW ? 3 : 2);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(&w.stats[SHADOW ? 2 : (depth == 0 ? 0 : 1)], (unsigned long long)count);
     const uint32_t lane = threadIdx.x & 31;
@@ -1323,8 +1343,8 @@ __global__ void __launch_bounds__(128, SHADOW ? 9 : 7)
                     idx = SHADOW ? shadow_entry(w, s_pre, j) : j;
                     if (SHADOW) {
                         const float4 o = w.sq_o[idx], d = w.sq_d[idx];
-                        const uint32_t p = __float_as_uint(d.w) & ((1u << 26) - 1u);
-                        const uint32_t root = BATCH ? b.items[w.path_item[p]].root : single_root;
+                        const uint32_t k = __float_as_uint(d.w) & ((1u << 26) - 1u);
+                        const uint32_t root = BATCH ? b.items[w.hit_item[k]].root : single_root;
                         t.init(root, o.x, o.y, o.z, d.x, d.y, d.z, KF_T_MIN, o.w);
                     } else {
                         const float4 o = w.q_o[cur][j], d = w.q_d[cur][j];
@@ -1380,19 +1400,18 @@ __global__ void __launch_bounds__(128, SHADOW ? 9 : 7)
 // (rchit:457-460), color += shadow_color * weight (rgen:111).
 // ---------------------------------------------------------------------------
 template <bool BATCH>
-__global__ void k_gather(SceneDev s, BatchDev b, WaveDev w, int cur, uint64_t chunk_start) {
-    const uint32_t count = w.counters[cur];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const uint32_t p = __float_as_uint(w.q_o[cur][i].w);
-        uint64_t req = w.req[p];
+__global__ void k_gather(SceneDev s, BatchDev b, WaveDev w, uint32_t depth, uint64_t chunk_start) {
+    const uint32_t count = w.counters[depth * kCounterRow + 1];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
+        uint64_t req = w.req[k];
         if (!req) continue;
-        const uint8_t* slot_group = BATCH ? b.items[w.path_item[p]].slot_group : nullptr;
+        const uint8_t* slot_group = BATCH ? b.items[w.hit_item[k]].slot_group : nullptr;
         v3 D = splat(0.0f), P = splat(0.0f), A = splat(0.0f);
         while (req) {
             const uint32_t j = __ffsll((long long)req) - 1;
             req &= req - 1;
-            if (!w.vis[(size_t)j * w.chunk_cap + p]) continue;
-            const float4 c4 = w.contrib[(size_t)j * w.chunk_cap + p];
+            if (!w.vis[(size_t)j * w.chunk_cap + k]) continue;
+            const float4 c4 = w.contrib[(size_t)j * w.chunk_cap + k];
             const v3 c = mk(c4.x, c4.y, c4.z);
             const uint32_t grp = BATCH ? slot_group[j] : s.slot_group[j];
             if (grp == 0) D = c;
@@ -1400,60 +1419,122 @@ __global__ void k_gather(SceneDev s, BatchDev b, WaveDev w, int cur, uint64_t ch
             else A = A + c;
         }
         const v3 shadow = (D + P) + A;
-        const float4 wn = w.nee_w[p];
-        const uint64_t g = chunk_start + p;
+        const float4 wn = w.nee_w[k];
+        const uint64_t g = chunk_start + (__float_as_uint(wn.w) & 0x3FFFFFFFu);
         const float4 col = w.radiance[g];
         const v3 color = mk(col.x, col.y, col.z) + shadow * mk(wn.x, wn.y, wn.z);
         w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
     }
 }
 
+// Linear value -> sRGB byte by binary search over the 256 thresholds (in shared memory: the
+// lanes of a warp search at different places).
+__device__ __forceinline__ unsigned char srgb8(const float* thresh, float v) {
+    if (!(v > 0.0f)) return 0;
+    int lo = 0;
+#pragma unroll
+    for (int step = 128; step >= 1; step >>= 1)
+        if (thresh[lo + step] <= v) lo += step;
+    return (unsigned char)lo;
+}
+
+__constant__ float c_srgb_thresh[256];
+
 // ---------------------------------------------------------------------------
 // Per-pixel resolve: finalColor = colors / spp (rgen:140-144) and the running
-// mean over frames (rgen:151-163); FP64 sum of finalColor alongside.
+// mean over frames (rgen:151-163); FP64 sum of finalColor alongside; the linear running mean
+// -> B8G8R8A8 sRGB (config.hpp:144, PostProcessing.frag:11-17).
+// Bound by HBM: 16 bytes per sample read once. A pixel's samples are consecutive and summed in
+// order by one lane; a warp brings 32 pixels x 8 samples at a time through shared memory, so
+// its loads are whole 128-byte lines (views of fewer samples are read in place).
 // ---------------------------------------------------------------------------
-__global__ void k_resolve(const FrameDev* __restrict__ fp, const float4* __restrict__ radiance, uint32_t npix,
-                          uint32_t spp, float4* accum, dbl4* sum64) {
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+constexpr uint32_t kResSamples = 8;
+template <bool BATCH>
+__global__ void __launch_bounds__(kResolvePix) k_resolve(const FrameDev* __restrict__ fp, BatchDev b,
+                                                         const float4* __restrict__ radiance, uint32_t npix,
+                                                         uint32_t spp, float4* accum, dbl4* sum64, uchar4* bgra) {
+    __shared__ float s_thresh[256];
+    __shared__ float4 s_buf[kResolvePix / 32][32 * (kResSamples + 1)];
+    for (uint32_t i = threadIdx.x; i < 256; i += kResolvePix) s_thresh[i] = c_srgb_thresh[i];
+    __syncthreads();
+    uint32_t block = blockIdx.x;
+    if (BATCH) {
+        uint32_t lo = 0, hi = b.num_items; // the item of this block
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (b.items[mid].block_start <= block) lo = mid;
+            else hi = mid;
+        }
+        const ItemDev& it = b.items[lo];
+        block -= it.block_start;
+        fp = &it.f;
+        radiance += it.path_start;
+        npix = it.f.npix;
+        spp = it.spp;
+        accum = it.accum;
+        sum64 = it.sum64;
+        bgra = it.bgra;
+    }
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t pix0 = block * kResolvePix + warp * 32, pix = pix0 + lane;
+    v3 colors = splat(0.0f);
+    if (spp < 4) {
+        if (pix < npix)
+            for (uint32_t sidx = 0; sidx < spp; ++sidx) colors = colors + xyz(radiance[(size_t)pix * spp + sidx]);
+    } else {
+        float4* buf = s_buf[warp];
+        for (uint32_t s0 = 0; s0 < spp; s0 += kResSamples) {
+            const uint32_t ns = min(kResSamples, spp - s0), sm = lane % kResSamples;
+#pragma unroll
+            for (uint32_t q = 0; q < kResSamples; ++q) {
+                const uint32_t px = q * (32 / kResSamples) + lane / kResSamples;
+                if (sm < ns && pix0 + px < npix)
+                    buf[px * (kResSamples + 1) + sm] = radiance[(size_t)(pix0 + px) * spp + s0 + sm];
+            }
+            __syncwarp();
+            if (pix < npix)
+                for (uint32_t q = 0; q < ns; ++q) colors = colors + xyz(buf[lane * (kResSamples + 1) + q]);
+            __syncwarp();
+        }
+    }
     if (pix >= npix) return;
     const int32_t frame_count = fp->pc.frame_count;
-    v3 colors = splat(0.0f);
-    for (uint32_t sidx = 0; sidx < spp; ++sidx) {
-        const float4 c = radiance[(size_t)sidx * npix + pix];
-        colors = colors + mk(c.x, c.y, c.z);
-    }
     const v3 fin = colors / (float)spp;
+    float4 out;
     if (frame_count <= 0) {
-        accum[pix] = make_float4(fin.x, fin.y, fin.z, 1.0f);
+        out = make_float4(fin.x, fin.y, fin.z, 1.0f);
         sum64[pix] = make_dbl4(fin.x, fin.y, fin.z, 1.0);
     } else {
         const float4 old = accum[pix];
         const float a = 1.0f / (float)(frame_count + 1);
         // mix(x, y, a) = x * (1 - a) + y * a
-        accum[pix] = make_float4(old.x * (1.0f - a) + fin.x * a, old.y * (1.0f - a) + fin.y * a,
-                                 old.z * (1.0f - a) + fin.z * a, 1.0f);
+        out = make_float4(old.x * (1.0f - a) + fin.x * a, old.y * (1.0f - a) + fin.y * a,
+                          old.z * (1.0f - a) + fin.z * a, 1.0f);
         const dbl4 s = sum64[pix];
         sum64[pix] = make_dbl4(s.x + fin.x, s.y + fin.y, s.z + fin.z, s.w + 1.0);
     }
+    accum[pix] = out;
+    bgra[pix] = make_uchar4(srgb8(s_thresh, out.z), srgb8(s_thresh, out.y), srgb8(s_thresh, out.x), 255);
 }
 
-__constant__ float c_srgb_thresh[256];
-
-__device__ __forceinline__ unsigned char srgb8(float v) {
-    if (!(v > 0.0f)) return 0;
-    int lo = 0;
-#pragma unroll
-    for (int step = 128; step >= 1; step >>= 1)
-        if (c_srgb_thresh[lo + step] <= v) lo += step;
-    return (unsigned char)lo;
+// One sample of a per-path buffer as an image (downloads of path data are sample-major).
+__global__ void k_sample_slice(const float4* __restrict__ src, uint32_t npix, uint32_t spp, uint32_t sample,
+                               uint32_t words, float4* dst) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= npix) return;
+    for (uint32_t q = 0; q < words; ++q)
+        dst[(size_t)i * words + q] = src[((size_t)i * spp + sample) * words + q];
 }
 
-// Linear RGBA32F -> B8G8R8A8 sRGB (config.hpp:144, PostProcessing.frag:11-17).
+// Linear RGBA32F -> B8G8R8A8 sRGB.
 __global__ void k_srgb(const float4* __restrict__ img, uint32_t npix, uchar4* out) {
+    __shared__ float s_thresh[256];
+    for (uint32_t k = threadIdx.x; k < 256; k += blockDim.x) s_thresh[k] = c_srgb_thresh[k];
+    __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npix) return;
     const float4 c = img[i];
-    out[i] = make_uchar4(srgb8(c.z), srgb8(c.y), srgb8(c.x), 255);
+    out[i] = make_uchar4(srgb8(s_thresh, c.z), srgb8(s_thresh, c.y), srgb8(s_thresh, c.x), 255);
 }
 
 // FP64 relative MSE: sum over rgb of (x - r)^2 / (r^2 + eps), per-block partials then one final block.
@@ -1538,18 +1619,18 @@ void launch_nee(const SceneDev& s, const FrameDev* f, const BatchDev& b, const W
         k_nee<false><<<grid, kShadeThreads, 0, st>>>(s, f, b, w, depth, chunk_start);
     KF_CUDA_CHECK(cudaGetLastError());
 }
-void launch_shadow(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t grid, bool count_mode,
-                   cudaStream_t st) {
+void launch_shadow(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t depth, uint32_t grid,
+                   bool count_mode, cudaStream_t st) {
     if (b.items) {
         if (count_mode)
-            k_shadow<true, true><<<grid, 128, 0, st>>>(s, b, w);
+            k_shadow<true, true><<<grid, 128, 0, st>>>(s, b, w, depth);
         else
-            k_shadow<false, true><<<grid, 128, 0, st>>>(s, b, w);
+            k_shadow<false, true><<<grid, 128, 0, st>>>(s, b, w, depth);
     } else {
         if (count_mode)
-            k_shadow<true, false><<<grid, 128, 0, st>>>(s, b, w);
+            k_shadow<true, false><<<grid, 128, 0, st>>>(s, b, w, depth);
         else
-            k_shadow<false, false><<<grid, 128, 0, st>>>(s, b, w);
+            k_shadow<false, false><<<grid, 128, 0, st>>>(s, b, w, depth);
     }
     KF_CUDA_CHECK(cudaGetLastError());
 }
@@ -1591,17 +1672,27 @@ uint32_t trace_dyn_blocks_per_sm(bool shadow) {
     return (uint32_t)std::max(1, a);
 }
 
-void launch_gather(const SceneDev& s, const BatchDev& b, const WaveDev& w, int cur, uint64_t chunk_start,
+void launch_gather(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t depth, uint64_t chunk_start,
                    uint32_t grid, cudaStream_t st) {
     if (b.items)
-        k_gather<true><<<grid, 256, 0, st>>>(s, b, w, cur, chunk_start);
+        k_gather<true><<<grid, 256, 0, st>>>(s, b, w, depth, chunk_start);
     else
-        k_gather<false><<<grid, 256, 0, st>>>(s, b, w, cur, chunk_start);
+        k_gather<false><<<grid, 256, 0, st>>>(s, b, w, depth, chunk_start);
     KF_CUDA_CHECK(cudaGetLastError());
 }
 void launch_resolve(const FrameDev* f, const float4* radiance, uint32_t npix, uint32_t spp, float4* accum,
-                    dbl4* sum64, cudaStream_t st) {
-    k_resolve<<<(npix + 255) / 256, 256, 0, st>>>(f, radiance, npix, spp, accum, sum64);
+                    dbl4* sum64, uchar4* bgra, cudaStream_t st) {
+    k_resolve<false><<<(npix + kResolvePix - 1) / kResolvePix, kResolvePix, 0, st>>>(
+        f, BatchDev{nullptr, 0, 0}, radiance, npix, spp, accum, sum64, bgra);
+    KF_CUDA_CHECK(cudaGetLastError());
+}
+void launch_resolve_batch(const BatchDev& b, const float4* radiance, uint32_t blocks, cudaStream_t st) {
+    k_resolve<true><<<blocks, kResolvePix, 0, st>>>(nullptr, b, radiance, 0, 0, nullptr, nullptr, nullptr);
+    KF_CUDA_CHECK(cudaGetLastError());
+}
+void launch_sample_slice(const float4* src, uint32_t npix, uint32_t spp, uint32_t sample, uint32_t words, float4* dst,
+                         cudaStream_t st) {
+    k_sample_slice<<<(npix + 255) / 256, 256, 0, st>>>(src, npix, spp, sample, words, dst);
     KF_CUDA_CHECK(cudaGetLastError());
 }
 void launch_srgb(const float4* img, uint32_t npix, uchar4* out, cudaStream_t st) {

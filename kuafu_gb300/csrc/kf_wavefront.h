@@ -55,6 +55,8 @@ constexpr uint32_t kNoRoot = 0xFFFFFFFFu;
 struct ItemDev {
     FrameDev f;
     uint64_t path_start;
+    uint32_t block_start;     // first block of the item in the batched resolve (kResolvePix pixels each)
+    uint32_t spp;
     uint32_t root;            // TLAS root node in the batch's node pool (kNoRoot: nothing to hit)
     uint32_t num_slots;
     uint8_t slot_group[kMaxLightSlots];
@@ -72,6 +74,9 @@ struct ItemDev {
     float4* normal;
     float* depth;
     uint4* seg;
+    float4* accum;            // resolve targets
+    dbl4* sum64;
+    uchar4* bgra;
 };
 
 // Batch description handed to the kernels (items == nullptr: a single-view frame).
@@ -81,25 +86,37 @@ struct BatchDev {
     uint32_t pad;
 };
 
-// Per-chunk wavefront state.
+// Counters of one bounce, cleared once per chunk for all its bounces: a row per depth, so that
+// no launch waits for a clear between bounces.
+constexpr int kCounterRow = 8; // [0] rays queued, [1] rays that hit, [2] / [3] fetch cursors (closest / shadow)
+constexpr int kSlotRow = 64;   // shadow rays queued per light slot
+
+// Per-chunk wavefront state. A path's number within its view is pixel * spp + sample: a pixel's
+// samples are neighbours in the radiance buffer as they are in the ray queues, so a warp's
+// radiance accesses fall into a few lines. Everything a bounce hands from kernel to kernel is
+// stored in queue order (rays) or hit-list order (hits) and read coalesced. Before, throughput,
+// radiance, requests, contributions and visibility were indexed by a sample-major path number,
+// which put a warp's 32 accesses into 32 lines: a Cornell room of 256 x 256 at 64 spp takes 3.49
+// instead of 4.57 ms (no NEE there: its three kernels and records, a quarter of that frame, are
+// skipped), the 256-icosphere frame at 1080p, 8 spp, 21.8 instead of 22.7 ms.
 struct WaveDev {
     float4* q_o[2];       // ray queue: origin.xyz + path id bits
-    float4* q_d[2];       // ray queue: direction.xyz
-    uint32_t* counters;   // [0],[1] ray queue counts, [2] shadow count, [3],[4] fetch cursors,
-                          // [5] rays of the bounce that hit
+    float4* q_d[2];       // ray queue: direction.xyz + throughput.x
+    float2* q_w[2];       // ray queue: throughput.yz (not written for camera rays: 1)
+    uint32_t* counters;   // kCounterRow words per depth
     float4* hit;          // t, u, v, instance bits
     uint32_t* hit_prim;
-    uint32_t* sel;        // queue positions of this bounce's rays that hit ([5] of them)
-    uint32_t* scount;     // per light slot j: shadow rays queued, at sq_o/sq_d[j * chunk_cap + k]
+    uint32_t* sel;        // queue positions of this bounce's rays that hit
+    uint32_t* scount;     // kSlotRow words per depth: slot j's shadow rays, at sq_o/sq_d[j * chunk_cap + k]
     uint32_t nslot;       // light slots with a shadow queue (scount entries)
-    float4* weight;       // throughput carried to the next bounce
-    float4* nee_w;        // throughput that scales this bounce's NEE
-    float4* nee_in;       // per hit (hit-list order), 6 float4: what k_nee needs of k_shade's shading
-    uint64_t* req;        // shadow slots requested this bounce (bit j = slot j)
-    float4* contrib;      // [slot][chunk] light contribution
-    uint8_t* vis;         // [slot][chunk] 1 = unoccluded
+    uint32_t lit;         // some view of the launch has a light slot (else no NEE is recorded)
+    float4* nee_w;        // per hit: throughput that scales this bounce's NEE + path id and flag bits
+    float4* nee_in;       // per hit, 5 arrays of chunk_cap: what k_nee needs of k_shade's shading
+    uint64_t* req;        // per hit: shadow slots requested this bounce (bit j = slot j)
+    float4* contrib;      // [slot][hit] light contribution
+    uint8_t* vis;         // [slot][hit] 1 = unoccluded
     float4* sq_o;         // shadow queue: origin.xyz + tmax
-    float4* sq_d;         // shadow queue: direction.xyz + (slot << 26 | path) bits
+    float4* sq_d;         // shadow queue: direction.xyz + (slot << 26 | hit) bits
     float4* radiance;     // per global path (frame): accumulated `color`
     kf_hit* primary;      // per global path, debug (may be null)
     float4* albedo;       // per pixel AOVs
@@ -108,6 +125,7 @@ struct WaveDev {
     uint4* seg;           // per pixel {instance, geometry, material, primitive} of sample 0's first hit
     unsigned long long* stats; // [0] primary, [1] extension, [2] shadow, [3] nodes, [4] tris, [5] inst
     uint16_t* path_item;       // batched launch: item of each path of the chunk
+    uint16_t* hit_item;        // batched launch: item of each hit
     uint32_t chunk_cap;
 };
 
@@ -126,20 +144,27 @@ void launch_miss(const SceneDev& s, const FrameDev* f, const BatchDev& b, const 
 // Light samples (shadow queues, contributions, NEE requests) of the hits k_shade shaded.
 void launch_nee(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, uint32_t depth,
                 uint64_t chunk_start, uint32_t grid, cudaStream_t st);
-void launch_shadow(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t grid, bool count_mode,
-                   cudaStream_t st);
+void launch_shadow(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t depth, uint32_t grid,
+                   bool count_mode, cudaStream_t st);
 // Persistent traversal with dynamic ray fetch (closest hit, or shadow rays when `shadow`).
-// Needs w.counters[3] (closest) / w.counters[4] (shadow) zeroed before the launch.
 // refill_below (1..32) and steps (1..64): the warp scheduling of the persistent kernel.
 void launch_trace_dyn(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
                       uint32_t depth, uint64_t chunk_start, bool shadow, uint32_t grid, bool count_mode,
                       uint32_t refill_below, uint32_t steps, cudaStream_t st);
 // resident blocks per SM of the persistent traversal kernel (closest-hit or shadow variant)
 uint32_t trace_dyn_blocks_per_sm(bool shadow);
-void launch_gather(const SceneDev& s, const BatchDev& b, const WaveDev& w, int cur, uint64_t chunk_start,
+void launch_gather(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t depth, uint64_t chunk_start,
                    uint32_t grid, cudaStream_t st);
+// Per-pixel mean, running mean, FP64 sum and the BGRA frame of one view.
+constexpr uint32_t kResolvePix = 256; // pixels per block
 void launch_resolve(const FrameDev* f, const float4* radiance, uint32_t npix, uint32_t spp, float4* accum,
-                    dbl4* sum64, cudaStream_t st);
+                    dbl4* sum64, uchar4* bgra, cudaStream_t st);
+// The same for every view of a batch in one launch (blocks: the items' resolve blocks in all).
+void launch_resolve_batch(const BatchDev& b, const float4* radiance, uint32_t blocks, cudaStream_t st);
+// dst[pix] = src[pix * spp + sample] of `words` float4 per path: one sample of a per-path buffer
+// as an image (downloads are sample-major).
+void launch_sample_slice(const float4* src, uint32_t npix, uint32_t spp, uint32_t sample, uint32_t words, float4* dst,
+                         cudaStream_t st);
 void launch_srgb(const float4* img, uint32_t npix, uchar4* out, cudaStream_t st);
 void upload_srgb_thresholds(const float* thresh256);
 void launch_relmse(const float4* x, const float4* ref, uint64_t n, double eps, double* partial, uint32_t blocks,

@@ -1,0 +1,112 @@
+"""Path numbering and queue layout: results do not depend on how a frame is cut into chunks,
+on which views of a batch have lights, or on lights that appear between batches.
+
+The reference is the same frame in one chunk (itself equal to the oracle in test_gpu_parity.py);
+every comparison is bit for bit.
+"""
+import numpy as np
+import pytest
+
+from kuafu_gb300 import _native as N
+from kuafu_gb300 import api, scenes
+
+pytestmark = pytest.mark.gpu
+
+AOVS = (N.KF_AOV_RADIANCE_F32, N.KF_AOV_ALBEDO_F32, N.KF_AOV_NORMAL_F32, N.KF_AOV_DEPTH_F32, N.KF_AOV_SEGMENTATION,
+        N.KF_AOV_PATH_RADIANCE, N.KF_AOV_PRIMARY_HITS)
+
+
+def _aov(r, cam, kind):
+    a = r.downloadAov(cam, kind)
+    if kind == N.KF_AOV_SEGMENTATION:
+        a = a[..., [0, 1, 3]]  # not the material: its number counts every material of the process
+    return a
+
+
+def _same(a, b):
+    return np.array_equal(np.ascontiguousarray(a).view(np.uint8), np.ascontiguousarray(b).view(np.uint8))
+
+
+def _frame(lit, w, h, spp, chunk):
+    cfg = scenes.icosphere_config(spp=spp, depth=5, count=6) if lit else scenes.cornell_config(spp=spp, depth=4)
+    cfg.setDebugOutputs(True)
+    if chunk:
+        cfg.setMaxPathsInFlight(chunk)
+    with api.Kuafu(cfg) as r:
+        cam = scenes.icospheres(r, w, h, count=6, level=2) if lit else scenes.cornell(r, w, h)
+        r.run()
+        return [_aov(r, cam, k) for k in AOVS] + [r.downloadLatestFrame(cam)]
+
+
+# odd sizes; chunks that end inside a pixel, inside a band of rows and at band ends (8 rows)
+@pytest.mark.parametrize("lit", [False, True])
+@pytest.mark.parametrize("w,h,spp,chunk", [(37, 19, 7, 1000), (33, 24, 9, 33 * 8 * 9), (41, 9, 3, 1), (64, 17, 12, 777)])
+def test_chunks_do_not_change_the_frame(lit, w, h, spp, chunk):
+    if chunk == 1:
+        w, h, spp, chunk = 5, 3, 2, 4
+    for kind, a, b in zip(AOVS + ("frame",), _frame(lit, w, h, spp, 0), _frame(lit, w, h, spp, chunk)):
+        assert _same(a, b), kind
+
+
+def test_resolve_sample_counts():
+    """Sample counts around the resolve's groups of 8: the mean of the downloaded paths, in order."""
+    for spp in (1, 3, 4, 8, 9, 17):
+        cfg = scenes.cornell_config(spp=spp, depth=2)
+        with api.Kuafu(cfg) as r:
+            cam = scenes.cornell(r, 45, 13)
+            r.run()
+            paths = r.downloadAov(cam, N.KF_AOV_PATH_RADIANCE, spp)[..., :3]
+            total = np.zeros_like(paths[0])
+            for k in range(spp):
+                total = total + paths[k]
+            assert _same(r.downloadAov(cam, N.KF_AOV_RADIANCE_F32)[..., :3], total / np.float32(spp)), spp
+
+
+def _mixed(r):
+    """A room without lights to sample, spheres with seven, and a second camera of the room."""
+    room, spheres = r.getScene(), r.createScene()
+    c0 = scenes.cornell(r, 40, 31, scene=room)
+    c1 = scenes.icospheres(r, 53, 27, count=5, level=2, scene=spheres)
+    c2 = room.createCamera(24, 24)
+    c2.setPosition((-3.0, 0.1, 0.2))
+    c2.setFront((1.0, 0.0, 0.0))
+    c2.setUp((0.0, 0.0, 1.0))
+    scenes.pinhole(c2, 24, 24, 50.0)
+    return room, [(room, c0, 5), (spheres, c1, 3), (room, c2, 9)]
+
+
+@pytest.mark.parametrize("chunk", [0, 1234])
+def test_batch_of_lit_and_unlit_views(chunk):
+    def render(pick):
+        cfg = scenes.icosphere_config(spp=1, depth=4, count=64)
+        if chunk:
+            cfg.setMaxPathsInFlight(chunk)
+        with api.Kuafu(cfg) as r:
+            _, items = _mixed(r)
+            part = [items[k] for k in pick]
+            r.runBatch(part)
+            return [_aov(r, c, k) for _, c, _ in part for k in AOVS[:5]]
+
+    alone = [x for k in range(3) for x in render([k])]  # one view each: a new renderer's first frame word
+    for a, b in zip(render([0, 1, 2]), alone):
+        assert _same(a, b)
+
+
+def test_lights_added_between_batches():
+    """The captured launch sequence is renewed when a batch gains lights (its buffers move)."""
+    light = lambda: api.PointLight(position=(0.0, 0.0, 0.5), color=(1.0, 0.9, 0.8), radius=0.1, strength=2.0)
+
+    def render(when):
+        with api.Kuafu(scenes.icosphere_config(spp=1, depth=4, count=64)) as r:
+            room, items = _mixed(r)
+            items = [items[0], items[2]]
+            for batch in range(2):
+                if batch == when:
+                    for _ in range(3):
+                        room.addPointLight(light())
+                r.runBatch(items)
+            return [r.downloadAov(c, N.KF_AOV_RADIANCE_F32) for _, c, _ in items]
+
+    for a, b, dark in zip(render(1), render(0), render(2)):
+        assert _same(a, b)
+        assert not _same(a, dark)
