@@ -244,8 +244,9 @@ KF_API int kf_renderer_create(const kf_config* cfg, kf_renderer* out) {
         r->grid_extend = (uint32_t)r->num_sms * 16;
         r->grid_shade = (uint32_t)r->num_sms * 16; // 16 blocks per SM measured fastest (4, 8, 16)
         if (!r->cfg.host_only) {
-            r->grid_dyn = (uint32_t)r->num_sms * trace_dyn_blocks_per_sm(false);
-            r->grid_dyn_shadow = (uint32_t)r->num_sms * trace_dyn_blocks_per_sm(true);
+            r->grid_dyn = (uint32_t)r->num_sms * trace_dyn_blocks_per_sm(TraceKind::bounce);
+            r->grid_dyn_camera = (uint32_t)r->num_sms * trace_dyn_blocks_per_sm(TraceKind::camera);
+            r->grid_dyn_shadow = (uint32_t)r->num_sms * trace_dyn_blocks_per_sm(TraceKind::shadow);
         }
         // Kuafu::Kuafu (kuafu.cpp:27-63): a scene with a 1x1 camera; present mode adds
         // a camera of the initial size and makes it current.

@@ -213,12 +213,20 @@ __host__ __device__ __forceinline__ int leaf_first(int child) { return (int)((ui
 // TLAS instance record, 64 B: world->object rows + BLAS addressing.
 struct alignas(16) InstanceRec {
     float4 w2o0, w2o1, w2o2;
-    uint32_t blas_root; // node index in the BLAS node pool
+    uint32_t blas_root; // node index in the BLAS node pool, or a leaf link into the triangle pool
     uint32_t geometry;  // geometry index
     uint32_t flags;     // bit0: opaque, bit1: hidden
     uint32_t pad;
 };
 static_assert(sizeof(InstanceRec) == 64, "InstanceRec must be 64 bytes");
+
+// An opaque geometry of up to this many triangles is entered as a leaf, without its BLAS root
+// node: a quad's two triangles have the quad's box each, so the root culls nothing, and one node
+// visit costs about as much as one triangle test. Five wall quads to a Cornell room: 3.59 instead
+// of 3.99 ms a frame of 256 x 256 at 64 spp, a batch of rooms with spheres 58.8 instead of 63.0 ms
+// (both of one build of the traversal). Up to 12 triangles (boxes): 3.68 and 66.7 ms.
+// Non-opaque geometry keeps its node: the any-hit draws follow the order of its candidates.
+constexpr uint32_t kRootLeafTris = 2;
 
 // Precomputed triangle, 48 B: the three object-space vertices; w of the first
 // float4 carries the primitive index within its geometry.

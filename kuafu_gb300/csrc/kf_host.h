@@ -87,6 +87,7 @@ struct SceneGpu {
     kf::DeviceBuffer<float4> env;
     uint64_t built_env_version = 0;
     std::vector<uint32_t> blas_root;                 // per geometry
+    std::vector<uint32_t> blas_tri;                  // per geometry: first triangle of its BLAS in the pool
     std::vector<std::array<float, 6>> blas_box;      // per geometry object-space box
     std::vector<std::array<double, 10>> blas_bound; // per geometry: vertex box and bounding sphere
     std::vector<uint32_t> tri_offset, vert_offset;   // per geometry
@@ -190,7 +191,7 @@ struct kf_renderer_s {
     kf_stats stats{};
     bool count_traversal = false;
     uint32_t grid_extend = 0, grid_shade = 0;
-    uint32_t grid_dyn = 0, grid_dyn_shadow = 0; // persistent traversal: one resident wave each
+    uint32_t grid_dyn = 0, grid_dyn_camera = 0, grid_dyn_shadow = 0; // persistent traversal: one resident wave each
     // CUDA graph of one frame's launch sequence
     cudaGraphExec_t graph_exec = nullptr;
     std::string graph_key;

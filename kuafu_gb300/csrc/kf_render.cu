@@ -267,8 +267,8 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
         for (uint32_t depth = 0; depth <= max_depth; ++depth) {
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[0], st));
             if (dyn)
-                launch_trace_dyn(sv, fd, b, w, cur, depth, start, false, r->grid_dyn, r->count_traversal,
-                                 r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
+                launch_trace_dyn(sv, fd, b, w, cur, depth, start, false, depth ? r->grid_dyn : r->grid_dyn_camera,
+                                 r->count_traversal, r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
             else
                 launch_extend(sv, fd, b, w, cur, depth, start, r->grid_extend, r->count_traversal, st);
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[1], st));

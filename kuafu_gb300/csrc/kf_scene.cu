@@ -312,6 +312,7 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
 
         // BLAS per geometry, appended to one node pool and one triangle pool.
         G.blas_root.assign(ng, 0);
+        G.blas_tri.assign(ng, 0);
         G.blas_box.assign(ng, {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY});
         G.blas_bound.resize(ng);
         for (size_t gi = 0; gi < ng; ++gi) G.blas_bound[gi] = geometry_bound(s->geometries[gi]);
@@ -405,10 +406,12 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
                 const size_t bi = build_of[gi];
                 if (share && bi != gi) { // the first geometry of this build was placed before
                     G.blas_root[gi] = G.blas_root[bi];
+                    G.blas_tri[gi] = G.blas_tri[bi];
                     G.blas_box[gi] = G.blas_box[bi];
                     continue;
                 }
                 G.blas_root[gi] = (uint32_t)pool.size();
+                G.blas_tri[gi] = geom[gi].y;
                 root_box(sah_nodes[bi][0], G.blas_box[gi]);
                 const uint32_t nb = (uint32_t)pool.size(), tb = geom[gi].y;
                 for (Node4 nd : sah_nodes[bi]) {
@@ -438,6 +441,7 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
             if (ntri == 0) continue;
             if (r->cfg.blas_share && build_of[gi] != gi) {
                 G.blas_root[gi] = G.blas_root[build_of[gi]];
+                G.blas_tri[gi] = G.blas_tri[build_of[gi]];
                 G.blas_box[gi] = G.blas_box[build_of[gi]];
                 continue;
             }
@@ -459,6 +463,7 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
             KF_CUDA_CHECK(cudaStreamSynchronize(st));
             root_box(root, G.blas_box[gi]);
             G.blas_root[gi] = node_base;
+            G.blas_tri[gi] = geom[gi].y;
             node_base += (uint32_t)nn;
         }
         G.blas_node_count = node_base;
@@ -540,6 +545,9 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
             rc.geometry = (uint32_t)gi;
             const kf_geometry_s* g = s->geometries[gi];
             const bool hidden = g->hide_render || g->indices.size() < 3;
+            const size_t ntri = g->indices.size() / 3;
+            if (!hidden && g->opaque && ntri <= kRootLeafTris)
+                rc.blas_root = (uint32_t)leaf_child((int)G.blas_tri[gi], (int)ntri);
             rc.flags = (g->opaque ? 1u : 0u) | (hidden ? 2u : 0u);
             rc.pad = 0;
             if (hidden) continue;
@@ -833,7 +841,7 @@ void batch_sync(kf_renderer_s* r, const std::vector<kf_scene_s*>& scenes) {
             KF_CUDA_CHECK(cudaMemcpyAsync(recs.data(), G.inst.ptr, sn * sizeof(InstanceRec), cudaMemcpyDeviceToHost, st));
             KF_CUDA_CHECK(cudaStreamSynchronize(st));
             for (InstanceRec& rc : recs) {
-                rc.blas_root += (uint32_t)obn;
+                rc.blas_root += (rc.blas_root & kLeafChildTag) ? (uint32_t)ot : (uint32_t)obn;
                 rc.geometry += (uint32_t)og;
                 inst.push_back(rc);
             }

@@ -88,9 +88,15 @@ __device__ __forceinline__ bool anyhit_accept(const SceneDev& s, uint32_t geomet
 
 // Traversal stack of one thread: the first kSmemStack entries live in shared
 // memory laid out entry-major (entry * blockDim + thread, so a warp's accesses hit
-// 32 different banks whatever each lane's depth), deeper entries in local memory.
-constexpr int kSmemStack = 40;
+// 32 different banks whatever each lane's depth), deeper entries in local memory. 16 entries:
+// shared memory is taken from the L1 that serves the nodes and triangles. With the world ray
+// beside the stack, the 256-icosphere 1080p frame takes 21.7 ms with 40 entries, 20.0 with 31,
+// 19.5 with 24 or 20, 19.4 with 16 to 12, 19.5 with 10 and 19.9 with 8 (a Cornell room 3.27,
+// 3.15, 3.08, 3.02, 3.02, 3.02, 3.04).
+constexpr int kSmemStack = 16;
+constexpr int kWorldRay = 9; // words of the world ray (origin, direction, 1 / direction), after the stack
 constexpr int kThreadsTrace = 128;
+constexpr int kSmemTrace = (kSmemStack + kWorldRay) * kThreadsTrace;
 struct TStack {
     uint32_t* sm; // &shared[threadIdx.x]
     uint32_t deep[kStack - kSmemStack];
@@ -105,47 +111,98 @@ struct TStack {
     }
 };
 
-// Resumable two-level traversal state: init() then step() until it returns true.
-// One step processes one stack entry (a node with its leaf children, an instance
-// entry or the return to the TLAS), so a warp can interleave rays step by step.
-// The slab test of box4 on a node read in place: the near and far planes of each axis are
-// loaded by the ray's direction signs (no selects), with the child links.
+// Two FP32 operations in one instruction (sm_100's f32x2), each rounded as the scalar one, and
+// the three-input minimum / maximum.
+__device__ __forceinline__ uint64_t pk2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void up2(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// The slab test of box4 on a node read in place, with the child links: the near and far planes
+// of each axis are loaded by the ray's direction signs (no selects) and tested two children per
+// instruction (18.9 instead of 19.3 ms on the 256-icosphere 1080p frame; no change while the
+// kernel still spilled).
 __device__ __forceinline__ int box4_dir(const PRay& r, const float4* p, float tmin, float tmax, float tn_out[4],
-                                        int4& child, int4& cnt) {
+                                        int4& child) {
     const int sx = r.ix >= 0.0f ? 0 : 1, sy = r.iy >= 0.0f ? 0 : 1, sz = r.iz >= 0.0f ? 0 : 1;
-    const float4 nx = __ldg(p + sx), fx = __ldg(p + (1 - sx));
-    const float4 ny = __ldg(p + 2 + sy), fy = __ldg(p + (3 - sy));
-    const float4 nz = __ldg(p + 4 + sz), fz = __ldg(p + (5 - sz));
     child = __ldg(reinterpret_cast<const int4*>(p + 6));
-    cnt = __ldg(reinterpret_cast<const int4*>(p + 7));
+    const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
+    const ulonglong2 nx = __ldg(q + sx), fx = __ldg(q + (1 - sx));
+    const ulonglong2 ny = __ldg(q + 2 + sy), fy = __ldg(q + (3 - sy));
+    const ulonglong2 nz = __ldg(q + 4 + sz), fz = __ldg(q + (5 - sz));
+    const uint64_t ox = pk2(-r.ox, -r.ox), oy = pk2(-r.oy, -r.oy), oz = pk2(-r.oz, -r.oz);
+    const uint64_t ix = pk2(r.ix, r.ix), iy = pk2(r.iy, r.iy), iz = pk2(r.iz, r.iz);
+    const uint64_t wd = pk2(KF_BOX_WIDEN, KF_BOX_WIDEN);
+    const float lim = tmax * KF_TMAX_WIDEN;
     int mask = 0;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float t1x, t1y, t1z;
-        const float t0x = slab1(lane(nx, c), lane(fx, c), r.ox, r.ix, t1x);
-        const float t0y = slab1(lane(ny, c), lane(fy, c), r.oy, r.iy, t1y);
-        const float t0z = slab1(lane(nz, c), lane(fz, c), r.oz, r.iz, t1z);
-        float tn = fmaxf(tmin, t0x);
-        float tf = fminf(__int_as_float(0x7f800000), t1x);
-        tn = fmaxf(tn, t0y);
-        tf = fminf(tf, t1y);
-        tn = fmaxf(tn, t0z);
-        tf = fminf(tf, t1z);
-        tn_out[c] = tn;
-        if (tn <= fminf(tf * KF_BOX_WIDEN, tmax * KF_TMAX_WIDEN)) mask |= 1 << c;
+    for (int h = 0; h < 2; ++h) {
+        float x0, x1, y0, y1, z0, z1, u0, u1, v0, v1, w0, w1;
+        up2(mul2(add2(h ? nx.y : nx.x, ox), ix), x0, x1);
+        up2(mul2(add2(h ? ny.y : ny.x, oy), iy), y0, y1);
+        up2(mul2(add2(h ? nz.y : nz.x, oz), iz), z0, z1);
+        up2(mul2(add2(h ? fx.y : fx.x, ox), ix), u0, u1);
+        up2(mul2(add2(h ? fy.y : fy.x, oy), iy), v0, v1);
+        up2(mul2(add2(h ? fz.y : fz.x, oz), iz), w0, w1);
+        float f0, f1;
+        up2(mul2(pk2(min3(u0, v0, w0), min3(u1, v1, w1)), wd), f0, f1);
+        tn_out[2 * h] = fmaxf(max3(tmin, x0, y0), z0);
+        tn_out[2 * h + 1] = fmaxf(max3(tmin, x1, y1), z1);
+        if (tn_out[2 * h] <= fminf(f0, lim)) mask |= 1 << (2 * h);
+        if (tn_out[2 * h + 1] <= fminf(f1, lim)) mask |= 2 << (2 * h);
     }
     return mask;
 }
 
-template <bool SHADOW, bool COUNT> struct Tracer {
-    PRay wr, r;
+// Resumable two-level traversal state: init() then step() until it returns true.
+// One step processes one stack entry (a node with its leaf children, an instance
+// entry or the return to the TLAS), so a warp can interleave rays step by step.
+template <bool SHADOW, bool COUNT, bool VOTE> struct Tracer {
+    PRay r; // the ray in the space of the nodes and triangles it meets
     TStack stack;
     int sp;
+    uint32_t e; // VOTE: the entry to process next, off the stack
     bool in_blas, cur_opaque;
     uint32_t cur_inst, cur_geom;
     float tmin, best;
     HitOut h;
     TraceCounters cnt;
+
+    // The world ray lives in shared memory: it is read at instance entries and on the way back
+    // to the TLAS only, and its nine registers would spill.
+    __device__ __forceinline__ float& world(int k) {
+        return reinterpret_cast<float*>(stack.sm)[(kSmemStack + k) * kThreadsTrace];
+    }
+    __device__ __forceinline__ void to_world() {
+        in_blas = false;
+        // back in the TLAS only boxes are tested: origin and reciprocal direction
+        // (copying the shear terms too would keep them live in registers)
+        r.ox = world(0); r.oy = world(1); r.oz = world(2);
+        r.ix = world(6); r.iy = world(7); r.iz = world(8);
+    }
 
     // root: the TLAS root node of the ray's scene (kNoRoot: the ray hits nothing)
     __device__ __forceinline__ void init(uint32_t root, float ox, float oy, float oz, float dx, float dy, float dz,
@@ -153,12 +210,15 @@ template <bool SHADOW, bool COUNT> struct Tracer {
         h.inst = kMiss;
         h.t = h.u = h.v = 0.0f;
         h.prim = 0;
-        wr.ox = ox; wr.oy = oy; wr.oz = oz;
-        wr.dx = dx; wr.dy = dy; wr.dz = dz;
-        prep_ray(wr);
-        r = wr;
+        r.ox = ox; r.oy = oy; r.oz = oz;
+        r.dx = dx; r.dy = dy; r.dz = dz;
+        prep_ray(r);
+        world(0) = ox; world(1) = oy; world(2) = oz;
+        world(3) = dx; world(4) = dy; world(5) = dz;
+        world(6) = r.ix; world(7) = r.iy; world(8) = r.iz;
         sp = 0;
-        if (root != kNoRoot) stack.put(sp++, root);
+        e = root;
+        if (!VOTE && root != kNoRoot) stack.put(sp++, root);
         in_blas = false;
         cur_inst = cur_geom = 0;
         cur_opaque = true;
@@ -172,16 +232,12 @@ template <bool SHADOW, bool COUNT> struct Tracer {
     // node index. Node child links are entries of these kinds as they are.
     // The rare, cheap entries do not take a step of their own: a return to the TLAS goes on
     // to the next entry (a TLAS node or instance), and an instance entry goes on to the root
-    // node of its BLAS, so the lanes of a warp mostly run the node or the leaf code together.
+    // of its BLAS, so the lanes of a warp mostly run the node or the leaf code together.
     __device__ __forceinline__ bool step(const SceneDev& s, AnyHitCtx* ah) {
         if (sp <= 0) return true;
         uint32_t e = stack.get(--sp);
         if (e == kPopTag) {
-            in_blas = false;
-            // back in the TLAS only boxes are tested: origin and reciprocal direction
-            // (copying the shear terms too would keep them live in registers)
-            r.ox = wr.ox; r.oy = wr.oy; r.oz = wr.oz;
-            r.ix = wr.ix; r.iy = wr.iy; r.iz = wr.iz;
+            to_world();
             if (sp <= 0) return true;
             e = stack.get(--sp); // below a return entry: a TLAS node or an instance entry
         }
@@ -193,28 +249,6 @@ template <bool SHADOW, bool COUNT> struct Tracer {
             for (uint32_t q = (e >> 26) & 0xFu; q > 0; --q)
                 if (sp < kStack) stack.put(sp++, kInstTag | __ldg(s.tlas_inst + first + q));
             e = kInstTag | __ldg(s.tlas_inst + first);
-        }
-        if ((e & 0xC0000000u) == kLeafTag) {
-            const uint32_t first = e & 0x03FFFFFFu, cnt_tri = ((e >> 26) & 0xFu) + 1u;
-#pragma unroll 1
-            for (uint32_t q = 0; q < cnt_tri; ++q) {
-                const float4* tp = reinterpret_cast<const float4*>(s.tris + first + q);
-                const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
-                if (COUNT) cnt.tris++;
-                float t, u, v;
-                if (!intersect_tri(r, a, b, cc, tmin, best, t, u, v)) continue;
-                const uint32_t prim = __float_as_uint(a.w);
-                if (SHADOW) {
-                    h.inst = cur_inst;
-                    sp = 0;
-                    return true;
-                }
-                if (!closer(t, cur_inst, prim, h.t, h.inst, h.prim)) continue;
-                if (!cur_opaque && ah && !anyhit_accept(s, cur_geom, prim, *ah)) continue;
-                h.t = t; h.u = u; h.v = v; h.inst = cur_inst; h.prim = prim;
-                best = t;
-            }
-            return sp <= 0;
         }
         if (e & kInstTag) {
             cur_inst = e & ~kInstTag;
@@ -228,16 +262,46 @@ template <bool SHADOW, bool COUNT> struct Tracer {
             if (meta.z & 2u) return sp <= 0; // hidden (dummy BLAS, rt.cpp:156)
             cur_geom = meta.y;
             cur_opaque = (meta.z & 1u) != 0;
-            to_object(in, wr.ox, wr.oy, wr.oz, wr.dx, wr.dy, wr.dz, r);
+            to_object(in, world(0), world(1), world(2), world(3), world(4), world(5), r);
             in_blas = true;
             if (sp + 2 > kStack) return sp <= 0;
             stack.put(sp++, kPopTag);
-            e = meta.x; // the BLAS root, visited in this step
+            e = meta.x; // the BLAS root (a node, or a leaf of few triangles), visited in this step
         }
-        Node4 n;
+        if ((e & 0xC0000000u) == kLeafTag) return leaf(s, ah, e) || sp <= 0;
+        node(s, e);
+        return sp <= 0;
+    }
+
+    // The triangles of a BLAS leaf; true: a shadow ray is done.
+    __device__ __forceinline__ bool leaf(const SceneDev& s, AnyHitCtx* ah, uint32_t e) {
+        const uint32_t first = e & 0x03FFFFFFu, cnt_tri = ((e >> 26) & 0xFu) + 1u;
+#pragma unroll 1
+        for (uint32_t q = 0; q < cnt_tri; ++q) {
+            const float4* tp = reinterpret_cast<const float4*>(s.tris + first + q);
+            const float4 a = __ldg(tp), b = __ldg(tp + 1), cc = __ldg(tp + 2);
+            if (COUNT) cnt.tris++;
+            float t, u, v;
+            if (!intersect_tri(r, a, b, cc, tmin, best, t, u, v)) continue;
+            const uint32_t prim = __float_as_uint(a.w);
+            if (SHADOW) {
+                h.inst = cur_inst;
+                return true;
+            }
+            if (!closer(t, cur_inst, prim, h.t, h.inst, h.prim)) continue;
+            if (!cur_opaque && ah && !anyhit_accept(s, cur_geom, prim, *ah)) continue;
+            h.t = t; h.u = u; h.v = v; h.inst = cur_inst; h.prim = prim;
+            best = t;
+        }
+        return false;
+    }
+
+    // Visits a node: the children it meets go on the stack, the one to visit first on top.
+    __device__ __forceinline__ void node(const SceneDev& s, uint32_t e) {
+        int4 child;
         float tn[4];
         const int mask = box4_dir(r, reinterpret_cast<const float4*>((in_blas ? s.blas_nodes : s.tlas_nodes) + e), tmin,
-                                  best, tn, n.child, n.cnt);
+                                  best, tn, child);
         if (COUNT) cnt.nodes++;
         // children to visit, as (entry distance, stack entry); misses get -inf. The child
         // links are stack entries already: node indices, and leaf entries (triangles in a
@@ -248,7 +312,7 @@ template <bool SHADOW, bool COUNT> struct Tracer {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             it[c] = ((mask >> c) & 1) ? tn[c] : __int_as_float(0xff800000);
-            ic[c] = (uint32_t)lanei(n.child, c);
+            ic[c] = (uint32_t)lanei(child, c);
         }
         // sort by entry distance (fixed network, registers only), then push. Closest-hit rays
         // sort descending, so the nearest child ends on top of the stack; shadow rays (ended by
@@ -283,7 +347,49 @@ template <bool SHADOW, bool COUNT> struct Tracer {
             for (int c = 0; c < 4; ++c)
                 if (it[c] != __int_as_float(0xff800000) && sp < kStack) stack.put(sp++, ic[c]);
         }
-        return sp <= 0;
+    }
+
+    // ---- vote scheduling: the same work, one kind per call, the next entry left in e ----
+    __device__ __forceinline__ bool is_node() const { return !(e & 0xC0000000u); }
+    __device__ __forceinline__ bool is_inst() const { return (e & kInstTag) != 0; }
+    __device__ __forceinline__ bool is_leaf() const { return (e & 0xC0000000u) == kLeafTag; }
+
+    // Takes the next entry off the stack; false when the traversal is over.
+    __device__ __forceinline__ bool pop(const SceneDev& s) {
+        if (sp <= 0) return false;
+        e = stack.get(--sp);
+        if (e == kPopTag) {
+            to_world();
+            if (sp <= 0) return false;
+            e = stack.get(--sp); // below a return entry: a TLAS node or an instance entry
+        }
+        if (!in_blas && is_leaf()) { // a TLAS leaf: its first instance, the others wait on the stack
+            const uint32_t first = e & 0x03FFFFFFu;
+#pragma unroll 1
+            for (uint32_t q = (e >> 26) & 0xFu; q > 0; --q)
+                if (sp < kStack) stack.put(sp++, kInstTag | __ldg(s.tlas_inst + first + q));
+            e = kInstTag | __ldg(s.tlas_inst + first);
+        }
+        return true;
+    }
+    // Enters the instance: the BLAS root is next. False: hidden, or no room for the return entry.
+    __device__ __forceinline__ bool inst(const SceneDev& s) {
+        cur_inst = e & ~kInstTag;
+        const InstanceRec* ip = s.inst + cur_inst;
+        InstanceRec in;
+        in.w2o0 = __ldg(&ip->w2o0);
+        in.w2o1 = __ldg(&ip->w2o1);
+        in.w2o2 = __ldg(&ip->w2o2);
+        const uint4 meta = __ldg(reinterpret_cast<const uint4*>(ip) + 3);
+        if (COUNT) cnt.insts++;
+        if ((meta.z & 2u) || sp + 2 > kStack) return false;
+        cur_geom = meta.y;
+        cur_opaque = (meta.z & 1u) != 0;
+        to_object(in, world(0), world(1), world(2), world(3), world(4), world(5), r);
+        in_blas = true;
+        stack.put(sp++, kPopTag);
+        e = meta.x;
+        return true;
     }
 };
 
@@ -292,7 +398,7 @@ template <bool SHADOW, bool COUNT>
 __device__ bool trace(const SceneDev& s, uint32_t root, uint32_t* smem, float ox, float oy, float oz, float dx,
                       float dy, float dz, float tmin, float tmax, HitOut& h, TraceCounters& cnt,
                       AnyHitCtx* ah = nullptr) {
-    Tracer<SHADOW, COUNT> t;
+    Tracer<SHADOW, COUNT, false> t;
     t.stack.sm = smem + threadIdx.x;
     t.init(root, ox, oy, oz, dx, dy, dz, tmin, tmax);
     t.cnt = cnt;
@@ -472,7 +578,7 @@ __global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
 template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(128) k_extend(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
                                                 int cur, uint32_t depth, uint64_t chunk_start) {
-    __shared__ uint32_t s_stack[kSmemStack * kThreadsTrace];
+    __shared__ uint32_t s_stack[kSmemTrace];
     const uint32_t count = w.counters[depth * kCounterRow];
     const float4* __restrict__ qo = w.q_o[cur];
     const float4* __restrict__ qd = w.q_d[cur];
@@ -1271,7 +1377,7 @@ __device__ __forceinline__ uint32_t shadow_entry(const WaveDev& w, const uint32_
 
 template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(128) k_shadow(SceneDev s, BatchDev b, WaveDev w, uint32_t depth) {
-    __shared__ uint32_t s_stack[kSmemStack * kThreadsTrace];
+    __shared__ uint32_t s_stack[kSmemTrace];
     __shared__ uint32_t s_pre[kMaxSlots + 1];
     const uint32_t count = shadow_prefix(w, depth, s_pre);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.stats[2], (unsigned long long)count);
@@ -1299,17 +1405,27 @@ __global__ void __launch_bounds__(128) k_shadow(SceneDev s, BatchDev b, WaveDev 
 // flight; whenever fewer than refill_below lanes are busy, the idle lanes take
 // the next rays of the queue (one ballot, one atomic per warp), so a warp does
 // not idle behind its slowest ray. Results are identical to k_extend / k_shadow:
-// each ray runs the same Tracer steps, only the interleaving changes.
+// each ray visits the same entries in the same order, only the interleaving changes.
+//
+// VOTE: a ray's work comes in three kinds (node, leaf, instance entry), and a warp whose lanes
+// are at different kinds runs the code of each in turn, with few lanes (11 of 32 on the diffuse
+// bounces of a room). Here the warp does one kind at a time: up to two nodes per ray while at
+// least half of its rays are at a node, else the leaves and instance entries that wait. The vote
+// costs two ballots and a convergence per turn, which pays where rays are incoherent and wait at
+// leaves: closest-hit rays after the first bounce (a room's: 586 -> 471 us, a batch of rooms
+// with spheres 3.5 -> 2.8 ms per bounce, the 256 icospheres' unchanged). Camera rays and shadow
+// rays run the same code at the same time mostly and lose up to 20 % by it; they keep
+// free-running steps.
 // ---------------------------------------------------------------------------
 // refill_below: a warp fetches rays when fewer lanes than this are busy; steps: traversal
-// steps between fetches (both tunable, kf_config.dyn_refill_below / dyn_steps).
-// Occupancy: 7 resident blocks per SM for closest-hit rays (72 registers, 2 bytes of spill)
-// and 9 for shadow rays (56 registers, no spill) measured fastest on the 256-icosphere frame.
-template <bool SHADOW, bool COUNT, bool BATCH>
-__global__ void __launch_bounds__(128, SHADOW ? 9 : 7)
+// steps (turns) between fetches (both tunable, kf_config.dyn_refill_below / dyn_steps).
+// Occupancy: 8 resident blocks per SM for the vote (64 registers; 9 and 10 spill: +3 and +10 %),
+// 7 for camera rays (72 registers; 8: no change) and 9 for shadow rays (56 registers; 10: no change).
+template <bool SHADOW, bool COUNT, bool BATCH, bool VOTE>
+__global__ void __launch_bounds__(128, SHADOW ? 9 : (VOTE ? 8 : 7))
     k_trace_dyn(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w, int cur, uint32_t depth,
                 uint64_t chunk_start, uint32_t refill_below, int steps) {
-    __shared__ uint32_t s_stack[kSmemStack * kThreadsTrace];
+    __shared__ uint32_t s_stack[kSmemTrace];
     __shared__ uint32_t s_pre[SHADOW ? kMaxSlots + 1 : 1];
     uint32_t* ctr = w.counters + depth * kCounterRow;
     const uint32_t count = SHADOW ? shadow_prefix(w, depth, s_pre) : ctr[0];
@@ -1318,7 +1434,7 @@ __global__ void __launch_bounds__(128, SHADOW ? 9 : 7)
         atomicAdd(&w.stats[SHADOW ? 2 : (depth == 0 ? 0 : 1)], (unsigned long long)count);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t single_root = s.has_tlas ? 0u : kNoRoot;
-    Tracer<SHADOW, COUNT> t;
+    Tracer<SHADOW, COUNT, VOTE> t;
     t.stack.sm = s_stack + threadIdx.x;
     t.cnt = TraceCounters{0, 0, 0};
     AnyHitCtx ah;
@@ -1360,32 +1476,61 @@ __global__ void __launch_bounds__(128, SHADOW ? 9 : 7)
             act = __ballot_sync(kFull, active);
         }
         if (act == 0) break;
-        if (active) {
-            bool done = false;
+        bool done = false;
+        if (VOTE) {
+            bool alive = active && t.e != kNoRoot;
+#pragma unroll 1
+            for (int k = 0; k < steps; ++k) {
+                const uint32_t mn = __ballot_sync(kFull, alive && t.is_node());
+                const bool at_node = mn >> lane & 1;
+                if (2 * __popc(mn) >= __popc(act)) {
+                    if (at_node) {
+                        t.node(s, t.e);
+                        alive = t.pop(s);
+                        if (alive && t.is_node()) {
+                            t.node(s, t.e);
+                            alive = t.pop(s);
+                        }
+                    }
+                } else if (alive && !at_node) {
+                    bool next = true;
+                    if (t.is_inst()) next = !t.inst(s);
+                    if (t.is_leaf()) {
+                        next = true;
+                        if (t.leaf(s, SHADOW ? nullptr : &ah, t.e)) { next = false; alive = false; }
+                    }
+                    if (next) alive = t.pop(s);
+                }
+                __syncwarp();
+                act = __ballot_sync(kFull, alive);
+                if (act == 0 || (!exhausted && (uint32_t)__popc(act) < refill_below)) break;
+            }
+            done = active && !alive;
+        } else if (active) {
 #pragma unroll 1
             for (int k = 0; k < steps && !done; ++k) done = t.step(s, SHADOW ? nullptr : &ah);
-            if (done) {
-                if (SHADOW) {
-                    if (t.h.inst == kMiss) {
-                        const uint32_t tag = __float_as_uint(w.sq_d[idx].w);
-                        w.vis[(size_t)(tag >> 26) * w.chunk_cap + (tag & ((1u << 26) - 1u))] = 1;
-                    }
-                } else {
-                    w.hit[idx] = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.inst));
-                    w.hit_prim[idx] = t.h.prim;
-                    if (depth == 0 && w.primary) {
-                        const uint32_t p = __float_as_uint(w.q_o[cur][idx].w);
-                        kf_hit ph;
-                        ph.t = t.h.t; ph.u = t.h.u; ph.v = t.h.v; ph.prim = t.h.prim;
-                        ph.instance = (BATCH && t.h.inst != kMiss)
-                                          ? t.h.inst - b.items[w.path_item[p]].inst_base // scene-local id
-                                          : t.h.inst;
-                        ph.pad[0] = ph.pad[1] = ph.pad[2] = 0;
-                        w.primary[chunk_start + p] = ph;
-                    }
+        }
+        if (done) {
+            if (SHADOW) {
+                if (t.h.inst == kMiss) {
+                    const uint32_t tag = __float_as_uint(w.sq_d[idx].w);
+                    w.vis[(size_t)(tag >> 26) * w.chunk_cap + (tag & ((1u << 26) - 1u))] = 1;
                 }
-                active = false;
+            } else {
+                w.hit[idx] = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.inst));
+                w.hit_prim[idx] = t.h.prim;
+                if (depth == 0 && w.primary) {
+                    const uint32_t p = __float_as_uint(w.q_o[cur][idx].w);
+                    kf_hit ph;
+                    ph.t = t.h.t; ph.u = t.h.u; ph.v = t.h.v; ph.prim = t.h.prim;
+                    ph.instance = (BATCH && t.h.inst != kMiss)
+                                      ? t.h.inst - b.items[w.path_item[p]].inst_base // scene-local id
+                                      : t.h.inst;
+                    ph.pad[0] = ph.pad[1] = ph.pad[2] = 0;
+                    w.primary[chunk_start + p] = ph;
+                }
             }
+            active = false;
         }
     }
     if (COUNT) {
@@ -1635,21 +1780,25 @@ void launch_shadow(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint3
     KF_CUDA_CHECK(cudaGetLastError());
 }
 
+template <bool SHADOW, bool VOTE, bool BATCH>
+static void trace_dyn_run(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
+                          uint32_t depth, uint64_t chunk_start, uint32_t grid, bool count_mode, uint32_t rb, int ns,
+                          cudaStream_t st) {
+    if (count_mode)
+        k_trace_dyn<SHADOW, true, BATCH, VOTE><<<grid, 128, 0, st>>>(s, f, b, w, cur, depth, chunk_start, rb, ns);
+    else
+        k_trace_dyn<SHADOW, false, BATCH, VOTE><<<grid, 128, 0, st>>>(s, f, b, w, cur, depth, chunk_start, rb, ns);
+}
 template <bool BATCH>
 static void trace_dyn_dispatch(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
                                uint32_t depth, uint64_t chunk_start, bool shadow, uint32_t grid, bool count_mode,
                                uint32_t rb, int ns, cudaStream_t st) {
-    if (shadow) {
-        if (count_mode)
-            k_trace_dyn<true, true, BATCH><<<grid, 128, 0, st>>>(s, f, b, w, cur, depth, chunk_start, rb, ns);
-        else
-            k_trace_dyn<true, false, BATCH><<<grid, 128, 0, st>>>(s, f, b, w, cur, depth, chunk_start, rb, ns);
-    } else {
-        if (count_mode)
-            k_trace_dyn<false, true, BATCH><<<grid, 128, 0, st>>>(s, f, b, w, cur, depth, chunk_start, rb, ns);
-        else
-            k_trace_dyn<false, false, BATCH><<<grid, 128, 0, st>>>(s, f, b, w, cur, depth, chunk_start, rb, ns);
-    }
+    if (shadow)
+        trace_dyn_run<true, false, BATCH>(s, f, b, w, cur, depth, chunk_start, grid, count_mode, rb, ns, st);
+    else if (depth == 0)
+        trace_dyn_run<false, false, BATCH>(s, f, b, w, cur, depth, chunk_start, grid, count_mode, rb, ns, st);
+    else
+        trace_dyn_run<false, true, BATCH>(s, f, b, w, cur, depth, chunk_start, grid, count_mode, rb, ns, st);
 }
 void launch_trace_dyn(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
                       uint32_t depth, uint64_t chunk_start, bool shadow, uint32_t grid, bool count_mode,
@@ -1663,12 +1812,14 @@ void launch_trace_dyn(const SceneDev& s, const FrameDev* f, const BatchDev& b, c
     KF_CUDA_CHECK(cudaGetLastError());
 }
 
-uint32_t trace_dyn_blocks_per_sm(bool shadow) {
+uint32_t trace_dyn_blocks_per_sm(TraceKind kind) {
     int a = 0;
-    if (shadow)
-        KF_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_trace_dyn<true, false, false>, 128, 0));
+    if (kind == TraceKind::shadow)
+        KF_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_trace_dyn<true, false, false, false>, 128, 0));
+    else if (kind == TraceKind::camera)
+        KF_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_trace_dyn<false, false, false, false>, 128, 0));
     else
-        KF_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_trace_dyn<false, false, false>, 128, 0));
+        KF_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_trace_dyn<false, false, false, true>, 128, 0));
     return (uint32_t)std::max(1, a);
 }
 

@@ -151,8 +151,10 @@ void launch_shadow(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint3
 void launch_trace_dyn(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
                       uint32_t depth, uint64_t chunk_start, bool shadow, uint32_t grid, bool count_mode,
                       uint32_t refill_below, uint32_t steps, cudaStream_t st);
-// resident blocks per SM of the persistent traversal kernel (closest-hit or shadow variant)
-uint32_t trace_dyn_blocks_per_sm(bool shadow);
+// resident blocks per SM of the persistent traversal kernel's variants: shadow rays, camera rays
+// (depth 0) and later closest-hit rays
+enum class TraceKind { shadow, camera, bounce };
+uint32_t trace_dyn_blocks_per_sm(TraceKind kind);
 void launch_gather(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t depth, uint64_t chunk_start,
                    uint32_t grid, cudaStream_t st);
 // Per-pixel mean, running mean, FP64 sum and the BGRA frame of one view.

@@ -299,3 +299,65 @@ def test_two_stream_schedule_matches_sequential():
             outs.append((r.downloadAov(cam, N.KF_AOV_RADIANCE_F32), r.downloadLatestFrame(cam)))
     assert np.array_equal(outs[0][0], outs[1][0])
     assert np.array_equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("builder", [0, 1, 2])
+@pytest.mark.parametrize("traversal", [0, 1])
+def test_tiny_geometries_entered_as_leaves(builder, traversal):
+    """Opaque geometries of 1 and 2 triangles (entered without a BLAS node), of 3 (with one), two
+    that share a BLAS, and a non-opaque quad that must stay invisible: hits and paths against the
+    oracle's brute force, alone and as the second scene of a batch (rebased pools)."""
+    corners = np.array([[-1, -1, 0], [1, -1, 0], [1, 1, 0], [-1, 1, 0], [0, 0, 0.8]], np.float32)
+    faces = {1: [0, 1, 2], 2: [0, 1, 2, 0, 2, 3], 3: [0, 1, 4, 1, 2, 4, 2, 3, 4]}
+    up = np.tile(np.array([0, 0, 1], np.float32), (5, 1))
+
+    def geometry(n, color, alpha=1.0):
+        g = api.Geometry.from_arrays(corners, faces[n], normals=up)
+        g.setMaterial(api.NiceMaterial(diffuseColor=color, roughness=0.6, alpha=alpha))
+        g.setFlags(opaque=alpha >= 1.0)
+        return g
+
+    spp, depth, w, h = 4, 4, 41, 29
+    cfg = scenes.cornell_config(spp=spp, depth=depth, debug=True)
+    cfg.setBvhBuilder(builder)
+    cfg.setTraversal(traversal)
+    with api.Kuafu(cfg) as r:
+        first = r.createScene()
+        cam0 = scenes.cornell(r, 24, 24, scene=first)
+        s = r.getScene()
+        rng = scenes.SplitMix64(5)
+        geoms = [geometry(1, (0.8, 0.3, 0.2)), geometry(2, (0.2, 0.8, 0.3)), geometry(2, (0.9, 0.9, 0.1)),
+                 geometry(3, (0.3, 0.3, 0.9)), geometry(2, (1.0, 1.0, 1.0), alpha=0.0)]
+        for g in geoms:
+            s.submitGeometry(g)
+        for k in range(30):
+            m = (scenes.translate(rng.uniform(-3, 3), rng.uniform(-3, 3), rng.uniform(-2, 2)) @
+                 scenes.quat_matrix(rng.uniform(), rng.uniform(), rng.uniform()) @ scenes.scale(1.0, 0.7, 1.3))
+            s.submitGeometryInstance(api.instance(geoms[k % 5], m))
+        s.setClearColor((0.3, 0.4, 0.5, 1.0))
+        s.addPointLight(api.PointLight(position=(-4.0, 1.0, 3.0), radius=0.2, strength=30.0))
+        cam = s.createCamera(w, h)
+        s.setCamera(cam)
+        cam.setPosition((-7.0, 0.0, 0.5))
+        cam.setFront((1.0, 0.0, 0.0))
+        cam.setUp((0.0, 0.0, 1.0))
+        scenes.pinhole(cam, w, h, 50.0)
+        paths, hits, rgba, ref = _render_pair(r, cam, spp, depth, clear=(0.3, 0.4, 0.5, 1.0))
+        rh = ref["hits"]
+        assert np.array_equal(hits["instance"], rh["instance"])
+        hit = rh["instance"] != 0xFFFFFFFF
+        assert 0.1 < hit.mean() < 0.95 and not np.isin(hits["instance"][hit] % 5, [4]).any()
+        for k in ("prim", "t", "u", "v"):
+            assert np.array_equal(hits[k][hit], rh[k][hit]), k
+        assert _check_paths(paths, ref["paths"]) > 0.999
+        # the same frame word as the first run: a new renderer would be needed for an equal image,
+        # so the batch is compared with a single run of its own frame word
+        r.runBatch([(first, cam0, 2), (s, cam, spp)])
+        batch = r.downloadAov(cam, N.KF_AOV_PRIMARY_HITS, spp)
+        flat = s.export()
+        ref = O.render(flat, cam.ubo(), w, h, O.push_constants(spp, depth, clear=(0.3, 0.4, 0.5, 1.0)),
+                       seed=r.config._c.seed, frame=1, camera_index=1)
+        for k in ("instance", "prim", "t"):
+            assert np.array_equal(batch[k][ref["hits"]["instance"] != 0xFFFFFFFF],
+                                  ref["hits"][k][ref["hits"]["instance"] != 0xFFFFFFFF]), k
+        assert _check_paths(r.downloadAov(cam, N.KF_AOV_PATH_RADIANCE, spp), ref["paths"]) > 0.999
