@@ -261,21 +261,28 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
     const size_t clear = ((size_t)max_depth + 2) * (kCounterRow + kSlotRow) * sizeof(uint32_t);
     for (uint64_t start = 0; start < npaths; start += chunk) {
         const uint32_t n = (uint32_t)std::min<uint64_t>(chunk, npaths - start);
+        // no more blocks than a bounce can have work for: a ray per thread in the shading kernels,
+        // kTraceMinBlockRays per block of the persistent traversal
+        const uint32_t rays = n, shadow_rays = (uint32_t)std::min<uint64_t>((uint64_t)n * w.nslot, 1u << 30);
+        const uint32_t grid_shade = std::min(r->grid_shade, (rays + 127) / 128);
+        auto trace_grid = [](uint32_t full, uint32_t count) {
+            return std::max(1u, std::min(full, (count + kTraceMinBlockRays - 1) / kTraceMinBlockRays));
+        };
         KF_CUDA_CHECK(cudaMemsetAsync(w.counters, 0, clear, st));
         launch_raygen(fd, b, w, start, n, st);
         int cur = 0;
         for (uint32_t depth = 0; depth <= max_depth; ++depth) {
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[0], st));
             if (dyn)
-                launch_trace_dyn(sv, fd, b, w, cur, depth, start, false, depth ? r->grid_dyn : r->grid_dyn_camera,
-                                 r->count_traversal, r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
+                launch_trace_dyn(sv, fd, b, w, cur, depth, start, false,
+                                 trace_grid(depth ? r->grid_dyn : r->grid_dyn_camera, rays), r->count_traversal, r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
             else
                 launch_extend(sv, fd, b, w, cur, depth, start, r->grid_extend, r->count_traversal, st);
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[1], st));
             if (fork && depth > 0) KF_CUDA_CHECK(cudaStreamWaitEvent(st, r->ev_join, 0)); // previous gather done
-            launch_miss(sv, fd, b, w, cur, depth, start, r->grid_shade, st);
-            launch_shade(sv, fd, b, w, cur, depth, start, r->grid_shade, st);
-            if (lit) launch_nee(sv, fd, b, w, depth, start, r->grid_shade, st);
+            launch_miss(sv, fd, b, w, cur, depth, start, grid_shade, st);
+            launch_shade(sv, fd, b, w, cur, depth, start, grid_shade, st);
+            if (lit) launch_nee(sv, fd, b, w, depth, start, grid_shade, st);
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[2], st));
             if (lit) {
                 if (fork) {
@@ -283,13 +290,14 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
                     KF_CUDA_CHECK(cudaStreamWaitEvent(st2, r->ev_fork, 0));
                 }
                 if (dyn)
-                    launch_trace_dyn(sv, fd, b, w, cur, depth, start, true, r->grid_dyn_shadow, r->count_traversal,
+                    launch_trace_dyn(sv, fd, b, w, cur, depth, start, true,
+                                     trace_grid(r->grid_dyn_shadow, shadow_rays), r->count_traversal,
                                      r->cfg.dyn_refill_below, r->cfg.dyn_steps, st2);
                 else
                     launch_shadow(sv, b, w, depth, r->grid_extend, r->count_traversal, st2);
             }
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[3], st));
-            if (lit) launch_gather(sv, b, w, depth, start, r->grid_shade, st2);
+            if (lit) launch_gather(sv, b, w, depth, start, grid_shade, st2);
             if (fork) KF_CUDA_CHECK(cudaEventRecord(r->ev_join, st2));
             if (profile) {
                 KF_CUDA_CHECK(cudaEventSynchronize(r->ev[3]));

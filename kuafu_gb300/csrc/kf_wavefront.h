@@ -153,6 +153,8 @@ void launch_trace_dyn(const SceneDev& s, const FrameDev* f, const BatchDev& b, c
                       uint32_t refill_below, uint32_t steps, cudaStream_t st);
 // resident blocks per SM of the persistent traversal kernel's variants: shadow rays, camera rays
 // (depth 0) and later closest-hit rays
+// rays a block of it takes at least (a launch has no more blocks than that gives work)
+constexpr uint32_t kTraceMinBlockRays = 16;
 enum class TraceKind { shadow, camera, bounce };
 uint32_t trace_dyn_blocks_per_sm(TraceKind kind);
 void launch_gather(const SceneDev& s, const BatchDev& b, const WaveDev& w, uint32_t depth, uint64_t chunk_start,
