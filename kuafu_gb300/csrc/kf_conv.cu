@@ -1,19 +1,16 @@
 // kf_conv.cu — tcgen05 tensor-core kernels of the learned denoiser:
 //
-//   * implicit 3x3 convolution (forward and backward-data): NHWC BF16 activations,
-//     per K step one 4D TMA box of 128 output pixels x 32 input channels shifted by
-//     the filter tap (shifts fall on W / H, the 64-byte channel slice stays aligned;
-//     out-of-image taps read TMA's zero fill = zero padding) and one 3D TMA box of
-//     weights, tcgen05.mma kind::f16 (M = 128, N = output channels) accumulating in
-//     TMEM, epilogue tcgen05.ld -> + bias -> ReLU -> BF16 NHWC store (into a channel
-//     slice, so skip concatenation costs nothing);
-//   * K-major GEMM D += A * B^T (weight gradients): 2D TMA, 128-byte swizzle,
-//     split-K with FP32 atomics in the epilogue.
+//   * 3x3 convolutions (forward and backward-data) of NHWC BF16 activations, FP32 accumulation
+//     in TMEM, bias / ReLU / pooling / ReLU-mask epilogues into a channel slice (so skip
+//     concatenation costs nothing): k_conv_halo for wide images, k_conv_tile for narrow ones,
+//     and k_tc for more input channels than k_conv_tile holds (one TMA box of 128 output pixels
+//     x 32 input channels per filter tap);
+//   * weight and bias gradients (k_wgrad);
+//   * K-major GEMM D += A * B^T (k_tc): 2D TMA, 128-byte swizzle, split-K with FP32 atomics.
 //
-// One CTA of 128 threads per output tile: warp 0 lane 0 issues TMA into a 2-, 3- or
-// 4-stage mbarrier ring, warp 1 lane 0 issues the MMAs, all four warps drain TMEM. Every
-// wait is bounded (~1 s of SM clock); on expiry the kernel records an error code,
-// drains its own copies and frees its TMEM.
+// In each, one thread issues TMA into mbarrier-guarded shared memory, another the MMAs, and
+// other warps drain TMEM. Every wait is bounded (~1 s of SM clock); on expiry the kernel records
+// an error code, drains its own copies and frees its TMEM.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -277,6 +274,18 @@ __device__ __forceinline__ void st_bf16x16(__nv_bfloat16* dst, const float (&v0)
                  : "memory");
 }
 
+// A ReLU's backward mask on 8 channels of one pixel: zero where the forward output is not positive.
+__device__ __forceinline__ void mask8(const __nv_bfloat16* m, float (&v)[8]) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(m));
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 t = __bfloat1622float2(h[k]);
+        if (!(t.x > 0.0f)) v[2 * k] = 0.0f;
+        if (!(t.y > 0.0f)) v[2 * k + 1] = 0.0f;
+    }
+}
+
 struct HaloParams {
     int N, H, W, Cin, Cout;
     int n_tile, R, kchunks;
@@ -294,6 +303,9 @@ struct HaloParams {
     int out_cstride, out_coff;
     float* outf;
     __nv_bfloat16* pool_out;   // fused 2x2 average pooling into a dense [N][H/2][W/2][Cout] tensor, or null
+    const __nv_bfloat16* mask; // ReLU backward mask (channel stride mask_cs, slice at mask_co), or null
+    int mask_cs, mask_co;
+    int settled;               // weights and bias may be read before the kernel before this one ends
 };
 
 // Constants of the MMA sequence that depend on n_tile: weight block offsets (in
@@ -365,6 +377,11 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
     const int n0 = blockIdx.y * p.n_tile;
     const int acc_cols = p.R * p.n_tile;
 
+    if (threadIdx.x == 32) {
+        tc::prefetch_map(&tmX);
+        tc::prefetch_map(&tmW);
+    }
+    if (!p.settled) grid_dependency_wait();
     if (warp == 0) tc::tmem_alloc(tmem_slot, p.tmem_cols);
     for (int i = threadIdx.x; i < p.n_tile; i += blockDim.x)
         sbias[i] = (p.bias && n0 + i < p.Cout) ? p.bias[n0 + i] : 0.0f;
@@ -411,6 +428,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
             tc::mbar_arrive_expect_tx(wbar, p.w_bytes);
             load_weights(wst, wbar, 0);
         }
+        if (p.settled) grid_dependency_wait();
         uint32_t it = 0;
         for (int t = blockIdx.x; t < p.num_tiles && ok; t += gridDim.x) {
             int n_img, y0, x0;
@@ -490,6 +508,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
         const bool wide = !p.outf && p.out && ((uintptr_t)p.out & 31) == 0 && (p.out_cstride & 15) == 0;
         const bool pool_wide = p.pool_out && ((uintptr_t)p.pool_out & 31) == 0 && (p.Cout & 15) == 0 &&
                                (n0 & 15) == 0;
+        if (p.settled) grid_dependency_wait();
         uint32_t j = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++j) {
             const uint32_t b = j & 1;
@@ -542,6 +561,10 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
             if (!p.pool_out) {
                 for (int r = 0; r < p.R; ++r) {
                     const uint32_t col0 = (b * (uint32_t)p.R + (uint32_t)r) * (uint32_t)p.n_tile;
+                    const __nv_bfloat16* mk =
+                        p.mask && px < p.W && y0 + r < p.H
+                            ? p.mask + ((size_t)((size_t)n_img * p.H + y0 + r) * p.W + px) * p.mask_cs + p.mask_co + n0
+                            : nullptr;
                     for (int c = cb; c < ce; c += 16) { // two TMEM loads per wait
                         uint32_t r0[8], r1[8];
                         const bool two = c + 16 <= ce;
@@ -553,6 +576,10 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
                         for (int q = 0; q < 8; ++q) {
                             v0[q] = act(r0[q], c + q);
                             v1[q] = two ? act(r1[q], c + 8 + q) : 0.0f;
+                        }
+                        if (mk) {
+                            if (n0 + c + 8 <= p.Cout) mask8(mk + c, v0);
+                            if (two && n0 + c + 16 <= p.Cout) mask8(mk + c + 8, v1);
                         }
                         if (two)
                             emit16(v0, v1, y0 + r, c);
@@ -630,6 +657,264 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
 }
 
 // ---------------------------------------------------------------------------
+// Tile convolution, for images that are narrow for the halo kernel above (training crops, the
+// deep levels of small frames): persistent, with all weights of its output channels resident.
+//
+// A tile is 8 x 16 output pixels x n_tile channels. Per 32 input channels one TMA box brings the
+// tile's halo (10 x 18 pixels) into shared memory as K-major rows of 64 bytes; the 128 rows of
+// the A operand are 16 groups of 8 pixels, one per image row, so their stride is the halo's row
+// (10 pixels) and a tap's view starts (dy * 10 + dx) rows further. The weights of the CTA's n_tile
+// output channels (9 taps x all input channels) are loaded once; the halo of the next tile loads
+// (two buffers where they fit) while this one multiplies, and the epilogue of the tile before
+// drains the other accumulator. Sums run over taps, then channels: the order of the per-tap kernel
+// k_tc, and so its bits.
+//
+// Bound: the tensor core's operand fetch (128 x 16 of A feed n_tile columns), and for a few tiles
+// the latency of one load, one multiplication and one epilogue. k_tc loads 9 shifted boxes per 32
+// channels through a ring of 2 or 3 stages, a round trip to L2 every few steps. 16 images, before
+// and after: 160 -> 160 channels at 8 x 8 26 -> 12 us, 288 -> 128 at 16 x 16 36 -> 19, 96 -> 96 at
+// 32 x 32 17 -> 11, 160 -> 64 at 64 x 64 28 -> 26; a 256 x 256 frame's whole network 391 -> 303 us
+// (with the weights loaded while the kernel before drains).
+//
+// Warp 0 lane 0: TMA, warp 1 lane 0: MMAs, warps 2-5: epilogue, one TMEM lane group (4 tile rows)
+// each. Every wait is bounded as in the kernels above.
+// ---------------------------------------------------------------------------
+constexpr int kTileThreads = 192;
+constexpr int kTileW = 8, kTileH = 16, kTileHaloW = kTileW + 2, kTileHaloH = kTileH + 2;
+constexpr uint32_t kTileHaloBytes = kTileHaloW * kTileHaloH * 64; // 32 channels
+constexpr uint32_t kTileHaloSlot = (kTileHaloBytes + 1023u) & ~1023u;
+
+struct TileParams {
+    int H, W, Cout;
+    int n_tile, bufs;
+    int tiles_x, tiles_y, num_tiles;
+    uint32_t tmem_cols;
+    const float* bias;
+    int relu;
+    __nv_bfloat16* out;
+    int out_cstride, out_coff;
+    float* outf;
+    __nv_bfloat16* pool_out; // fused 2x2 average pooling into a dense [N][H/2][W/2][Cout] tensor, or null
+    const __nv_bfloat16* mask; // ReLU backward mask (channel stride mask_cs, slice at mask_co), or null
+    int mask_cs, mask_co;
+    int settled; // weights and bias may be read before the kernel before this one ends
+};
+
+// The MMAs of a tile over KC chunks of 32 input channels, unrolled at compile time: the one
+// issuing thread then spends a few instructions on each (in a loop over run-time chunks the
+// 160 -> 64 layer of 16 x 64 x 64 pixels took 34.9 us, bound by their issue).
+template <int KC>
+__device__ __forceinline__ void tile_mmas(uint32_t acc, uint64_t ad0, uint64_t bd0, uint32_t tap_units, uint32_t idesc) {
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            const uint64_t ad = ad0 + (uint32_t)(((tap / 3) * kTileHaloW + tap % 3) * 4 + c * (kTileHaloSlot >> 4));
+            const uint64_t bd = bd0 + (uint32_t)(c * 9 + tap) * tap_units;
+            tc::mma_bf16(acc, ad, bd, idesc, (tap > 0 || c > 0) ? 1u : 0u);
+            tc::mma_bf16(acc, ad + 2, bd + 2, idesc, 1u);
+        }
+    }
+}
+
+template <int KC>
+__global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constant__ CUtensorMap tmX,
+                                                               const __grid_constant__ CUtensorMap tmW,
+                                                               const TileParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t tap_bytes = (uint32_t)p.n_tile * 64u;           // one tap, 32 channels
+    const uint32_t buf_bytes = (uint32_t)KC * kTileHaloSlot;
+    uint8_t* wst = smem + (uint32_t)p.bufs * buf_bytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(wst + (uint32_t)KC * 9u * tap_bytes);
+    uint64_t* empty = full + 2;
+    uint64_t* acc_full = empty + 2;
+    uint64_t* acc_empty = acc_full + 2;
+    uint64_t* wbar = acc_empty + 2;
+    uint64_t* mma_done = wbar + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
+    float* sbias = reinterpret_cast<float*>(tmem_slot + 4);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = blockIdx.y * p.n_tile;
+
+    if (threadIdx.x == 32) {
+        tc::prefetch_map(&tmX);
+        tc::prefetch_map(&tmW);
+    }
+    if (!p.settled) grid_dependency_wait();
+    if (warp == 0) tc::tmem_alloc(tmem_slot, p.tmem_cols);
+    for (int i = threadIdx.x; i < p.n_tile; i += blockDim.x)
+        sbias[i] = (p.bias && n0 + i < p.Cout) ? p.bias[n0 + i] : 0.0f;
+    if (threadIdx.x == 32) {
+        for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&full[b], 1);
+            tc::mbar_init(&empty[b], 1);
+            tc::mbar_init(&acc_full[b], 1);
+            tc::mbar_init(&acc_empty[b], 4);
+        }
+        tc::mbar_init(wbar, 1);
+        tc::mbar_init(mma_done, 1);
+        tc::fence_barrier_init();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = *tmem_slot;
+
+    auto tile_origin = [&](int t, int& n_img, int& y0, int& x0) {
+        const int per_img = p.tiles_x * p.tiles_y;
+        n_img = t / per_img;
+        const int r = t % per_img;
+        y0 = (r / p.tiles_x) * kTileH;
+        x0 = (r % p.tiles_x) * kTileW;
+    };
+
+    if (warp == 0 && lane == 0) {
+        // ---- producer: the weights first, while the kernel before this one may still run ----
+        const bool any = (int)blockIdx.x < p.num_tiles;
+        if (any) {
+            tc::mbar_arrive_expect_tx(wbar, (uint32_t)KC * 9u * tap_bytes);
+            for (int c = 0; c < KC; ++c)
+                tc::tma_load_3d(wst + (uint32_t)c * 9u * tap_bytes, &tmW, wbar, c * 32, n0, 0);
+        }
+        if (p.settled) grid_dependency_wait();
+        uint32_t it = 0;
+        for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
+            const uint32_t b = p.bufs == 2 ? (it & 1) : 0, use = p.bufs == 2 ? it >> 1 : it;
+            if (use > 0 && !tc::mbar_wait(&empty[b], (use - 1) & 1, kWaitBudget)) {
+                set_error(31);
+                break;
+            }
+            int n_img, y0, x0;
+            tile_origin(t, n_img, y0, x0);
+            tc::mbar_arrive_expect_tx(&full[b], (uint32_t)KC * kTileHaloBytes);
+            for (int c = 0; c < KC; ++c)
+                tc::tma_load_4d(smem + b * buf_bytes + c * kTileHaloSlot, &tmX, &full[b], c * 32, x0 - 1, y0 - 1, n_img);
+        }
+        // drain: every issued copy must have landed before the CTA may exit
+        for (uint32_t b = 0; b < (uint32_t)p.bufs && b < it; ++b) {
+            const uint32_t uses = p.bufs == 2 ? (it - b + 1) / 2 : it;
+            if (!tc::mbar_wait(&full[b], (uses - 1) & 1, kWaitBudget)) set_error(32);
+        }
+        if (any && !tc::mbar_wait(wbar, 0, kWaitBudget)) set_error(33);
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMA issuer ----
+        const uint32_t idesc = tc::idesc_bf16(128, (uint32_t)p.n_tile);
+        const uint32_t halo0 = tc::smem_u32(smem);
+        const uint64_t bd0 = tc::smem_desc(tc::smem_u32(wst), 512u, 4u);
+        bool ok = (int)blockIdx.x >= p.num_tiles || tc::mbar_wait(wbar, 0, kWaitBudget);
+        if (!ok) set_error(34);
+        uint32_t it = 0;
+        for (int t = blockIdx.x; t < p.num_tiles && ok; t += gridDim.x, ++it) {
+            const uint32_t b = p.bufs == 2 ? (it & 1) : 0, use = p.bufs == 2 ? it >> 1 : it, a = it & 1;
+            if (it >= 2 && !tc::mbar_wait(&acc_empty[a], ((it / 2) - 1) & 1, kWaitBudget)) {
+                set_error(35);
+                break;
+            }
+            if (!tc::mbar_wait(&full[b], use & 1, kWaitBudget)) {
+                set_error(36);
+                break;
+            }
+            tc::fence_after_sync();
+            const uint32_t acc = tmem + a * (uint32_t)p.n_tile;
+            const uint64_t ad0 = tc::smem_desc(halo0 + b * buf_bytes, kTileHaloW * 64u, 4u);
+            tile_mmas<KC>(acc, ad0, bd0, tap_bytes >> 4, idesc);
+            tc::mma_commit(&empty[b]);
+            tc::mma_commit(&acc_full[a]);
+        }
+        // every MMA of this CTA completes before the TMEM is freed
+        tc::mma_commit(mma_done);
+        if (!tc::mbar_wait(mma_done, 0, kWaitBudget)) set_error(37);
+    } else if (warp >= 2) {
+        // ---- epilogue: lane = pixel (4 rows of 8 per warp) ----
+        const int lg = warp & 3, m = lg * 32 + lane;
+        const bool wide = !p.outf && ((uintptr_t)p.out & 31) == 0 && (p.out_cstride & 15) == 0;
+        if (p.settled) grid_dependency_wait();
+        uint32_t it = 0;
+        for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
+            const uint32_t a = it & 1;
+            const bool ready = tc::mbar_wait(&acc_full[a], (it / 2) & 1, kWaitBudget);
+            __syncwarp();
+            if (!ready) {
+                set_error(38);
+                break;
+            }
+            tc::fence_after_sync();
+            int n_img, y0, x0;
+            tile_origin(t, n_img, y0, x0);
+            const int px = x0 + (m & 7), py = y0 + (m >> 3);
+            const bool valid = px < p.W && py < p.H;
+            const size_t base = ((size_t)((size_t)n_img * p.H + py) * p.W + px) * p.out_cstride + p.out_coff;
+            const uint32_t col0 = tmem + ((uint32_t)(lg * 32) << 16) + a * (uint32_t)p.n_tile;
+            for (int c = 0; c < p.n_tile; c += 16) {
+                uint32_t r0[8], r1[8];
+                tc::tmem_ld8(col0 + (uint32_t)c, r0);
+                tc::tmem_ld8(col0 + (uint32_t)(c + 8), r1);
+                tc::tmem_ld_wait();
+                const int co = n0 + c;
+                float v0[8], v1[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    v0[q] = __uint_as_float(r0[q]) + sbias[c + q];
+                    v1[q] = __uint_as_float(r1[q]) + sbias[c + 8 + q];
+                    if (p.relu) {
+                        v0[q] = fmaxf(v0[q], 0.0f);
+                        v1[q] = fmaxf(v1[q], 0.0f);
+                    }
+                }
+                if (p.mask && valid) {
+                    const __nv_bfloat16* mk =
+                        p.mask + ((size_t)((size_t)n_img * p.H + py) * p.W + px) * p.mask_cs + p.mask_co + co;
+                    if (co + 8 <= p.Cout) mask8(mk, v0);
+                    if (co + 16 <= p.Cout) mask8(mk + 8, v1);
+                }
+                if (valid) {
+                    if (p.outf) { // FP32 output (a network head)
+                        for (int q = 0; q < 16 && co + q < p.Cout; ++q) p.outf[base + co + q] = q < 8 ? v0[q & 7] : v1[q & 7];
+                    } else if (wide && co + 16 <= p.Cout && ((p.out_coff + co) & 15) == 0) {
+                        st_bf16x16(p.out + base + co, v0, v1);
+                    } else {
+                        __nv_bfloat16* dst = p.out + base + co;
+                        const bool al = ((p.out_coff + co) & 7) == 0 && (p.out_cstride & 7) == 0;
+                        if (al && co + 8 <= p.Cout) st_bf16x8(dst, v0);
+                        else
+                            for (int q = 0; q < 8 && co + q < p.Cout; ++q) dst[q] = __float2bfloat16_rn(v0[q]);
+                        if (al && co + 16 <= p.Cout) st_bf16x8(dst + 8, v1);
+                        else
+                            for (int q = 0; q < 8 && co + 8 + q < p.Cout; ++q) dst[8 + q] = __float2bfloat16_rn(v1[q]);
+                    }
+                }
+                if (p.pool_out) {
+                    // the 2x2 average of the BF16 outputs, ((a + b) + c) + d in row order as the
+                    // separate pass computes it: the neighbours are lanes 1 and 8 further
+                    float o0[8], o1[8];
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) {
+                        const float av = __bfloat162float(__float2bfloat16_rn(q < 8 ? v0[q & 7] : v1[q & 7]));
+                        const float bv = __shfl_xor_sync(0xFFFFFFFFu, av, 1);
+                        const float cv = __shfl_xor_sync(0xFFFFFFFFu, av, 8);
+                        const float dv = __shfl_xor_sync(0xFFFFFFFFu, av, 9);
+                        (q < 8 ? o0 : o1)[q & 7] = 0.25f * (((av + bv) + cv) + dv);
+                    }
+                    if (valid && !(lane & 9) && co < p.Cout) {
+                        __nv_bfloat16* dst = p.pool_out +
+                                             ((size_t)((size_t)n_img * (p.H / 2) + py / 2) * (p.W / 2) + px / 2) * p.Cout + co;
+                        st_bf16x8(dst, o0);
+                        if (co + 8 < p.Cout) st_bf16x8(dst + 8, o1);
+                    }
+                }
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&acc_empty[a]);
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, p.tmem_cols);
+}
+
+// ---------------------------------------------------------------------------
 // Weight gradients of a 3x3 convolution: dW[dy][dx][co][ci] += sum over pixels p of
 // dZ[p][co] * X[p + (dy - 1, dx - 1)][ci], as one tcgen05 contraction over pixels.
 //
@@ -651,8 +936,9 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
 // pass take 0.34 ms in this form (9 to 38 us each, cold cache); as 9 shifted transposes and 9
 // GEMMs a layer, each reading its operands from HBM again, they took 12.8 ms.
 //
-// One CTA of 128 threads: warp 0 lane 0 issues TMA, warp 1 lane 0 the MMAs, warps 0-2 (one per
-// dx) drain TMEM. Every wait is bounded as in the kernels above.
+// One CTA of 128 threads: warp 0 lane 0 issues TMA, warp 1 lane 0 the MMAs, warps 2 and 3 sum the
+// bias gradient from the dZ tiles in shared memory (a pass over dZ of its own before), warps 0-2
+// (one per dx) drain TMEM. Every wait is bounded as in the kernels above.
 // ---------------------------------------------------------------------------
 constexpr int kWgRows = 8;     // X rows of a tile
 constexpr int kWgMaxCi = 5;    // blocks of 32 input channels per CTA (5 x 96 TMEM columns)
@@ -670,6 +956,7 @@ struct WgradParams {
     uint32_t tmem_cols;
     int Cin, Cout;
     float* dw;
+    float* db;
 };
 
 __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtensorMap tmX,
@@ -680,26 +967,73 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
     uint64_t* empty = full + kWgMaxStages;
     uint64_t* done = empty + kWgMaxStages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+    float* s_db = reinterpret_cast<float*>(tmem_slot + 4); // bias sums of the CTA's channels
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int co0 = blockIdx.y * p.co_block;
+    const bool bias = blockIdx.z == 0; // one CTA of a dZ tile's readers also sums it
     const int ci0 = blockIdx.z * p.n_ci * 32;
     const int n_ci = min(p.n_ci, p.Cin / 32 - (int)blockIdx.z * p.n_ci);
     const uint32_t acc_cols = 3u * (uint32_t)p.co_block;
 
+    if (threadIdx.x == 32) {
+        tc::prefetch_map(&tmX);
+        tc::prefetch_map(&tmZ);
+    }
     if (warp == 0) tc::tmem_alloc(tmem_slot, p.tmem_cols);
     if (threadIdx.x == 32) {
         for (int s = 0; s < p.stages; ++s) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], 1);
+            tc::mbar_init(&empty[s], bias ? 3 : 1); // the MMAs, and the two warps that sum dZ
         }
         tc::mbar_init(done, 1);
         tc::fence_barrier_init();
     }
+    if (threadIdx.x < 64) s_db[threadIdx.x] = 0.0f;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
 
+    grid_dependency_wait();
+    if (warp >= 2 && bias) {
+        // ---- bias sums: thread = 8 channels of every (64 / groups)-th pixel of the tile's own rows
+        const uint32_t groups = (uint32_t)p.co_block / 8, zrow = 2u * (uint32_t)p.co_block;
+        const uint32_t tid = threadIdx.x - 64, g = tid % groups, pl = tid / groups, per = 64 / groups;
+        float sum[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) sum[q] = 0.0f;
+        uint32_t it = 0, s = 0;
+        for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
+            const bool ready = tc::mbar_wait(&full[s], (it / p.stages) & 1, kWaitBudget);
+            __syncwarp();
+            if (!ready) {
+                set_error(25);
+                break;
+            }
+            // rows past the image are zero; the halo rows above and below are other tiles' own
+            const uint8_t* z = smem + s * p.stage_stride;
+            for (uint32_t r = (uint32_t)p.bw + pl; r < (uint32_t)p.bw * (kWgRows + 1); r += per) {
+                const uint32_t piece = p.co_block == 64 ? (g ^ (r & 7)) : (g ^ ((r >> 1) & 3)); // TMA's swizzle
+                const uint4 v = *reinterpret_cast<const uint4*>(z + r * zrow + piece * 16);
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 f = __bfloat1622float2(h[q]);
+                    sum[2 * q] += f.x;
+                    sum[2 * q + 1] += f.y;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&empty[s]);
+            if (++s == (uint32_t)p.stages) s = 0;
+        }
+        // lanes of the same channels first, then one shared add per warp and channel
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            for (uint32_t o = groups; o < 32; o <<= 1) sum[q] += __shfl_xor_sync(0xFFFFFFFFu, sum[q], o);
+            if ((uint32_t)lane < groups) atomicAdd(&s_db[8 * g + q], sum[q]);
+        }
+    }
     if (warp == 0 && lane == 0) {
         uint32_t it = 0, s = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
@@ -782,6 +1116,8 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
     }
     tc::fence_before_sync();
     __syncthreads();
+    if (bias && threadIdx.x < (unsigned)p.co_block && co0 + (int)threadIdx.x < p.Cout)
+        atomicAdd(p.db + co0 + threadIdx.x, s_db[threadIdx.x]);
     if (warp == 0) tc::tmem_dealloc(tmem, p.tmem_cols);
 }
 
@@ -904,8 +1240,7 @@ void launch_halo(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const Ha
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         configured = true;
     }
-    k_conv_halo<CK, R, STACK, STAGES><<<grid, kHaloThreads, smem, st>>>(x, w, p);
-    KF_CUDA_CHECK(cudaGetLastError());
+    launch_overlapped(k_conv_halo<CK, R, STACK, STAGES>, grid, dim3(kHaloThreads), smem, st, x, w, p);
 }
 
 // One instantiation per (rows per tile, stacked rows, stages): R = 8 comes with n_tile <= 32
@@ -972,6 +1307,12 @@ int conv3x3_halo(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __n
     p.outf = y_f32;
     p.out_cstride = y_cstride;
     p.out_coff = y_coff;
+    p.settled = fuse && fuse->settled ? 1 : 0;
+    if (fuse && fuse->mask) {
+        p.mask = fuse->mask;
+        p.mask_cs = fuse->mask_cs;
+        p.mask_co = fuse->mask_co;
+    }
     bool fused = false;
     // pooling pairs rows inside a tile (R even) and reads the right neighbour's lane
     if (fuse && fuse->pool_out && y && !y_f32 && Cout % 8 == 0 && n_tile % 8 == 0 && h.R % 2 == 0 && H % 2 == 0 &&
@@ -986,6 +1327,94 @@ int conv3x3_halo(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __n
         launch_halo_ck<32>(grid, mx, mw, p, h.stages, h.smem, st);
     else
         launch_halo_ck<16>(grid, mx, mw, p, h.stages, h.smem, st);
+    return fused ? 2 : 1;
+}
+
+template <int KC>
+void launch_tile(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const TileParams& p, size_t smem,
+                 cudaStream_t st) {
+    static bool configured = false;
+    if (!configured) {
+        KF_CUDA_CHECK(cudaFuncSetAttribute(k_conv_tile<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        configured = true;
+    }
+    launch_overlapped(k_conv_tile<KC>, grid, dim3(kTileThreads), smem, st, x, w, p);
+}
+
+// The tile kernel, for up to 288 input channels (one instantiation per 32; with more, the weights
+// of 32 output channels and a halo no longer fit). Returns 0 for more (the caller takes k_tc), 1
+// when it ran, 2 when it also did the fused work.
+int conv3x3_tile(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __nv_bfloat16* w, int Cout_rows,
+                 const float* bias, int Cout, bool relu, __nv_bfloat16* y, int y_cstride, int y_coff,
+                 cudaStream_t st, float* y_f32, const ConvFuse* fuse) {
+    if (Cin % 32 || Cin > 288) return 0;
+    TileParams p{};
+    const int kchunks = Cin / 32;
+    p.tiles_x = (W + kTileW - 1) / kTileW;
+    p.tiles_y = (H + kTileH - 1) / kTileH;
+    const int64_t tiles = (int64_t)p.tiles_x * p.tiles_y * N;
+    if (tiles > (1 << 30)) return 0;
+    p.num_tiles = (int)tiles;
+    const int sms = num_sms();
+    const size_t limit = 227 * 1024, halo = (size_t)kchunks * kTileHaloSlot;
+    auto bytes = [&](int n, int bufs) {
+        return 1024 + (size_t)bufs * halo + (size_t)kchunks * 9 * n * 64 + 256 + 4u * (size_t)n;
+    };
+    // Output channels per CTA: as many as fit (fewer reads of the halo, more columns per operand
+    // fetch) while every SM still gets a tile; fewer, down to 16, where there are few tiles.
+    int best = 0;
+    for (int n = 16; n <= std::min(256, Cout_rows); n += 16) {
+        const int slices = (Cout_rows + n - 1) / n;
+        if (n > 16 && slices == (Cout_rows + n - 17) / (n - 16)) continue; // no fewer slices than n - 16
+        if (bytes(n, 1) > limit) break;
+        if (best && tiles * slices < sms) break;
+        best = n;
+    }
+    if (!best) return 0;
+    p.n_tile = best;
+    const int slices = (Cout_rows + best - 1) / best;
+    p.bufs = bytes(best, 2) <= limit && tiles * slices > sms ? 2 : 1;
+    const size_t smem = bytes(best, p.bufs);
+    const int per_sm = std::max<int>(1, std::min<int>((int)(limit / (smem + 1024)), 512 / (int)pow2_at_least(2u * best)));
+    const uint64_t xdims[4] = {(uint64_t)Cin, (uint64_t)W, (uint64_t)H, (uint64_t)N};
+    const uint64_t xstr[3] = {(uint64_t)Cin * 2, (uint64_t)W * Cin * 2, (uint64_t)H * W * Cin * 2};
+    const uint32_t xbox[4] = {32, kTileHaloW, kTileHaloH, 1};
+    const CUtensorMap mx = make_map(x, 4, xdims, xstr, xbox, CU_TENSOR_MAP_SWIZZLE_64B);
+    const uint64_t wdims[3] = {(uint64_t)Cin, (uint64_t)Cout_rows, 9};
+    const uint64_t wstr[2] = {(uint64_t)Cin * 2, (uint64_t)Cout_rows * Cin * 2};
+    const uint32_t wbox[3] = {32, (uint32_t)best, 9};
+    const CUtensorMap mw = make_map(w, 3, wdims, wstr, wbox, CU_TENSOR_MAP_SWIZZLE_64B);
+    p.H = H; p.W = W; p.Cout = Cout;
+    p.tmem_cols = pow2_at_least((uint32_t)(2 * best));
+    p.bias = bias;
+    p.relu = relu ? 1 : 0;
+    p.out = y;
+    p.outf = y_f32;
+    p.out_cstride = y_cstride;
+    p.out_coff = y_coff;
+    p.settled = fuse && fuse->settled ? 1 : 0;
+    if (fuse && fuse->mask) {
+        p.mask = fuse->mask;
+        p.mask_cs = fuse->mask_cs;
+        p.mask_co = fuse->mask_co;
+    }
+    bool fused = false;
+    if (fuse && fuse->pool_out && y && !y_f32 && Cout % 8 == 0 && H % 2 == 0 && W % 2 == 0) {
+        p.pool_out = fuse->pool_out;
+        fused = true;
+    }
+    const dim3 grid((unsigned)std::min<int64_t>(tiles, std::max(1, sms * per_sm / slices)), (unsigned)slices, 1);
+    switch (kchunks) {
+        case 1: launch_tile<1>(grid, mx, mw, p, smem, st); break;
+        case 2: launch_tile<2>(grid, mx, mw, p, smem, st); break;
+        case 3: launch_tile<3>(grid, mx, mw, p, smem, st); break;
+        case 4: launch_tile<4>(grid, mx, mw, p, smem, st); break;
+        case 5: launch_tile<5>(grid, mx, mw, p, smem, st); break;
+        case 6: launch_tile<6>(grid, mx, mw, p, smem, st); break;
+        case 7: launch_tile<7>(grid, mx, mw, p, smem, st); break;
+        case 8: launch_tile<8>(grid, mx, mw, p, smem, st); break;
+        default: launch_tile<9>(grid, mx, mw, p, smem, st); break;
+    }
     return fused ? 2 : 1;
 }
 
@@ -1007,12 +1436,18 @@ bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __
                KF_ERR_INVALID_ARGUMENT, "conv3x3: tensors must be 16-byte aligned (FP32 output: 4-byte)");
     KF_REQUIRE(!fuse || !fuse->pool_out || (((uintptr_t)fuse->pool_out & 15) == 0 && Cout % 8 == 0),
                KF_ERR_INVALID_ARGUMENT, "conv3x3: pooled output must be 16-byte aligned with Cout % 8 == 0");
+    KF_REQUIRE(!fuse || !fuse->mask || (((uintptr_t)fuse->mask & 15) == 0 && Cout % 8 == 0 && fuse->mask_cs % 8 == 0 &&
+                                        fuse->mask_co % 8 == 0 && Cin <= 288 && y && !fuse->pool_out),
+               KF_ERR_INVALID_ARGUMENT, "conv3x3: mask layout");
     const int halo = conv3x3_halo(x, N, H, W, Cin, w, Cout_rows, bias, Cout, relu, y, y_cstride, y_coff, st, y_f32,
                                   fuse);
     if (halo) return halo == 2;
     KF_REQUIRE(Cin % 32 == 0, KF_ERR_INVALID_ARGUMENT,
                "conv3x3: 16 input channels need an image the halo kernel takes (at least 96 wide)");
-    // narrow images: one CTA per tile of bw x bh = 128 pixels, 9 tap-shifted boxes per chunk
+    const int tile = conv3x3_tile(x, N, H, W, Cin, w, Cout_rows, bias, Cout, relu, y, y_cstride, y_coff, st, y_f32, fuse);
+    if (tile) return tile == 2;
+    // more input channels than the tile kernel holds: one CTA per tile of bw x bh = 128 pixels,
+    // 9 tap-shifted boxes per chunk
     int bw = 128;
     while (bw > W && bw > 8) bw >>= 1;
     const int bh = 128 / bw;
@@ -1042,12 +1477,7 @@ bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __
     p.out_coff = y_coff;
     p.tmem_cols = pow2_at_least((uint32_t)n_tile);
     const dim3 grid((unsigned)(p.tiles_x * p.tiles_y * N), (unsigned)((Cout_rows + n_tile - 1) / n_tile), 1);
-    // short K loops (Cin <= 64: 9 or 18 steps) take a 2-stage ring: half the shared memory,
-    // twice the resident CTAs, so one CTA's epilogue overlaps the others' loads and MMAs
-    if (p.k_iters <= 18)
-        launch_tc<0, 64, 2>(grid, ma, mb, p, st);
-    else
-        launch_tc<0, 64, 3>(grid, ma, mb, p, st);
+    launch_tc<0, 64, 3>(grid, ma, mb, p, st);
     return false;
 }
 
@@ -1084,7 +1514,7 @@ void gemm_bf16_tn(const __nv_bfloat16* a, int M, const __nv_bfloat16* b, int N, 
 }
 
 void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int W, int Cin, const __nv_bfloat16* dz,
-                        int dz_channels, int Cout, float* dw, cudaStream_t st) {
+                        int dz_channels, int Cout, float* dw, float* db, cudaStream_t st) {
     KF_REQUIRE(N > 0 && H > 0 && W > 0, KF_ERR_INVALID_ARGUMENT, "wgrad: empty tensor");
     KF_REQUIRE(Cin > 0 && Cin % 32 == 0 && dz_channels % 32 == 0 && Cout > 0 && Cout <= dz_channels,
                KF_ERR_INVALID_ARGUMENT, "wgrad: channels must be multiples of 32");
@@ -1101,6 +1531,7 @@ void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int
     p.Cin = Cin;
     p.Cout = Cout;
     p.dw = dw;
+    p.db = db;
     p.x_bytes = (uint32_t)(kWgRows * (p.bw + 2) * 64);
     p.x_stride = (p.x_bytes + 64 + 1023u) & ~1023u; // the unused fourth shift reads one pixel past the tile
     p.z_bytes = (uint32_t)((kWgRows + 2) * p.bw * 2 * p.co_block);
@@ -1116,7 +1547,7 @@ void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int
     p.stage_stride = p.n_ci * p.x_stride + z_stride;
     p.stages = std::min<int>(kWgMaxStages, (int)(220u * 1024u / p.stage_stride));
     p.tmem_cols = pow2_at_least((uint32_t)(p.n_ci * 3 * p.co_block));
-    const size_t smem = 1024 + (size_t)p.stages * p.stage_stride + 128;
+    const size_t smem = 1024 + (size_t)p.stages * p.stage_stride + 128 + 256;
     const uint64_t xdims[4] = {(uint64_t)Cin, (uint64_t)W, (uint64_t)H, (uint64_t)N};
     const uint64_t xstr[3] = {(uint64_t)x_cstride * 2, (uint64_t)W * x_cstride * 2, (uint64_t)H * W * x_cstride * 2};
     const uint32_t xbox[4] = {32, (uint32_t)p.bw + 2, kWgRows, 1};
@@ -1135,8 +1566,7 @@ void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int
     const int blocks = co_blocks * ((ci_blocks + p.n_ci - 1) / p.n_ci);
     const int splits = std::max(1, std::min(p.num_tiles, sms / std::max(1, blocks)));
     const dim3 grid((unsigned)splits, (unsigned)co_blocks, (unsigned)((ci_blocks + p.n_ci - 1) / p.n_ci));
-    k_wgrad<<<grid, 128, smem, st>>>(mx, mz, p);
-    KF_CUDA_CHECK(cudaGetLastError());
+    launch_overlapped(k_wgrad, grid, dim3(128), smem, st, mx, mz, p);
 }
 
 namespace {

@@ -11,8 +11,16 @@ namespace kf {
 // Work a convolution can take over from the pass that follows it: 2x2 average pooling of
 // its BF16 output into a dense [N][H/2][W/2][Cout] tensor. The values equal those of the
 // separate pass (both read the BF16-rounded outputs).
+// And a ReLU's backward mask: outputs whose place in `mask` (NHWC, channel stride mask_cs, slice
+// starting at mask_co, both multiples of 8) is not positive become zero.
+// settled: the weights and bias were complete before the kernel that precedes this one in the
+// stream started (the previous launch is one of a chain that waited): they may be loaded while
+// that kernel still runs.
 struct ConvFuse {
+    bool settled = false;
     __nv_bfloat16* pool_out = nullptr;
+    const __nv_bfloat16* mask = nullptr;
+    int mask_cs = 0, mask_co = 0;
 };
 
 // y[n, y, x, y_coff + co] = act(bias[co] + sum_{tap, ci} x[n, y+dy, x+dx, ci] * w[tap][co][ci])
@@ -20,8 +28,9 @@ struct ConvFuse {
 // Cout_rows a multiple of 16 (rows >= Cout are computed and dropped); Cin % 32 == 0, or
 // Cin == 16 for images at least 96 wide.
 // With y_f32 set, the output is written there in FP32 (same strides) and y is unused.
-// Returns true when it also did the fused work asked for in `fuse` (the persistent halo
-// kernel does it for suitable shapes; otherwise the caller runs the separate pass).
+// Returns true when it also did the pooling asked for in `fuse` (the persistent kernels do it for
+// suitable shapes; otherwise the caller runs the separate pass). A mask is always applied (at
+// most 288 input channels then).
 bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __nv_bfloat16* w, int Cout_rows,
                   const float* bias, int Cout, bool relu, __nv_bfloat16* y, int y_cstride, int y_coff,
                   cudaStream_t st, float* y_f32 = nullptr, const ConvFuse* fuse = nullptr);
@@ -30,11 +39,11 @@ bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __
 void gemm_bf16_tn(const __nv_bfloat16* a, int M, const __nv_bfloat16* b, int N, int K, float* d, int ldd, int splits,
                   cudaStream_t st);
 
-// dw[tap][co][ci] += sum over pixels of dz[p][co] * x[p shifted by tap][ci] for co < Cout (FP32
-// atomics; x NHWC with channel stride x_cstride, dz dense [N][H][W][dz_channels], Cin and
-// dz_channels multiples of 32).
+// dw[tap][co][ci] += sum over pixels of dz[p][co] * x[p shifted by tap][ci] and db[co] += sum
+// over pixels of dz[p][co], for co < Cout (FP32 atomics; x NHWC with channel stride x_cstride, dz
+// dense [N][H][W][dz_channels], Cin and dz_channels multiples of 32).
 void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int W, int Cin, const __nv_bfloat16* dz,
-                        int dz_channels, int Cout, float* dw, cudaStream_t st);
+                        int dz_channels, int Cout, float* dw, float* db, cudaStream_t st);
 
 // Reads and clears the error word the tensor-core kernels set when a bounded wait expires.
 uint32_t tc_take_error();

@@ -58,6 +58,7 @@ __device__ __forceinline__ void st8(bf16* p, const F8& f) {
 
 // y (dense, H/2 x W/2) = 2x2 average of x[slice] (H x W)
 __global__ void k_pool_fwd(const bf16* __restrict__ x, int xs, int xo, int C, int N, int H, int W, bf16* y) {
+    grid_dependency_wait();
     const int Ho = H / 2, Wo = W / 2, G = C / 8;
     const size_t total = (size_t)N * Ho * Wo * G;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -74,9 +75,18 @@ __global__ void k_pool_fwd(const bf16* __restrict__ x, int xs, int xo, int C, in
     }
 }
 
-// gx (dense, H x W) = broadcast(gy / 4) + gskip[slice] (optional)
+// ReLU's backward mask on the BF16-rounded gradient: zero where the forward output y is not positive
+__device__ __forceinline__ void mask8(F8& v, const bf16* y) {
+    const F8 m = ld8(y);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (!(m.v[k] > 0.0f)) v.v[k] = 0.0f;
+}
+
+// gx (dense, H x W) = broadcast(gy / 4) + gskip[slice], masked by the forward output y[slice]
 __global__ void k_pool_bwd_add(const bf16* __restrict__ gy, const bf16* __restrict__ gskip, int ss, int so, int C,
-                               int N, int H, int W, bf16* gx) {
+                               int N, int H, int W, const bf16* __restrict__ y, int ys, int yo, bf16* gx) {
+    grid_dependency_wait();
     const int G = C / 8;
     const size_t total = (size_t)N * H * W * G;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -86,19 +96,17 @@ __global__ void k_pool_bwd_add(const bf16* __restrict__ gy, const bf16* __restri
         const size_t ny = pix / W; // n * H + y
         const size_t low = (ny / 2) * (W / 2) + xw / 2;
         F8 v = ld8(gy + low * C + 8 * g);
+        const F8 sk = ld8(gskip + pix * ss + so + 8 * g);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v.v[k] *= 0.25f;
-        if (gskip) {
-            const F8 sk = ld8(gskip + pix * ss + so + 8 * g);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v.v[k] += sk.v[k];
-        }
+        for (int k = 0; k < 8; ++k) v.v[k] = v.v[k] * 0.25f + sk.v[k];
+        mask8(v, y + pix * ys + yo + 8 * g);
         st8(gx + pix * C + 8 * g, v);
     }
 }
 
 // nearest 2x upsampling of x (dense, H/2 x W/2) into y[slice] (H x W)
 __global__ void k_up_fwd(const bf16* __restrict__ x, int C, int N, int H, int W, bf16* y, int ys, int yo) {
+    grid_dependency_wait();
     const int Ho = H / 2, Wo = W / 2, G = C / 8;
     const size_t total = (size_t)N * Ho * Wo * G;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -115,8 +123,11 @@ __global__ void k_up_fwd(const bf16* __restrict__ x, int C, int N, int H, int W,
     }
 }
 
-// gx (dense, H/2 x W/2) = sum of the 2x2 block of gy[slice] (H x W)
-__global__ void k_up_bwd(const bf16* __restrict__ gy, int gs, int go, int C, int N, int H, int W, bf16* gx) {
+// gx (dense, H/2 x W/2) = sum of the 2x2 block of gy[slice] (H x W), masked by the forward
+// output y (dense, H/2 x W/2)
+__global__ void k_up_bwd(const bf16* __restrict__ gy, int gs, int go, int C, int N, int H, int W,
+                         const bf16* __restrict__ y, bf16* gx) {
+    grid_dependency_wait();
     const int Ho = H / 2, Wo = W / 2, G = C / 8;
     const size_t total = (size_t)N * Ho * Wo * G;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -129,85 +140,66 @@ __global__ void k_up_bwd(const bf16* __restrict__ gy, int gs, int go, int C, int
         const F8 c = ld8(gy + (row0 + W) * gs + go + 8 * g), d = ld8(gy + (row0 + W + 1) * gs + go + 8 * g);
 #pragma unroll
         for (int k = 0; k < 8; ++k) a.v[k] = ((a.v[k] + b.v[k]) + c.v[k]) + d.v[k];
+        mask8(a, y + pix * C + 8 * g);
         st8(gx + pix * C + 8 * g, a);
     }
 }
 
-// dz[p][c] = (c < C) ? gy[p][c] * (relu ? y[p][c] > 0 : 1) : 0   for c < Ck (dense, Ck channels),
-// and db[c] += sum_p dz[p][c] of the rounded values. Bound by HBM: one read of gy and y, one
-// write of dz; the bias sums ride along in registers (a thread keeps its 8 channels for all its
-// pixels), where a pass of their own read dz again with one 2-byte load per value: 19 layers of
-// a 16 x 128 x 128 batch take 0.27 ms, in two passes they took 0.38 ms. All strides and offsets are multiples
-// of 8 (16-byte accesses).
-constexpr int kMaskThreads = 256, kMaskMaxC = 160;
-__global__ void __launch_bounds__(kMaskThreads) k_relu_mask_bias(const bf16* __restrict__ gy, int gs, int go,
-                                                                 const bf16* __restrict__ y, int ys, int yo, int C,
-                                                                 int Ck, size_t P, int relu, bf16* __restrict__ dz,
-                                                                 float* db) {
-    __shared__ float s_db[kMaskMaxC];
-    const int G = Ck / 8, per = kMaskThreads / G; // pixels per block and step
-    const int g = threadIdx.x % G, pl = threadIdx.x / G;
-    for (int c = threadIdx.x; c < Ck; c += kMaskThreads) s_db[c] = 0.0f;
-    __syncthreads();
-    float sum[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) sum[k] = 0.0f;
-    if (pl < per) {
-        for (size_t p = (size_t)blockIdx.x * per + pl; p < P; p += (size_t)gridDim.x * per) {
-            F8 v = ld8(gy + p * gs + go + 8 * g);
-            if (relu) {
-                const F8 m = ld8(y + p * ys + yo + 8 * g);
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (!(m.v[k] > 0.0f)) v.v[k] = 0.0f;
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (8 * g + k >= C) v.v[k] = 0.0f;
-                sum[k] += v.v[k];
-            }
-            st8(dz + p * Ck + 8 * g, v);
+// Where each layer's parameters and packed weights lie, for k_update (a kernel parameter).
+struct UpdateTable {
+    int first[20]; // first block of each layer: a block per tap and 32 x 32 weights
+    int cin[19], cout[19], rows[19], cout_k[19];
+    uint32_t w_off[19], b_off[19], wf_off[19], wb_off[19];
+};
+
+// One pass over all parameters: Adam on the FP32 master weights (Kingma & Ba 2015; skipped when
+// !step) and the BF16 weights the convolutions read: forward wf[tap][co][ci], backward-data
+// wb[8 - tap][ci][co], and the first layer's input channels 0..15 alone (wf16: the inference path
+// feeds it 16-channel features). Rows and columns of the padding stay zero from their allocation.
+// A block holds 32 x 32 weights of one tap, transposed through shared memory so that both layouts
+// are written in whole lines. Bound by HBM (36 bytes a parameter): 21 us for the 1.8 M
+// parameters (cold cache); Adam and 20 packing launches took 92 us.
+constexpr int kUpdateThreads = 256;
+__global__ void __launch_bounds__(kUpdateThreads) k_update(UpdateTable tab, float* __restrict__ w,
+                                                           const float* __restrict__ grad, float* __restrict__ m,
+                                                           float* __restrict__ v, bf16* __restrict__ wf,
+                                                           bf16* __restrict__ wb, bf16* __restrict__ wf16, int step,
+                                                           float lr, float b1, float b2, float eps, float bc1,
+                                                           float bc2) {
+    __shared__ bf16 tile[32][34];
+    int l = 0;
+    while ((int)blockIdx.x >= tab.first[l + 1]) ++l;
+    const int cin = tab.cin[l], cout = tab.cout[l], rows = tab.rows[l], cout_k = tab.cout_k[l];
+    const int nci = cin / 32, k = (int)blockIdx.x - tab.first[l];
+    const int ci0 = (k % nci) * 32, co0 = (k / nci) % (cout_k / 32) * 32, tap = k / (nci * (cout_k / 32));
+    auto adam = [&](size_t i) {
+        float x = w[i];
+        if (step) {
+            const float gi = grad[i];
+            const float mi = b1 * m[i] + (1.0f - b1) * gi;
+            const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+            m[i] = mi;
+            v[i] = vi;
+            x -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+            w[i] = x;
         }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) atomicAdd(&s_db[8 * g + k], sum[k]);
+        return x;
+    };
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < 32; r += kUpdateThreads / 32) {
+        const int co = co0 + r, ci = ci0 + lane;
+        bf16 q = __float2bfloat16_rn(0.0f);
+        if (co < cout) {
+            q = __float2bfloat16_rn(adam(tab.w_off[l] + ((size_t)tap * cout + co) * cin + ci));
+            wf[tab.wf_off[l] + ((size_t)tap * rows + co) * cin + ci] = q;
+            if (l == 0 && ci < 16) wf16[((size_t)tap * rows + co) * 16 + ci] = q;
+        }
+        tile[r][lane] = q;
     }
+    if (tap == 0 && ci0 == 0 && threadIdx.x < 32 && co0 + lane < cout && step) adam(tab.b_off[l] + co0 + lane);
     __syncthreads();
-    for (int c = threadIdx.x; c < C; c += kMaskThreads) atomicAdd(db + c, s_db[c]);
-}
-
-// Adam on FP32 master weights (Kingma & Ba 2015).
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       size_t n, float lr, float b1, float b2, float eps, float bc1, float bc2) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    }
-}
-
-// BF16 forward weights wf[tap][co][ci] (rows >= cout zero) and backward-data weights
-// wb[8 - tap][ci][co] (co >= cout zero) from FP32 master W[tap][co][ci].
-__global__ void k_pack_layer(const float* __restrict__ W, int cin, int cout, int rows, int cout_k, bf16* wf, bf16* wb) {
-    const size_t total = (size_t)9 * rows * cin;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int ci = (int)(i % cin);
-        const size_t r = i / cin;
-        const int co = (int)(r % rows);
-        const int tap = (int)(r / rows);
-        const float v = co < cout ? W[((size_t)tap * cout + co) * cin + ci] : 0.0f;
-        wf[i] = __float2bfloat16_rn(v);
-        if (co < cout_k) wb[((size_t)(8 - tap) * cin + ci) * cout_k + co] = __float2bfloat16_rn(v);
-    }
-}
-
-// out[r][c] = in[r][c] for c < cout of rows of cin channels (BF16).
-__global__ void k_slice_cin(const bf16* __restrict__ in, int rows, int cin, int cout, bf16* out) {
-    const size_t total = (size_t)rows * cout;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = in[(i / cout) * cin + i % cout];
+    for (int r = threadIdx.x >> 5; r < 32; r += kUpdateThreads / 32)
+        wb[tab.wb_off[l] + ((size_t)(8 - tap) * cin + ci0 + r) * cout_k + co0 + lane] = tile[lane][r];
 }
 
 // The network works on g(x) = tone(x) of linear radiance (kf_tone.cuh).
@@ -281,53 +273,82 @@ __global__ void k_unpack_residual(const float4* __restrict__ pred, const float4*
 
 
 // L = mean|p - t| + lambda * mean(|dx p - dx t| + |dy p - dy t|) in g space, p the FP32
-// prediction [P][4], t = g(target); writes dL/dp as the BF16 [P][32] gradient of the head.
-__global__ void k_loss(const float* __restrict__ pred, const float4* __restrict__ target, int N, int H, int W,
-                       float lambda, float* loss, bf16* gpred) {
+// prediction [P][4] (+ base, the residual, where given), t = g(target); writes dL/dp as the BF16
+// [P][32] gradient of the head. A block takes 32 x 8 pixels and brings predictions and g(target)
+// with a border of one pixel to shared memory once, so that g is evaluated 1.3 times a pixel
+// (with every neighbour read and mapped in place 5 times, and the 64-byte gradient written in
+// 2-byte pieces, 16 x 128 x 128 pixels took 63 us; this form 11).
+constexpr int kLossW = 32, kLossH = 8;
+__global__ void __launch_bounds__(kLossW * kLossH) k_loss(const float4* __restrict__ pred,
+                                                          const float4* __restrict__ base,
+                                                          const float4* __restrict__ target, int N, int H, int W,
+                                                          float lambda, float* loss, bf16* gpred) {
+    __shared__ float sp[3][kLossH + 2][kLossW + 2], st[3][kLossH + 2][kLossW + 2];
+    __shared__ float s_acc[kLossW * kLossH / 32];
+    const int tx = (W + kLossW - 1) / kLossW, ty = (H + kLossH - 1) / kLossH;
+    const int n = blockIdx.x / (tx * ty), r = blockIdx.x % (tx * ty);
+    const int x0 = r % tx * kLossW, y0 = r / tx * kLossH;
+    for (int i = threadIdx.x; i < (kLossH + 2) * (kLossW + 2); i += kLossW * kLossH) {
+        const int lx = i % (kLossW + 2), ly = i / (kLossW + 2), x = x0 + lx - 1, y = y0 + ly - 1;
+        if (x < 0 || x >= W || y < 0 || y >= H) continue;
+        const size_t j = ((size_t)n * H + y) * W + x;
+        float4 p = pred[j];
+        const float4 t = target[j];
+        if (base) {
+            const float4 b = base[j];
+            p.x += b.x;
+            p.y += b.y;
+            p.z += b.z;
+        }
+        sp[0][ly][lx] = p.x; sp[1][ly][lx] = p.y; sp[2][ly][lx] = p.z;
+        st[0][ly][lx] = tone(t.x); st[1][ly][lx] = tone(t.y); st[2][ly][lx] = tone(t.z);
+    }
+    __syncthreads();
     const size_t total = (size_t)N * H * W;
     const float inv = 1.0f / (float)(total * 3);
+    const int lx = (int)threadIdx.x % kLossW + 1, ly = (int)threadIdx.x / kLossW + 1;
+    const int x = x0 + lx - 1, y = y0 + ly - 1;
     float acc = 0.0f;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % W);
-        const int y = (int)((i / W) % H);
-        const float4 t4 = target[i];
-        const float tv[3] = {tone(t4.x), tone(t4.y), tone(t4.z)};
-        bf16* g = gpred + i * 32;
+    if (x < W && y < H) {
+        F8 g;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) g.v[c] = 0.0f;
+        auto sign = [](float e) { return e > 0.0f ? 1.0f : (e < 0.0f ? -1.0f : 0.0f); };
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
-            auto P = [&](size_t j) { return pred[j * 4 + c]; };
-            auto T = [&](size_t j) {
-                const float4 q = target[j];
-                return tone(c == 0 ? q.x : (c == 1 ? q.y : q.z));
-            };
-            const float p = P(i);
-            float d = p - tv[c];
+            const float p = sp[c][ly][lx], tv = st[c][ly][lx];
+            const float d = p - tv;
             acc += fabsf(d);
-            float gr = (d > 0.0f ? 1.0f : (d < 0.0f ? -1.0f : 0.0f));
-            // forward differences touching pixel i: (i, i+1) and (i-1, i) in x, same in y
+            float gr = sign(d);
+            // forward differences touching the pixel: (i, i+1) and (i-1, i) in x, same in y
             if (x + 1 < W) {
-                const float e = (P(i + 1) - p) - (T(i + 1) - tv[c]);
+                const float e = (sp[c][ly][lx + 1] - p) - (st[c][ly][lx + 1] - tv);
                 acc += lambda * fabsf(e);
-                gr -= lambda * (e > 0.0f ? 1.0f : (e < 0.0f ? -1.0f : 0.0f));
+                gr -= lambda * sign(e);
             }
-            if (x > 0) {
-                const float e = (p - P(i - 1)) - (tv[c] - T(i - 1));
-                gr += lambda * (e > 0.0f ? 1.0f : (e < 0.0f ? -1.0f : 0.0f));
-            }
+            if (x > 0) gr += lambda * sign((p - sp[c][ly][lx - 1]) - (tv - st[c][ly][lx - 1]));
             if (y + 1 < H) {
-                const float e = (P(i + W) - p) - (T(i + W) - tv[c]);
+                const float e = (sp[c][ly + 1][lx] - p) - (st[c][ly + 1][lx] - tv);
                 acc += lambda * fabsf(e);
-                gr -= lambda * (e > 0.0f ? 1.0f : (e < 0.0f ? -1.0f : 0.0f));
+                gr -= lambda * sign(e);
             }
-            if (y > 0) {
-                const float e = (p - P(i - W)) - (tv[c] - T(i - W));
-                gr += lambda * (e > 0.0f ? 1.0f : (e < 0.0f ? -1.0f : 0.0f));
-            }
-            g[c] = __float2bfloat16_rn(gr * inv);
+            if (y > 0) gr += lambda * sign((p - sp[c][ly - 1][lx]) - (tv - st[c][ly - 1][lx]));
+            g.v[c] = gr * inv;
         }
-        for (int c = 3; c < 32; ++c) g[c] = __float2bfloat16_rn(0.0f);
+        bf16* o = gpred + (((size_t)n * H + y) * W + x) * 32;
+        st8(o, g);
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int q = 1; q < 4; ++q) reinterpret_cast<uint4*>(o)[q] = zero;
     }
     for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc * inv);
+    if ((threadIdx.x & 31) == 0) s_acc[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float a = 0.0f;
+        for (int k = 0; k < kLossW * kLossH / 32; ++k) a += s_acc[k];
+        atomicAdd(loss, a * inv);
+    }
 }
 
 // A training target from the FP64 accumulation: sum of the frames' pixel means / frames.
@@ -394,7 +415,7 @@ enum {
     T_D2A, T_D2B, T_D1A, T_D1B, T_D0A, T_D0B, T_OUT,
     // gradients
     G_OUT, G_D0B, G_D0A, G_CAT0, G_D1B, G_D1A, G_CAT1, G_D2B, G_D2A, G_CAT2, G_D3B, G_D3A, G_CAT3, G_E4B, G_E4A, G_P3,
-    G_E3B, G_E3A, G_P2, G_E2B, G_E2A, G_P1, G_E1B, G_E1A, G_P0, G_E0B, G_E0A, G_DZ,
+    G_E3B, G_E3A, G_P2, G_E2B, G_E2A, G_P1, G_E1B, G_E1A, G_P0, G_E0B, G_E0A,
     T_COUNT
 };
 
@@ -476,27 +497,42 @@ void init_params(kf_denoiser_impl& d, uint32_t seed, cudaStream_t st) {
     KF_CUDA_CHECK(cudaMemsetAsync(d.v.ptr, 0, d.v.bytes(), st));
     d.wf.resize(d.nwf, st);
     d.wb.resize(d.nwb, st);
+    d.wf0_16.resize((size_t)9 * d.L[0].rows * 16, st);
+    KF_CUDA_CHECK(cudaMemsetAsync(d.wf.ptr, 0, d.wf.bytes(), st));
+    KF_CUDA_CHECK(cudaMemsetAsync(d.wf0_16.ptr, 0, d.wf0_16.bytes(), st));
     KF_CUDA_CHECK(cudaMemsetAsync(d.wb.ptr, 0, d.wb.bytes(), st));
     d.loss.resize(4, st);
     d.packed = false;
     d.step = 0;
 }
 
-void pack(kf_denoiser_impl& d, cudaStream_t st) {
-    for (const Layer& l : d.L) {
-        const size_t n = (size_t)9 * l.rows * l.cin;
-        k_pack_layer<<<grid_for(n), 256, 0, st>>>(d.params.ptr + l.w_off, l.cin, l.cout, l.rows, l.cout_k,
-                                                  d.wf.ptr + l.wf_off, d.wb.ptr + l.wb_off);
+// The BF16 weights from the master weights, after an Adam step on them when `step` is its number
+// (0: no step).
+void update(kf_denoiser_impl& d, int step, float lr, cudaStream_t st) {
+    UpdateTable t{};
+    int blocks = 0;
+    for (size_t k = 0; k < d.L.size(); ++k) {
+        const Layer& l = d.L[k];
+        t.first[k] = blocks;
+        blocks += 9 * (l.cin / 32) * (l.cout_k / 32);
+        t.cin[k] = l.cin;
+        t.cout[k] = l.cout;
+        t.rows[k] = l.rows;
+        t.cout_k[k] = l.cout_k;
+        t.w_off[k] = (uint32_t)l.w_off;
+        t.b_off[k] = (uint32_t)l.b_off;
+        t.wf_off[k] = (uint32_t)l.wf_off;
+        t.wb_off[k] = (uint32_t)l.wb_off;
     }
-    // the first convolution's weights of input channels 0..15 alone: the inference path
-    // feeds it 16-channel features (channels 11..31 of the input are always zero)
-    const Layer& l0 = d.L[0];
-    d.wf0_16.resize((size_t)9 * l0.rows * 16, st);
-    k_slice_cin<<<grid_for((size_t)9 * l0.rows * 16), 256, 0, st>>>(d.wf.ptr + l0.wf_off, 9 * l0.rows, l0.cin, 16,
-                                                                   d.wf0_16.ptr);
+    t.first[d.L.size()] = blocks;
+    const float b1 = 0.9f, b2 = 0.999f;
+    const float bc1 = 1.0f - std::pow(b1, (float)step), bc2 = 1.0f - std::pow(b2, (float)step);
+    k_update<<<blocks, kUpdateThreads, 0, st>>>(t, d.params.ptr, d.grads.ptr, d.m.ptr, d.v.ptr, d.wf.ptr, d.wb.ptr,
+                                                d.wf0_16.ptr, step, lr, b1, b2, 1e-8f, bc1, bc2);
     KF_CUDA_CHECK(cudaGetLastError());
     d.packed = true;
 }
+void pack(kf_denoiser_impl& d, cudaStream_t st) { update(d, 0, 0.0f, st); }
 
 // channel counts and spatial level of every tensor
 struct TDesc {
@@ -508,8 +544,7 @@ const TDesc kT[T_COUNT] = {
     // gradients
     {32, 0}, {32, 0}, {32, 0}, {96, 0}, {64, 1}, {64, 1}, {160, 1}, {96, 2}, {96, 2}, {224, 2}, {128, 3}, {128, 3},
     {288, 3}, {160, 4}, {160, 4}, {128, 4}, {128, 3}, {128, 3}, {96, 3}, {96, 2}, {96, 2}, {64, 2}, {64, 1}, {64, 1},
-    {32, 1}, {32, 0}, {32, 0},
-    {0, 0}};
+    {32, 1}, {32, 0}, {32, 0}};
 
 void ensure_acts(kf_denoiser_impl& d, int n, int h, int w, cudaStream_t st) {
     Acts& a = d.acts;
@@ -518,17 +553,11 @@ void ensure_acts(kf_denoiser_impl& d, int n, int h, int w, cudaStream_t st) {
     a.off.assign(T_COUNT, 0);
     size_t total = 0;
     const size_t P0 = (size_t)n * h * w;
-    for (int k = 0; k < G_DZ; ++k) {
+    for (int k = 0; k < T_COUNT; ++k) {
         a.off[k] = total;
         total += (P0 >> (2 * kT[k].level)) * kT[k].c;
         total = (total + 127) / 128 * 128;
     }
-    // scratch: masked gradient of one layer
-    size_t dz_max = 0;
-    const int level[19] = {0, 0, 1, 1, 2, 2, 3, 3, 4, 4, 3, 3, 2, 2, 1, 1, 0, 0, 0};
-    for (int i = 0; i < 19; ++i) dz_max = std::max(dz_max, (P0 >> (2 * level[i])) * (size_t)pad32(kLayers[i][1]));
-    a.off[G_DZ] = total;
-    total += (dz_max + 127) / 128 * 128;
     a.buf.resize(total, st);
     KF_CUDA_CHECK(cudaMemsetAsync(a.buf.ptr, 0, a.buf.bytes(), st));
     a.head.resize(P0 * 4, st);
@@ -549,28 +578,30 @@ struct Ctx {
 
 // The convolution, and (when `fuse` is given) the pooling / upsampling pass after it: the
 // persistent conv kernel does that work in its epilogue where it can, else the pass runs here.
-bool conv_fwd(Ctx& c, int li, int level, TRef x, TRef y, const ConvFuse* fuse = nullptr) {
+bool conv_fwd(Ctx& c, int li, int level, TRef x, TRef y, ConvFuse f = ConvFuse()) {
     const Layer& l = c.d.L[li];
+    f.settled = li > 0; // behind the first convolution, whatever wrote the weights is complete
     return conv3x3_bf16(x.p, c.n, c.H(level), c.W(level), x.cs, c.d.wf.ptr + l.wf_off, l.rows,
-                        c.d.params.ptr + l.b_off, l.cout, l.relu, y.p, y.cs, y.co, c.st, nullptr, fuse);
+                        c.d.params.ptr + l.b_off, l.cout, l.relu, y.p, y.cs, y.co, c.st, nullptr, &f);
 }
 
-// Backward of y = act(conv(x) + b): accumulates dW, db; writes gx (if gx.p) = dL/dx.
-void conv_bwd(Ctx& c, int li, int level, TRef x, TRef y, TRef gy, TRef gx) {
+// Backward of z = conv(x) + b from dz = dL/dz (dense, the layer's channels padded to 32): adds dW
+// and db; with gx.p, gx = dL/dx, masked by x > 0 where x is a ReLU's output that nothing else
+// reads (mask: gx is then the dL/dz of the layer before).
+void conv_bwd(Ctx& c, int li, int level, TRef x, TRef dz, TRef gx, bool mask) {
     const Layer& l = c.d.L[li];
-    Acts& a = c.d.acts;
-    const size_t P = c.P(level);
-    bf16* dz = a.at(G_DZ);
-    // a few pixels per thread at least, two resident waves of blocks at most
-    const size_t per = (size_t)(kMaskThreads / (l.cout_k / 8));
-    const unsigned blocks = (unsigned)std::max<size_t>(1, std::min<size_t>((P + 4 * per - 1) / (4 * per), 152 * 16));
-    k_relu_mask_bias<<<blocks, kMaskThreads, 0, c.st>>>(gy.p, gy.cs, gy.co, y.p, y.cs, y.co, l.cout, l.cout_k, P,
-                                                        l.relu ? 1 : 0, dz, c.d.grads.ptr + l.b_off);
-    conv3x3_wgrad_bf16(x.p + x.co, x.cs, c.n, c.H(level), c.W(level), l.cin, dz, l.cout_k, l.cout,
-                       c.d.grads.ptr + l.w_off, c.st);
+    conv3x3_wgrad_bf16(x.p + x.co, x.cs, c.n, c.H(level), c.W(level), l.cin, dz.p, l.cout_k, l.cout,
+                       c.d.grads.ptr + l.w_off, c.d.grads.ptr + l.b_off, c.st);
     if (gx.p) {
-        conv3x3_bf16(dz, c.n, c.H(level), c.W(level), l.cout_k, c.d.wb.ptr + l.wb_off, l.cin, nullptr, l.cin, false,
-                     gx.p, gx.cs, gx.co, c.st);
+        ConvFuse f;
+        f.settled = true; // the weight-gradient kernel runs between
+        if (mask) {
+            f.mask = x.p;
+            f.mask_cs = x.cs;
+            f.mask_co = x.co;
+        }
+        conv3x3_bf16(dz.p, c.n, c.H(level), c.W(level), l.cout_k, c.d.wb.ptr + l.wb_off, l.cin, nullptr, l.cin, false,
+                     gx.p, gx.cs, gx.co, c.st, nullptr, &f);
     }
     KF_CUDA_CHECK(cudaGetLastError());
 }
@@ -580,17 +611,17 @@ TRef S(Acts& a, int k, int off, int cnt) { return TRef{a.at(k), kT[k].c, off, cn
 
 void pool_fwd(Ctx& c, TRef x, int level, TRef y) {
     const size_t n = c.P(level + 1) * x.c / 8;
-    k_pool_fwd<<<grid_for(n), 256, 0, c.st>>>(x.p, x.cs, x.co, x.c, c.n, c.H(level), c.W(level), y.p);
+    launch_overlapped(k_pool_fwd, dim3(grid_for(n)), dim3(256), 0, c.st, x.p, x.cs, x.co, x.c, c.n, c.H(level), c.W(level), y.p);
 }
 void up_fwd(Ctx& c, TRef x, int level_hi, TRef y) {
     const size_t n = c.P(level_hi + 1) * x.c / 8;
-    k_up_fwd<<<grid_for(n), 256, 0, c.st>>>(x.p, x.c, c.n, c.H(level_hi), c.W(level_hi), y.p, y.cs, y.co);
+    launch_overlapped(k_up_fwd, dim3(grid_for(n)), dim3(256), 0, c.st, x.p, x.c, c.n, c.H(level_hi), c.W(level_hi), y.p, y.cs, y.co);
 }
 // conv into y, then 2x2 pooling of y into `pooled` (at level + 1)
 void conv_pool(Ctx& c, int li, int level, TRef x, TRef y, TRef pooled) {
     ConvFuse f;
     f.pool_out = pooled.p;
-    if (!conv_fwd(c, li, level, x, y, &f)) pool_fwd(c, y, level, pooled);
+    if (!conv_fwd(c, li, level, x, y, f)) pool_fwd(c, y, level, pooled);
 }
 // conv into y, then nearest 2x upsampling of y into the channel slice `up` (at level - 1).
 // A separate pass: both forms are bound by the same HBM writes of the four copies, and
@@ -631,55 +662,60 @@ void forward(Ctx& c, const float4* base, bool in16 = false) {
     conv_fwd(c, 17, 0, T(a, T_D0A), T(a, T_D0B));
     {
         const Layer& l = c.d.L[18];
+        ConvFuse f;
+        f.settled = true;
         conv3x3_bf16(a.at(T_D0B), c.n, c.h, c.w, 32, c.d.wf.ptr + l.wf_off, l.rows, c.d.params.ptr + l.b_off, l.cout,
-                     false, nullptr, 4, 0, c.st, a.head.ptr);
+                     false, nullptr, 4, 0, c.st, a.head.ptr, &f);
     }
     if (base)
         k_add_base<<<grid_for(c.P(0)), 256, 0, c.st>>>(reinterpret_cast<float4*>(a.head.ptr), base, c.P(0));
     KF_CUDA_CHECK(cudaGetLastError());
 }
 
-void pool_bwd_add(Ctx& c, TRef gy_low, TRef gskip, int level_hi, TRef gx) {
+void pool_bwd_add(Ctx& c, TRef gy_low, TRef gskip, int level_hi, TRef y, TRef gx) {
     const size_t n = c.P(level_hi) * gx.c / 8;
-    k_pool_bwd_add<<<grid_for(n), 256, 0, c.st>>>(gy_low.p, gskip.p, gskip.cs, gskip.co, gx.c, c.n, c.H(level_hi),
-                                                   c.W(level_hi), gx.p);
+    launch_overlapped(k_pool_bwd_add, dim3(grid_for(n)), dim3(256), 0, c.st, gy_low.p, gskip.p, gskip.cs, gskip.co, gx.c, c.n, c.H(level_hi),
+                                                   c.W(level_hi), y.p, y.cs, y.co, gx.p);
 }
-void up_bwd(Ctx& c, TRef gy_slice, int level_hi, TRef gx_low) {
+void up_bwd(Ctx& c, TRef gy_slice, int level_hi, TRef y, TRef gx_low) {
     const size_t n = c.P(level_hi + 1) * gx_low.c / 8;
-    k_up_bwd<<<grid_for(n), 256, 0, c.st>>>(gy_slice.p, gy_slice.cs, gy_slice.co, gx_low.c, c.n, c.H(level_hi),
-                                             c.W(level_hi), gx_low.p);
+    launch_overlapped(k_up_bwd, dim3(grid_for(n)), dim3(256), 0, c.st, gy_slice.p, gy_slice.cs, gy_slice.co, gx_low.c, c.n, c.H(level_hi),
+                                             c.W(level_hi), y.p, gx_low.p);
 }
 
+// Every gradient tensor G_* of a ReLU layer's output holds dL/dz: the ReLU's mask is applied by
+// whatever writes it (the backward-data convolution's epilogue, the upsampling and pooling
+// passes), with the rounded values a separate pass over gradient and output would mask.
 void backward(Ctx& c) {
     Acts& a = c.d.acts;
     TRef none{nullptr, 0, 0, 0};
-    conv_bwd(c, 18, 0, T(a, T_D0B), TRef{a.at(T_OUT), 32, 0, 3}, T(a, G_OUT), T(a, G_D0B));
-    conv_bwd(c, 17, 0, T(a, T_D0A), T(a, T_D0B), T(a, G_D0B), T(a, G_D0A));
-    conv_bwd(c, 16, 0, T(a, T_CAT0), T(a, T_D0A), T(a, G_D0A), T(a, G_CAT0));
-    up_bwd(c, S(a, G_CAT0, 0, 64), 0, T(a, G_D1B));
-    conv_bwd(c, 15, 1, T(a, T_D1A), T(a, T_D1B), T(a, G_D1B), T(a, G_D1A));
-    conv_bwd(c, 14, 1, T(a, T_CAT1), T(a, T_D1A), T(a, G_D1A), T(a, G_CAT1));
-    up_bwd(c, S(a, G_CAT1, 0, 96), 1, T(a, G_D2B));
-    conv_bwd(c, 13, 2, T(a, T_D2A), T(a, T_D2B), T(a, G_D2B), T(a, G_D2A));
-    conv_bwd(c, 12, 2, T(a, T_CAT2), T(a, T_D2A), T(a, G_D2A), T(a, G_CAT2));
-    up_bwd(c, S(a, G_CAT2, 0, 128), 2, T(a, G_D3B));
-    conv_bwd(c, 11, 3, T(a, T_D3A), T(a, T_D3B), T(a, G_D3B), T(a, G_D3A));
-    conv_bwd(c, 10, 3, T(a, T_CAT3), T(a, T_D3A), T(a, G_D3A), T(a, G_CAT3));
-    up_bwd(c, S(a, G_CAT3, 0, 160), 3, T(a, G_E4B));
-    conv_bwd(c, 9, 4, T(a, T_E4A), T(a, T_E4B), T(a, G_E4B), T(a, G_E4A));
-    conv_bwd(c, 8, 4, T(a, T_P3), T(a, T_E4A), T(a, G_E4A), T(a, G_P3));
-    pool_bwd_add(c, T(a, G_P3), S(a, G_CAT3, 160, 128), 3, T(a, G_E3B));
-    conv_bwd(c, 7, 3, T(a, T_E3A), S(a, T_CAT3, 160, 128), T(a, G_E3B), T(a, G_E3A));
-    conv_bwd(c, 6, 3, T(a, T_P2), T(a, T_E3A), T(a, G_E3A), T(a, G_P2));
-    pool_bwd_add(c, T(a, G_P2), S(a, G_CAT2, 128, 96), 2, T(a, G_E2B));
-    conv_bwd(c, 5, 2, T(a, T_E2A), S(a, T_CAT2, 128, 96), T(a, G_E2B), T(a, G_E2A));
-    conv_bwd(c, 4, 2, T(a, T_P1), T(a, T_E2A), T(a, G_E2A), T(a, G_P1));
-    pool_bwd_add(c, T(a, G_P1), S(a, G_CAT1, 96, 64), 1, T(a, G_E1B));
-    conv_bwd(c, 3, 1, T(a, T_E1A), S(a, T_CAT1, 96, 64), T(a, G_E1B), T(a, G_E1A));
-    conv_bwd(c, 2, 1, T(a, T_P0), T(a, T_E1A), T(a, G_E1A), T(a, G_P0));
-    pool_bwd_add(c, T(a, G_P0), S(a, G_CAT0, 64, 32), 0, T(a, G_E0B));
-    conv_bwd(c, 1, 0, T(a, T_E0A), S(a, T_CAT0, 64, 32), T(a, G_E0B), T(a, G_E0A));
-    conv_bwd(c, 0, 0, T(a, T_IN), T(a, T_E0A), T(a, G_E0A), none);
+    conv_bwd(c, 18, 0, T(a, T_D0B), T(a, G_OUT), T(a, G_D0B), true);
+    conv_bwd(c, 17, 0, T(a, T_D0A), T(a, G_D0B), T(a, G_D0A), true);
+    conv_bwd(c, 16, 0, T(a, T_CAT0), T(a, G_D0A), T(a, G_CAT0), false);
+    up_bwd(c, S(a, G_CAT0, 0, 64), 0, T(a, T_D1B), T(a, G_D1B));
+    conv_bwd(c, 15, 1, T(a, T_D1A), T(a, G_D1B), T(a, G_D1A), true);
+    conv_bwd(c, 14, 1, T(a, T_CAT1), T(a, G_D1A), T(a, G_CAT1), false);
+    up_bwd(c, S(a, G_CAT1, 0, 96), 1, T(a, T_D2B), T(a, G_D2B));
+    conv_bwd(c, 13, 2, T(a, T_D2A), T(a, G_D2B), T(a, G_D2A), true);
+    conv_bwd(c, 12, 2, T(a, T_CAT2), T(a, G_D2A), T(a, G_CAT2), false);
+    up_bwd(c, S(a, G_CAT2, 0, 128), 2, T(a, T_D3B), T(a, G_D3B));
+    conv_bwd(c, 11, 3, T(a, T_D3A), T(a, G_D3B), T(a, G_D3A), true);
+    conv_bwd(c, 10, 3, T(a, T_CAT3), T(a, G_D3A), T(a, G_CAT3), false);
+    up_bwd(c, S(a, G_CAT3, 0, 160), 3, T(a, T_E4B), T(a, G_E4B));
+    conv_bwd(c, 9, 4, T(a, T_E4A), T(a, G_E4B), T(a, G_E4A), true);
+    conv_bwd(c, 8, 4, T(a, T_P3), T(a, G_E4A), T(a, G_P3), false);
+    pool_bwd_add(c, T(a, G_P3), S(a, G_CAT3, 160, 128), 3, S(a, T_CAT3, 160, 128), T(a, G_E3B));
+    conv_bwd(c, 7, 3, T(a, T_E3A), T(a, G_E3B), T(a, G_E3A), true);
+    conv_bwd(c, 6, 3, T(a, T_P2), T(a, G_E3A), T(a, G_P2), false);
+    pool_bwd_add(c, T(a, G_P2), S(a, G_CAT2, 128, 96), 2, S(a, T_CAT2, 128, 96), T(a, G_E2B));
+    conv_bwd(c, 5, 2, T(a, T_E2A), T(a, G_E2B), T(a, G_E2A), true);
+    conv_bwd(c, 4, 2, T(a, T_P1), T(a, G_E2A), T(a, G_P1), false);
+    pool_bwd_add(c, T(a, G_P1), S(a, G_CAT1, 96, 64), 1, S(a, T_CAT1, 96, 64), T(a, G_E1B));
+    conv_bwd(c, 3, 1, T(a, T_E1A), T(a, G_E1B), T(a, G_E1A), true);
+    conv_bwd(c, 2, 1, T(a, T_P0), T(a, G_E1A), T(a, G_P0), false);
+    pool_bwd_add(c, T(a, G_P0), S(a, G_CAT0, 64, 32), 0, S(a, T_CAT0, 64, 32), T(a, G_E0B));
+    conv_bwd(c, 1, 0, T(a, T_E0A), T(a, G_E0B), T(a, G_E0A), true);
+    conv_bwd(c, 0, 0, T(a, T_IN), T(a, G_E0A), none, false);
 }
 
 } // namespace
@@ -731,24 +767,21 @@ void denoiser_forward(kf_denoiser_impl* d, const void* feat, const void* base, i
 float denoiser_train_step(kf_denoiser_impl* d, const void* feat, const void* base, const float* tgt, int n, int h,
                           int w, float lr, float* grads_out, bool apply_update) {
     cudaStream_t st = d->r->stream;
-    denoiser_forward(d, feat, base, n, h, w, nullptr);
+    denoiser_forward(d, feat, nullptr, n, h, w, nullptr); // the loss adds the residual
     Acts& a = d->acts;
     KF_CUDA_CHECK(cudaMemsetAsync(d->loss.ptr, 0, sizeof(float), st));
-    const size_t P = (size_t)n * h * w;
-    k_loss<<<grid_for(P), 256, 0, st>>>(a.head.ptr, reinterpret_cast<const float4*>(tgt), n, h, w, 0.5f, d->loss.ptr,
-                                        a.at(G_OUT));
+    const unsigned tiles = (unsigned)n * (unsigned)((w + kLossW - 1) / kLossW) * (unsigned)((h + kLossH - 1) / kLossH);
+    k_loss<<<tiles, kLossW * kLossH, 0, st>>>(reinterpret_cast<const float4*>(a.head.ptr),
+                                              static_cast<const float4*>(base), reinterpret_cast<const float4*>(tgt), n,
+                                              h, w, 0.5f, d->loss.ptr, a.at(G_OUT));
+    KF_CUDA_CHECK(cudaGetLastError());
     KF_CUDA_CHECK(cudaMemsetAsync(d->grads.ptr, 0, d->grads.bytes(), st));
     Ctx c{*d, st, n, h, w};
     backward(c);
     if (grads_out)
         KF_CUDA_CHECK(cudaMemcpyAsync(grads_out, d->grads.ptr, d->nparams * 4, cudaMemcpyDeviceToDevice, st));
     if (apply_update) {
-        ++d->step;
-        const float b1 = 0.9f, b2 = 0.999f;
-        const float bc1 = 1.0f - std::pow(b1, (float)d->step), bc2 = 1.0f - std::pow(b2, (float)d->step);
-        k_adam<<<grid_for(d->nparams), 256, 0, st>>>(d->params.ptr, d->grads.ptr, d->m.ptr, d->v.ptr, d->nparams, lr,
-                                                     b1, b2, 1e-8f, bc1, bc2);
-        d->packed = false;
+        update(*d, ++d->step, lr, st);
     }
     float loss = 0.0f;
     KF_CUDA_CHECK(cudaMemcpyAsync(&loss, d->loss.ptr, sizeof(float), cudaMemcpyDeviceToHost, st));

@@ -84,6 +84,34 @@ template <class T> struct DeviceBuffer {
     size_t bytes() const { return sizeof(T) * count; }
 };
 
+// Launches a kernel that may start while its predecessor in the stream drains (programmatic
+// dependent launch). Such a kernel calls grid_dependency_wait() before it touches anything the
+// predecessor reads or writes.
+template <class... KArgs, class... Args>
+void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    KF_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+}
+
+#ifdef __CUDACC__
+// Waits until every kernel before this one in the stream is complete and its writes are visible
+// (returns at once in a kernel launched the usual way), then lets the next kernel's blocks start
+// their own prologue as this one's leave room.
+__device__ __forceinline__ void grid_dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // Stream-ordered temporaries (cudaMallocAsync), freed on the same stream at scope exit.
 struct TempAlloc {
     cudaStream_t st;

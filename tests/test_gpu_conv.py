@@ -68,6 +68,24 @@ def test_conv3x3_matches_torch(n, h, w, cin, cout, rows, relu, cstride, coff):
         assert (rest == 0).all()
 
 
+# The tile kernel (images under 96 wide, up to 288 input channels): tiles of 8 x 16 pixels with
+# remainders of 1 and all but 1, more tiles than CTAs (two halo buffers), channel slices of 16, one
+# and several output-channel blocks, the largest resident weights; and the per-tile kernel beyond.
+@pytest.mark.parametrize("n,h,w,cin,cout,rows,relu,cstride,coff", [
+    (1, 1, 1, 32, 16, 16, False, 16, 0),
+    (2, 17, 9, 32, 32, 32, True, 48, 16),
+    (3, 15, 7, 64, 24, 32, False, 24, 0),
+    (40, 33, 25, 96, 96, 96, True, 96, 0),
+    (1, 16, 8, 160, 160, 160, True, 288, 128),
+    (2, 31, 95, 224, 48, 48, False, 48, 0),
+    (1, 20, 40, 288, 128, 128, True, 128, 0),
+    (5, 64, 64, 160, 64, 64, True, 64, 0),
+    (1, 10, 12, 320, 32, 32, True, 32, 0),
+])
+def test_conv3x3_tiles_of_narrow_images(n, h, w, cin, cout, rows, relu, cstride, coff):
+    test_conv3x3_matches_torch(n, h, w, cin, cout, rows, relu, cstride, coff)
+
+
 @pytest.mark.parametrize("m,n,k,splits", [(200, 96, 4096, 4), (128, 32, 64, 1), (77, 160, 1000, 3)])
 def test_gemm_tn_matches_torch(m, n, k, splits):
     import torch

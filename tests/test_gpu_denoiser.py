@@ -238,6 +238,41 @@ def test_training_reduces_loss(renderer):
     d.close()
 
 
+def test_update_is_adam_and_reaches_the_convolutions(renderer):
+    """Two steps from known gradients equal Adam evaluated in FP64 (FP32 state: 1e-5 of the largest
+    step), and the network then computes with the new weights, bit for bit those of a denoiser that
+    is given them."""
+    import torch
+
+    d = api.Denoiser(renderer, seed=4)
+    n, h, w, lr = 2, 32, 112, 1e-3
+    feat, target = _inputs(torch, n, h, w, 41)
+    x = d.getParams().astype(np.float64)
+    m, v = np.zeros_like(x), np.zeros_like(x)
+    grads = torch.zeros(x.size, device="cuda")
+    torch.cuda.synchronize()
+    for step in (1, 2):
+        d.trainStep(feat.data_ptr(), target.data_ptr(), n, h, w, lr=lr, grads_ptr=grads.data_ptr(), apply=True)
+        torch.cuda.synchronize()
+        g = grads.cpu().numpy().astype(np.float64)
+        m, v = 0.9 * m + 0.1 * g, 0.999 * v + 0.001 * g * g
+        x -= lr * (m / (1 - 0.9 ** step)) / (np.sqrt(v / (1 - 0.999 ** step)) + 1e-8)
+        got = d.getParams()
+        # bias corrections are FP32 (1 - 0.999 keeps 13 bits of its 24: 2^-13 of a step)
+        assert np.abs(got - x).max() <= lr * 2.0 ** -11 + 1e-7 * np.abs(x).max()
+        x = got.astype(np.float64)
+    e = api.Denoiser(renderer, seed=6)
+    e.setParams(got)
+    out = [torch.zeros((n, h, w, 4), device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    for k, net in enumerate((d, e)):
+        net.forward(feat.data_ptr(), n, h, w, out[k].data_ptr())
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], out[1]) and _tc_error() == 0
+    d.close()
+    e.close()
+
+
 def test_params_roundtrip(renderer, tmp_path):
     d = api.Denoiser(renderer, seed=1)
     p = d.getParams()
