@@ -1015,8 +1015,11 @@ __global__ void __launch_bounds__(kMissThreads) k_miss(SceneDev s, const FrameDe
 constexpr uint32_t kShadeThreads = 128, kShadeWarps = kShadeThreads / 32;
 
 template <bool BATCH>
-// 4 resident blocks per SM (128 registers, no spill) measured fastest; unbounded it takes 148.
-__global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
+// Bound by the latency of its five dependent levels of loads (list, hit, instance, indices,
+// vertices): 8 resident blocks per SM (64 registers, 44 bytes spilled) hide more of it than 4 to 6
+// without a spill. A Cornell room of 256 x 256 at 64 spp takes 3.03 ms with 4 or 5 blocks, 2.85 with 6,
+// 2.67 with 8, 2.69 with 9, 2.75 with 10; a batch of rooms with spheres 56.2, 53.1, 51.3, 51.4, 52.0.
+__global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
                                                int cur, uint32_t depth, uint64_t chunk_start) {
     const uint32_t count = w.counters[depth * kCounterRow + 1]; // rays that hit (k_miss takes the others)
     const int nxt = cur ^ 1;
@@ -1275,8 +1278,10 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(SceneDev s, const Fr
 // light slots, one ballot per slot. A kernel of its own, beside k_shade: each of the two is
 // small enough for the instruction cache.
 // ---------------------------------------------------------------------------
+// 7 blocks per SM (72 registers; 101 unbounded, 5 blocks): 18.4 instead of 18.8 ms on the 256-icosphere
+// 1080p frame; 8 to 12 gain nothing there and cost small views up to 4 %.
 template <bool BATCH>
-__global__ void __launch_bounds__(kShadeThreads) k_nee(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
+__global__ void __launch_bounds__(kShadeThreads, 7) k_nee(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
                                              uint32_t depth, uint64_t chunk_start) {
     const uint32_t count = w.counters[depth * kCounterRow + 1];
     const uint32_t lane = threadIdx.x & 31;
