@@ -81,6 +81,7 @@ struct SceneGpu {
     kf::DeviceBuffer<kf_dir_light_ubo> dlight;
     kf::DeviceBuffer<kf_point_lights_ubo> plights;
     kf::DeviceBuffer<kf_active_lights_ubo> alights;
+    std::vector<unsigned char> light_bytes;          // what the three light buffers hold
     kf::DeviceBuffer<uint4> tex_info;
     kf::DeviceBuffer<uchar4> texels;
     kf::DeviceBuffer<float> srgb_decode;

@@ -110,3 +110,27 @@ def test_lights_added_between_batches():
     for a, b, dark in zip(render(1), render(0), render(2)):
         assert _same(a, b)
         assert not _same(a, dark)
+
+
+def test_changed_lights_reach_the_next_frame():
+    """Lights are uploaded when they change: a point light recoloured and a directional light added
+    between frames give the frame of a renderer that had them from the start."""
+    import ctypes as C
+
+    def render(when):
+        with api.Kuafu(scenes.icosphere_config(spp=2, depth=3, count=64)) as r:
+            s = r.getScene()
+            cam = scenes.cornell(r, 31, 22, scene=s)
+            light = api.PointLight(position=(0.0, 0.0, 0.5), color=(1.0, 0.2, 0.1), radius=0.1, strength=2.0)
+            s.addPointLight(light)
+            for frame in range(2):
+                if frame == when:
+                    c = N.kf_point_light((C.c_float * 3)(0.1, 0.0, 0.5), (C.c_float * 3)(0.2, 1.0, 0.4), 0.1, 3.0)
+                    N.check(N.load().kf_light_update_point(s._lights[id(light)][1], C.byref(c)))
+                    s.setDirectionalLight(api.DirectionalLight(direction=(1.0, 0.1, -0.4), strength=1.5))
+                r.resetFrame()
+                r.run()
+            return r.downloadAov(cam, N.KF_AOV_RADIANCE_F32)
+
+    assert _same(render(1), render(0))
+    assert not _same(render(1), render(2))
