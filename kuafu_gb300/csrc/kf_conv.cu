@@ -254,36 +254,79 @@ constexpr int kHaloW = 130;     // 128 output pixels + 2 halo pixels
 // tiles, or 32-channel chunks with streamed weights).
 constexpr int kHaloThreads = 320;  // producer warp, MMA warp, 8 epilogue warps
 
-// 8 or 16 FP32 values stored as BF16 with one 16- or 32-byte store (dst 16- / 32-byte aligned)
-__device__ __forceinline__ void st_bf16x8(__nv_bfloat16* dst, const float (&v)[8]) {
-    __nv_bfloat162 q2[4];
+// ---- epilogue pieces of the two persistent kernels: a lane holds 16 output channels of a pixel ----
+// The epilogue warps run a few instructions deep in each other's results, so its length is what
+// the narrow layers (16 and 32 input channels) wait for: bias in registers for all rows of a
+// channel group, two groups of accumulators per TMEM wait, and pooling neighbours exchanged as
+// packed BF16 pairs.
+struct Bias16 {
+    float v[16];
+    __device__ __forceinline__ void load(const float* s) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) q2[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(q2);
-}
-__device__ __forceinline__ void st_bf16x16(__nv_bfloat16* dst, const float (&v0)[8], const float (&v1)[8]) {
-    __nv_bfloat162 q2[8];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        q2[q] = __floats2bfloat162_rn(v0[2 * q], v0[2 * q + 1]);
-        q2[4 + q] = __floats2bfloat162_rn(v1[2 * q], v1[2 * q + 1]);
+        for (int q = 0; q < 4; ++q) {
+            const float4 b = *reinterpret_cast<const float4*>(s + 4 * q);
+            v[4 * q] = b.x; v[4 * q + 1] = b.y; v[4 * q + 2] = b.z; v[4 * q + 3] = b.w;
+        }
     }
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(q2);
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]),
-                 "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+};
+__device__ __forceinline__ void activate(const uint32_t (&raw)[16], const Bias16& b, int relu, float (&v)[16]) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(raw[q]) + b.v[q];
+    if (relu) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = fmaxf(v[q], 0.0f);
+    }
+}
+__device__ __forceinline__ void pack16(const float (&v)[16], uint32_t (&w)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+        w[q] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+}
+// 16 BF16 channels with one 32-byte store (dst 32-byte aligned)
+__device__ __forceinline__ void store16(__nv_bfloat16* dst, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                  : "memory");
 }
-
-// A ReLU's backward mask on 8 channels of one pixel: zero where the forward output is not positive.
-__device__ __forceinline__ void mask8(const __nv_bfloat16* m, float (&v)[8]) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(m));
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+// the first n of 16 channels, at any alignment (16-byte stores where they fit)
+__device__ __forceinline__ void store16_any(__nv_bfloat16* dst, const uint32_t (&w)[8], int n) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float2 t = __bfloat1622float2(h[k]);
-        if (!(t.x > 0.0f)) v[2 * k] = 0.0f;
-        if (!(t.y > 0.0f)) v[2 * k + 1] = 0.0f;
+    for (int h = 0; h < 2; ++h) {
+        const int m = n - 8 * h;
+        if (m >= 8 && ((uintptr_t)(dst + 8 * h) & 15) == 0) {
+            *reinterpret_cast<uint4*>(dst + 8 * h) = make_uint4(w[4 * h], w[4 * h + 1], w[4 * h + 2], w[4 * h + 3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (q < m) reinterpret_cast<uint16_t*>(dst)[8 * h + q] = (uint16_t)(w[4 * h + q / 2] >> (16 * (q & 1)));
+        }
     }
+}
+// A ReLU's backward mask on the packed channels of one pixel: zero where the forward output is
+// not positive. m: 16 channels, 16-byte aligned.
+__device__ __forceinline__ void mask16(const __nv_bfloat16* m, uint32_t (&w)[8]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(m) + h);
+        const uint32_t y[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float lo = __uint_as_float(y[k] << 16), hi = __uint_as_float(y[k] & 0xFFFF0000u);
+            w[4 * h + k] &= (lo > 0.0f ? 0x0000FFFFu : 0u) | (hi > 0.0f ? 0xFFFF0000u : 0u);
+        }
+    }
+}
+// ((a + b) + c) + d, quartered, of packed BF16 pairs: the order of the separate pooling pass
+__device__ __forceinline__ uint32_t pool_pair(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    const float lo = 0.25f * (((__uint_as_float(a << 16) + __uint_as_float(b << 16)) + __uint_as_float(c << 16)) +
+                              __uint_as_float(d << 16));
+    const float hi = 0.25f * (((__uint_as_float(a & 0xFFFF0000u) + __uint_as_float(b & 0xFFFF0000u)) +
+                               __uint_as_float(c & 0xFFFF0000u)) +
+                              __uint_as_float(d & 0xFFFF0000u));
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 struct HaloParams {
@@ -499,15 +542,16 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
         tc::mma_commit(mma_done);
         if (!tc::mbar_wait(mma_done, 0, kWaitBudget)) set_error(17);
     } else if (warp >= 2) {
-        // ---- epilogue: 8 warps, two per TMEM lane group, each taking half the channels ----
+        // ---- epilogue: 8 warps, two per TMEM lane group, each taking half of the channel groups ----
         const int lg = warp & 3;                 // TMEM lane group of this warp
         const int px_in_tile = lg * 32 + lane;
-        const int half = (warp - 2) >> 2;
-        const int cb = half * (p.n_tile / 2), ce = cb + p.n_tile / 2;  // multiples of 8
-        // 32-byte stores need 32-byte aligned rows: the tensor, the channel stride and slice
-        const bool wide = !p.outf && p.out && ((uintptr_t)p.out & 31) == 0 && (p.out_cstride & 15) == 0;
-        const bool pool_wide = p.pool_out && ((uintptr_t)p.pool_out & 31) == 0 && (p.Cout & 15) == 0 &&
-                               (n0 & 15) == 0;
+        const int ng = p.n_tile >> 4;            // groups of 16 channels
+        const int g0 = warp < 6 ? 0 : (ng + 1) / 2, g1 = warp < 6 ? (ng + 1) / 2 : ng;
+        // whole 32-byte stores: the tensor, the channel stride and the slice are aligned to them
+        const bool fast = !p.outf && p.out && ((uintptr_t)p.out & 31) == 0 && (p.out_cstride & 15) == 0 &&
+                          ((p.out_coff + n0) & 15) == 0 && n0 + p.n_tile <= p.Cout;
+        const bool pool_fast = p.pool_out && ((uintptr_t)p.pool_out & 31) == 0 && (p.Cout & 15) == 0;
+        const uint32_t lanes = (uint32_t)(lg * 32) << 16;
         if (p.settled) grid_dependency_wait();
         uint32_t j = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++j) {
@@ -522,128 +566,59 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
             int n_img, y0, x0;
             tile_origin(t, n_img, y0, x0);
             const int px = x0 + px_in_tile;
-            // one output row's 8 channels [cc, cc + 8) of this pixel (BF16 or FP32)
-            auto emit8 = [&](const float(&v)[8], int py, int cc) {
-                const int co = n0 + cc;
-                if (!(px < p.W && py < p.H) || co >= p.Cout) return;
-                const size_t base = ((size_t)((size_t)n_img * p.H + py) * p.W + px) * p.out_cstride + p.out_coff;
-                if (p.outf) {
-                    for (int q = 0; q < 8 && co + q < p.Cout; ++q) p.outf[base + co + q] = v[q];
+            const int rows = px < p.W ? min(R, p.H - y0) : 0; // this pixel column's rows inside the image
+            const size_t pix = ((size_t)n_img * p.H + y0) * p.W + px;
+            const size_t row_step = (size_t)p.W * p.out_cstride;
+            // one row's 16 channels of this pixel
+            auto emit = [&](int r, int g, const float(&v)[16], uint32_t(&w)[8]) {
+                const int co = n0 + 16 * g;
+                if (r >= rows || co >= p.Cout) return;
+                const size_t at = pix * p.out_cstride + p.out_coff + co + r * row_step;
+                if (p.outf) { // FP32 output (a network head)
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        if (co + q < p.Cout) p.outf[at + q] = v[q];
                     return;
                 }
-                __nv_bfloat162 q2[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) q2[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-                const uint4 packed = *reinterpret_cast<const uint4*>(q2);
-                __nv_bfloat16* dst = p.out + base + co;
-                if (co + 8 <= p.Cout && ((p.out_coff + co) & 7) == 0 && (p.out_cstride & 7) == 0)
-                    *reinterpret_cast<uint4*>(dst) = packed;
-                else
-                    for (int q = 0; q < 8 && co + q < p.Cout; ++q) dst[q] = __float2bfloat16_rn(v[q]);
+                if (p.mask) mask16(p.mask + (pix + (size_t)r * p.W) * p.mask_cs + p.mask_co + co, w);
+                if (fast) store16(p.out + at, w);
+                else store16_any(p.out + at, w, p.Cout - co);
             };
-            // 16 channels [cc, cc + 16): one 32-byte store (a whole L2 sector) when aligned
-            auto emit16 = [&](const float(&v0)[8], const float(&v1)[8], int py, int cc) {
-                const int co = n0 + cc;
-                if (wide && co + 16 <= p.Cout && ((p.out_coff + co) & 15) == 0) {
-                    if (!(px < p.W && py < p.H)) return;
-                    const size_t base = ((size_t)((size_t)n_img * p.H + py) * p.W + px) * p.out_cstride + p.out_coff;
-                    st_bf16x16(p.out + base + co, v0, v1);
-                    return;
-                }
-                emit8(v0, py, cc);
-                emit8(v1, py, cc + 8);
-            };
-            auto act = [&](uint32_t raw, int cc) {
-                const float v = __uint_as_float(raw) + sbias[cc];
-                return p.relu ? fmaxf(v, 0.0f) : v;
-            };
-            const uint32_t lanes = (uint32_t)(lg * 32) << 16;
-            if (!p.pool_out) {
-                for (int r = 0; r < p.R; ++r) {
-                    const uint32_t col0 = (b * (uint32_t)p.R + (uint32_t)r) * (uint32_t)p.n_tile;
-                    const __nv_bfloat16* mk =
-                        p.mask && px < p.W && y0 + r < p.H
-                            ? p.mask + ((size_t)((size_t)n_img * p.H + y0 + r) * p.W + px) * p.mask_cs + p.mask_co + n0
-                            : nullptr;
-                    for (int c = cb; c < ce; c += 16) { // two TMEM loads per wait
-                        uint32_t r0[8], r1[8];
-                        const bool two = c + 16 <= ce;
-                        tc::tmem_ld8(tmem + lanes + col0 + (uint32_t)c, r0);
-                        if (two) tc::tmem_ld8(tmem + lanes + col0 + (uint32_t)(c + 8), r1);
-                        tc::tmem_ld_wait();
-                        float v0[8], v1[8];
+            for (int g = g0; g < g1; ++g) {
+                Bias16 bias;
+                bias.load(sbias + 16 * g);
+                const uint32_t col0 = tmem + lanes + b * (uint32_t)acc_cols + 16u * (uint32_t)g;
+#pragma unroll 1
+                for (int r = 0; r < R; r += 2) { // two rows per TMEM wait (R = 1: one)
+                    uint32_t r0[16], r1[16], w0[8], w1[8];
+                    float v0[16], v1[16];
+                    tc::tmem_ld16(col0 + (uint32_t)(r * p.n_tile), r0);
+                    if (R > 1) tc::tmem_ld16(col0 + (uint32_t)((r + 1) * p.n_tile), r1);
+                    tc::tmem_ld_wait();
+                    activate(r0, bias, p.relu, v0);
+                    pack16(v0, w0);
+                    if (R > 1) {
+                        activate(r1, bias, p.relu, v1);
+                        pack16(v1, w1);
+                        if (p.pool_out) {
+                            // R and y0 are even: the 2x2 average of the BF16 outputs over (2y, 2x),
+                            // (2y, 2x+1), (2y+1, 2x), (2y+1, 2x+1); the right neighbour is the next lane
+                            uint32_t pw[8];
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            v0[q] = act(r0[q], c + q);
-                            v1[q] = two ? act(r1[q], c + 8 + q) : 0.0f;
-                        }
-                        if (mk) {
-                            if (n0 + c + 8 <= p.Cout) mask8(mk + c, v0);
-                            if (two && n0 + c + 16 <= p.Cout) mask8(mk + c + 8, v1);
-                        }
-                        if (two)
-                            emit16(v0, v1, y0 + r, c);
-                        else
-                            emit8(v0, y0 + r, c);
-                    }
-                }
-            } else {
-                // rows in pairs (R and y0 are even): the 2x2 average of the BF16 outputs, as the
-                // separate pooling pass computes it ((a + b) + c) + d over (2y, 2x), (2y, 2x+1),
-                // (2y+1, 2x), (2y+1, 2x+1); the right neighbour is the next lane
-                const int Hh = p.H / 2, Wh = p.W / 2;
-                for (int r = 0; r < p.R; r += 2) {
-                    const int py = y0 + r;
-                    const uint32_t col0 = (b * (uint32_t)p.R + (uint32_t)r) * (uint32_t)p.n_tile;
-                    for (int c = cb; c < ce; c += 16) {
-                        const bool two = c + 16 <= ce;
-                        uint32_t ra[16], rc[16];
-                        tc::tmem_ld8(tmem + lanes + col0 + (uint32_t)c, *reinterpret_cast<uint32_t(*)[8]>(ra));
-                        tc::tmem_ld8(tmem + lanes + col0 + (uint32_t)(p.n_tile + c),
-                                     *reinterpret_cast<uint32_t(*)[8]>(rc));
-                        if (two) {
-                            tc::tmem_ld8(tmem + lanes + col0 + (uint32_t)(c + 8),
-                                         *reinterpret_cast<uint32_t(*)[8]>(ra + 8));
-                            tc::tmem_ld8(tmem + lanes + col0 + (uint32_t)(p.n_tile + c + 8),
-                                         *reinterpret_cast<uint32_t(*)[8]>(rc + 8));
-                        }
-                        tc::tmem_ld_wait();
-                        float va[16], vc[16], pooled[16];
-#pragma unroll
-                        for (int q = 0; q < 16; ++q) {
-                            const bool live = q < 8 || two;
-                            va[q] = live ? act(ra[q], c + q) : 0.0f;
-                            vc[q] = live ? act(rc[q], c + q) : 0.0f;
-                            const float a = __bfloat162float(__float2bfloat16_rn(va[q]));
-                            const float cv = __bfloat162float(__float2bfloat16_rn(vc[q]));
-                            const float bv = __shfl_xor_sync(0xFFFFFFFFu, a, 1);
-                            const float dv = __shfl_xor_sync(0xFFFFFFFFu, cv, 1);
-                            pooled[q] = 0.25f * (((a + bv) + cv) + dv);
-                        }
-                        const float(&va0)[8] = *reinterpret_cast<const float(*)[8]>(va);
-                        const float(&va1)[8] = *reinterpret_cast<const float(*)[8]>(va + 8);
-                        const float(&vc0)[8] = *reinterpret_cast<const float(*)[8]>(vc);
-                        const float(&vc1)[8] = *reinterpret_cast<const float(*)[8]>(vc + 8);
-                        if (two) {
-                            emit16(va0, va1, py, c);
-                            emit16(vc0, vc1, py + 1, c);
-                        } else {
-                            emit8(va0, py, c);
-                            emit8(vc0, py + 1, c);
-                        }
-                        const int co = n0 + c;
-                        if ((lane & 1) == 0 && px + 1 < p.W && py + 1 < p.H && co < p.Cout) {
-                            const size_t pb = ((size_t)((size_t)n_img * Hh + py / 2) * Wh + px / 2) * p.Cout + co;
-                            const float(&p0)[8] = *reinterpret_cast<const float(*)[8]>(pooled);
-                            const float(&p1)[8] = *reinterpret_cast<const float(*)[8]>(pooled + 8);
-                            if (two && pool_wide && co + 16 <= p.Cout && (co & 15) == 0)
-                                st_bf16x16(p.pool_out + pb, p0, p1);
-                            else {
-                                st_bf16x8(p.pool_out + pb, p0);
-                                if (two && co + 8 < p.Cout) st_bf16x8(p.pool_out + pb + 8, p1);
+                            for (int q = 0; q < 8; ++q)
+                                pw[q] = pool_pair(w0[q], __shfl_xor_sync(0xFFFFFFFFu, w0[q], 1), w1[q],
+                                                  __shfl_xor_sync(0xFFFFFFFFu, w1[q], 1));
+                            const int co = n0 + 16 * g;
+                            if (!(lane & 1) && px + 1 < p.W && r + 1 < rows && co < p.Cout) {
+                                __nv_bfloat16* dst = p.pool_out +
+                                    (((size_t)n_img * (p.H / 2) + (y0 + r) / 2) * (p.W / 2) + px / 2) * p.Cout + co;
+                                if (pool_fast) store16(dst, pw);
+                                else store16_any(dst, pw, p.Cout - co);
                             }
                         }
                     }
+                    emit(r, g, v0, w0);
+                    if (R > 1) emit(r + 1, g, v1, w1);
                 }
             }
             tc::fence_before_sync();
@@ -676,10 +651,10 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
 // 32 x 32 17 -> 11, 160 -> 64 at 64 x 64 28 -> 26; a 256 x 256 frame's whole network 391 -> 303 us
 // (with the weights loaded while the kernel before drains).
 //
-// Warp 0 lane 0: TMA, warp 1 lane 0: MMAs, warps 2-5: epilogue, one TMEM lane group (4 tile rows)
-// each. Every wait is bounded as in the kernels above.
+// Warp 0 lane 0: TMA, warp 1 lane 0: MMAs, warps 2-9: epilogue, two to a TMEM lane group (4 tile
+// rows), each taking half of the channel groups. Every wait is bounded as in the kernels above.
 // ---------------------------------------------------------------------------
-constexpr int kTileThreads = 192;
+constexpr int kTileThreads = 320;
 constexpr int kTileW = 8, kTileH = 16, kTileHaloW = kTileW + 2, kTileHaloH = kTileH + 2;
 constexpr uint32_t kTileHaloBytes = kTileHaloW * kTileHaloH * 64; // 32 channels
 constexpr uint32_t kTileHaloSlot = (kTileHaloBytes + 1023u) & ~1023u;
@@ -705,14 +680,18 @@ struct TileParams {
 // 160 -> 64 layer of 16 x 64 x 64 pixels took 34.9 us, bound by their issue).
 template <int KC>
 __device__ __forceinline__ void tile_mmas(uint32_t acc, uint64_t ad0, uint64_t bd0, uint32_t tap_units, uint32_t idesc) {
+#pragma unroll 1
+    for (int dy = 0; dy < 3; ++dy) { // a filter row at a time: all 9 taps at once spill from 160 channels on
+        const uint64_t ar = ad0 + (uint32_t)(dy * kTileHaloW * 4), br = bd0 + (uint32_t)dy * 3u * tap_units;
 #pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
+        for (int dx = 0; dx < 3; ++dx) {
 #pragma unroll
-        for (int c = 0; c < KC; ++c) {
-            const uint64_t ad = ad0 + (uint32_t)(((tap / 3) * kTileHaloW + tap % 3) * 4 + c * (kTileHaloSlot >> 4));
-            const uint64_t bd = bd0 + (uint32_t)(c * 9 + tap) * tap_units;
-            tc::mma_bf16(acc, ad, bd, idesc, (tap > 0 || c > 0) ? 1u : 0u);
-            tc::mma_bf16(acc, ad + 2, bd + 2, idesc, 1u);
+            for (int c = 0; c < KC; ++c) {
+                const uint64_t ad = ar + (uint32_t)(dx * 4 + c * (kTileHaloSlot >> 4));
+                const uint64_t bd = br + (uint32_t)(c * 9 + dx) * tap_units;
+                tc::mma_bf16(acc, ad, bd, idesc, (dy > 0 || dx > 0 || c > 0) ? 1u : 0u);
+                tc::mma_bf16(acc, ad + 2, bd + 2, idesc, 1u);
+            }
         }
     }
 }
@@ -750,7 +729,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
             tc::mbar_init(&full[b], 1);
             tc::mbar_init(&empty[b], 1);
             tc::mbar_init(&acc_full[b], 1);
-            tc::mbar_init(&acc_empty[b], 4);
+            tc::mbar_init(&acc_empty[b], 8);
         }
         tc::mbar_init(wbar, 1);
         tc::mbar_init(mma_done, 1);
@@ -826,9 +805,13 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
         tc::mma_commit(mma_done);
         if (!tc::mbar_wait(mma_done, 0, kWaitBudget)) set_error(37);
     } else if (warp >= 2) {
-        // ---- epilogue: lane = pixel (4 rows of 8 per warp) ----
+        // ---- epilogue: lane = pixel (4 rows of 8 per lane group) ----
         const int lg = warp & 3, m = lg * 32 + lane;
-        const bool wide = !p.outf && ((uintptr_t)p.out & 31) == 0 && (p.out_cstride & 15) == 0;
+        const int ng = p.n_tile >> 4;
+        const int g0 = warp < 6 ? 0 : (ng + 1) / 2, g1 = warp < 6 ? (ng + 1) / 2 : ng;
+        const bool fast = !p.outf && ((uintptr_t)p.out & 31) == 0 && (p.out_cstride & 15) == 0 &&
+                          ((p.out_coff + n0) & 15) == 0 && n0 + p.n_tile <= p.Cout;
+        const bool pool_fast = p.pool_out && ((uintptr_t)p.pool_out & 31) == 0 && (p.Cout & 15) == 0;
         if (p.settled) grid_dependency_wait();
         uint32_t it = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
@@ -844,65 +827,50 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
             tile_origin(t, n_img, y0, x0);
             const int px = x0 + (m & 7), py = y0 + (m >> 3);
             const bool valid = px < p.W && py < p.H;
-            const size_t base = ((size_t)((size_t)n_img * p.H + py) * p.W + px) * p.out_cstride + p.out_coff;
+            const size_t pix = ((size_t)n_img * p.H + py) * p.W + px;
             const uint32_t col0 = tmem + ((uint32_t)(lg * 32) << 16) + a * (uint32_t)p.n_tile;
-            for (int c = 0; c < p.n_tile; c += 16) {
-                uint32_t r0[8], r1[8];
-                tc::tmem_ld8(col0 + (uint32_t)c, r0);
-                tc::tmem_ld8(col0 + (uint32_t)(c + 8), r1);
-                tc::tmem_ld_wait();
-                const int co = n0 + c;
-                float v0[8], v1[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    v0[q] = __uint_as_float(r0[q]) + sbias[c + q];
-                    v1[q] = __uint_as_float(r1[q]) + sbias[c + 8 + q];
-                    if (p.relu) {
-                        v0[q] = fmaxf(v0[q], 0.0f);
-                        v1[q] = fmaxf(v1[q], 0.0f);
-                    }
-                }
-                if (p.mask && valid) {
-                    const __nv_bfloat16* mk =
-                        p.mask + ((size_t)((size_t)n_img * p.H + py) * p.W + px) * p.mask_cs + p.mask_co + co;
-                    if (co + 8 <= p.Cout) mask8(mk, v0);
-                    if (co + 16 <= p.Cout) mask8(mk + 8, v1);
-                }
-                if (valid) {
-                    if (p.outf) { // FP32 output (a network head)
-                        for (int q = 0; q < 16 && co + q < p.Cout; ++q) p.outf[base + co + q] = q < 8 ? v0[q & 7] : v1[q & 7];
-                    } else if (wide && co + 16 <= p.Cout && ((p.out_coff + co) & 15) == 0) {
-                        st_bf16x16(p.out + base + co, v0, v1);
-                    } else {
-                        __nv_bfloat16* dst = p.out + base + co;
-                        const bool al = ((p.out_coff + co) & 7) == 0 && (p.out_cstride & 7) == 0;
-                        if (al && co + 8 <= p.Cout) st_bf16x8(dst, v0);
-                        else
-                            for (int q = 0; q < 8 && co + q < p.Cout; ++q) dst[q] = __float2bfloat16_rn(v0[q]);
-                        if (al && co + 16 <= p.Cout) st_bf16x8(dst + 8, v1);
-                        else
-                            for (int q = 0; q < 8 && co + 8 + q < p.Cout; ++q) dst[8 + q] = __float2bfloat16_rn(v1[q]);
-                    }
-                }
+            auto finish = [&](int g, const uint32_t(&raw)[16]) {
+                Bias16 bias;
+                bias.load(sbias + 16 * g);
+                float v[16];
+                uint32_t w[8];
+                activate(raw, bias, p.relu, v);
+                pack16(v, w);
+                const int co = n0 + 16 * g;
                 if (p.pool_out) {
-                    // the 2x2 average of the BF16 outputs, ((a + b) + c) + d in row order as the
-                    // separate pass computes it: the neighbours are lanes 1 and 8 further
-                    float o0[8], o1[8];
+                    // the 2x2 average of the BF16 outputs: the neighbours are lanes 1, 8 and 9 further
+                    uint32_t pw[8];
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        const float av = __bfloat162float(__float2bfloat16_rn(q < 8 ? v0[q & 7] : v1[q & 7]));
-                        const float bv = __shfl_xor_sync(0xFFFFFFFFu, av, 1);
-                        const float cv = __shfl_xor_sync(0xFFFFFFFFu, av, 8);
-                        const float dv = __shfl_xor_sync(0xFFFFFFFFu, av, 9);
-                        (q < 8 ? o0 : o1)[q & 7] = 0.25f * (((av + bv) + cv) + dv);
-                    }
+                    for (int q = 0; q < 8; ++q)
+                        pw[q] = pool_pair(w[q], __shfl_xor_sync(0xFFFFFFFFu, w[q], 1),
+                                          __shfl_xor_sync(0xFFFFFFFFu, w[q], 8), __shfl_xor_sync(0xFFFFFFFFu, w[q], 9));
                     if (valid && !(lane & 9) && co < p.Cout) {
-                        __nv_bfloat16* dst = p.pool_out +
-                                             ((size_t)((size_t)n_img * (p.H / 2) + py / 2) * (p.W / 2) + px / 2) * p.Cout + co;
-                        st_bf16x8(dst, o0);
-                        if (co + 8 < p.Cout) st_bf16x8(dst + 8, o1);
+                        __nv_bfloat16* dst =
+                            p.pool_out + (((size_t)n_img * (p.H / 2) + py / 2) * (p.W / 2) + px / 2) * p.Cout + co;
+                        if (pool_fast) store16(dst, pw);
+                        else store16_any(dst, pw, p.Cout - co);
                     }
                 }
+                if (!valid || co >= p.Cout) return;
+                const size_t at = pix * p.out_cstride + p.out_coff + co;
+                if (p.outf) { // FP32 output (a network head)
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        if (co + q < p.Cout) p.outf[at + q] = v[q];
+                    return;
+                }
+                if (p.mask) mask16(p.mask + pix * p.mask_cs + p.mask_co + co, w);
+                if (fast) store16(p.out + at, w);
+                else store16_any(p.out + at, w, p.Cout - co);
+            };
+#pragma unroll 1
+            for (int g = g0; g < g1; g += 2) { // two groups per TMEM wait
+                uint32_t r0[16], r1[16];
+                tc::tmem_ld16(col0 + 16u * (uint32_t)g, r0);
+                if (g + 1 < g1) tc::tmem_ld16(col0 + 16u * (uint32_t)(g + 1), r1);
+                tc::tmem_ld_wait();
+                finish(g, r0);
+                if (g + 1 < g1) finish(g + 1, r1);
             }
             tc::fence_before_sync();
             __syncwarp();
@@ -1436,7 +1404,7 @@ bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __
                KF_ERR_INVALID_ARGUMENT, "conv3x3: tensors must be 16-byte aligned (FP32 output: 4-byte)");
     KF_REQUIRE(!fuse || !fuse->pool_out || (((uintptr_t)fuse->pool_out & 15) == 0 && Cout % 8 == 0),
                KF_ERR_INVALID_ARGUMENT, "conv3x3: pooled output must be 16-byte aligned with Cout % 8 == 0");
-    KF_REQUIRE(!fuse || !fuse->mask || (((uintptr_t)fuse->mask & 15) == 0 && Cout % 8 == 0 && fuse->mask_cs % 8 == 0 &&
+    KF_REQUIRE(!fuse || !fuse->mask || (((uintptr_t)fuse->mask & 15) == 0 && Cout % 16 == 0 && fuse->mask_cs % 8 == 0 &&
                                         fuse->mask_co % 8 == 0 && Cin <= 288 && y && !fuse->pool_out),
                KF_ERR_INVALID_ARGUMENT, "conv3x3: mask layout");
     const int halo = conv3x3_halo(x, N, H, W, Cin, w, Cout_rows, bias, Cout, relu, y, y_cstride, y_coff, st, y_f32,
