@@ -258,6 +258,12 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
                           const WaveDev& w, uint32_t max_depth, uint64_t npaths, uint32_t chunk, bool profile) {
     cudaStream_t st = r->stream, st2 = profile ? r->stream : r->stream2;
     const bool dyn = r->cfg.traversal == 1, lit = w.lit != 0, fork = lit && !profile;
+    // a small launch without lights: whole paths in one kernel (the thread-per-ray setting, profiling
+    // and counting ask for the wavefront's kernels)
+    if (!lit && dyn && !profile && !r->count_traversal && npaths <= chunk && npaths <= kPathsMax) {
+        launch_paths(sv, fd, b, w, (uint32_t)npaths, max_depth, (uint32_t)r->num_sms, st);
+        return;
+    }
     const size_t clear = ((size_t)max_depth + 2) * (kCounterRow + kSlotRow) * sizeof(uint32_t);
     for (uint64_t start = 0; start < npaths; start += chunk) {
         const uint32_t n = (uint32_t)std::min<uint64_t>(chunk, npaths - start);

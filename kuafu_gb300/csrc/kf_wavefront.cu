@@ -493,40 +493,47 @@ __device__ __forceinline__ uint32_t tiled_pixel(uint32_t idx, uint32_t width, ui
     return (rb * kTileH + k / wb) * width + cb * kTileW + k % wb;
 }
 
+// Queue position j of a chunk: its path's view, pixel, sample and global number, with the pixels'
+// AOVs cleared (those of pixels that hit no material stay zero).
+// A pixel's samples are queued one after the other, so a warp's camera rays start in few
+// neighbouring pixels (+5 % over queuing each sample's pixels together); a band of kTileH rows
+// that lies in this chunk is queued in tile order.
 template <bool BATCH>
-__global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w, uint64_t chunk_start,
-                         uint32_t chunk_n) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; // queue position
-    if (j == 0) w.counters[0] = chunk_n;
-    if (j >= chunk_n) return;
+__device__ __forceinline__ View<BATCH> camera_path(const FrameDev* __restrict__ fp, const BatchDev& b, const WaveDev& w,
+                                                   uint64_t chunk_start, uint32_t chunk_n, uint32_t j, uint32_t& item,
+                                                   uint32_t& pix, uint32_t& sample, uint64_t& G) {
     uint64_t g = chunk_start + j;
     uint64_t view_start = 0; // global index of the view's first path
-    const FrameDev* fsel = fp;
-    uint32_t item = 0;
+    View<BATCH> v;
+    v.f = fp;
+    v.it = nullptr;
+    item = 0;
     if (BATCH) {
         item = find_item(b, g);
-        fsel = &b.items[item].f;
-        view_start = b.items[item].path_start;
+        v.it = b.items + item;
+        v.f = &v.it->f;
+        view_start = v.it->path_start;
     }
-    const FrameDev& f = *fsel;
+    const FrameDev& f = *v.f;
     g -= view_start;
-    // a pixel's samples are queued one after the other, so a warp's camera rays start in few
-    // neighbouring pixels (+5 % over queuing each sample's pixels together); a band of kTileH
-    // rows that lies in this chunk is queued in tile order
-    uint32_t sample, pix;
     split_path(g, f.pc.spp, pix, sample);
     const uint32_t band = f.width * kTileH, first = pix / band * band;
     const uint64_t b0 = view_start + (uint64_t)first * f.pc.spp;
     const uint64_t b1 = view_start + (uint64_t)min(first + band, f.npix) * f.pc.spp;
     if (b0 >= chunk_start && b1 <= chunk_start + chunk_n) pix = tiled_pixel(pix, f.width, f.height);
-    const uint32_t p = (uint32_t)(view_start + (uint64_t)pix * f.pc.spp + sample - chunk_start);
-    if (BATCH) w.path_item[p] = (uint16_t)item;
-    if (sample == 0) { // the AOVs of pixels that hit no material stay zero
-        (BATCH ? b.items[item].albedo : w.albedo)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        (BATCH ? b.items[item].normal : w.normal)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    v.g = (uint64_t)pix * f.pc.spp + sample;
+    G = view_start + v.g;
+    if (sample == 0) {
+        (BATCH ? v.it->albedo : w.albedo)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        (BATCH ? v.it->normal : w.normal)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+    return v;
+}
+
+// The camera ray of a pixel's sample (PathTrace.rgen:35-75).
+__device__ __forceinline__ void camera_ray(const FrameDev& f, uint32_t pix, const PathKey& pk, float (&origin)[4],
+                                           float (&dir)[4]) {
     const uint32_t px = pix % f.width, py = pix / f.width;
-    PathKey pk{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
     Stream js;
     js.init(0, KF_RNG_JITTER);
     const float jx = js.next(pk);
@@ -552,7 +559,6 @@ __global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
     const float tin[4] = {dxn, dyn, 1.0f, 1.0f};
     float target[4];
     mat4_mul(f.cam.proj_inv, tin, target);
-    float origin[4], dir[4];
     if (aperture > 0.0f) {
         const float oin[4] = {offx, offy, 0.0f, 1.0f};
         mat4_mul(f.cam.view_inv, oin, origin);
@@ -567,9 +573,26 @@ __global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
         const float din[4] = {nd.x, nd.y, nd.z, 0.0f};
         mat4_mul(f.cam.view_inv, din, dir);
     }
+}
+
+template <bool BATCH>
+__global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w, uint64_t chunk_start,
+                         uint32_t chunk_n) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; // queue position
+    if (j == 0) w.counters[0] = chunk_n;
+    if (j >= chunk_n) return;
+    uint32_t item, pix, sample;
+    uint64_t G;
+    const View<BATCH> v = camera_path<BATCH>(fp, b, w, chunk_start, chunk_n, j, item, pix, sample, G);
+    const FrameDev& f = *v.f;
+    const uint32_t p = (uint32_t)(G - chunk_start);
+    if (BATCH) w.path_item[p] = (uint16_t)item;
+    const PathKey pk{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
+    float origin[4], dir[4];
+    camera_ray(f, pix, pk, origin, dir);
     w.q_o[0][j] = make_float4(origin[0], origin[1], origin[2], __uint_as_float(p));
     w.q_d[0][j] = make_float4(dir[0], dir[1], dir[2], 1.0f);
-    w.radiance[chunk_start + p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    w.radiance[G] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
 
 // ---------------------------------------------------------------------------
@@ -925,27 +948,12 @@ __device__ bool light_sample(const SceneDev& s, const LS& ls, uint32_t slot, uin
 // that its warps shade hits only.
 // ---------------------------------------------------------------------------
 template <bool BATCH>
-__device__ __forceinline__ void miss_path(const SceneDev& s, const FrameDev* fp, const BatchDev& b, const WaveDev& w,
-                                          int cur, uint32_t depth, uint64_t chunk_start, uint32_t i) {
-    const float4 qd = w.q_d[cur][i];
-    const uint32_t p = __float_as_uint(w.q_o[cur][i].w);
-    const uint64_t g = chunk_start + p;
-    const View<BATCH> vw = view_of<BATCH>(fp, b, w, chunk_start, p);
+__device__ __forceinline__ v3 miss_emission(const SceneDev& s, const WaveDev& w, const View<BATCH>& vw, uint32_t depth,
+                                            v3 dir) {
     const FrameDev& f = *vw.f;
     const float4* env = BATCH ? vw.it->env : s.env;
     const uint32_t env_size = BATCH ? vw.it->env_size : s.env_size;
-    // camera rays carry weight 1 and find the radiance still zero
-    v3 wold = splat(1.0f), color = splat(0.0f);
-    if (depth > 0) {
-        const float2 wyz = w.q_w[cur][i];
-        wold = mk(qd.w, wyz.x, wyz.y);
-        color = xyz(w.radiance[g]);
-    }
-    const v3 emission = (f.pc.use_env_map && env) ? env_lookup(env, env_size, mk(qd.x, qd.y, qd.z))
-                                                   : ld3(f.pc.clear_color) * f.pc.clear_color[3];
-    color = color + emission * wold;
-    w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
-    if (depth == 0) { // sample 0 of the first bounce
+    if (depth == 0) { // AOVs of sample 0 of the first bounce
         uint32_t pix, sample;
         split_path(vw.g, f.pc.spp, pix, sample);
         if (sample == 0) {
@@ -954,6 +962,25 @@ __device__ __forceinline__ void miss_path(const SceneDev& s, const FrameDev* fp,
             if (aov_seg) aov_seg[pix] = make_uint4(kMiss, kMiss, kMiss, 0u);
         }
     }
+    return (f.pc.use_env_map && env) ? env_lookup(env, env_size, dir)
+                                      : ld3(f.pc.clear_color) * f.pc.clear_color[3];
+}
+template <bool BATCH>
+__device__ __forceinline__ void miss_path(const SceneDev& s, const FrameDev* fp, const BatchDev& b, const WaveDev& w,
+                                          int cur, uint32_t depth, uint64_t chunk_start, uint32_t i) {
+    const float4 qd = w.q_d[cur][i];
+    const uint32_t p = __float_as_uint(w.q_o[cur][i].w);
+    const uint64_t g = chunk_start + p;
+    const View<BATCH> vw = view_of<BATCH>(fp, b, w, chunk_start, p);
+    // camera rays carry weight 1 and find the radiance still zero
+    v3 wold = splat(1.0f), color = splat(0.0f);
+    if (depth > 0) {
+        const float2 wyz = w.q_w[cur][i];
+        wold = mk(qd.w, wyz.x, wyz.y);
+        color = xyz(w.radiance[g]);
+    }
+    color = color + miss_emission<BATCH>(s, w, vw, depth, mk(qd.x, qd.y, qd.z)) * wold;
+    w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
 }
 
 // One block of kMissThreads takes tiles of kMissThreads * kMissPer rays, kMissPer consecutive
@@ -1011,6 +1038,186 @@ __global__ void __launch_bounds__(kMissThreads) k_miss(SceneDev s, const FrameDe
     }
 }
 
+// One hit shaded (rchit:322-468, rgen:109-138): emission, or the PrincipledBSDF's sample, the
+// throughput after it and whether the path goes on. Writes the AOVs of sample 0 of the first bounce.
+struct HitShade {
+    bool emissive, is_mat, cont;
+    v3 worldPos, N, V, L;
+    v3 wnew, wcont; // throughput after the sample, and after Russian roulette; emissive: the radiance in wnew
+    Shading sh;
+};
+template <bool BATCH>
+__device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, const View<BATCH>& vw, uint32_t depth,
+                                          const PathKey& pk, uint32_t pix, uint32_t sample, v3 rayO, v3 rayD, v3 wold,
+                                          float4 hv, uint32_t prim, HitShade& o) {
+    const FrameDev& f = *vw.f;
+    float4* aov_albedo = BATCH ? vw.it->albedo : w.albedo;
+    float4* aov_normal = BATCH ? vw.it->normal : w.normal;
+    float* aov_depth = BATCH ? vw.it->depth : w.depth;
+    const uint32_t inst = __float_as_uint(hv.w); // never kMiss here
+    const InstanceRec* ip = s.inst + inst;
+    const float4 m0 = __ldg(&ip->w2o0), m1 = __ldg(&ip->w2o1), m2 = __ldg(&ip->w2o2);
+    const uint32_t geom = __ldg(&ip->geometry);
+    const uint4 gi = __ldg(s.geom + geom);
+    const uint32_t tri = gi.y + prim;
+    const uint32_t i0 = __ldg(s.indices + 3 * (size_t)tri + 0) + gi.x;
+    const uint32_t i1 = __ldg(s.indices + 3 * (size_t)tri + 1) + gi.x;
+    const uint32_t i2 = __ldg(s.indices + 3 * (size_t)tri + 2) + gi.x;
+    const float4 a0 = __ldg(s.verts + 3 * (size_t)i0), a1 = __ldg(s.verts + 3 * (size_t)i0 + 1),
+                 a2v = __ldg(s.verts + 3 * (size_t)i0 + 2);
+    const float4 b0 = __ldg(s.verts + 3 * (size_t)i1), b1 = __ldg(s.verts + 3 * (size_t)i1 + 1),
+                 b2 = __ldg(s.verts + 3 * (size_t)i1 + 2);
+    const float4 c0 = __ldg(s.verts + 3 * (size_t)i2), c1 = __ldg(s.verts + 3 * (size_t)i2 + 1),
+                 c2 = __ldg(s.verts + 3 * (size_t)i2 + 2);
+    const kf_material_gpu mat = s.materials[__ldg(s.matidx + tri)];
+    const v3 emission = ld3(mat.emission) * mat.emission[3];
+    if (emission != splat(0.0f)) {
+        // emissive hit ends the path (rchit:330-335)
+        o.emissive = true;
+        o.wnew = (ld3(mat.emission) * mat.emission[3]) * wold;
+    } else {
+        // getShadingData (rchit:66-98); unpackVertex: pos = d0.xyz,
+        // normal = (d0.w, d1.x, d1.y), uv = (d2.y, d2.z)
+        const float bx = 1.0f - hv.y - hv.z, by = hv.y, bz = hv.z;
+        const v3 n0 = mk(a0.w, a1.x, a1.y), n1 = mk(b0.w, b1.x, b1.y), n2 = mk(c0.w, c1.x, c1.y);
+        const v3 ln = n0 * bx + n1 * by + n2 * bz;
+        const v3 wn = mk(ln.x * m0.x + ln.y * m1.x + ln.z * m2.x, ln.x * m0.y + ln.y * m1.y + ln.z * m2.y,
+                         ln.x * m0.z + ln.y * m1.z + ln.z * m2.z);
+        o.N = normalize(wn);
+                            o.worldPos = rayO + rayD * hv.x;
+        const float uvx = a2v.y * bx + b2.y * by + c2.y * bz;
+        const float uvy = a2v.z * bx + b2.z * by + c2.z * bz;
+        // facing in object space: front when dir opposes (v1-v0)x(v2-v0)
+        bool backface;
+        {
+            const float odx = m0.x * rayD.x + m0.y * rayD.y + m0.z * rayD.z;
+            const float ody = m1.x * rayD.x + m1.y * rayD.y + m1.z * rayD.z;
+            const float odz = m2.x * rayD.x + m2.y * rayD.y + m2.z * rayD.z;
+            const v3 e1 = mk(b0.x, b0.y, b0.z) - mk(a0.x, a0.y, a0.z);
+            const v3 e2 = mk(c0.x, c0.y, c0.z) - mk(a0.x, a0.y, a0.z);
+            backface = dot(mk(odx, ody, odz), cross(e1, e2)) > 0.0f;
+        }
+        v3 baseColor = ld3(mat.diffuse);
+        if (mat.diffuse_tex >= 0) baseColor = texture_rgb(s, mat.diffuse_tex, uvx, uvy);
+        baseColor = baseColor / KF_REF_PI;
+        const float metallic =
+            mat.metallic_tex >= 0 ? texture_rgb(s, mat.metallic_tex, uvx, uvy).x : mat.metallic;
+        const float roughness =
+            mat.roughness_tex >= 0 ? texture_rgb(s, mat.roughness_tex, uvx, uvy).x : mat.roughness;
+        const float a2 = roughness * roughness;
+        const float transmission = mat.transmission_tex >= 0
+                                       ? texture_rgb(s, mat.transmission_tex, uvx, uvy).x
+                                       : mat.transmission;
+        const float fi = fmaxf(mat.ior, 1e-5f);
+        const float diffuse_weight =
+            (1.0f - clampf(metallic, 0.0f, 1.0f)) * (1.0f - clampf(transmission, 0.0f, 1.0f));
+        const float final_transmission =
+            clampf(transmission, 0.0f, 1.0f) * (1.0f - clampf(metallic, 0.0f, 1.0f));
+        const float specular_weight = (1.0f - final_transmission);
+        v3 weight = splat(0.0f);
+        o.V = normalize(-rayD);
+        const bool isInside = backface;
+        o.N = isInside ? -o.N : o.N;
+        o.L = splat(0.0f);
+        const float NdotV = dot(o.N, o.V);
+        const v3 diffuseColor = diffuse_weight * baseColor;
+        const v3 specularColor =
+            specular_weight * (baseColor * metallic + (mat.specular * 0.08f * splat(1.0f)) * (1.0f - metallic));
+        const v3 transmissionColor = transmission * baseColor;
+        const float diffuseLum = length(diffuseColor);
+        const float specularLum = length(specularColor);
+        float probDiffuse = diffuseLum / (diffuseLum + specularLum);
+        if (diffuseLum == 0.0f && specularLum == 0.0f) {
+            if (baseColor == splat(0.0f)) {
+                if (diffuse_weight == 1.0f) probDiffuse = 1.0f;
+                else if (diffuse_weight == 0.0f) probDiffuse = 0.0f;
+                else probDiffuse = 0.5f;
+            } else
+                probDiffuse = 0.0f;
+        } else {
+            probDiffuse *= specular_weight;
+        }
+        Stream bs;
+        bs.init(depth, KF_RNG_BSDF);
+        const bool chooseDiffuse = bs.next(pk) < probDiffuse;
+        if (chooseDiffuse) {
+            const float u0 = bs.next(pk), u1 = bs.next(pk);
+            o.L = cosineHemisphereSampling(u0, u1, o.N);
+            const float NdotL = clampf(dot(o.N, o.L), 0.0f, 1.0f);
+            weight = KF_REF_PI * diffuseColor * NdotL / probDiffuse;
+        }
+        if (!chooseDiffuse) {
+            if (final_transmission == 0.0f) {
+                const float u0 = bs.next(pk), u1 = bs.next(pk);
+                const v3 H = sampleGGX(u0, u1, a2, o.N);
+                const float HdotV = dot(H, o.V);
+                o.L = 2.0f * HdotV * H - o.V;
+                const float NoV = fmaxf(dot(o.N, o.V), 1e-7f);
+                const float NoL = dot(o.N, o.L);
+                const float NoH = fmaxf(dot(o.N, H), 1e-7f);
+                const float VoH = fmaxf(dot(o.V, H), 1e-7f);
+                if (NoL >= 0.0f) {
+                    const float G = GeometricShadowing(NoV, NoL, a2);
+                    const v3 F = schlickFresnel(specularColor, VoH);
+                    weight = KF_REF_PI * F * G * VoH / (NoH * NoV * (1.0f - probDiffuse));
+                } else
+                    weight = splat(0.0f);
+            } else {
+                const float ior = isInside ? 1.0f / fi : fi;
+                const float _dot = isInside ? NdotV * ior : NdotV;
+                const v3 refractedL = refract(-o.V, o.N, 1.0f / fi);
+                const float reflectProb = refractedL != splat(0.0f) ? Schlick(_dot, fi) : 1.0f;
+                if (bs.next(pk) >= reflectProb) {
+                    o.L = refractedL;
+                    weight = KF_REF_PI * transmissionColor / (1.0f - probDiffuse);
+                } else {
+                    o.L = reflect(-o.V, o.N);
+                    weight = KF_REF_PI * transmissionColor / (1.0f - probDiffuse);
+                }
+            }
+        }
+        o.sh.f = fi;
+        o.sh.a2 = a2;
+        o.sh.diffuseColor = diffuseColor;
+        o.sh.specularColor = specularColor;
+        o.sh.transmissionColor = transmissionColor;
+        o.sh.isInside = isInside;
+        // AOVs of sample 0, first bounce (rgen:114-117)
+        if (depth == 0 && sample == 0) {
+            aov_albedo[pix] = make_float4(baseColor.x, baseColor.y, baseColor.z, 1.0f);
+            aov_normal[pix] = make_float4(o.N.x, o.N.y, o.N.z, 1.0f);
+        }
+        // rgen:110  weight *= ray.weight
+        o.wnew = wold * weight;
+        if (o.wnew != splat(0.0f)) {
+            o.is_mat = true;
+            bool alive = true;
+            o.wcont = o.wnew;
+            if (f.pc.russian_roulette && depth >= f.pc.rr_min_bounces) { // rgen:124-138
+                const float pr = fmaxf(o.wnew.x, fmaxf(o.wnew.y, o.wnew.z));
+                Stream rs;
+                rs.init(depth, KF_RNG_RR);
+                const float rnd = rs.next(pk);
+                if (rnd > pr)
+                    alive = false;
+                else
+                    o.wcont = o.wnew * (1.0f / pr);
+            }
+            o.cont = alive && (depth + 1 <= f.pc.max_path_depth);
+        }
+    }
+    if (depth == 0 && sample == 0) {
+        aov_depth[pix] = hv.x;
+        uint4* aov_seg = BATCH ? vw.it->seg : w.seg;
+        if (aov_seg) {
+            const uint32_t gidx = __ldg(&s.inst[inst].geometry);
+                const uint32_t midx = __ldg(s.matidx + __ldg(s.geom + gidx).y + prim);
+            aov_seg[pix] = BATCH ? make_uint4(inst - vw.it->inst_base, gidx - vw.it->geom_base, midx, prim)
+                                 : make_uint4(inst, gidx, midx, prim);
+        }
+    }
+}
+
 // Blocks of the shading kernels (k_shade, k_nee); k_shade's block scan keeps one count per warp.
 constexpr uint32_t kShadeThreads = 128, kShadeWarps = kShadeThreads / 32;
 
@@ -1032,202 +1239,32 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
         const bool valid = base + lane < count;
         const uint32_t i = valid ? w.sel[base + lane] : 0u; // queue position of the ray
         uint32_t p = 0;
-        uint64_t g = 0;
-        PathKey pk;
-        bool is_mat = false, cont = false;
-        v3 worldPos = splat(0.0f), N = splat(0.0f), V = splat(0.0f), L = splat(0.0f);
-        v3 wnew = splat(0.0f), wcont = splat(0.0f);
-        Shading sh;
-        sh.f = 1.0f; sh.a2 = 0.0f;
-        sh.diffuseColor = sh.specularColor = sh.transmissionColor = splat(0.0f);
-        sh.isInside = false;
+        HitShade o;
+        o.emissive = o.is_mat = o.cont = false;
+        o.worldPos = o.N = o.V = o.L = o.wnew = o.wcont = splat(0.0f);
+        o.sh.f = 1.0f; o.sh.a2 = 0.0f;
+        o.sh.diffuseColor = o.sh.specularColor = o.sh.transmissionColor = splat(0.0f);
+        o.sh.isInside = false;
         View<BATCH> vw{fp, nullptr, 0};
         if (valid) {
             const float4 qo = w.q_o[cur][i], qd = w.q_d[cur][i];
             p = __float_as_uint(qo.w);
-            g = chunk_start + p; // radiance index (the batch's path space)
             vw = view_of<BATCH>(fp, b, w, chunk_start, p);
             const FrameDev& f = *vw.f;
             uint32_t sample, pix;
             split_path(vw.g, f.pc.spp, pix, sample);
-            pk = PathKey{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
-            float4* aov_albedo = BATCH ? vw.it->albedo : w.albedo;
-            float4* aov_normal = BATCH ? vw.it->normal : w.normal;
-            float* aov_depth = BATCH ? vw.it->depth : w.depth;
-            const float4 hv = w.hit[i];
-            const uint32_t inst = __float_as_uint(hv.w); // never kMiss here
+            const PathKey pk{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
             v3 wold = splat(1.0f); // camera rays
             if (depth > 0) {
                 const float2 wyz = w.q_w[cur][i];
                 wold = mk(qd.w, wyz.x, wyz.y);
             }
-            const v3 rayD = mk(qd.x, qd.y, qd.z);
-            {
-                const uint32_t prim = w.hit_prim[i];
-                const InstanceRec* ip = s.inst + inst;
-                const float4 m0 = __ldg(&ip->w2o0), m1 = __ldg(&ip->w2o1), m2 = __ldg(&ip->w2o2);
-                const uint32_t geom = __ldg(&ip->geometry);
-                const uint4 gi = __ldg(s.geom + geom);
-                const uint32_t tri = gi.y + prim;
-                const uint32_t i0 = __ldg(s.indices + 3 * (size_t)tri + 0) + gi.x;
-                const uint32_t i1 = __ldg(s.indices + 3 * (size_t)tri + 1) + gi.x;
-                const uint32_t i2 = __ldg(s.indices + 3 * (size_t)tri + 2) + gi.x;
-                const float4 a0 = __ldg(s.verts + 3 * (size_t)i0), a1 = __ldg(s.verts + 3 * (size_t)i0 + 1),
-                             a2v = __ldg(s.verts + 3 * (size_t)i0 + 2);
-                const float4 b0 = __ldg(s.verts + 3 * (size_t)i1), b1 = __ldg(s.verts + 3 * (size_t)i1 + 1),
-                             b2 = __ldg(s.verts + 3 * (size_t)i1 + 2);
-                const float4 c0 = __ldg(s.verts + 3 * (size_t)i2), c1 = __ldg(s.verts + 3 * (size_t)i2 + 1),
-                             c2 = __ldg(s.verts + 3 * (size_t)i2 + 2);
-                const kf_material_gpu mat = s.materials[__ldg(s.matidx + tri)];
-                const v3 emission = ld3(mat.emission) * mat.emission[3];
-                if (emission != splat(0.0f)) {
-                    // emissive hit ends the path (rchit:330-335)
-                    v3 color = depth > 0 ? xyz(w.radiance[g]) : splat(0.0f);
-                    color = color + (ld3(mat.emission) * mat.emission[3]) * wold;
-                    w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
-                } else {
-                    // getShadingData (rchit:66-98); unpackVertex: pos = d0.xyz,
-                    // normal = (d0.w, d1.x, d1.y), uv = (d2.y, d2.z)
-                    const float bx = 1.0f - hv.y - hv.z, by = hv.y, bz = hv.z;
-                    const v3 n0 = mk(a0.w, a1.x, a1.y), n1 = mk(b0.w, b1.x, b1.y), n2 = mk(c0.w, c1.x, c1.y);
-                    const v3 ln = n0 * bx + n1 * by + n2 * bz;
-                    const v3 wn = mk(ln.x * m0.x + ln.y * m1.x + ln.z * m2.x, ln.x * m0.y + ln.y * m1.y + ln.z * m2.y,
-                                     ln.x * m0.z + ln.y * m1.z + ln.z * m2.z);
-                    N = normalize(wn);
-                    const v3 rayO = mk(qo.x, qo.y, qo.z);
-                    worldPos = rayO + rayD * hv.x;
-                    const float uvx = a2v.y * bx + b2.y * by + c2.y * bz;
-                    const float uvy = a2v.z * bx + b2.z * by + c2.z * bz;
-                    // facing in object space: front when dir opposes (v1-v0)x(v2-v0)
-                    bool backface;
-                    {
-                        const float odx = m0.x * rayD.x + m0.y * rayD.y + m0.z * rayD.z;
-                        const float ody = m1.x * rayD.x + m1.y * rayD.y + m1.z * rayD.z;
-                        const float odz = m2.x * rayD.x + m2.y * rayD.y + m2.z * rayD.z;
-                        const v3 e1 = mk(b0.x, b0.y, b0.z) - mk(a0.x, a0.y, a0.z);
-                        const v3 e2 = mk(c0.x, c0.y, c0.z) - mk(a0.x, a0.y, a0.z);
-                        backface = dot(mk(odx, ody, odz), cross(e1, e2)) > 0.0f;
-                    }
-                    v3 baseColor = ld3(mat.diffuse);
-                    if (mat.diffuse_tex >= 0) baseColor = texture_rgb(s, mat.diffuse_tex, uvx, uvy);
-                    baseColor = baseColor / KF_REF_PI;
-                    const float metallic =
-                        mat.metallic_tex >= 0 ? texture_rgb(s, mat.metallic_tex, uvx, uvy).x : mat.metallic;
-                    const float roughness =
-                        mat.roughness_tex >= 0 ? texture_rgb(s, mat.roughness_tex, uvx, uvy).x : mat.roughness;
-                    const float a2 = roughness * roughness;
-                    const float transmission = mat.transmission_tex >= 0
-                                                   ? texture_rgb(s, mat.transmission_tex, uvx, uvy).x
-                                                   : mat.transmission;
-                    const float fi = fmaxf(mat.ior, 1e-5f);
-                    const float diffuse_weight =
-                        (1.0f - clampf(metallic, 0.0f, 1.0f)) * (1.0f - clampf(transmission, 0.0f, 1.0f));
-                    const float final_transmission =
-                        clampf(transmission, 0.0f, 1.0f) * (1.0f - clampf(metallic, 0.0f, 1.0f));
-                    const float specular_weight = (1.0f - final_transmission);
-                    v3 weight = splat(0.0f);
-                    V = normalize(-rayD);
-                    const bool isInside = backface;
-                    N = isInside ? -N : N;
-                    L = splat(0.0f);
-                    const float NdotV = dot(N, V);
-                    const v3 diffuseColor = diffuse_weight * baseColor;
-                    const v3 specularColor =
-                        specular_weight * (baseColor * metallic + (mat.specular * 0.08f * splat(1.0f)) * (1.0f - metallic));
-                    const v3 transmissionColor = transmission * baseColor;
-                    const float diffuseLum = length(diffuseColor);
-                    const float specularLum = length(specularColor);
-                    float probDiffuse = diffuseLum / (diffuseLum + specularLum);
-                    if (diffuseLum == 0.0f && specularLum == 0.0f) {
-                        if (baseColor == splat(0.0f)) {
-                            if (diffuse_weight == 1.0f) probDiffuse = 1.0f;
-                            else if (diffuse_weight == 0.0f) probDiffuse = 0.0f;
-                            else probDiffuse = 0.5f;
-                        } else
-                            probDiffuse = 0.0f;
-                    } else {
-                        probDiffuse *= specular_weight;
-                    }
-                    Stream bs;
-                    bs.init(depth, KF_RNG_BSDF);
-                    const bool chooseDiffuse = bs.next(pk) < probDiffuse;
-                    if (chooseDiffuse) {
-                        const float u0 = bs.next(pk), u1 = bs.next(pk);
-                        L = cosineHemisphereSampling(u0, u1, N);
-                        const float NdotL = clampf(dot(N, L), 0.0f, 1.0f);
-                        weight = KF_REF_PI * diffuseColor * NdotL / probDiffuse;
-                    }
-                    if (!chooseDiffuse) {
-                        if (final_transmission == 0.0f) {
-                            const float u0 = bs.next(pk), u1 = bs.next(pk);
-                            const v3 H = sampleGGX(u0, u1, a2, N);
-                            const float HdotV = dot(H, V);
-                            L = 2.0f * HdotV * H - V;
-                            const float NoV = fmaxf(dot(N, V), 1e-7f);
-                            const float NoL = dot(N, L);
-                            const float NoH = fmaxf(dot(N, H), 1e-7f);
-                            const float VoH = fmaxf(dot(V, H), 1e-7f);
-                            if (NoL >= 0.0f) {
-                                const float G = GeometricShadowing(NoV, NoL, a2);
-                                const v3 F = schlickFresnel(specularColor, VoH);
-                                weight = KF_REF_PI * F * G * VoH / (NoH * NoV * (1.0f - probDiffuse));
-                            } else
-                                weight = splat(0.0f);
-                        } else {
-                            const float ior = isInside ? 1.0f / fi : fi;
-                            const float _dot = isInside ? NdotV * ior : NdotV;
-                            const v3 refractedL = refract(-V, N, 1.0f / fi);
-                            const float reflectProb = refractedL != splat(0.0f) ? Schlick(_dot, fi) : 1.0f;
-                            if (bs.next(pk) >= reflectProb) {
-                                L = refractedL;
-                                weight = KF_REF_PI * transmissionColor / (1.0f - probDiffuse);
-                            } else {
-                                L = reflect(-V, N);
-                                weight = KF_REF_PI * transmissionColor / (1.0f - probDiffuse);
-                            }
-                        }
-                    }
-                    sh.f = fi;
-                    sh.a2 = a2;
-                    sh.diffuseColor = diffuseColor;
-                    sh.specularColor = specularColor;
-                    sh.transmissionColor = transmissionColor;
-                    sh.isInside = isInside;
-                    // AOVs of sample 0, first bounce (rgen:114-117)
-                    if (depth == 0 && sample == 0) {
-                        aov_albedo[pix] = make_float4(baseColor.x, baseColor.y, baseColor.z, 1.0f);
-                        aov_normal[pix] = make_float4(N.x, N.y, N.z, 1.0f);
-                    }
-                    // rgen:110  weight *= ray.weight
-                    wnew = wold * weight;
-                    if (wnew != splat(0.0f)) {
-                        is_mat = true;
-                        bool alive = true;
-                        wcont = wnew;
-                        if (f.pc.russian_roulette && depth >= f.pc.rr_min_bounces) { // rgen:124-138
-                            const float pr = fmaxf(wnew.x, fmaxf(wnew.y, wnew.z));
-                            Stream rs;
-                            rs.init(depth, KF_RNG_RR);
-                            const float rnd = rs.next(pk);
-                            if (rnd > pr)
-                                alive = false;
-                            else
-                                wcont = wnew * (1.0f / pr);
-                        }
-                        cont = alive && (depth + 1 <= f.pc.max_path_depth);
-                    }
-                }
-            }
-            if (depth == 0 && sample == 0) {
-                aov_depth[pix] = hv.x;
-                uint4* aov_seg = BATCH ? vw.it->seg : w.seg;
-                if (aov_seg) {
-                    const uint32_t gidx = __ldg(&s.inst[inst].geometry);
-                    const uint32_t prim = w.hit_prim[i];
-                    const uint32_t midx = __ldg(s.matidx + __ldg(s.geom + gidx).y + prim);
-                    aov_seg[pix] = BATCH ? make_uint4(inst - vw.it->inst_base, gidx - vw.it->geom_base, midx, prim)
-                                         : make_uint4(inst, gidx, midx, prim);
-                }
+            shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, mk(qo.x, qo.y, qo.z), mk(qd.x, qd.y, qd.z), wold, w.hit[i],
+                             w.hit_prim[i], o);
+            if (o.emissive) {
+                const uint64_t g = chunk_start + p; // radiance index (the batch's path space)
+                const v3 color = (depth > 0 ? xyz(w.radiance[g]) : splat(0.0f)) + o.wnew;
+                w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
             }
         }
         // what the light samples of this hit need, for k_nee (hit-list order, one array per
@@ -1237,23 +1274,23 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
             const uint32_t k = base + lane;
             if (BATCH) {
                 w.hit_item[k] = w.path_item[p];
-                is_mat = is_mat && vw.it->num_slots > 0;
+                o.is_mat = o.is_mat && vw.it->num_slots > 0;
             }
-            w.nee_w[k] = make_float4(wnew.x, wnew.y, wnew.z,
-                                     __uint_as_float(p | (is_mat ? 0x80000000u : 0u) | (sh.isInside ? 0x40000000u : 0u)));
-            if (is_mat) {
+            w.nee_w[k] = make_float4(o.wnew.x, o.wnew.y, o.wnew.z,
+                                     __uint_as_float(p | (o.is_mat ? 0x80000000u : 0u) | (o.sh.isInside ? 0x40000000u : 0u)));
+            if (o.is_mat) {
                 float4* rec = w.nee_in + k;
                 const size_t n = w.chunk_cap;
-                rec[0] = make_float4(worldPos.x, worldPos.y, worldPos.z, sh.f);
-                rec[n] = make_float4(N.x, N.y, N.z, sh.a2);
-                rec[2 * n] = make_float4(V.x, V.y, V.z, sh.diffuseColor.x);
-                rec[3 * n] = make_float4(sh.diffuseColor.y, sh.diffuseColor.z, sh.specularColor.x, sh.specularColor.y);
-                rec[4 * n] = make_float4(sh.specularColor.z, sh.transmissionColor.x, sh.transmissionColor.y,
-                                         sh.transmissionColor.z);
+                rec[0] = make_float4(o.worldPos.x, o.worldPos.y, o.worldPos.z, o.sh.f);
+                rec[n] = make_float4(o.N.x, o.N.y, o.N.z, o.sh.a2);
+                rec[2 * n] = make_float4(o.V.x, o.V.y, o.V.z, o.sh.diffuseColor.x);
+                rec[3 * n] = make_float4(o.sh.diffuseColor.y, o.sh.diffuseColor.z, o.sh.specularColor.x, o.sh.specularColor.y);
+                rec[4 * n] = make_float4(o.sh.specularColor.z, o.sh.transmissionColor.x, o.sh.transmissionColor.y,
+                                         o.sh.transmissionColor.z);
             }
         }
         // next rays in hit-list order: one atomic per block tile
-        const uint32_t m = __ballot_sync(kFull, cont);
+        const uint32_t m = __ballot_sync(kFull, o.cont);
         if (lane == 0) s_cnt[par][wid] = __popc(m);
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1264,12 +1301,84 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
         __syncthreads();
         uint32_t pos = s_base[par] + __popc(m & lanemask_lt());
         for (uint32_t k = 0; k < wid; ++k) pos += s_cnt[par][k];
-        if (cont) {
-            w.q_o[nxt][pos] = make_float4(worldPos.x, worldPos.y, worldPos.z, __uint_as_float(p));
-            w.q_d[nxt][pos] = make_float4(L.x, L.y, L.z, wcont.x);
-            w.q_w[nxt][pos] = make_float2(wcont.y, wcont.z);
+        if (o.cont) {
+            w.q_o[nxt][pos] = make_float4(o.worldPos.x, o.worldPos.y, o.worldPos.z, __uint_as_float(p));
+            w.q_d[nxt][pos] = make_float4(o.L.x, o.L.y, o.L.z, o.wcont.x);
+            w.q_w[nxt][pos] = make_float2(o.wcont.y, o.wcont.z);
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Whole paths of a small launch without lights to sample: one thread per path, from the camera
+// ray to its end, with the radiance in a register. Same steps and random streams per path as the
+// wavefront kernels, so the same results.
+//
+// Bound by the longest path's chain of dependent instructions. A wavefront of a few thousand rays
+// is, too, but pays it per bounce and kernel: three launches, three cold instruction caches and the
+// slowest ray of each bounce. Cornell rooms of depth 5, wavefront and whole paths: 256 paths 166 and
+// 61 us, 16 384 208 and 111, 65 536 256 and 148, 131 072 294 and 251, 262 144 367 and 444; rooms with
+// up to 300 spheres: 40 thousand paths 495 and 292, 163 thousand 650 and 432. Hence the limit
+// kPathsMax: past it the wavefront's compacted, sorted work wins back its launches.
+// Paths are spread over all warps the GPU holds (share lanes of each), as rays are in k_trace_dyn.
+// 4 blocks per SM: 3 the same, 5 slower by 6 % at 16 384 paths and faster by 8 % at 262 144, 8 by 38 %
+// slower and 5 % faster.
+// ---------------------------------------------------------------------------
+constexpr int kPathsBlocks = 4;
+template <bool BATCH>
+__global__ void __launch_bounds__(kThreadsTrace, kPathsBlocks) k_paths(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b,
+                                                             WaveDev w, uint32_t n, uint32_t max_depth, uint32_t share) {
+    __shared__ uint32_t s_stack[kSmemTrace];
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t j = (blockIdx.x * (kThreadsTrace / 32) + (threadIdx.x >> 5)) * share + lane;
+    uint32_t extension = 0;
+    if (lane < share && j < n) {
+        uint32_t item, pix, sample;
+        uint64_t G;
+        const View<BATCH> vw = camera_path<BATCH>(fp, b, w, 0, n, j, item, pix, sample, G);
+        const FrameDev& f = *vw.f;
+        const PathKey pk{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
+        float origin[4], dir[4];
+        camera_ray(f, pix, pk, origin, dir);
+        v3 O = mk(origin[0], origin[1], origin[2]), D = mk(dir[0], dir[1], dir[2]);
+        v3 weight = splat(1.0f), color = splat(0.0f);
+        TraceCounters cnt{0, 0, 0};
+#pragma unroll 1
+        for (uint32_t depth = 0;; ++depth) {
+            HitOut h;
+            AnyHitCtx ah;
+            ah.f = vw.f;
+            ah.g = vw.g;
+            ah.st.init(depth, KF_RNG_ANYHIT);
+            const bool hit = trace<false, false>(s, root_of<BATCH>(s, vw), s_stack, O.x, O.y, O.z, D.x, D.y, D.z,
+                                                 KF_T_MIN, KF_T_MAX, h, cnt, &ah);
+            if (depth == 0 && w.primary) {
+                kf_hit ph;
+                ph.t = h.t; ph.u = h.u; ph.v = h.v; ph.prim = h.prim;
+                ph.instance = (BATCH && hit) ? h.inst - vw.it->inst_base : h.inst; // scene-local id
+                ph.pad[0] = ph.pad[1] = ph.pad[2] = 0;
+                w.primary[G] = ph;
+            }
+            if (!hit) {
+                color = color + miss_emission<BATCH>(s, w, vw, depth, D) * weight;
+                break;
+            }
+            HitShade o;
+            o.emissive = o.cont = false;
+            shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, O, D, weight,
+                             make_float4(h.t, h.u, h.v, __uint_as_float(h.inst)), h.prim, o);
+            if (o.emissive) color = color + o.wnew;
+            if (!o.cont || depth == max_depth) break;
+            O = o.worldPos;
+            D = o.L;
+            weight = o.wcont;
+            ++extension;
+        }
+        w.radiance[G] = make_float4(color.x, color.y, color.z, 0.0f);
+    }
+    __syncwarp();
+    warp_add_stat(&w.stats[1], extension);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.stats[0], (unsigned long long)n);
 }
 
 // ---------------------------------------------------------------------------
@@ -1747,6 +1856,18 @@ void launch_raygen(const FrameDev* f, const BatchDev& b, const WaveDev& w, uint6
         k_raygen<true><<<grid, 256, 0, st>>>(f, b, w, chunk_start, chunk_n);
     else
         k_raygen<false><<<grid, 256, 0, st>>>(f, b, w, chunk_start, chunk_n);
+    KF_CUDA_CHECK(cudaGetLastError());
+}
+void launch_paths(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, uint32_t n,
+                  uint32_t max_depth, uint32_t sms, cudaStream_t st) {
+    const uint32_t warps = sms * kPathsBlocks * (kThreadsTrace / 32); // what the GPU holds
+    const uint32_t share = std::min(32u, (n + warps - 1) / warps);
+    const uint32_t block_paths = share * (kThreadsTrace / 32);
+    const dim3 grid((n + block_paths - 1) / block_paths);
+    if (b.items)
+        k_paths<true><<<grid, kThreadsTrace, 0, st>>>(s, f, b, w, n, max_depth, share);
+    else
+        k_paths<false><<<grid, kThreadsTrace, 0, st>>>(s, f, b, w, n, max_depth, share);
     KF_CUDA_CHECK(cudaGetLastError());
 }
 void launch_extend(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,

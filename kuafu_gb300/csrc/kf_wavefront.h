@@ -134,6 +134,12 @@ struct WaveDev {
 // takes its frame constants, TLAS root, lights and AOV targets from its item.
 void launch_raygen(const FrameDev* f, const BatchDev& b, const WaveDev& w, uint64_t chunk_start, uint32_t chunk_n,
                    cudaStream_t st);
+// Every path of a launch of n paths without lights to sample (w.lit == 0, no chunks), one thread
+// each: raygen to the end of the path. sms: SMs of the GPU.
+// The wavefront is faster from more than kPathsMax paths on.
+constexpr uint64_t kPathsMax = 163840;
+void launch_paths(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, uint32_t n,
+                  uint32_t max_depth, uint32_t sms, cudaStream_t st);
 void launch_extend(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
                    uint32_t depth, uint64_t chunk_start, uint32_t grid, bool count_mode, cudaStream_t st);
 // k_miss ends the paths whose ray missed and lists the others in w.sel; k_shade shades those.

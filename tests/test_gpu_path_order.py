@@ -2,7 +2,8 @@
 on which views of a batch have lights, or on lights that appear between batches.
 
 The reference is the same frame in one chunk (itself equal to the oracle in test_gpu_parity.py);
-every comparison is bit for bit.
+every comparison is bit for bit. Small frames without lights are rendered path by path in one
+kernel: cut into chunks they take the wavefront, so the two are compared here as well.
 """
 import numpy as np
 import pytest
@@ -46,6 +47,38 @@ def test_chunks_do_not_change_the_frame(lit, w, h, spp, chunk):
         w, h, spp, chunk = 5, 3, 2, 4
     for kind, a, b in zip(AOVS + ("frame",), _frame(lit, w, h, spp, 0), _frame(lit, w, h, spp, chunk)):
         assert _same(a, b), kind
+
+
+@pytest.mark.parametrize("w,h", [(512, 320), (641, 256), (163841, 1)])
+def test_whole_paths_and_wavefront_agree(w, h):
+    """Both sides of the limit between whole paths and the wavefront, with spheres (metal, glass and
+    mirror paths), Russian roulette, an environment map and textures: one launch against the
+    thread-per-ray wavefront."""
+    spp = 1  # 163840 paths, 164096, and 163841 of a one-row frame (nearly all of them miss)
+    rng = np.random.default_rng(3)
+    env = rng.random((6, 8, 8, 4), dtype=np.float32)
+    tex = api.createTexture(rng.integers(0, 256, (16, 16, 4), dtype=np.uint8))
+    out = []
+    for traversal in (1, 0):
+        cfg = scenes.icosphere_config(spp=spp, depth=6, count=64)
+        cfg.setTraversal(traversal)
+        cfg.setDebugOutputs(True)
+        with api.Kuafu(cfg) as r:
+            cam = scenes.icospheres(r, w, h, count=40, level=2, seed=1)
+            s = r.getScene()
+            s.removeLights()
+            s.setEnvironmentMap(env)
+            ground = api.createYZPlane(False, api.NiceMaterial(diffuseTex=tex, roughness=0.8))
+            s.submitGeometry(ground)
+            s.submitGeometryInstance(api.instance(ground, scenes.translate(0, 0, -22) @ scenes.rot_axis("y", -90) @
+                                                  scenes.scale(30.0, 30.0, 30.0)))
+            r.run()
+            st = r.stats()
+            out.append([_aov(r, cam, k) for k in AOVS] + [r.downloadLatestFrame(cam),
+                                                           np.array([st.rays_primary, st.rays_extension])])
+    for k, (a, b) in enumerate(zip(*out)):
+        assert _same(a, b), k
+    assert h == 1 or out[0][-1][1] > 1000
 
 
 def test_resolve_sample_counts():
