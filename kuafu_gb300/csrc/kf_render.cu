@@ -251,16 +251,18 @@ WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, bool lit
 // queue and writes visibility, the gather reads bounce d's hit records of the NEE and adds to
 // the radiance. What bounce d+1 writes of that (the NEE records, requests, contributions and
 // the radiance of the paths) is written by k_miss / k_shade, which wait for the gather (the
-// join). Counters are per bounce and cleared once per chunk, after the last gather of the
+// join). The tail (k_paths), which finishes the paths when few are left, reads and writes what
+// the gather does and sits behind the join, too. Counters are per bounce and cleared once per chunk, after the last gather of the
 // chunk before it. A launch without lights has no NEE: one stream, three kernels per bounce.
 // With `profile` everything runs on one stream with events around the kernel groups.
 static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* fd, const BatchDev& b,
                           const WaveDev& w, uint32_t max_depth, uint64_t npaths, uint32_t chunk, bool profile) {
     cudaStream_t st = r->stream, st2 = profile ? r->stream : r->stream2;
     const bool dyn = r->cfg.traversal == 1, lit = w.lit != 0, fork = lit && !profile;
-    // a small launch without lights: whole paths in one kernel (the thread-per-ray setting, profiling
-    // and counting ask for the wavefront's kernels)
-    if (!lit && dyn && !profile && !r->count_traversal && npaths <= chunk && npaths <= kPathsMax) {
+    // a small launch: whole paths in one kernel, and one for the last of a lit wavefront's paths (the
+    // thread-per-ray setting, profiling and counting ask for the wavefront's kernels)
+    const bool whole = dyn && !profile && !r->count_traversal;
+    if (whole && npaths <= chunk && npaths <= (lit ? kPathsMaxLit : kPathsMax)) {
         launch_paths(sv, fd, b, w, (uint32_t)npaths, max_depth, (uint32_t)r->num_sms, st);
         return;
     }
@@ -286,6 +288,8 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
                 launch_extend(sv, fd, b, w, cur, depth, start, r->grid_extend, r->count_traversal, st);
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[1], st));
             if (fork && depth > 0) KF_CUDA_CHECK(cudaStreamWaitEvent(st, r->ev_join, 0)); // previous gather done
+            if (whole && lit && depth > 0)
+                launch_tail(sv, fd, b, w, cur, depth, start, max_depth, (uint32_t)r->num_sms, st);
             launch_miss(sv, fd, b, w, cur, depth, start, grid_shade, st);
             launch_shade(sv, fd, b, w, cur, depth, start, grid_shade, st);
             if (lit) launch_nee(sv, fd, b, w, depth, start, grid_shade, st);

@@ -1310,75 +1310,165 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
 }
 
 // ---------------------------------------------------------------------------
-// Whole paths of a small launch without lights to sample: one thread per path, from the camera
-// ray to its end, with the radiance in a register. Same steps and random streams per path as the
-// wavefront kernels, so the same results.
+// Whole paths: the paths of a small launch from the camera ray to the end, with the radiance in a
+// register, or (QUEUE) the rest of the paths a lit wavefront still has at some bounce. Same steps
+// and random streams per path as the wavefront kernels, so the same results. With lights, up to
+// kPathsLanes lanes share a path: they run the same steps, take a light slot each (sample and
+// shadow ray) and sum the slots in order; the lanes of a path, and paths to a warp, are as few as
+// keep every path on the GPU at once.
 //
 // Bound by the longest path's chain of dependent instructions. A wavefront of a few thousand rays
-// is, too, but pays it per bounce and kernel: three launches, three cold instruction caches and the
-// slowest ray of each bounce. Cornell rooms of depth 5, wavefront and whole paths: 256 paths 166 and
-// 61 us, 16 384 208 and 111, 65 536 256 and 148, 131 072 294 and 251, 262 144 367 and 444; rooms with
-// up to 300 spheres: 40 thousand paths 495 and 292, 163 thousand 650 and 432. Hence the limit
-// kPathsMax: past it the wavefront's compacted, sorted work wins back its launches.
-// Paths are spread over all warps the GPU holds (share lanes of each), as rays are in k_trace_dyn.
-// 4 blocks per SM: 3 the same, 5 slower by 6 % at 16 384 paths and faster by 8 % at 262 144, 8 by 38 %
-// slower and 5 % faster.
+// is, too, but pays it per bounce and kernel: three to six launches, as many cold instruction
+// caches and the slowest ray of each bounce. Cornell rooms of depth 5, wavefront and whole paths:
+// 256 paths 166 and 61 us, 16 384 208 and 111, 65 536 256 and 148, 131 072 294 and 251, 262 144 367
+// and 444; rooms with up to 300 spheres: 40 thousand paths 495 and 292, 163 thousand 650 and 432.
+// Hence the limit kPathsMax: past it the wavefront's compacted, sorted work wins back its launches.
+// With seven lights: 256 spheres 4096 paths 430 and 295, 16 384 550 and 548, 23 040 630 and 757; 64
+// spheres 23 040 350 and 287, 36 864 354 and 307: kPathsMaxLit.
+// The tail of a lit wavefront is taken from kTailMax rays on down: 641 x 363 pixels among moving
+// spheres 916 -> 850 us, the active-light rig 6.32 -> 6.14 ms, 12 thousand paths 357 -> 290; with
+// 4096 or 16 384 the same, from 20 thousand on slower again. (Without lights it gains nothing.)
+// 4 blocks per SM: 3 the same, 5 slower by 6 % at 16 384 unlit paths and faster by 8 % at 262 144, 8
+// by 38 % slower and 5 % faster.
 // ---------------------------------------------------------------------------
 constexpr int kPathsBlocks = 4;
-template <bool BATCH>
-__global__ void __launch_bounds__(kThreadsTrace, kPathsBlocks) k_paths(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b,
-                                                             WaveDev w, uint32_t n, uint32_t max_depth, uint32_t share) {
+constexpr uint32_t kTailMax = 12288, kPathsLanes = 8;
+template <bool BATCH, bool LIT, bool QUEUE>
+__global__ void __launch_bounds__(kThreadsTrace, kPathsBlocks)
+    k_paths(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w, int cur, uint32_t depth0,
+            uint64_t chunk_start, uint32_t n_paths, uint32_t max_depth) {
     __shared__ uint32_t s_stack[kSmemTrace];
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t j = (blockIdx.x * (kThreadsTrace / 32) + (threadIdx.x >> 5)) * share + lane;
-    uint32_t extension = 0;
-    if (lane < share && j < n) {
-        uint32_t item, pix, sample;
-        uint64_t G;
-        const View<BATCH> vw = camera_path<BATCH>(fp, b, w, 0, n, j, item, pix, sample, G);
-        const FrameDev& f = *vw.f;
-        const PathKey pk{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
-        float origin[4], dir[4];
-        camera_ray(f, pix, pk, origin, dir);
-        v3 O = mk(origin[0], origin[1], origin[2]), D = mk(dir[0], dir[1], dir[2]);
-        v3 weight = splat(1.0f), color = splat(0.0f);
-        TraceCounters cnt{0, 0, 0};
-#pragma unroll 1
-        for (uint32_t depth = 0;; ++depth) {
+    uint32_t* ctr = w.counters + depth0 * kCounterRow;
+    const uint32_t n = QUEUE ? ctr[0] : n_paths;
+    if (QUEUE && (n == 0 || n > kTailMax)) return;
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * (kThreadsTrace / 32);
+    // lanes per path: a power of two, as many as the light slots use while every path has its lanes
+    uint32_t L = 1;
+    if (LIT)
+        while (L < kPathsLanes && L < w.nslot && n * 2 * L <= warps * 32) L *= 2;
+    const uint32_t sub = lane % L, per_warp = min(32 / L, (n + warps - 1) / warps);
+    const uint32_t gmask = (L == 32 ? kFull : (1u << L) - 1u) << (lane - sub);
+    uint32_t extension = 0, shadow = 0;
+    if (lane / L < per_warp)
+        for (uint32_t j = (blockIdx.x * (kThreadsTrace / 32) + (threadIdx.x >> 5)) * per_warp + lane / L; j < n;
+             j += warps * per_warp) {
+            uint32_t pix, sample;
+            uint64_t G;
+            View<BATCH> vw;
+            v3 O, D, weight = splat(1.0f), color = splat(0.0f);
             HitOut h;
-            AnyHitCtx ah;
-            ah.f = vw.f;
-            ah.g = vw.g;
-            ah.st.init(depth, KF_RNG_ANYHIT);
-            const bool hit = trace<false, false>(s, root_of<BATCH>(s, vw), s_stack, O.x, O.y, O.z, D.x, D.y, D.z,
-                                                 KF_T_MIN, KF_T_MAX, h, cnt, &ah);
-            if (depth == 0 && w.primary) {
-                kf_hit ph;
-                ph.t = h.t; ph.u = h.u; ph.v = h.v; ph.prim = h.prim;
-                ph.instance = (BATCH && hit) ? h.inst - vw.it->inst_base : h.inst; // scene-local id
-                ph.pad[0] = ph.pad[1] = ph.pad[2] = 0;
-                w.primary[G] = ph;
+            PathKey pk;
+            if (QUEUE) {
+                const float4 qo = w.q_o[cur][j], qd = w.q_d[cur][j], hv = w.hit[j];
+                const float2 wyz = w.q_w[cur][j];
+                G = chunk_start + __float_as_uint(qo.w);
+                vw = view_of<BATCH>(fp, b, w, chunk_start, __float_as_uint(qo.w));
+                split_path(vw.g, vw.f->pc.spp, pix, sample);
+                O = mk(qo.x, qo.y, qo.z);
+                D = mk(qd.x, qd.y, qd.z);
+                weight = mk(qd.w, wyz.x, wyz.y);
+                color = xyz(w.radiance[G]);
+                h = HitOut{hv.x, hv.y, hv.z, __float_as_uint(hv.w), w.hit_prim[j]};
+                pk = PathKey{make_uint2(vw.f->seed ^ pix, vw.f->camera_index), sample, vw.f->frame};
+            } else {
+                uint32_t item;
+                vw = camera_path<BATCH>(fp, b, w, 0, n, j, item, pix, sample, G);
+                pk = PathKey{make_uint2(vw.f->seed ^ pix, vw.f->camera_index), sample, vw.f->frame};
+                float origin[4], dir[4];
+                camera_ray(*vw.f, pix, pk, origin, dir);
+                O = mk(origin[0], origin[1], origin[2]);
+                D = mk(dir[0], dir[1], dir[2]);
             }
-            if (!hit) {
-                color = color + miss_emission<BATCH>(s, w, vw, depth, D) * weight;
-                break;
+            TraceCounters cnt{0, 0, 0};
+#pragma unroll 1
+            for (uint32_t depth = depth0;; ++depth) {
+                if (!QUEUE || depth != depth0) {
+                    AnyHitCtx ah;
+                    ah.f = vw.f;
+                    ah.g = vw.g;
+                    ah.st.init(depth, KF_RNG_ANYHIT);
+                    trace<false, false>(s, root_of<BATCH>(s, vw), s_stack, O.x, O.y, O.z, D.x, D.y, D.z, KF_T_MIN,
+                                        KF_T_MAX, h, cnt, &ah);
+                    if (!QUEUE && depth == 0 && w.primary && sub == 0) {
+                        kf_hit ph;
+                        ph.t = h.t; ph.u = h.u; ph.v = h.v; ph.prim = h.prim;
+                        ph.instance = (BATCH && h.inst != kMiss) ? h.inst - vw.it->inst_base : h.inst; // scene-local id
+                        ph.pad[0] = ph.pad[1] = ph.pad[2] = 0;
+                        w.primary[G] = ph;
+                    }
+                }
+                if (h.inst == kMiss) {
+                    color = color + miss_emission<BATCH>(s, w, vw, depth, D) * weight;
+                    break;
+                }
+                HitShade o;
+                o.emissive = o.is_mat = o.cont = false;
+                shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, O, D, weight,
+                                 make_float4(h.t, h.u, h.v, __uint_as_float(h.inst)), h.prim, o);
+                if (o.emissive) color = color + o.wnew;
+                if (LIT && o.is_mat) {
+                    // the path's lanes take a light slot each, then all sum them in slot order (k_nee,
+                    // k_trace_dyn<shadow> and k_gather of the wavefront)
+                    const uint32_t slots = BATCH ? vw.it->num_slots : s.num_slots;
+                    v3 Ld = splat(0.0f), Lp = splat(0.0f), La = splat(0.0f);
+                    bool any = false;
+                    for (uint32_t j0 = 0; j0 < slots; j0 += L) {
+                        v3 Ls, c = splat(0.0f);
+                        float tmax;
+                        uint32_t state = 0; // 1: a shadow ray was traced, 2: unoccluded
+                        if (j0 + sub < slots) {
+                            bool emit;
+                            if (BATCH)
+                                emit = light_sample(s, ItemLights{vw.it}, j0 + sub, depth, pk, o.worldPos, o.N, o.V, o.sh,
+                                                    Ls, tmax, c);
+                            else
+                                emit = light_sample(s, SceneLights{s}, j0 + sub, depth, pk, o.worldPos, o.N, o.V, o.sh,
+                                                    Ls, tmax, c);
+                            if (emit) {
+                                HitOut sh;
+                                ++shadow;
+                                state = trace<true, false>(s, root_of<BATCH>(s, vw), s_stack, o.worldPos.x, o.worldPos.y,
+                                                           o.worldPos.z, Ls.x, Ls.y, Ls.z, KF_T_MIN, tmax, sh, cnt)
+                                            ? 1u
+                                            : 3u;
+                            }
+                        }
+                        __syncwarp(gmask);
+                        for (uint32_t q = 0; q < L && j0 + q < slots; ++q) {
+                            const uint32_t st = __shfl_sync(gmask, state, q, L);
+                            const v3 cq = mk(__shfl_sync(gmask, c.x, q, L), __shfl_sync(gmask, c.y, q, L),
+                                             __shfl_sync(gmask, c.z, q, L));
+                            any |= st != 0;
+                            if (!(st & 2u)) continue;
+                            const uint32_t grp = BATCH ? vw.it->slot_group[j0 + q] : s.slot_group[j0 + q];
+                            if (grp == 0) Ld = cq;
+                            else if (grp == 1) Lp = Lp + cq;
+                            else La = La + cq;
+                        }
+                    }
+                    if (any) color = color + ((Ld + Lp) + La) * o.wnew;
+                }
+                if (!o.cont || depth == max_depth) break;
+                O = o.worldPos;
+                D = o.L;
+                weight = o.wcont;
+                if (sub == 0) ++extension;
             }
-            HitShade o;
-            o.emissive = o.cont = false;
-            shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, O, D, weight,
-                             make_float4(h.t, h.u, h.v, __uint_as_float(h.inst)), h.prim, o);
-            if (o.emissive) color = color + o.wnew;
-            if (!o.cont || depth == max_depth) break;
-            O = o.worldPos;
-            D = o.L;
-            weight = o.wcont;
-            ++extension;
+            if (sub == 0) w.radiance[G] = make_float4(color.x, color.y, color.z, 0.0f);
         }
-        w.radiance[G] = make_float4(color.x, color.y, color.z, 0.0f);
-    }
     __syncwarp();
     warp_add_stat(&w.stats[1], extension);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.stats[0], (unsigned long long)n);
+    if (LIT) warp_add_stat(&w.stats[2], shadow);
+    if (!QUEUE) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.stats[0], (unsigned long long)n);
+    } else {
+        // the last block empties the bounce's queue: the kernels behind find nothing to do
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(ctr + 4, 1u) == gridDim.x - 1) ctr[0] = 0;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1858,17 +1948,26 @@ void launch_raygen(const FrameDev* f, const BatchDev& b, const WaveDev& w, uint6
         k_raygen<false><<<grid, 256, 0, st>>>(f, b, w, chunk_start, chunk_n);
     KF_CUDA_CHECK(cudaGetLastError());
 }
+template <bool BATCH, bool QUEUE>
+static void paths_run(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur, uint32_t depth0,
+                      uint64_t chunk_start, uint32_t n, uint32_t max_depth, uint32_t grid, cudaStream_t st) {
+    if (w.lit)
+        k_paths<BATCH, true, QUEUE><<<grid, kThreadsTrace, 0, st>>>(s, f, b, w, cur, depth0, chunk_start, n, max_depth);
+    else
+        k_paths<BATCH, false, QUEUE><<<grid, kThreadsTrace, 0, st>>>(s, f, b, w, cur, depth0, chunk_start, n, max_depth);
+    KF_CUDA_CHECK(cudaGetLastError());
+}
 void launch_paths(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, uint32_t n,
                   uint32_t max_depth, uint32_t sms, cudaStream_t st) {
-    const uint32_t warps = sms * kPathsBlocks * (kThreadsTrace / 32); // what the GPU holds
-    const uint32_t share = std::min(32u, (n + warps - 1) / warps);
-    const uint32_t block_paths = share * (kThreadsTrace / 32);
-    const dim3 grid((n + block_paths - 1) / block_paths);
-    if (b.items)
-        k_paths<true><<<grid, kThreadsTrace, 0, st>>>(s, f, b, w, n, max_depth, share);
-    else
-        k_paths<false><<<grid, kThreadsTrace, 0, st>>>(s, f, b, w, n, max_depth, share);
-    KF_CUDA_CHECK(cudaGetLastError());
+    const uint32_t grid = std::max(1u, std::min(sms * kPathsBlocks, n)); // what the GPU holds
+    if (b.items) paths_run<true, false>(s, f, b, w, 0, 0, 0, n, max_depth, grid, st);
+    else paths_run<false, false>(s, f, b, w, 0, 0, 0, n, max_depth, grid, st);
+}
+void launch_tail(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur, uint32_t depth,
+                 uint64_t chunk_start, uint32_t max_depth, uint32_t sms, cudaStream_t st) {
+    const uint32_t grid = sms * kPathsBlocks;
+    if (b.items) paths_run<true, true>(s, f, b, w, cur, depth, chunk_start, 0, max_depth, grid, st);
+    else paths_run<false, true>(s, f, b, w, cur, depth, chunk_start, 0, max_depth, grid, st);
 }
 void launch_extend(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
                    uint32_t depth, uint64_t chunk_start, uint32_t grid, bool count_mode, cudaStream_t st) {

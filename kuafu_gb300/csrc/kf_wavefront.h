@@ -88,7 +88,8 @@ struct BatchDev {
 
 // Counters of one bounce, cleared once per chunk for all its bounces: a row per depth, so that
 // no launch waits for a clear between bounces.
-constexpr int kCounterRow = 8; // [0] rays queued, [1] rays that hit, [2] / [3] fetch cursors (closest / shadow)
+constexpr int kCounterRow = 8; // [0] rays queued, [1] rays that hit, [2] / [3] fetch cursors (closest / shadow),
+                               // [4] finished blocks of k_paths
 constexpr int kSlotRow = 64;   // shadow rays queued per light slot
 
 // Per-chunk wavefront state. A path's number within its view is pixel * spp + sample: a pixel's
@@ -134,12 +135,16 @@ struct WaveDev {
 // takes its frame constants, TLAS root, lights and AOV targets from its item.
 void launch_raygen(const FrameDev* f, const BatchDev& b, const WaveDev& w, uint64_t chunk_start, uint32_t chunk_n,
                    cudaStream_t st);
-// Every path of a launch of n paths without lights to sample (w.lit == 0, no chunks), one thread
-// each: raygen to the end of the path. sms: SMs of the GPU.
-// The wavefront is faster from more than kPathsMax paths on.
-constexpr uint64_t kPathsMax = 163840;
+// Every path of a launch of n paths (one chunk), from raygen to the end of the path. sms: SMs of
+// the GPU. The wavefront is faster from more than kPathsMax paths on, or kPathsMaxLit where some
+// view has lights to sample.
+constexpr uint64_t kPathsMax = 163840, kPathsMaxLit = 16384;
 void launch_paths(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, uint32_t n,
                   uint32_t max_depth, uint32_t sms, cudaStream_t st);
+// The rest of every path of bounce `depth` of a chunk (its closest hits found, the NEE of the
+// bounces before gathered), if there are few enough of them; the bounce's queue is then empty.
+void launch_tail(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur, uint32_t depth,
+                 uint64_t chunk_start, uint32_t max_depth, uint32_t sms, cudaStream_t st);
 void launch_extend(const SceneDev& s, const FrameDev* f, const BatchDev& b, const WaveDev& w, int cur,
                    uint32_t depth, uint64_t chunk_start, uint32_t grid, bool count_mode, cudaStream_t st);
 // k_miss ends the paths whose ray missed and lists the others in w.sel; k_shade shades those.

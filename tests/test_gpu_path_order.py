@@ -81,6 +81,39 @@ def test_whole_paths_and_wavefront_agree(w, h):
     assert h == 1 or out[0][-1][1] > 1000
 
 
+# lights of every kind, more slots than lanes of a path, and none that emit; a small frame (whole
+# paths), one just past that limit and larger ones whose tail is finished path by path, in one and
+# several chunks
+@pytest.mark.parametrize("w,h,spp,chunk,points", [(64, 64, 4, 0, 4), (31, 17, 3, 0, 11), (16385, 1, 1, 0, 1),
+                                                  (200, 150, 2, 0, 4), (200, 150, 2, 17000, 11), (8, 8, 1, 0, 0)])
+def test_whole_paths_with_lights(w, h, spp, chunk, points):
+    out = []
+    for traversal in (1, 0):
+        cfg = scenes.icosphere_config(spp=spp, depth=7, count=64)
+        cfg.setTraversal(traversal)
+        cfg.setDebugOutputs(True)
+        if chunk:
+            cfg.setMaxPathsInFlight(chunk)
+        with api.Kuafu(cfg) as r:
+            cam = scenes.icospheres(r, w, h, count=48, level=2, seed=2)
+            s = r.getScene()
+            s.removeLights()
+            for k in range(points):
+                s.addPointLight(api.PointLight(position=(-10.0 + 3 * k, 5.0 - k, 4.0 + k), color=(1.0, 0.5 + 0.04 * k, 0.3),
+                                               radius=0.4 * (k % 2), strength=200.0))
+            s.setDirectionalLight(api.DirectionalLight(direction=(-1.0, 0.2, -1.0), strength=1.0, softness=0.05))
+            s.addActiveLight(api.ActiveLight(viewMat=scenes.look_at_view((0.0, 3.0, 25.0), (0, 0, 0), (0, 1, 0)),
+                                             fov=1.0, strength=500.0, softness=0.1))
+            r.run()
+            st = r.stats()
+            out.append([_aov(r, cam, k) for k in AOVS] + [np.array([st.rays_primary, st.rays_extension, st.rays_shadow])])
+            if not chunk:
+                r.runBatch([(s, cam, spp)])
+                out[-1].append(_aov(r, cam, N.KF_AOV_PATH_RADIANCE))
+    for k, (a, b) in enumerate(zip(*out)):
+        assert _same(a, b), k
+
+
 def test_resolve_sample_counts():
     """Sample counts around the resolve's groups of 8: the mean of the downloaded paths, in order."""
     for spp in (1, 3, 4, 8, 9, 17):
