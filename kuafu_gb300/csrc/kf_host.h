@@ -163,7 +163,7 @@ struct BatchState {
 struct WaveBuffers {
     kf::DeviceBuffer<float4> q_o0, q_o1, q_d0, q_d1, hit, nee_w, nee_in, contrib, sq_o, sq_d;
     kf::DeviceBuffer<float2> q_w0, q_w1;
-    kf::DeviceBuffer<uint32_t> counters, hit_prim, sel, scount;
+    kf::DeviceBuffer<uint32_t> counters, hit_inst, sel, scount;
     kf::DeviceBuffer<uint64_t> req;
     kf::DeviceBuffer<uint8_t> vis;
     kf::DeviceBuffer<float4> radiance;      // per path of the frame

@@ -184,7 +184,7 @@ void ensure_wave(kf_renderer_s* r, uint32_t chunk, uint32_t slots, uint64_t npat
         W.q_o0.resize(chunk, st); W.q_o1.resize(chunk, st);
         W.q_d0.resize(chunk, st); W.q_d1.resize(chunk, st);
         W.q_w0.resize(chunk, st); W.q_w1.resize(chunk, st);
-        W.hit.resize(chunk, st); W.hit_prim.resize(chunk, st); W.sel.resize(chunk, st);
+        W.hit.resize(chunk, st); W.hit_inst.resize(chunk, st); W.sel.resize(chunk, st);
         W.nee_w.resize(chunk, st); W.nee_in.resize((size_t)5 * chunk, st);
         W.req.resize(chunk, st);
         W.chunk_cap = chunk;
@@ -220,7 +220,7 @@ WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, bool lit
     w.q_w[0] = W.q_w0.ptr; w.q_w[1] = W.q_w1.ptr;
     w.counters = W.counters.ptr;
     w.hit = W.hit.ptr;
-    w.hit_prim = W.hit_prim.ptr;
+    w.hit_inst = W.hit_inst.ptr;
     w.sel = W.sel.ptr;
     w.scount = W.counters.ptr + ((size_t)max_depth + 2) * kCounterRow;
     w.lit = lit ? 1u : 0u;

@@ -617,8 +617,8 @@ __global__ void __launch_bounds__(128) k_extend(SceneDev s, const FrameDev* __re
         ah.st.init(depth, KF_RNG_ANYHIT);
         trace<false, COUNT>(s, root_of<BATCH>(s, v), s_stack, o.x, o.y, o.z, d.x, d.y, d.z, KF_T_MIN, KF_T_MAX, h,
                             cnt, &ah);
-        w.hit[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.inst));
-        w.hit_prim[i] = h.prim;
+        w.hit[i] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
+        w.hit_inst[i] = h.inst;
         if (depth == 0 && w.primary) {
             const uint32_t p = __float_as_uint(o.w);
             kf_hit ph;
@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(kMissThreads) k_miss(SceneDev s, const FrameDe
         for (uint32_t q = 0; q < kMissPer; ++q) {
             const uint32_t i = base + threadIdx.x * per + q;
             if (q < per && i < count) {
-                if (__float_as_uint(w.hit[i].w) == kMiss) {
+                if (w.hit_inst[i] == kMiss) {
                     missm |= 1u << q;
                 } else {
                     hitm |= 1u << q;
@@ -1049,12 +1049,12 @@ struct HitShade {
 template <bool BATCH>
 __device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, const View<BATCH>& vw, uint32_t depth,
                                           const PathKey& pk, uint32_t pix, uint32_t sample, v3 rayO, v3 rayD, v3 wold,
-                                          float4 hv, uint32_t prim, HitShade& o) {
+                                          float4 hv, uint32_t inst, HitShade& o) {
     const FrameDev& f = *vw.f;
     float4* aov_albedo = BATCH ? vw.it->albedo : w.albedo;
     float4* aov_normal = BATCH ? vw.it->normal : w.normal;
     float* aov_depth = BATCH ? vw.it->depth : w.depth;
-    const uint32_t inst = __float_as_uint(hv.w); // never kMiss here
+    const uint32_t prim = __float_as_uint(hv.w);
     const InstanceRec* ip = s.inst + inst;
     const float4 m0 = __ldg(&ip->w2o0), m1 = __ldg(&ip->w2o1), m2 = __ldg(&ip->w2o2);
     const uint32_t geom = __ldg(&ip->geometry);
@@ -1260,7 +1260,7 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
                 wold = mk(qd.w, wyz.x, wyz.y);
             }
             shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, mk(qo.x, qo.y, qo.z), mk(qd.x, qd.y, qd.z), wold, w.hit[i],
-                             w.hit_prim[i], o);
+                             w.hit_inst[i], o);
             if (o.emissive) {
                 const uint64_t g = chunk_start + p; // radiance index (the batch's path space)
                 const v3 color = (depth > 0 ? xyz(w.radiance[g]) : splat(0.0f)) + o.wnew;
@@ -1368,7 +1368,7 @@ __global__ void __launch_bounds__(kThreadsTrace, kPathsBlocks)
                 D = mk(qd.x, qd.y, qd.z);
                 weight = mk(qd.w, wyz.x, wyz.y);
                 color = xyz(w.radiance[G]);
-                h = HitOut{hv.x, hv.y, hv.z, __float_as_uint(hv.w), w.hit_prim[j]};
+                h = HitOut{hv.x, hv.y, hv.z, w.hit_inst[j], __float_as_uint(hv.w)};
                 pk = PathKey{make_uint2(vw.f->seed ^ pix, vw.f->camera_index), sample, vw.f->frame};
             } else {
                 uint32_t item;
@@ -1404,7 +1404,7 @@ __global__ void __launch_bounds__(kThreadsTrace, kPathsBlocks)
                 HitShade o;
                 o.emissive = o.is_mat = o.cont = false;
                 shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, O, D, weight,
-                                 make_float4(h.t, h.u, h.v, __uint_as_float(h.inst)), h.prim, o);
+                                 make_float4(h.t, h.u, h.v, __uint_as_float(h.prim)), h.inst, o);
                 if (o.emissive) color = color + o.wnew;
                 if (LIT && o.is_mat) {
                     // the path's lanes take a light slot each, then all sum them in slot order (k_nee,
@@ -1740,8 +1740,8 @@ __global__ void __launch_bounds__(128, SHADOW ? 9 : (VOTE ? 8 : 7))
                     w.vis[(size_t)(tag >> 26) * w.chunk_cap + (tag & ((1u << 26) - 1u))] = 1;
                 }
             } else {
-                w.hit[idx] = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.inst));
-                w.hit_prim[idx] = t.h.prim;
+                w.hit[idx] = make_float4(t.h.t, t.h.u, t.h.v, __uint_as_float(t.h.prim));
+                w.hit_inst[idx] = t.h.inst;
                 if (depth == 0 && w.primary) {
                     const uint32_t p = __float_as_uint(w.q_o[cur][idx].w);
                     kf_hit ph;

@@ -105,8 +105,8 @@ struct WaveDev {
     float4* q_d[2];       // ray queue: direction.xyz + throughput.x
     float2* q_w[2];       // ray queue: throughput.yz (not written for camera rays: 1)
     uint32_t* counters;   // kCounterRow words per depth
-    float4* hit;          // t, u, v, instance bits
-    uint32_t* hit_prim;
+    float4* hit;          // t, u, v, primitive bits
+    uint32_t* hit_inst;   // instance, or all ones on a miss (apart: k_miss reads this word of every ray only)
     uint32_t* sel;        // queue positions of this bounce's rays that hit
     uint32_t* scount;     // kSlotRow words per depth: slot j's shadow rays, at sq_o/sq_d[j * chunk_cap + k]
     uint32_t nslot;       // light slots with a shadow queue (scount entries)
