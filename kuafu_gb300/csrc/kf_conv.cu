@@ -899,9 +899,11 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
 // one image row for B (N = 3 x co_block: dZ rows y - 1, y, y + 1, that is dy = 2, 1, 0). The
 // shifted views start at any pixel: swizzling works on absolute shared-memory addresses.
 //
-// A CTA owns n_ci blocks of 32 input channels and one block of output channels, walks its
-// share of the tiles and adds its FP32 sums to dW by atomics (lane = input channel, so a warp's
-// add is one 128-byte line).
+// A CTA owns 32 input channels and one block of output channels, walks its share of the tiles and
+// adds its FP32 sums to dW by atomics (lane = input channel, so a warp's add is one 128-byte
+// line). It keeps to 110 KB of shared memory where two stages fit them, so that a convolution of
+// the backward-data chain fits beside it. (Up to 5 blocks of input channels per CTA share dZ tiles,
+// but leave fewer, larger CTAs: 904 against 892 us a step by itself, 877 against 838 beside the chain.)
 //
 // Bound: operand fetch of the tensor core at full resolution, launch and first-tile latency at
 // the deep levels. On a batch of 16 crops of 128 x 128 the 19 layers of the denoiser's backward
@@ -913,13 +915,11 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
 // (one per dx) drain TMEM. Every wait is bounded as in the kernels above.
 // ---------------------------------------------------------------------------
 constexpr int kWgRows = 8;     // X rows of a tile
-constexpr int kWgMaxCi = 5;    // blocks of 32 input channels per CTA (5 x 96 TMEM columns)
 constexpr int kWgMaxStages = 4;
 
 struct WgradParams {
     int tiles_x, tiles_y, num_tiles;
     int bw;                   // tile width: 8, 16 or 32
-    int n_ci;                 // blocks of 32 input channels per CTA
     int co_block;             // 32 or 64 output channels
     int stages;
     uint32_t x_stride;        // bytes of one 32-channel X tile (1024-aligned slot)
@@ -943,9 +943,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int co0 = blockIdx.y * p.co_block;
     const bool bias = blockIdx.z == 0; // one CTA of a dZ tile's readers also sums it
-    const int ci0 = blockIdx.z * p.n_ci * 32;
-    const int n_ci = min(p.n_ci, p.Cin / 32 - (int)blockIdx.z * p.n_ci);
-    const uint32_t acc_cols = 3u * (uint32_t)p.co_block;
+    const int ci0 = blockIdx.z * 32;
 
     if (threadIdx.x == 32) {
         tc::prefetch_map(&tmX);
@@ -1017,11 +1015,9 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
             const int n_img = t / per_img, r = t % per_img;
             const int y0 = (r / p.tiles_x) * kWgRows, x0 = (r % p.tiles_x) * p.bw;
             uint8_t* st = smem + s * p.stage_stride;
-            tc::mbar_arrive_expect_tx(&full[s], (uint32_t)n_ci * p.x_bytes + p.z_bytes);
+            tc::mbar_arrive_expect_tx(&full[s], p.x_bytes + p.z_bytes);
             tc::tma_load_4d(st, &tmZ, &full[s], co0, x0, y0 - 1, n_img);
-            st += p.stage_stride - p.n_ci * p.x_stride;
-            for (int c = 0; c < n_ci; ++c)
-                tc::tma_load_4d(st + c * p.x_stride, &tmX, &full[s], ci0 + 32 * c, x0 - 1, y0, n_img);
+            tc::tma_load_4d(st + p.stage_stride - p.x_stride, &tmX, &full[s], ci0, x0 - 1, y0, n_img);
             if (++s == (uint32_t)p.stages) s = 0;
         }
         // drain: every issued copy must have landed before the CTA may exit
@@ -1046,14 +1042,13 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
             }
             tc::fence_after_sync();
             const uint32_t z = tc::smem_u32(smem + s * p.stage_stride);
-            const uint32_t x = z + p.stage_stride - p.n_ci * p.x_stride;
-            for (int c = 0; c < n_ci; ++c)
-                for (uint32_t r = 0; r < (uint32_t)kWgRows; r += row_step)
-                    for (uint32_t q = 0; q < segs; ++q) {
-                        const uint64_t ad = ax + ((x + c * p.x_stride + r * ximg + q * 16 * xrow) >> 4);
-                        const uint64_t bd = bz + ((z + (r * p.bw + q * 16) * zrow) >> 4);
-                        tc::mma_bf16(tmem + c * acc_cols, ad, bd, idesc, (it > 0 || r > 0 || q > 0) ? 1u : 0u);
-                    }
+            const uint32_t x = z + p.stage_stride - p.x_stride;
+            for (uint32_t r = 0; r < (uint32_t)kWgRows; r += row_step)
+                for (uint32_t q = 0; q < segs; ++q) {
+                    const uint64_t ad = ax + ((x + r * ximg + q * 16 * xrow) >> 4);
+                    const uint64_t bd = bz + ((z + (r * p.bw + q * 16) * zrow) >> 4);
+                    tc::mma_bf16(tmem, ad, bd, idesc, (it > 0 || r > 0 || q > 0) ? 1u : 0u);
+                }
             tc::mma_commit(&empty[s]);
             if (++s == (uint32_t)p.stages) s = 0;
         }
@@ -1066,23 +1061,17 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
     __syncwarp();
     tc::fence_after_sync();
     if (ready && warp < 3) {
-        for (int c = 0; c < n_ci; ++c) {
-            const int ci = ci0 + 32 * c + lane;
-            for (int j = 0; j < 3; ++j) {
-                const int tap = (2 - j) * 3 + warp;
-                for (int k = 0; k < p.co_block; k += 16) {
-                    uint32_t r0[8], r1[8];
-                    const uint32_t col = tmem + ((uint32_t)(warp * 32) << 16) + c * acc_cols +
-                                         (uint32_t)(j * p.co_block + k);
-                    tc::tmem_ld8(col, r0);
-                    tc::tmem_ld8(col + 8, r1);
-                    tc::tmem_ld_wait();
-                    float* dst = p.dw + ((size_t)tap * p.Cout + co0 + k) * p.Cin + ci;
+        const int ci = ci0 + lane;
+        for (int j = 0; j < 3; ++j) {
+            const int tap = (2 - j) * 3 + warp;
+            for (int k = 0; k < p.co_block; k += 16) {
+                uint32_t r0[16];
+                tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * p.co_block + k), r0);
+                tc::tmem_ld_wait();
+                float* dst = p.dw + ((size_t)tap * p.Cout + co0 + k) * p.Cin + ci;
 #pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        if (co0 + k + q < p.Cout)
-                            atomicAdd(dst + (size_t)q * p.Cin, __uint_as_float(q < 8 ? r0[q & 7] : r1[q & 7]));
-                }
+                for (int q = 0; q < 16; ++q)
+                    if (co0 + k + q < p.Cout) atomicAdd(dst + (size_t)q * p.Cin, __uint_as_float(r0[q]));
             }
         }
     }
@@ -1509,16 +1498,9 @@ void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int
     p.z_bytes = (uint32_t)((kWgRows + 2) * p.bw * 2 * p.co_block);
     const uint32_t z_stride = (p.z_bytes + 1023u) & ~1023u;
     const int ci_blocks = Cin / 32, co_blocks = dz_channels / p.co_block, sms = num_sms();
-    // several input-channel blocks per CTA share the dZ tile: as many as TMEM and two stages
-    // of shared memory hold, while the CTAs that are left still have a tile each on every SM
-    p.n_ci = 1;
-    for (int c = 2; c <= std::min(kWgMaxCi, ci_blocks); ++c)
-        if (c * 3 * p.co_block <= 512 && 2 * (c * p.x_stride + z_stride) <= 220u * 1024u &&
-            (int64_t)p.num_tiles * co_blocks * ((ci_blocks + c - 1) / c) >= 2 * sms)
-            p.n_ci = c;
-    p.stage_stride = p.n_ci * p.x_stride + z_stride;
-    p.stages = std::min<int>(kWgMaxStages, (int)(220u * 1024u / p.stage_stride));
-    p.tmem_cols = pow2_at_least((uint32_t)(p.n_ci * 3 * p.co_block));
+    p.stage_stride = p.x_stride + z_stride;
+    p.stages = std::max(2, std::min<int>(kWgMaxStages, (int)(110u * 1024u / p.stage_stride)));
+    p.tmem_cols = pow2_at_least((uint32_t)(3 * p.co_block));
     const size_t smem = 1024 + (size_t)p.stages * p.stage_stride + 128 + 256;
     const uint64_t xdims[4] = {(uint64_t)Cin, (uint64_t)W, (uint64_t)H, (uint64_t)N};
     const uint64_t xstr[3] = {(uint64_t)x_cstride * 2, (uint64_t)W * x_cstride * 2, (uint64_t)H * W * x_cstride * 2};
@@ -1535,9 +1517,9 @@ void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int
         KF_CUDA_CHECK(cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         configured = true;
     }
-    const int blocks = co_blocks * ((ci_blocks + p.n_ci - 1) / p.n_ci);
+    const int blocks = co_blocks * ci_blocks;
     const int splits = std::max(1, std::min(p.num_tiles, sms / std::max(1, blocks)));
-    const dim3 grid((unsigned)splits, (unsigned)co_blocks, (unsigned)((ci_blocks + p.n_ci - 1) / p.n_ci));
+    const dim3 grid((unsigned)splits, (unsigned)co_blocks, (unsigned)ci_blocks);
     launch_overlapped(k_wgrad, grid, dim3(128), smem, st, mx, mz, p);
 }
 
