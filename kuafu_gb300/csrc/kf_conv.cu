@@ -134,8 +134,9 @@ __global__ void __launch_bounds__(128, 1) k_tc(const __grid_constant__ CUtensorM
             const int last = ((nk - 1 - s) / kStages) * kStages + s;
             if (!tc::mbar_wait(&full[s], (last / kStages) & 1, kWaitBudget)) set_error(2);
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer ----
+    } else if (warp == 1) {
+        // ---- MMA issuer: the warp stays converged, one elected lane issues ----
+        const uint32_t elected = tc::elect_one();
         const uint32_t idesc = tc::idesc_bf16(128, (uint32_t)p.n_tile);
         for (int i = 0; i < nk; ++i) {
             const int s = i % kStages;
@@ -150,11 +151,11 @@ __global__ void __launch_bounds__(128, 1) k_tc(const __grid_constant__ CUtensorM
             for (int kk = 0; kk < CK / 16; ++kk) {
                 const uint64_t ad = tc::smem_desc(a_addr + kk * 32, SBO, LAYOUT);
                 const uint64_t bd = tc::smem_desc(b_addr + kk * 32, SBO, LAYOUT);
-                tc::mma_bf16(tmem, ad, bd, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                tc::mma_bf16(tmem, ad, bd, idesc, (i > 0 || kk > 0) ? 1u : 0u, elected);
             }
-            tc::mma_commit(&empty[s]);
+            if (elected) tc::mma_commit(&empty[s]);
         }
-        tc::mma_commit(done);
+        if (elected) tc::mma_commit(done);
     }
 
     // ---- epilogue: all 4 warps, warp w owns TMEM lanes [32w, 32w + 32) ----
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(128, 1) k_tc(const __grid_constant__ CUtensorM
 // 2x2 average pooling that follows some layers (rows are paired inside a tile, the right
 // neighbour is the next lane), saving the pass that would read the layer's output again.
 //
-// Warp 0 lane 0: TMA producer (a ring of STAGES stages). Warp 1 lane 0: MMA issuer.
+// Warp 0 lane 0: TMA producer (a ring of STAGES stages). Warp 1: MMA issuer.
 // Warps 2-9: epilogue, warp w owning TMEM lanes [32 (w % 4), +32) = tile pixels, warps 2-5
 // the first half of the channels and warps 6-9 the second.
 // Every wait is bounded; on expiry the kernel records an error code, lets its own
@@ -362,7 +363,7 @@ struct HaloMmaConsts {
     uint32_t dcol[8];
 };
 
-// The MMAs of one chunk, unrolled at compile time (the single issuing thread then spends a
+// The MMAs of one chunk, unrolled at compile time (the single issuing warp then spends a
 // few instructions per MMA; built from a table at run time they took half again as long).
 // Halo row hr with shift dx feeds output rows hr - 2 .. hr (tap dy = hr - r); their
 // accumulators are adjacent TMEM columns and their weight blocks ([dx][dy = 2, 1, 0])
@@ -372,7 +373,8 @@ struct HaloMmaConsts {
 // tile's first chunk the row a halo row reaches first (r = hr, at dx = 0, kk = 0) starts
 // its accumulator with a non-accumulating MMA of its own.
 template <int CK, int R, int STACK, bool FIRST>
-__device__ __forceinline__ void halo_chunk_mmas(uint64_t ad0, uint64_t bd0, uint32_t acc, const HaloMmaConsts& k) {
+__device__ __forceinline__ void halo_chunk_mmas(uint64_t ad0, uint64_t bd0, uint32_t acc, const HaloMmaConsts& k,
+                                                uint32_t elected) {
     constexpr uint32_t W_ROW = CK * 2, HALO_ROW = kHaloW * W_ROW;
 #pragma unroll
     for (int hr = 0; hr < R + 2; ++hr) {
@@ -384,14 +386,14 @@ __device__ __forceinline__ void halo_chunk_mmas(uint64_t ad0, uint64_t bd0, uint
                 const int lo = hr - 2 > 0 ? hr - 2 : 0;
                 int hi = hr < R - 1 ? hr : R - 1;
                 if (FIRST && dx == 0 && kk == 0 && hi == hr) {
-                    tc::mma_bf16(acc + k.dcol[hr], ad, bd0 + k.boff[dx * 3 + 2] + kk * 2, k.idesc[0], 0u);
+                    tc::mma_bf16(acc + k.dcol[hr], ad, bd0 + k.boff[dx * 3 + 2] + kk * 2, k.idesc[0], 0u, elected);
                     --hi;
                 }
 #pragma unroll
                 for (int r0 = lo; r0 <= hi; r0 += STACK) {
                     const int r1 = r0 + STACK - 1 < hi ? r0 + STACK - 1 : hi;
                     tc::mma_bf16(acc + k.dcol[r0], ad, bd0 + k.boff[dx * 3 + 2 - (hr - r0)] + kk * 2,
-                                 k.idesc[r1 - r0], 1u);
+                                 k.idesc[r1 - r0], 1u, elected);
                 }
             }
         }
@@ -497,8 +499,9 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
             if (!tc::mbar_wait(&full[s], (last / STAGES) & 1, kWaitBudget)) set_error(12);
         }
         if (p.w_resident && !tc::mbar_wait(wbar, 0, kWaitBudget)) set_error(13);
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer ----
+    } else if (warp == 1) {
+        // ---- MMA issuer: the warp stays converged, one elected lane issues ----
+        const uint32_t elected = tc::elect_one();
         const uint32_t halo0 = tc::smem_u32(halo), w0 = tc::smem_u32(wst);
         // per-CTA constants of the unrolled MMA sequence (halo_chunk_mmas)
         HaloMmaConsts k;
@@ -532,16 +535,16 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
                 const uint64_t ad0 = tc::smem_desc(ha, 8u * W_ROW, W_LAYOUT);
                 const uint64_t bd0 = tc::smem_desc(wa, 8u * W_ROW, W_LAYOUT);
                 if (c == 0)
-                    halo_chunk_mmas<CK, R, STACK, true>(ad0, bd0, acc, k);
+                    halo_chunk_mmas<CK, R, STACK, true>(ad0, bd0, acc, k, elected);
                 else
-                    halo_chunk_mmas<CK, R, STACK, false>(ad0, bd0, acc, k);
-                tc::mma_commit(&empty[s]);
+                    halo_chunk_mmas<CK, R, STACK, false>(ad0, bd0, acc, k, elected);
+                if (elected) tc::mma_commit(&empty[s]);
             }
             if (!ok) break;
-            tc::mma_commit(&acc_full[b]);
+            if (elected) tc::mma_commit(&acc_full[b]);
         }
         // every MMA of this CTA completes before the TMEM is freed
-        tc::mma_commit(mma_done);
+        if (elected) tc::mma_commit(mma_done);
         if (!tc::mbar_wait(mma_done, 0, kWaitBudget)) set_error(17);
     } else if (warp >= 2) {
         // ---- epilogue: 8 warps, two per TMEM lane group, each taking half of the channel groups ----
@@ -650,12 +653,12 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
 // the latency of one load, one multiplication and one epilogue. k_tc loads 9 shifted boxes per 32
 // channels through a ring of 2 or 3 stages, a round trip to L2 every few steps. 16 images, before
 // and after: 160 -> 160 channels at 8 x 8 26 -> 12 us, 288 -> 128 at 16 x 16 36 -> 19, 96 -> 96 at
-// 32 x 32 17 -> 10, 64 -> 160 at 64 x 64 38 -> 15, 160 -> 64 there 28 -> 27 (32 output channels per
-// CTA are all that fit beside its halos, and an MMA costs its 65 to 70 cycles of operand fetch with
+// 32 x 32 17 -> 10, 64 -> 160 at 64 x 64 38 -> 15, 160 -> 64 there 28 -> 23 (32 output channels per
+// CTA are all that fit beside its halos, and an MMA costs 40 to 48 cycles of operand fetch with
 // 32 columns as with 64); a 256 x 256 frame's whole network 391 -> 190 us (with the weights loaded
 // while the kernel before drains).
 //
-// Warp 0 lane 0: TMA, warp 1 lane 0: MMAs, warps 2-9: epilogue, two to a TMEM lane group (4 tile
+// Warp 0 lane 0: TMA, warp 1: MMAs, warps 2-9: epilogue, two to a TMEM lane group (4 tile
 // rows), each taking half of the channel groups. Every wait is bounded as in the kernels above.
 // ---------------------------------------------------------------------------
 constexpr int kTileThreads = 320;
@@ -681,9 +684,10 @@ struct TileParams {
 
 // The MMAs of a tile over KC chunks of 32 input channels, unrolled at compile time: the one
 // issuing thread then spends a few instructions on each (in a loop over run-time chunks the
-// 160 -> 64 layer of 16 x 64 x 64 pixels took 34.9 us, bound by their issue; now 27).
+// 160 -> 64 layer of 16 x 64 x 64 pixels took 34.9 us, bound by their issue; now 23).
 template <int KC>
-__device__ __forceinline__ void tile_mmas(uint32_t acc, uint64_t ad0, uint64_t bd0, uint32_t tap_units, uint32_t idesc) {
+__device__ __forceinline__ void tile_mmas(uint32_t acc, uint64_t ad0, uint64_t bd0, uint32_t tap_units, uint32_t idesc,
+                                          uint32_t elected) {
 #pragma unroll 1
     for (int dy = 0; dy < 3; ++dy) { // a filter row at a time: all 9 taps at once spill from 160 channels on
         const uint64_t ar = ad0 + (uint32_t)(dy * kTileHaloW * 4), br = bd0 + (uint32_t)dy * 3u * tap_units;
@@ -693,8 +697,8 @@ __device__ __forceinline__ void tile_mmas(uint32_t acc, uint64_t ad0, uint64_t b
             for (int c = 0; c < KC; ++c) {
                 const uint64_t ad = ar + (uint32_t)(dx * 4 + c * (kTileHaloSlot >> 4));
                 const uint64_t bd = br + (uint32_t)(c * 9 + dx) * tap_units;
-                tc::mma_bf16(acc, ad, bd, idesc, (dy > 0 || dx > 0 || c > 0) ? 1u : 0u);
-                tc::mma_bf16(acc, ad + 2, bd + 2, idesc, 1u);
+                tc::mma_bf16(acc, ad, bd, idesc, (dy > 0 || dx > 0 || c > 0) ? 1u : 0u, elected);
+                tc::mma_bf16(acc, ad + 2, bd + 2, idesc, 1u, elected);
             }
         }
     }
@@ -780,8 +784,9 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
             if (!tc::mbar_wait(&full[b], (uses - 1) & 1, kWaitBudget)) set_error(32);
         }
         if (any && !tc::mbar_wait(wbar, 0, kWaitBudget)) set_error(33);
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer ----
+    } else if (warp == 1) {
+        // ---- MMA issuer: the warp stays converged, one elected lane issues ----
+        const uint32_t elected = tc::elect_one();
         const uint32_t idesc = tc::idesc_bf16(128, (uint32_t)p.n_tile);
         const uint32_t halo0 = tc::smem_u32(smem);
         const uint64_t bd0 = tc::smem_desc(tc::smem_u32(wst), 512u, 4u);
@@ -801,12 +806,14 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
             tc::fence_after_sync();
             const uint32_t acc = tmem + a * (uint32_t)p.n_tile;
             const uint64_t ad0 = tc::smem_desc(halo0 + b * buf_bytes, kTileHaloW * 64u, 4u);
-            tile_mmas<KC>(acc, ad0, bd0, tap_bytes >> 4, idesc);
-            tc::mma_commit(&empty[b]);
-            tc::mma_commit(&acc_full[a]);
+            tile_mmas<KC>(acc, ad0, bd0, tap_bytes >> 4, idesc, elected);
+            if (elected) {
+                tc::mma_commit(&empty[b]);
+                tc::mma_commit(&acc_full[a]);
+            }
         }
         // every MMA of this CTA completes before the TMEM is freed
-        tc::mma_commit(mma_done);
+        if (elected) tc::mma_commit(mma_done);
         if (!tc::mbar_wait(mma_done, 0, kWaitBudget)) set_error(37);
     } else if (warp >= 2) {
         // ---- epilogue: lane = pixel (4 rows of 8 per lane group) ----
@@ -910,7 +917,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
 // pass take 0.34 ms in this form (9 to 38 us each, cold cache); as 9 shifted transposes and 9
 // GEMMs a layer, each reading its operands from HBM again, they took 12.8 ms.
 //
-// One CTA of 128 threads: warp 0 lane 0 issues TMA, warp 1 lane 0 the MMAs, warps 2 and 3 sum the
+// One CTA of 128 threads: warp 0 lane 0 issues TMA, warp 1 the MMAs, warps 2 and 3 sum the
 // bias gradient from the dZ tiles in shared memory (a pass over dZ of its own before), warps 0-2
 // (one per dx) drain TMEM. Every wait is bounded as in the kernels above.
 // ---------------------------------------------------------------------------
@@ -1025,7 +1032,8 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
             const uint32_t last = ((it - 1 - q) / p.stages) * p.stages + q;
             if (!tc::mbar_wait(&full[q], (last / p.stages) & 1, kWaitBudget)) set_error(22);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) { // converged; one elected lane issues
+        const uint32_t elected = tc::elect_one();
         const uint32_t zrow = 2u * (uint32_t)p.co_block;     // bytes of one dZ pixel (its swizzle width)
         const uint32_t xrow = 64u;
         const uint32_t ximg = (uint32_t)(p.bw + 2) * xrow;   // one image row of the X tile
@@ -1047,12 +1055,12 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
                 for (uint32_t q = 0; q < segs; ++q) {
                     const uint64_t ad = ax + ((x + r * ximg + q * 16 * xrow) >> 4);
                     const uint64_t bd = bz + ((z + (r * p.bw + q * 16) * zrow) >> 4);
-                    tc::mma_bf16(tmem, ad, bd, idesc, (it > 0 || r > 0 || q > 0) ? 1u : 0u);
+                    tc::mma_bf16(tmem, ad, bd, idesc, (it > 0 || r > 0 || q > 0) ? 1u : 0u, elected);
                 }
-            tc::mma_commit(&empty[s]);
+            if (elected) tc::mma_commit(&empty[s]);
             if (++s == (uint32_t)p.stages) s = 0;
         }
-        tc::mma_commit(done);
+        if (elected) tc::mma_commit(done);
     }
 
     const bool any = (int)blockIdx.x < p.num_tiles;

@@ -99,14 +99,28 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, M x N x 16, BF16 inputs, FP32 accumulator.
+// One lane of a converged warp: 1 there, 0 in the others. The warp that issues MMAs runs its whole
+// sequence converged and only the MMA and commit instructions are predicated with this, which keeps
+// the descriptors in uniform registers. An M = 128, N = 32, K = 16 MMA then takes 40 cycles, the
+// operand fetch; issued from a branch that lane 0 takes it took 49, and up to 77 beside working
+// epilogue warps (16 x 64 x 64 pixels 160 -> 64 channels 27.1 -> 22.8 us, 1920 x 1088 pixels
+// 96 -> 32 107.4 -> 104.7, a training step on 16 crops of 128 x 128 814 -> 776).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p;
+}
+
+// D[tmem] (+)= A[smem] * B[smem]^T, M x N x 16, BF16 inputs, FP32 accumulator;
+// issued by the elected lane of a converged warp.
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
+                                         uint32_t accumulate, uint32_t elected) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
 // Arrives on `bar` once every previously issued tcgen05.mma of this thread has completed.
