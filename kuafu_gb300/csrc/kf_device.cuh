@@ -199,6 +199,28 @@ struct alignas(16) Node4 {
 };
 static_assert(sizeof(Node4) == 128, "Node4 must be 128 bytes");
 
+// The node arrays that rays are traced through are swizzled: the 16-byte chunk c of node i lies
+// at chunk c ^ (i & 7) of its 128 bytes, so that lanes at different nodes read one field from
+// different banks (k_trace_dyn's comment has the figures). Builders and refits work on plain nodes.
+__host__ __device__ __forceinline__ void store_swizzled(Node4* out, uint32_t i, const Node4& n) {
+    float4* p = reinterpret_cast<float4*>(out + i);
+    const float4* q = reinterpret_cast<const float4*>(&n);
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (uint32_t c = 0; c < 8; ++c) p[c ^ (i & 7u)] = q[c];
+}
+__host__ __device__ __forceinline__ Node4 load_swizzled(const Node4* in, uint32_t i) {
+    Node4 n;
+    const float4* p = reinterpret_cast<const float4*>(in + i);
+    float4* q = reinterpret_cast<float4*>(&n);
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (uint32_t c = 0; c < 8; ++c) q[c] = p[c ^ (i & 7u)];
+    return n;
+}
+
 // Leaf child link: bit 30 set, count - 1 (<= 15) in bits 26..29, first primitive in bits
 // 0..25, so that the traversal pushes the link as it is. Rebasing a leaf by a primitive
 // offset is a plain addition (the sum stays below 2^26).
@@ -324,46 +346,15 @@ KF_DEV bool intersect_tri(const PRay& r, float4 a, float4 b, float4 c, float tmi
     return true;
 }
 
-// Conservative slab test against the four children of a node: far distances
+// The slab test against the children of a node is conservative: far distances are
 // widened by 1 + 2*gamma(3) (Ize, JCGT 2013) so no box is culled by rounding.
-// Returns a 4-bit mask of children hit and their entry distances.
 #define KF_BOX_WIDEN (1.0f + 2.0f * (3.0f * 0x1.0p-24f) / (1.0f - 3.0f * 0x1.0p-24f))
 // The current closest hit is widened too before a box is culled against it: a triangle
 // whose computed t ties the closest hit (two walls meeting at a corner) may sit in a box
 // whose computed entry distance lies a few ulp beyond that t; the tie rule needs it tested.
 #define KF_TMAX_WIDEN (1.0f + 0x1.0p-19f)
 
-KF_DEV float lane(float4 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
 KF_DEV int lanei(int4 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
-
-KF_DEV float slab1(float nearp, float farp, float o, float inv, float& tf) {
-    tf = (farp - o) * inv;
-    return (nearp - o) * inv;
-}
-
-KF_DEV int box4(const PRay& r, const Node4& n, float tmin, float tmax, float tn_out[4]) {
-    int mask = 0;
-    const bool px = r.ix >= 0.0f, py = r.iy >= 0.0f, pz = r.iz >= 0.0f;
-    const float4 nx = px ? n.lox : n.hix, fx = px ? n.hix : n.lox;
-    const float4 ny = py ? n.loy : n.hiy, fy = py ? n.hiy : n.loy;
-    const float4 nz = pz ? n.loz : n.hiz, fz = pz ? n.hiz : n.loz;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float t1x, t1y, t1z;
-        const float t0x = slab1(lane(nx, c), lane(fx, c), r.ox, r.ix, t1x);
-        const float t0y = slab1(lane(ny, c), lane(fy, c), r.oy, r.iy, t1y);
-        const float t0z = slab1(lane(nz, c), lane(fz, c), r.oz, r.iz, t1z);
-        float tn = fmaxf(tmin, t0x);
-        float tf = fminf(__int_as_float(0x7f800000), t1x);
-        tn = fmaxf(tn, t0y);
-        tf = fminf(tf, t1y);
-        tn = fmaxf(tn, t0z);
-        tf = fminf(tf, t1z);
-        tn_out[c] = tn;
-        if (tn <= fminf(tf * KF_BOX_WIDEN, tmax * KF_TMAX_WIDEN)) mask |= 1 << c;
-    }
-    return mask;
-}
 
 // Closest-hit ordering with a deterministic tie rule (smallest t, then instance, then primitive).
 KF_DEV bool closer(float t, uint32_t inst, uint32_t prim, float bt, uint32_t binst, uint32_t bprim) {
@@ -374,20 +365,5 @@ KF_DEV bool closer(float t, uint32_t inst, uint32_t prim, float bt, uint32_t bin
 }
 
 KF_DEV float4 ldg4(const float4* p) { return __ldg(p); }
-
-KF_DEV Node4 load_node(const Node4* nodes, uint32_t i) {
-    const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    Node4 n;
-    n.lox = __ldg(p + 0);
-    n.hix = __ldg(p + 1);
-    n.loy = __ldg(p + 2);
-    n.hiy = __ldg(p + 3);
-    n.loz = __ldg(p + 4);
-    n.hiz = __ldg(p + 5);
-    const int4* q = reinterpret_cast<const int4*>(p + 6);
-    n.child = __ldg(q);
-    n.cnt = __ldg(q + 1);
-    return n;
-}
 
 } // namespace kf

@@ -53,12 +53,14 @@ __global__ void k_tri_gather(const float4* __restrict__ verts, const uint32_t* _
 }
 
 // Rebase a freshly built node array into a pool: inner children += node_base, leaf
-// children += leaf_base, instance links (TLAS leaves of one instance) += inst_base.
+// children += leaf_base, instance links (TLAS leaves of one instance) += inst_base. The nodes go
+// to places node_base, node_base + 1, ... of the (swizzled) pool.
+template <bool SWIZZLED_IN>
 __global__ void k_rebase(const Node4* __restrict__ in, uint32_t n, uint32_t node_base, uint32_t leaf_base,
-                         uint32_t inst_base, Node4* out) {
+                         uint32_t inst_base, Node4* pool) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    Node4 o = in[i];
+    Node4 o = SWIZZLED_IN ? load_swizzled(in, i) : in[i];
     int c[4] = {o.child.x, o.child.y, o.child.z, o.child.w};
     const int k[4] = {o.cnt.x, o.cnt.y, o.cnt.z, o.cnt.w};
     for (int q = 0; q < 4; ++q) {
@@ -66,7 +68,7 @@ __global__ void k_rebase(const Node4* __restrict__ in, uint32_t n, uint32_t node
         else if (k[q] > 0) c[q] += (int)(((uint32_t)c[q] & kInstChildTag) ? inst_base : leaf_base);
     }
     o.child = make_int4(c[0], c[1], c[2], c[3]);
-    out[i] = o;
+    store_swizzled(pool, node_base + i, o);
 }
 
 // k_tri_gather over every geometry at once: out[j] for j in the triangle pool, the
@@ -145,6 +147,13 @@ void root_box(const Node4& n, std::array<float, 6>& b) {
         b[0] = std::min(b[0], lx[c]); b[1] = std::min(b[1], ly[c]); b[2] = std::min(b[2], lz[c]);
         b[3] = std::max(b[3], hx[c]); b[4] = std::max(b[4], hy[c]); b[5] = std::max(b[5], hz[c]);
     }
+}
+
+// The TLAS nodes as rays are traced through them, from the plain host copy.
+void upload_tlas(SceneGpu& G, cudaStream_t st) {
+    std::vector<Node4> nodes(G.tlas_host_nodes.size());
+    for (size_t i = 0; i < nodes.size(); ++i) store_swizzled(nodes.data(), (uint32_t)i, G.tlas_host_nodes[i]);
+    if (!nodes.empty()) G.tlas_nodes.upload(nodes.data(), nodes.size(), st);
 }
 
 } // namespace
@@ -424,7 +433,8 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
                         if (k[q] == 0) c[q] += (int)nb;
                         else if (k[q] > 0) c[q] += (int)tb;
                     }
-                    pool.push_back(nd);
+                    pool.emplace_back();
+                    store_swizzled(pool.data(), (uint32_t)pool.size() - 1, nd);
                 }
                 std::copy(sah_order[bi].begin(), sah_order[bi].end(), order_all.begin() + tb);
             }
@@ -458,8 +468,8 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
                                r->cfg.bvh_builder == 2);
             k_tri_gather<<<(ntri + 255) / 256, 256, 0, st>>>(G.verts.ptr, G.indices.ptr, order.ptr, geom[gi].x,
                                                              geom[gi].y, ntri, G.tris.ptr + geom[gi].y);
-            k_rebase<<<(nn + 127) / 128, 128, 0, st>>>(nodes.ptr, (uint32_t)nn, node_base, geom[gi].y, 0u,
-                                                       G.blas_nodes.ptr + node_base);
+            k_rebase<false><<<(nn + 127) / 128, 128, 0, st>>>(nodes.ptr, (uint32_t)nn, node_base, geom[gi].y, 0u,
+                                                              G.blas_nodes.ptr);
             KF_CUDA_CHECK(cudaGetLastError());
             Node4 root;
             KF_CUDA_CHECK(cudaMemcpyAsync(&root, nodes.ptr, sizeof(Node4), cudaMemcpyDeviceToHost, st));
@@ -634,7 +644,7 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
             nd.hiy = make_float4(hy[0], hy[1], hy[2], hy[3]);
             nd.hiz = make_float4(hz[0], hz[1], hz[2], hz[3]);
         }
-        if (!nodes.empty()) G.tlas_nodes.upload(nodes.data(), nodes.size(), st);
+        upload_tlas(G, st);
         G.built_xform_stamp = s->xform_stamp;
         ++G.tlas_refits;
     }
@@ -695,7 +705,7 @@ void scene_sync_gpu(kf_renderer_s* r, kf_scene_s* s) {
                 for (int c = 0; c < 4; ++c)
                     if (cn[c] == 1) ch[c] = (int)(kInstChildTag | G.tlas_host_inst[leaf_first(ch[c])]);
             }
-            G.tlas_nodes.upload(G.tlas_host_nodes.data(), G.tlas_host_nodes.size(), st);
+            upload_tlas(G, st);
         } else {
             G.tlas_node_count = 0;
             G.tlas_nodes.resize(1, st);
@@ -862,15 +872,14 @@ void batch_sync(kf_renderer_s* r, const std::vector<kf_scene_s*>& scenes) {
             }
         }
         if (G.blas_node_count) {
-            k_rebase<<<(G.blas_node_count + 127) / 128, 128, 0, st>>>(G.blas_nodes.ptr, G.blas_node_count,
-                                                                      (uint32_t)obn, (uint32_t)ot, 0u,
-                                                                      B.blas_nodes.ptr + obn);
+            k_rebase<true><<<(G.blas_node_count + 127) / 128, 128, 0, st>>>(
+                G.blas_nodes.ptr, G.blas_node_count, (uint32_t)obn, (uint32_t)ot, 0u, B.blas_nodes.ptr);
             KF_CUDA_CHECK(cudaGetLastError());
         }
         if (G.tlas_node_count) {
-            k_rebase<<<(G.tlas_node_count + 127) / 128, 128, 0, st>>>(G.tlas_nodes.ptr, G.tlas_node_count,
-                                                                      (uint32_t)otn, (uint32_t)oti,
-                                                                      (uint32_t)oinst, B.tlas_nodes.ptr + otn);
+            k_rebase<true><<<(G.tlas_node_count + 127) / 128, 128, 0, st>>>(G.tlas_nodes.ptr, G.tlas_node_count,
+                                                                            (uint32_t)otn, (uint32_t)oti, (uint32_t)oinst,
+                                                                            B.tlas_nodes.ptr);
             KF_CUDA_CHECK(cudaGetLastError());
             std::vector<uint32_t> ti(G.tlas_inst.count);
             KF_CUDA_CHECK(cudaMemcpyAsync(ti.data(), G.tlas_inst.ptr, ti.size() * 4, cudaMemcpyDeviceToHost, st));

@@ -141,18 +141,20 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
-// The slab test of box4 on a node read in place, with the child links: the near and far planes
-// of each axis are loaded by the ray's direction signs (no selects) and tested two children per
-// instruction (18.9 instead of 19.3 ms on the 256-icosphere 1080p frame; no change while the
-// kernel still spilled).
-__device__ __forceinline__ int box4_dir(const PRay& r, const float4* p, float tmin, float tmax, float tn_out[4],
-                                        int4& child) {
-    const int sx = r.ix >= 0.0f ? 0 : 1, sy = r.iy >= 0.0f ? 0 : 1, sz = r.iz >= 0.0f ? 0 : 1;
-    child = __ldg(reinterpret_cast<const int4*>(p + 6));
-    const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
-    const ulonglong2 nx = __ldg(q + sx), fx = __ldg(q + (1 - sx));
-    const ulonglong2 ny = __ldg(q + 2 + sy), fy = __ldg(q + (3 - sy));
-    const ulonglong2 nz = __ldg(q + 4 + sz), fz = __ldg(q + (5 - sz));
+// The slab test on node i read in place, with the child links: a 4-bit mask of the children met
+// and their entry distances. The near and far planes of each axis are loaded by the ray's
+// direction signs (no selects) and tested two children per instruction (18.9 instead of 19.3 ms
+// on the 256-icosphere 1080p frame; no change while the kernel still spilled).
+__device__ __forceinline__ int box4_dir(const PRay& r, const Node4* nodes, uint32_t i, float tmin, float tmax,
+                                        float tn_out[4], int4& child) {
+    const uint32_t sx = r.ix >= 0.0f ? 0u : 16u, sy = r.iy >= 0.0f ? 0u : 16u, sz = r.iz >= 0.0f ? 0u : 16u;
+    // chunk c of the swizzled node: byte c * 16 of it, with the address bits of i & 7 flipped
+    const uint64_t p = reinterpret_cast<uint64_t>(nodes + i) + ((i & 7u) << 4);
+    const auto chunk = [p](uint32_t byte) { return reinterpret_cast<const ulonglong2*>(p ^ byte); };
+    child = __ldg(reinterpret_cast<const int4*>(p ^ 96u));
+    const ulonglong2 nx = __ldg(chunk(sx)), fx = __ldg(chunk(sx ^ 16u));
+    const ulonglong2 ny = __ldg(chunk(sy ^ 32u)), fy = __ldg(chunk(sy ^ 48u));
+    const ulonglong2 nz = __ldg(chunk(sz ^ 64u)), fz = __ldg(chunk(sz ^ 80u));
     const uint64_t ox = pk2(-r.ox, -r.ox), oy = pk2(-r.oy, -r.oy), oz = pk2(-r.oz, -r.oz);
     const uint64_t ix = pk2(r.ix, r.ix), iy = pk2(r.iy, r.iy), iz = pk2(r.iz, r.iz);
     const uint64_t wd = pk2(KF_BOX_WIDEN, KF_BOX_WIDEN);
@@ -300,8 +302,7 @@ template <bool SHADOW, bool COUNT, bool VOTE> struct Tracer {
     __device__ __forceinline__ void node(const SceneDev& s, uint32_t e) {
         int4 child;
         float tn[4];
-        const int mask = box4_dir(r, reinterpret_cast<const float4*>((in_blas ? s.blas_nodes : s.tlas_nodes) + e), tmin,
-                                  best, tn, child);
+        const int mask = box4_dir(r, in_blas ? s.blas_nodes : s.tlas_nodes, e, tmin, best, tn, child);
         if (COUNT) cnt.nodes++;
         // children to visit, as (entry distance, stack entry); misses get -inf. The child
         // links are stack entries already: node indices, and leaf entries (triangles in a
@@ -1628,6 +1629,12 @@ __global__ void __launch_bounds__(128) k_shadow(SceneDev s, BatchDev b, WaveDev 
 // rays run the same code at the same time mostly and lose up to 20 % by it; they keep
 // free-running steps.
 // ---------------------------------------------------------------------------
+// Bound by the L1's data stage (79 % busy on incoherent bounces) and then by issue (64 %): a node
+// read is seven 16-byte loads per ray, and lanes at different nodes ask for the same chunk of
+// their 128 bytes, one bank group. Nodes lie swizzled by their index (store_swizzled), which
+// spreads them: 20 % fewer passes for shadow rays, 12 % for the bounces; the 256 icospheres 18.2 -> 17.1 ms
+// a frame, the batch of rooms with spheres 49.8 -> 46.5 ms, a room 2.62 -> 2.59 ms.
+//
 // refill_below: a warp fetches rays when fewer lanes than this are busy; steps: traversal
 // steps (turns) between fetches (both tunable, kf_config.dyn_refill_below / dyn_steps).
 // Occupancy: 8 resident blocks per SM for the vote (64 registers; 9 and 10 spill: +3 and +10 %),
