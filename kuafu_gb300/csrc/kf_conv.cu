@@ -293,6 +293,24 @@ __device__ __forceinline__ void store16(__nv_bfloat16* dst, const uint32_t (&w)[
                  "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                  : "memory");
 }
+// a pixel of the network's head, with the residual added
+__device__ __forceinline__ void store_head(float* dst, const float* base, const float (&v)[16]) {
+    float4 o = make_float4(v[0], v[1], v[2], 0.0f);
+    if (base) {
+        const float4 b = *reinterpret_cast<const float4*>(base);
+        o.x += b.x;
+        o.y += b.y;
+        o.z += b.z;
+    }
+    *reinterpret_cast<float4*>(dst) = o;
+}
+// the four copies of a pixel in an upsampled image
+__device__ __forceinline__ void store16_up(__nv_bfloat16* dst, int px_step, size_t row_step, const uint32_t (&w)[8]) {
+    store16(dst, w);
+    store16(dst + px_step, w);
+    store16(dst + row_step, w);
+    store16(dst + row_step + px_step, w);
+}
 // the first n of 16 channels, at any alignment (16-byte stores where they fit)
 __device__ __forceinline__ void store16_any(__nv_bfloat16* dst, const uint32_t (&w)[8], int n) {
 #pragma unroll
@@ -349,8 +367,12 @@ struct HaloParams {
     int out_cstride, out_coff;
     float* outf;
     __nv_bfloat16* pool_out;   // fused 2x2 average pooling into a dense [N][H/2][W/2][Cout] tensor, or null
-    const __nv_bfloat16* mask; // ReLU backward mask (channel stride mask_cs, slice at mask_co), or null
-    int mask_cs, mask_co;
+    union {                    // what the epilogue does besides (one at most; null: nothing)
+        const __nv_bfloat16* mask; // ReLU backward mask: channel stride aux_cs, slice at aux_co
+        __nv_bfloat16* up_out;     // EXTRA, BF16: 2x upsampling into a slice of [N][2H][2W][aux_cs]; out may be null
+        const float* base;         // EXTRA, FP32: the residual of a head of 3 channels in float4 pixels
+    };
+    int aux_cs, aux_co;
     int settled;               // weights and bias may be read before the kernel before this one ends
 };
 
@@ -400,7 +422,7 @@ __device__ __forceinline__ void halo_chunk_mmas(uint64_t ad0, uint64_t bd0, uint
     }
 }
 
-template <int CK, int R, int STACK, int STAGES>
+template <int CK, int R, int STACK, int STAGES, bool EXTRA>
 __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_constant__ CUtensorMap tmX,
                                                                  const __grid_constant__ CUtensorMap tmW,
                                                                  const HaloParams p) {
@@ -561,6 +583,16 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
         uint32_t j = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++j) {
             const uint32_t b = j & 1;
+            // the residual's rows, while the tile is still multiplied (the network 796 -> 777 us)
+            if (EXTRA && p.outf && p.base && g0 == 0) {
+                int n_img, y0, x0;
+                tile_origin(t, n_img, y0, x0);
+                const int px = x0 + px_in_tile;
+                if (px < p.W)
+                    for (int r = 0; r < min(R, p.H - y0); ++r)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                            p.base + (((size_t)n_img * p.H + y0 + r) * p.W + px) * 4));
+            }
             const bool ready = tc::mbar_wait(&acc_full[b], (j / 2) & 1, kWaitBudget);
             __syncwarp();
             if (!ready) {
@@ -579,13 +611,22 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
                 const int co = n0 + 16 * g;
                 if (r >= rows || co >= p.Cout) return;
                 const size_t at = pix * p.out_cstride + p.out_coff + co + r * row_step;
+                if (EXTRA && p.outf) {
+                    if (co == 0) store_head(p.outf + at, p.base ? p.base + at : nullptr, v);
+                    return;
+                }
                 if (p.outf) { // FP32 output (a network head)
 #pragma unroll
                     for (int q = 0; q < 16; ++q)
                         if (co + q < p.Cout) p.outf[at + q] = v[q];
                     return;
                 }
-                if (p.mask) mask16(p.mask + (pix + (size_t)r * p.W) * p.mask_cs + p.mask_co + co, w);
+                if (!EXTRA && p.mask) mask16(p.mask + (pix + (size_t)r * p.W) * p.aux_cs + p.aux_co + co, w);
+                if (EXTRA) {
+                    store16_up(p.up_out + (((size_t)n_img * p.H + y0 + r) * 4 * p.W + 2 * px) * p.aux_cs + p.aux_co + co,
+                               p.aux_cs, (size_t)(2 * p.W) * p.aux_cs, w);
+                    if (!p.out) return;
+                }
                 if (fast) store16(p.out + at, w);
                 else store16_any(p.out + at, w, p.Cout - co);
             };
@@ -677,8 +718,12 @@ struct TileParams {
     int out_cstride, out_coff;
     float* outf;
     __nv_bfloat16* pool_out; // fused 2x2 average pooling into a dense [N][H/2][W/2][Cout] tensor, or null
-    const __nv_bfloat16* mask; // ReLU backward mask (channel stride mask_cs, slice at mask_co), or null
-    int mask_cs, mask_co;
+    union {                    // what the epilogue does besides (one at most; null: nothing)
+        const __nv_bfloat16* mask; // ReLU backward mask: channel stride aux_cs, slice at aux_co
+        __nv_bfloat16* up_out;     // EXTRA, BF16: 2x upsampling into a slice of [N][2H][2W][aux_cs]; out may be null
+        const float* base;         // EXTRA, FP32: the residual of a head of 3 channels in float4 pixels
+    };
+    int aux_cs, aux_co;
     int settled; // weights and bias may be read before the kernel before this one ends
 };
 
@@ -704,7 +749,7 @@ __device__ __forceinline__ void tile_mmas(uint32_t acc, uint64_t ad0, uint64_t b
     }
 }
 
-template <int KC>
+template <int KC, bool EXTRA>
 __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constant__ CUtensorMap tmX,
                                                                const __grid_constant__ CUtensorMap tmW,
                                                                const TileParams p) {
@@ -864,13 +909,22 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
                 }
                 if (!valid || co >= p.Cout) return;
                 const size_t at = pix * p.out_cstride + p.out_coff + co;
+                if (EXTRA && p.outf) {
+                    if (co == 0) store_head(p.outf + at, p.base ? p.base + at : nullptr, v);
+                    return;
+                }
                 if (p.outf) { // FP32 output (a network head)
 #pragma unroll
                     for (int q = 0; q < 16; ++q)
                         if (co + q < p.Cout) p.outf[at + q] = v[q];
                     return;
                 }
-                if (p.mask) mask16(p.mask + pix * p.mask_cs + p.mask_co + co, w);
+                if (!EXTRA && p.mask) mask16(p.mask + pix * p.aux_cs + p.aux_co + co, w);
+                if (EXTRA) {
+                    store16_up(p.up_out + (((size_t)n_img * p.H + py) * 4 * p.W + 2 * px) * p.aux_cs + p.aux_co + co,
+                               p.aux_cs, (size_t)(2 * p.W) * p.aux_cs, w);
+                    if (!p.out) return;
+                }
                 if (fast) store16(p.out + at, w);
                 else store16_any(p.out + at, w, p.Cout - co);
             };
@@ -1200,16 +1254,24 @@ int num_sms() {
     return std::max(1, n);
 }
 
-template <int CK, int R, int STACK, int STAGES>
-void launch_halo(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const HaloParams& p, size_t smem,
+template <int CK, int R, int STACK, int STAGES, bool EXTRA>
+void launch_halo_kernel(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const HaloParams& p, size_t smem,
                  cudaStream_t st) {
     static bool configured = false;
     if (!configured) {
-        KF_CUDA_CHECK(cudaFuncSetAttribute(k_conv_halo<CK, R, STACK, STAGES>,
+        KF_CUDA_CHECK(cudaFuncSetAttribute(k_conv_halo<CK, R, STACK, STAGES, EXTRA>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         configured = true;
     }
-    launch_overlapped(k_conv_halo<CK, R, STACK, STAGES>, grid, dim3(kHaloThreads), smem, st, x, w, p);
+    launch_overlapped(k_conv_halo<CK, R, STACK, STAGES, EXTRA>, grid, dim3(kHaloThreads), smem, st, x, w, p);
+}
+// EXTRA: with an upsampled or a head output, in an instantiation of its own (its branches cost the
+// layers without them 3 to 6 %: 96 -> 32 at 1920 x 1088 104 and 110 us).
+template <int CK, int R, int STACK, int STAGES>
+void launch_halo(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const HaloParams& p, size_t smem,
+                 cudaStream_t st, bool extra) {
+    if (extra) launch_halo_kernel<CK, R, STACK, STAGES, true>(grid, x, w, p, smem, st);
+    else launch_halo_kernel<CK, R, STACK, STAGES, false>(grid, x, w, p, smem, st);
 }
 
 // One instantiation per (rows per tile, stacked rows, stages): R = 8 comes with n_tile <= 32
@@ -1217,19 +1279,19 @@ void launch_halo(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const Ha
 // with n_tile > 128 (STACK 1). halo_shape takes no other pair.
 template <int CK, int STAGES>
 bool launch_halo_stages(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const HaloParams& p, size_t smem,
-                        cudaStream_t st) {
-    if (p.R == 8 && p.stack == 3 && STAGES == 2) launch_halo<CK, 8, 3, 2>(grid, x, w, p, smem, st);
-    else if (p.R == 4 && p.stack == 3) launch_halo<CK, 4, 3, STAGES>(grid, x, w, p, smem, st);
-    else if (p.R == 2 && p.stack == 2) launch_halo<CK, 2, 2, STAGES>(grid, x, w, p, smem, st);
-    else if (p.R == 2 && p.stack == 3) launch_halo<CK, 2, 3, STAGES>(grid, x, w, p, smem, st);
-    else if (p.R == 1 && p.stack == 1) launch_halo<CK, 1, 1, STAGES>(grid, x, w, p, smem, st);
+                        cudaStream_t st, bool extra) {
+    if (p.R == 8 && p.stack == 3 && STAGES == 2) launch_halo<CK, 8, 3, 2>(grid, x, w, p, smem, st, extra);
+    else if (p.R == 4 && p.stack == 3) launch_halo<CK, 4, 3, STAGES>(grid, x, w, p, smem, st, extra);
+    else if (p.R == 2 && p.stack == 2) launch_halo<CK, 2, 2, STAGES>(grid, x, w, p, smem, st, extra);
+    else if (p.R == 2 && p.stack == 3) launch_halo<CK, 2, 3, STAGES>(grid, x, w, p, smem, st, extra);
+    else if (p.R == 1 && p.stack == 1) launch_halo<CK, 1, 1, STAGES>(grid, x, w, p, smem, st, extra);
     else return false;
     return true;
 }
 template <int CK> void launch_halo_ck(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const HaloParams& p,
-                                      int stages, size_t smem, cudaStream_t st) {
-    const bool ok = stages == 2 ? launch_halo_stages<CK, 2>(grid, x, w, p, smem, st)
-                                : launch_halo_stages<CK, 3>(grid, x, w, p, smem, st);
+                                      int stages, size_t smem, cudaStream_t st, bool extra) {
+    const bool ok = stages == 2 ? launch_halo_stages<CK, 2>(grid, x, w, p, smem, st, extra)
+                                : launch_halo_stages<CK, 3>(grid, x, w, p, smem, st, extra);
     if (!ok) throw KfError(KF_ERR_INTERNAL, "conv3x3: no halo kernel for this tile shape");
 }
 
@@ -1279,8 +1341,8 @@ int conv3x3_halo(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __n
     p.settled = fuse && fuse->settled ? 1 : 0;
     if (fuse && fuse->mask) {
         p.mask = fuse->mask;
-        p.mask_cs = fuse->mask_cs;
-        p.mask_co = fuse->mask_co;
+        p.aux_cs = fuse->mask_cs;
+        p.aux_co = fuse->mask_co;
     }
     bool fused = false;
     // pooling pairs rows inside a tile (R even) and reads the right neighbour's lane
@@ -1289,25 +1351,40 @@ int conv3x3_halo(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __n
         p.pool_out = fuse->pool_out;
         fused = true;
     }
+    const bool extra = fuse && (fuse->up_out || fuse->head4);
+    if (fuse && fuse->up_out) {
+        p.up_out = fuse->up_out;
+        p.aux_cs = fuse->up_cs;
+        p.aux_co = fuse->up_co;
+        if (fuse->up_only) p.out = nullptr;
+    }
+    if (fuse && fuse->head4) p.base = fuse->base;
     const int slices = (Cout_rows + n_tile - 1) / n_tile;
     const int per_slice = std::max(1, num_sms() / slices);
     const dim3 grid((unsigned)std::min(p.num_tiles, per_slice), (unsigned)slices, 1);
     if (h.CK == 32)
-        launch_halo_ck<32>(grid, mx, mw, p, h.stages, h.smem, st);
+        launch_halo_ck<32>(grid, mx, mw, p, h.stages, h.smem, st, extra);
     else
-        launch_halo_ck<16>(grid, mx, mw, p, h.stages, h.smem, st);
+        launch_halo_ck<16>(grid, mx, mw, p, h.stages, h.smem, st, extra);
     return fused ? 2 : 1;
 }
 
-template <int KC>
-void launch_tile(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const TileParams& p, size_t smem,
-                 cudaStream_t st) {
+template <int KC, bool EXTRA>
+void launch_tile_kernel(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const TileParams& p, size_t smem,
+                        cudaStream_t st) {
     static bool configured = false;
     if (!configured) {
-        KF_CUDA_CHECK(cudaFuncSetAttribute(k_conv_tile<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        KF_CUDA_CHECK(
+            cudaFuncSetAttribute(k_conv_tile<KC, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         configured = true;
     }
-    launch_overlapped(k_conv_tile<KC>, grid, dim3(kTileThreads), smem, st, x, w, p);
+    launch_overlapped(k_conv_tile<KC, EXTRA>, grid, dim3(kTileThreads), smem, st, x, w, p);
+}
+template <int KC>
+void launch_tile(dim3 grid, const CUtensorMap& x, const CUtensorMap& w, const TileParams& p, size_t smem,
+                 cudaStream_t st, bool extra) {
+    if (extra) launch_tile_kernel<KC, true>(grid, x, w, p, smem, st);
+    else launch_tile_kernel<KC, false>(grid, x, w, p, smem, st);
 }
 
 // The tile kernel, for up to 288 input channels (one instantiation per 32; with more, the weights
@@ -1364,25 +1441,33 @@ int conv3x3_tile(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __n
     p.settled = fuse && fuse->settled ? 1 : 0;
     if (fuse && fuse->mask) {
         p.mask = fuse->mask;
-        p.mask_cs = fuse->mask_cs;
-        p.mask_co = fuse->mask_co;
+        p.aux_cs = fuse->mask_cs;
+        p.aux_co = fuse->mask_co;
     }
     bool fused = false;
     if (fuse && fuse->pool_out && y && !y_f32 && Cout % 8 == 0 && H % 2 == 0 && W % 2 == 0) {
         p.pool_out = fuse->pool_out;
         fused = true;
     }
+    const bool extra = fuse && (fuse->up_out || fuse->head4);
+    if (fuse && fuse->up_out) {
+        p.up_out = fuse->up_out;
+        p.aux_cs = fuse->up_cs;
+        p.aux_co = fuse->up_co;
+        if (fuse->up_only) p.out = nullptr;
+    }
+    if (fuse && fuse->head4) p.base = fuse->base;
     const dim3 grid((unsigned)std::min<int64_t>(tiles, std::max(1, sms * per_sm / slices)), (unsigned)slices, 1);
     switch (kchunks) {
-        case 1: launch_tile<1>(grid, mx, mw, p, smem, st); break;
-        case 2: launch_tile<2>(grid, mx, mw, p, smem, st); break;
-        case 3: launch_tile<3>(grid, mx, mw, p, smem, st); break;
-        case 4: launch_tile<4>(grid, mx, mw, p, smem, st); break;
-        case 5: launch_tile<5>(grid, mx, mw, p, smem, st); break;
-        case 6: launch_tile<6>(grid, mx, mw, p, smem, st); break;
-        case 7: launch_tile<7>(grid, mx, mw, p, smem, st); break;
-        case 8: launch_tile<8>(grid, mx, mw, p, smem, st); break;
-        default: launch_tile<9>(grid, mx, mw, p, smem, st); break;
+        case 1: launch_tile<1>(grid, mx, mw, p, smem, st, extra); break;
+        case 2: launch_tile<2>(grid, mx, mw, p, smem, st, extra); break;
+        case 3: launch_tile<3>(grid, mx, mw, p, smem, st, extra); break;
+        case 4: launch_tile<4>(grid, mx, mw, p, smem, st, extra); break;
+        case 5: launch_tile<5>(grid, mx, mw, p, smem, st, extra); break;
+        case 6: launch_tile<6>(grid, mx, mw, p, smem, st, extra); break;
+        case 7: launch_tile<7>(grid, mx, mw, p, smem, st, extra); break;
+        case 8: launch_tile<8>(grid, mx, mw, p, smem, st, extra); break;
+        default: launch_tile<9>(grid, mx, mw, p, smem, st, extra); break;
     }
     return fused ? 2 : 1;
 }
@@ -1408,6 +1493,14 @@ bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __
     KF_REQUIRE(!fuse || !fuse->mask || (((uintptr_t)fuse->mask & 15) == 0 && Cout % 16 == 0 && fuse->mask_cs % 8 == 0 &&
                                         fuse->mask_co % 8 == 0 && Cin <= 288 && y && !fuse->pool_out),
                KF_ERR_INVALID_ARGUMENT, "conv3x3: mask layout");
+    KF_REQUIRE(!fuse || !fuse->up_out ||
+                   (((uintptr_t)fuse->up_out & 31) == 0 && Cout % 16 == 0 && fuse->up_cs % 16 == 0 &&
+                    fuse->up_co % 16 == 0 && !fuse->pool_out && !fuse->mask && y && !y_f32 && Cin <= 288),
+               KF_ERR_INVALID_ARGUMENT, "conv3x3: upsampled output layout");
+    KF_REQUIRE(!fuse || !fuse->head4 ||
+                   (y_f32 && ((uintptr_t)y_f32 & 15) == 0 && ((uintptr_t)fuse->base & 15) == 0 && Cout == 3 &&
+                    y_cstride == 4 && y_coff == 0 && !fuse->mask && !fuse->up_out && Cin <= 288),
+               KF_ERR_INVALID_ARGUMENT, "conv3x3: head layout");
     const int halo = conv3x3_halo(x, N, H, W, Cin, w, Cout_rows, bias, Cout, relu, y, y_cstride, y_coff, st, y_f32,
                                   fuse);
     if (halo) return halo == 2;

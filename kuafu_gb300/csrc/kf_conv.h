@@ -13,6 +13,11 @@ namespace kf {
 // separate pass (both read the BF16-rounded outputs).
 // And a ReLU's backward mask: outputs whose place in `mask` (NHWC, channel stride mask_cs, slice
 // starting at mask_co, both multiples of 8) is not positive become zero.
+// And nearest 2x upsampling of the BF16 output into the channel slice up_co of an NHWC tensor
+// [N][2H][2W][up_cs] (up_out 32-byte aligned, up_cs, up_co and Cout multiples of 16); with
+// up_only the output itself is not written. Always done (at most 288 input channels then).
+// head4: the FP32 output has 3 channels at stride 4 (y_f32 16-byte aligned): the fourth becomes
+// zero, and `base`, if any, is added to the three (same layout, may be y_f32 itself).
 // settled: the weights and bias were complete before the kernel that precedes this one in the
 // stream started (the previous launch is one of a chain that waited): they may be loaded while
 // that kernel still runs.
@@ -21,6 +26,11 @@ struct ConvFuse {
     __nv_bfloat16* pool_out = nullptr;
     const __nv_bfloat16* mask = nullptr;
     int mask_cs = 0, mask_co = 0;
+    __nv_bfloat16* up_out = nullptr;
+    int up_cs = 0, up_co = 0;
+    bool up_only = false;
+    bool head4 = false;
+    const float* base = nullptr;
 };
 
 // y[n, y, x, y_coff + co] = act(bias[co] + sum_{tap, ci} x[n, y+dy, x+dx, ci] * w[tap][co][ci])

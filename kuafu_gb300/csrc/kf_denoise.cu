@@ -104,25 +104,6 @@ __global__ void k_pool_bwd_add(const bf16* __restrict__ gy, const bf16* __restri
     }
 }
 
-// nearest 2x upsampling of x (dense, H/2 x W/2) into y[slice] (H x W)
-__global__ void k_up_fwd(const bf16* __restrict__ x, int C, int N, int H, int W, bf16* y, int ys, int yo) {
-    grid_dependency_wait();
-    const int Ho = H / 2, Wo = W / 2, G = C / 8;
-    const size_t total = (size_t)N * Ho * Wo * G;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int g = (int)(i % G);
-        const size_t pix = i / G;
-        const int xw = (int)(pix % Wo);
-        const size_t ny = pix / Wo;
-        const uint4 q = *reinterpret_cast<const uint4*>(x + pix * C + 8 * g);
-        const size_t row0 = (2 * ny) * W + 2 * xw;
-        *reinterpret_cast<uint4*>(y + row0 * ys + yo + 8 * g) = q;
-        *reinterpret_cast<uint4*>(y + (row0 + 1) * ys + yo + 8 * g) = q;
-        *reinterpret_cast<uint4*>(y + (row0 + W) * ys + yo + 8 * g) = q;
-        *reinterpret_cast<uint4*>(y + (row0 + W + 1) * ys + yo + 8 * g) = q;
-    }
-}
-
 // gx (dense, H/2 x W/2) = sum of the 2x2 block of gy[slice] (H x W), masked by the forward
 // output y (dense, H/2 x W/2)
 __global__ void k_up_bwd(const bf16* __restrict__ gy, int gs, int go, int C, int N, int H, int W,
@@ -243,18 +224,6 @@ __global__ void k_pack_features(const float4* __restrict__ rad, const float4* __
             st8(o + 8 * g, q);
         }
         if (base) base[i] = make_float4(f[0], f[1], f[2], 0.0f);
-    }
-}
-
-// head[p].xyz += base[p].xyz (the residual connection around the network)
-__global__ void k_add_base(float4* __restrict__ head, const float4* __restrict__ base, size_t P) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < P; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 b = base[i];
-        float4 h = head[i];
-        h.x += b.x;
-        h.y += b.y;
-        h.z += b.z;
-        head[i] = h;
     }
 }
 
@@ -571,6 +540,8 @@ struct Ctx {
     kf_denoiser_impl& d;
     cudaStream_t st;
     int n, h, w;
+    TRef in;           // the 32-channel input (16 channels when the first convolution takes those)
+    bool keep = false; // a backward pass follows
     int H(int level) const { return h >> level; }
     int W(int level) const { return w >> level; }
     size_t P(int level) const { return (size_t)n * H(level) * W(level); }
@@ -619,35 +590,38 @@ void pool_fwd(Ctx& c, TRef x, int level, TRef y) {
     const size_t n = c.P(level + 1) * x.c / 8;
     launch_overlapped(k_pool_fwd, dim3(grid_for(n)), dim3(256), 0, c.st, x.p, x.cs, x.co, x.c, c.n, c.H(level), c.W(level), y.p);
 }
-void up_fwd(Ctx& c, TRef x, int level_hi, TRef y) {
-    const size_t n = c.P(level_hi + 1) * x.c / 8;
-    launch_overlapped(k_up_fwd, dim3(grid_for(n)), dim3(256), 0, c.st, x.p, x.c, c.n, c.H(level_hi), c.W(level_hi), y.p, y.cs, y.co);
-}
 // conv into y, then 2x2 pooling of y into `pooled` (at level + 1)
 void conv_pool(Ctx& c, int li, int level, TRef x, TRef y, TRef pooled) {
     ConvFuse f;
     f.pool_out = pooled.p;
     if (!conv_fwd(c, li, level, x, y, f)) pool_fwd(c, y, level, pooled);
 }
-// conv into y, then nearest 2x upsampling of y into the channel slice `up` (at level - 1).
-// A separate pass: both forms are bound by the same HBM writes of the four copies, and
-// written from the conv epilogue (32-byte stores) the layer grew by what the pass takes.
+// conv, then nearest 2x upsampling of its output into the channel slice `up` (at level - 1), both
+// in the convolution's epilogue; the output itself goes to y where a backward pass will read it.
+// The four copies are what HBM has to take; a pass of its own read the output again and added its
+// length to the multiplication's, which now hides most of the stores. At 1920 x 1088, convolution
+// and pass: 92 -> 82 us into the full resolution, 43 -> 35 and 21 -> 20 below; the network 801 -> 777.
 void conv_up(Ctx& c, int li, int level, TRef x, TRef y, TRef up) {
-    conv_fwd(c, li, level, x, y);
-    up_fwd(c, y, level - 1, up);
+    ConvFuse f;
+    f.up_out = up.p;
+    f.up_cs = up.cs;
+    f.up_co = up.co;
+    f.up_only = !c.keep;
+    conv_fwd(c, li, level, x, y, f);
 }
 
-// prediction (in a.head) = network(T_IN) + base (FP32 residual, optional). in16: T_IN holds
-// 16-channel features (the first convolution then reads half the bytes and does half the
-// MMAs; channels 16..31 of the 32-channel input are zero, so the values are the same).
-void forward(Ctx& c, const float4* base, bool in16 = false) {
+// out (float4 pixels; the activations' head buffer or the caller's) = network(c.in) + base (FP32
+// residual, optional), channel 3 zero. in16: c.in holds 16-channel features (the first convolution
+// then reads half the bytes and does half the MMAs; channels 16..31 of the 32-channel input are
+// zero, so the values are the same).
+void forward(Ctx& c, const float* base, float* out, bool in16 = false) {
     Acts& a = c.d.acts;
     if (in16) {
         const Layer& l = c.d.L[0];
-        conv3x3_bf16(a.at(T_IN), c.n, c.h, c.w, 16, c.d.wf0_16.ptr, l.rows, c.d.params.ptr + l.b_off, l.cout, l.relu,
+        conv3x3_bf16(c.in.p, c.n, c.h, c.w, 16, c.d.wf0_16.ptr, l.rows, c.d.params.ptr + l.b_off, l.cout, l.relu,
                      a.at(T_E0A), 32, 0, c.st);
     } else {
-        conv_fwd(c, 0, 0, T(a, T_IN), T(a, T_E0A));
+        conv_fwd(c, 0, 0, c.in, T(a, T_E0A));
     }
     conv_pool(c, 1, 0, T(a, T_E0A), S(a, T_CAT0, 64, 32), T(a, T_P0));
     conv_fwd(c, 2, 1, T(a, T_P0), T(a, T_E1A));
@@ -670,11 +644,11 @@ void forward(Ctx& c, const float4* base, bool in16 = false) {
         const Layer& l = c.d.L[18];
         ConvFuse f;
         f.settled = true;
+        f.head4 = true;
+        f.base = base;
         conv3x3_bf16(a.at(T_D0B), c.n, c.h, c.w, 32, c.d.wf.ptr + l.wf_off, l.rows, c.d.params.ptr + l.b_off, l.cout,
-                     false, nullptr, 4, 0, c.st, a.head.ptr, &f);
+                     false, nullptr, 4, 0, c.st, out, &f);
     }
-    if (base)
-        k_add_base<<<grid_for(c.P(0)), 256, 0, c.st>>>(reinterpret_cast<float4*>(a.head.ptr), base, c.P(0));
     KF_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -721,7 +695,7 @@ void backward(Ctx& c) {
     conv_bwd(c, 2, 1, T(a, T_P0), T(a, G_E1A), T(a, G_P0), false);
     pool_bwd_add(c, T(a, G_P0), S(a, G_CAT0, 64, 32), 0, S(a, T_CAT0, 64, 32), T(a, G_E0B));
     conv_bwd(c, 1, 0, T(a, T_E0A), T(a, G_E0B), T(a, G_E0A), true);
-    conv_bwd(c, 0, 0, T(a, T_IN), T(a, G_E0A), none, false);
+    conv_bwd(c, 0, 0, c.in, T(a, G_E0A), none, false);
     KF_CUDA_CHECK(cudaEventRecord(c.d.r->ev_join, c.d.r->stream2));
     KF_CUDA_CHECK(cudaStreamWaitEvent(c.st, c.d.r->ev_join, 0));
 }
@@ -759,23 +733,55 @@ void denoiser_set_params(kf_denoiser_impl* d, const float* in, size_t n) {
     d->step = 0;
 }
 
-// out: [n, h, w, 4] FP32 device buffer (channels 0..2 = prediction in g space, 3 = 0);
-// base: optional FP32 residual [n, h, w] float4 added to the network output.
-void denoiser_forward(kf_denoiser_impl* d, const void* feat, const void* base, int n, int h, int w, void* out) {
+namespace {
+
+// The network over the caller's tensors. They are read and written in place where the kernels can
+// (this device's memory at 16-byte boundaries), else through the activations' buffers. At
+// 1920 x 1088 the copy of the input costs 41 us and that of the output 10 (778 us without both);
+// the residual is added in the last convolution's epilogue, a pass of 12 us before. The API calls
+// return when the stream is done, so nothing outlives the caller's tensors.
+Ctx run_forward(kf_denoiser_impl* d, const void* feat, const void* base, int n, int h, int w, void* out, bool keep) {
     cudaStream_t st = d->r->stream;
     ensure_acts(*d, n, h, w, st);
     if (!d->packed) pack(*d, st);
-    KF_CUDA_CHECK(cudaMemcpyAsync(d->acts.at(T_IN), feat, (size_t)n * h * w * 32 * 2, cudaMemcpyDeviceToDevice, st));
-    Ctx c{*d, st, n, h, w};
-    forward(c, static_cast<const float4*>(base));
-    if (out)
-        KF_CUDA_CHECK(cudaMemcpyAsync(out, d->acts.head.ptr, (size_t)n * h * w * 16, cudaMemcpyDeviceToDevice, st));
+    const auto in_place = [](const void* p) {
+        cudaPointerAttributes at{};
+        int dev = -1;
+        if (((uintptr_t)p & 15) != 0) return false;
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return at.type == cudaMemoryTypeDevice && at.device == dev;
+    };
+    Acts& a = d->acts;
+    Ctx c{*d, st, n, h, w, T(a, T_IN), keep};
+    if (in_place(feat))
+        c.in.p = static_cast<bf16*>(const_cast<void*>(feat));
+    else
+        KF_CUDA_CHECK(cudaMemcpyAsync(c.in.p, feat, (size_t)n * h * w * 32 * 2, cudaMemcpyDeviceToDevice, st));
+    // the head is written pixel by pixel while the residual is read: the same tensor, or one apart
+    const uintptr_t ob = (uintptr_t)out, bb = (uintptr_t)base, bytes = (uintptr_t)n * h * w * 16;
+    const bool apart = !base || ob == bb || ob + bytes <= bb || bb + bytes <= ob;
+    const bool direct = out && apart && in_place(out);
+    forward(c, static_cast<const float*>(base), direct ? static_cast<float*>(out) : a.head.ptr);
+    if (out && !direct)
+        KF_CUDA_CHECK(cudaMemcpyAsync(out, a.head.ptr, (size_t)n * h * w * 16, cudaMemcpyDeviceToDevice, st));
+    return c;
+}
+
+} // namespace
+
+// out: [n, h, w, 4] FP32 device buffer (channels 0..2 = prediction in g space, 3 = 0);
+// base: optional FP32 residual [n, h, w] float4 added to the network output.
+void denoiser_forward(kf_denoiser_impl* d, const void* feat, const void* base, int n, int h, int w, void* out) {
+    run_forward(d, feat, base, n, h, w, out, false);
 }
 
 float denoiser_train_step(kf_denoiser_impl* d, const void* feat, const void* base, const float* tgt, int n, int h,
                           int w, float lr, float* grads_out, bool apply_update) {
     cudaStream_t st = d->r->stream;
-    denoiser_forward(d, feat, nullptr, n, h, w, nullptr); // the loss adds the residual
+    Ctx c = run_forward(d, feat, nullptr, n, h, w, nullptr, true); // the loss adds the residual
     Acts& a = d->acts;
     KF_CUDA_CHECK(cudaMemsetAsync(d->loss.ptr, 0, sizeof(float), st));
     const unsigned tiles = (unsigned)n * (unsigned)((w + kLossW - 1) / kLossW) * (unsigned)((h + kLossH - 1) / kLossH);
@@ -784,7 +790,6 @@ float denoiser_train_step(kf_denoiser_impl* d, const void* feat, const void* bas
                                               h, w, 0.5f, d->loss.ptr, a.at(G_OUT));
     KF_CUDA_CHECK(cudaGetLastError());
     KF_CUDA_CHECK(cudaMemsetAsync(d->grads.ptr, 0, d->grads.bytes(), st));
-    Ctx c{*d, st, n, h, w};
     backward(c);
     if (grads_out)
         KF_CUDA_CHECK(cudaMemcpyAsync(grads_out, d->grads.ptr, d->nparams * 4, cudaMemcpyDeviceToDevice, st));
@@ -927,8 +932,8 @@ void denoiser_apply(kf_denoiser_impl* d, kf_camera_s* c) {
     // frames the halo convolution takes (at least 96 wide) use the 16-channel input
     const bool in16 = Wp >= 96;
     camera_features(c, frames * std::max(r->stats.last_spp, 1u), d->acts.at(T_IN), nullptr, Hp, Wp, st, in16);
-    Ctx cx{*d, st, 1, Hp, Wp};
-    forward(cx, nullptr, in16);
+    Ctx cx{*d, st, 1, Hp, Wp, T(d->acts, T_IN)};
+    forward(cx, nullptr, d->acts.head.ptr, in16);
     const size_t npix = (size_t)c->target_w * c->target_h;
     if (c->denoised.count != npix) c->denoised.resize(npix, st);
     k_unpack_residual<<<grid_for(npix), 256, 0, st>>>(reinterpret_cast<const float4*>(d->acts.head.ptr),

@@ -131,6 +131,40 @@ def test_forward_matches_torch(renderer, h, w):
     d.close()
 
 
+@pytest.mark.parametrize("n,h,w", [(1, 16, 16), (2, 96, 208)])
+def test_forward_reads_and_writes_in_place_or_through_copies(renderer, n, h, w):
+    """The same bits whether the kernels use the caller's tensors or copies of them: misaligned
+    features and output, the residual in the output's memory or overlapping it, and after a
+    training step's forward pass, which keeps the outputs that are only upsampled otherwise."""
+    import torch
+
+    d = api.Denoiser(renderer, seed=7)
+    feat, target = _inputs(torch, n, h, w, 3)
+    base = torch.randn((n, h, w, 4), device="cuda")
+
+    def forward(feat_ptr, out, base_ptr):
+        torch.cuda.synchronize()
+        d.forward(feat_ptr, n, h, w, out.data_ptr(), base_ptr=base_ptr)
+        assert _tc_error() == 0
+        return out.clone()
+
+    want = forward(feat.data_ptr(), torch.full((n, h, w, 4), 7.0, device="cuda"), base.data_ptr())
+    size = n * h * w * 4
+    odd = torch.zeros(feat.numel() + 8, device="cuda", dtype=torch.bfloat16)[1 : 1 + feat.numel()]
+    odd.copy_(feat.reshape(-1))
+    out = torch.zeros(size + 4, device="cuda")[1 : 1 + size]
+    assert odd.data_ptr() % 16 and out.data_ptr() % 16
+    assert torch.equal(forward(odd.data_ptr(), out, base.data_ptr()).reshape(n, h, w, 4), want)
+    inplace = base.clone()
+    assert torch.equal(forward(feat.data_ptr(), inplace, inplace.data_ptr()), want)
+    both = torch.zeros(size + 64, device="cuda")
+    both[64:].copy_(base.reshape(-1))  # the residual 16 pixels behind the output
+    assert torch.equal(forward(feat.data_ptr(), both[:size], both[64:].data_ptr()).reshape(n, h, w, 4), want)
+    d.trainStep(feat.data_ptr(), target.data_ptr(), n, h, w, base_ptr=base.data_ptr())
+    assert torch.equal(forward(feat.data_ptr(), torch.empty((n, h, w, 4), device="cuda"), base.data_ptr()), want)
+    d.close()
+
+
 @pytest.mark.parametrize("h,w", [(32, 48), (32, 256)])
 def test_gradients_match_autograd(renderer, h, w):
     import torch
