@@ -966,17 +966,22 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
 // the backward-data chain fits beside it. (Up to 5 blocks of input channels per CTA share dZ tiles,
 // but leave fewer, larger CTAs: 904 against 892 us a step by itself, 877 against 838 beside the chain.)
 //
-// Bound: operand fetch of the tensor core at full resolution, launch and first-tile latency at
+// Bound: the TMA's rate of 64-byte rows at full resolution (with a quarter of the MMAs, no bias
+// sums and no atomics the 96 -> 32 layer still takes 28 of 33 us), launch and first-tile latency at
 // the deep levels. On a batch of 16 crops of 128 x 128 the 19 layers of the denoiser's backward
-// pass take 0.34 ms in this form (9 to 38 us each, cold cache); as 9 shifted transposes and 9
-// GEMMs a layer, each reading its operands from HBM again, they took 12.8 ms.
+// pass take 0.29 ms in this form (8 to 33 us each); as 9 shifted transposes and 9 GEMMs a layer,
+// each reading its operands from HBM again, they took 12.8 ms.
 //
-// One CTA of 128 threads: warp 0 lane 0 issues TMA, warp 1 the MMAs, warps 2 and 3 sum the
-// bias gradient from the dZ tiles in shared memory (a pass over dZ of its own before), warps 0-2
-// (one per dx) drain TMEM. Every wait is bounded as in the kernels above.
+// One CTA of 192 threads: warp 0 lane 0 issues TMA, warp 1 the MMAs, warps 2 to 5 sum the bias
+// gradient from the dZ tiles in shared memory (a pass over dZ of its own before), warps 0-2 (one
+// per dx) drain TMEM. A stage is free when it is summed: with 2 warps the sums held the loads up
+// (0.32 ms, a step 762 us; with 4 735, 6 739, 8 752, which leave less room for the other chain).
+// Every wait is bounded as in the kernels above.
 // ---------------------------------------------------------------------------
 constexpr int kWgRows = 8;     // X rows of a tile
 constexpr int kWgMaxStages = 4;
+constexpr int kWgSumWarps = 4; // warps that sum the bias gradient
+constexpr int kWgThreads = 64 + 32 * kWgSumWarps;
 
 struct WgradParams {
     int tiles_x, tiles_y, num_tiles;
@@ -992,7 +997,7 @@ struct WgradParams {
     float* db;
 };
 
-__global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtensorMap tmX,
+__global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(const __grid_constant__ CUtensorMap tmX,
                                                   const __grid_constant__ CUtensorMap tmZ, const WgradParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1014,7 +1019,7 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
     if (threadIdx.x == 32) {
         for (int s = 0; s < p.stages; ++s) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], bias ? 3 : 1); // the MMAs, and the two warps that sum dZ
+            tc::mbar_init(&empty[s], bias ? 1 + kWgSumWarps : 1); // the MMAs, and the warps that sum dZ
         }
         tc::mbar_init(done, 1);
         tc::fence_barrier_init();
@@ -1027,9 +1032,9 @@ __global__ void __launch_bounds__(128, 1) k_wgrad(const __grid_constant__ CUtens
 
     grid_dependency_wait();
     if (warp >= 2 && bias) {
-        // ---- bias sums: thread = 8 channels of every (64 / groups)-th pixel of the tile's own rows
+        // ---- bias sums: thread = 8 channels of every `per`-th pixel of the tile's own rows
         const uint32_t groups = (uint32_t)p.co_block / 8, zrow = 2u * (uint32_t)p.co_block;
-        const uint32_t tid = threadIdx.x - 64, g = tid % groups, pl = tid / groups, per = 64 / groups;
+        const uint32_t tid = threadIdx.x - 64, g = tid % groups, pl = tid / groups, per = 32 * kWgSumWarps / groups;
         float sum[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) sum[q] = 0.0f;
@@ -1621,7 +1626,7 @@ void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int
     const int blocks = co_blocks * ci_blocks;
     const int splits = std::max(1, std::min(p.num_tiles, sms / std::max(1, blocks)));
     const dim3 grid((unsigned)splits, (unsigned)co_blocks, (unsigned)ci_blocks);
-    launch_overlapped(k_wgrad, grid, dim3(128), smem, st, mx, mz, p);
+    launch_overlapped(k_wgrad, grid, dim3(kWgThreads), smem, st, mx, mz, p);
 }
 
 namespace {
