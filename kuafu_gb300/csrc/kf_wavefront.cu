@@ -411,6 +411,27 @@ __device__ bool trace(const SceneDev& s, uint32_t root, uint32_t* smem, float ox
     return h.inst != kMiss;
 }
 
+// Loads of ray and hit records, which a kernel reads once: they do not take the L1's place from nodes
+// and vertices (k_trace_dyn's rays, k_shade's inputs; its next rays are stored streaming as well). A
+// room of 256 x 256 at 64 spp 2.54 -> 2.50 ms, a batch of rooms with spheres 46.2 -> 45.9, 256
+// icospheres no change.
+__device__ __forceinline__ float4 ld_once(const float4* p) {
+    float4 r;
+    asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+                 : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float2 ld_once(const float2* p) {
+    float2 r;
+    asm volatile("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint32_t ld_once(const uint32_t* p) {
+    uint32_t r;
+    asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(r) : "l"(p));
+    return r;
+}
 __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << (threadIdx.x & 31)) - 1u; }
 
 // Warp-aggregated append: one atomic per warp, positions by ballot prefix.
@@ -1253,7 +1274,7 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
         o.sh.isInside = false;
         View<BATCH> vw{fp, nullptr, 0};
         if (valid) {
-            const float4 qo = w.q_o[cur][i], qd = w.q_d[cur][i];
+            const float4 qo = ld_once(w.q_o[cur] + i), qd = ld_once(w.q_d[cur] + i);
             p = __float_as_uint(qo.w);
             vw = view_of<BATCH>(fp, b, w, chunk_start, p);
             const FrameDev& f = *vw.f;
@@ -1262,11 +1283,11 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
             const PathKey pk{make_uint2(f.seed ^ pix, f.camera_index), sample, f.frame};
             v3 wold = splat(1.0f); // camera rays
             if (depth > 0) {
-                const float2 wyz = w.q_w[cur][i];
+                const float2 wyz = ld_once(w.q_w[cur] + i);
                 wold = mk(qd.w, wyz.x, wyz.y);
             }
-            shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, mk(qo.x, qo.y, qo.z), mk(qd.x, qd.y, qd.z), wold, w.hit[i],
-                             w.hit_inst[i], o);
+            shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, mk(qo.x, qo.y, qo.z), mk(qd.x, qd.y, qd.z), wold,
+                             ld_once(w.hit + i), ld_once(w.hit_inst + i), o);
             if (o.emissive) {
                 const uint64_t g = chunk_start + p; // radiance index (the batch's path space)
                 const v3 color = (depth > 0 ? xyz(w.radiance[g]) : splat(0.0f)) + o.wnew;
@@ -1318,9 +1339,9 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
         __syncthreads();
         const uint32_t pos = o.cont ? s_cnt[par][key * kShadeWarps + wid] + rank : 0u;
         if (o.cont) {
-            w.q_o[nxt][pos] = make_float4(o.worldPos.x, o.worldPos.y, o.worldPos.z, __uint_as_float(p));
-            w.q_d[nxt][pos] = make_float4(o.L.x, o.L.y, o.L.z, o.wcont.x);
-            w.q_w[nxt][pos] = make_float2(o.wcont.y, o.wcont.z);
+            __stcs(w.q_o[nxt] + pos, make_float4(o.worldPos.x, o.worldPos.y, o.worldPos.z, __uint_as_float(p)));
+            __stcs(w.q_d[nxt] + pos, make_float4(o.L.x, o.L.y, o.L.z, o.wcont.x));
+            __stcs(w.q_w[nxt] + pos, make_float2(o.wcont.y, o.wcont.z));
         }
     }
 }
@@ -1703,12 +1724,12 @@ __global__ void __launch_bounds__(128, SHADOW ? 9 : (VOTE ? 8 : 7))
                 if (j < count) {
                     idx = SHADOW ? shadow_entry(w, s_pre, j) : j;
                     if (SHADOW) {
-                        const float4 o = w.sq_o[idx], d = w.sq_d[idx];
+                        const float4 o = ld_once(w.sq_o + idx), d = ld_once(w.sq_d + idx);
                         const uint32_t k = __float_as_uint(d.w) & ((1u << 26) - 1u);
                         const uint32_t root = BATCH ? b.items[w.hit_item[k]].root : single_root;
                         t.init(root, o.x, o.y, o.z, d.x, d.y, d.z, KF_T_MIN, o.w);
                     } else {
-                        const float4 o = w.q_o[cur][j], d = w.q_d[cur][j];
+                        const float4 o = ld_once(w.q_o[cur] + j), d = ld_once(w.q_d[cur] + j);
                         const View<BATCH> v = view_of<BATCH>(fp, b, w, chunk_start, __float_as_uint(o.w));
                         ah.f = v.f;
                         ah.g = v.g;
