@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(128, 1) k_tc(const __grid_constant__ CUtensorM
         const uint32_t idesc = tc::idesc_bf16(128, (uint32_t)p.n_tile);
         for (int i = 0; i < nk; ++i) {
             const int s = i % kStages;
-            if (!tc::mbar_wait(&full[s], (i / kStages) & 1, kWaitBudget)) {
+            if (!tc::mbar_wait_warp(&full[s], (i / kStages) & 1, kWaitBudget)) {
                 set_error(3);
                 break;
             }
@@ -533,12 +533,12 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
         for (int q = 0; q < 3; ++q) k.idesc[q] = tc::idesc_bf16(128, (uint32_t)((q + 1) * p.n_tile));
 #pragma unroll
         for (int r = 0; r < R; ++r) k.dcol[r] = (uint32_t)(r * p.n_tile);
-        bool ok = !p.w_resident || tc::mbar_wait(wbar, 0, kWaitBudget);
+        bool ok = !p.w_resident || tc::mbar_wait_warp(wbar, 0, kWaitBudget);
         if (!ok) set_error(14);
         uint32_t it = 0, j = 0;
         for (int t = blockIdx.x; t < p.num_tiles && ok; t += gridDim.x, ++j) {
             const uint32_t b = j & 1;
-            if (j >= 2 && !tc::mbar_wait(&acc_empty[b], ((j / 2) - 1) & 1, kWaitBudget)) {
+            if (j >= 2 && !tc::mbar_wait_warp(&acc_empty[b], ((j / 2) - 1) & 1, kWaitBudget)) {
                 set_error(15);
                 break;
             }
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
             const uint32_t acc = tmem + b * (uint32_t)acc_cols;
             for (int c = 0; c < p.kchunks; ++c, ++it) {
                 const uint32_t s = it % STAGES;
-                if (!tc::mbar_wait(&full[s], (it / STAGES) & 1, kWaitBudget)) {
+                if (!tc::mbar_wait_warp(&full[s], (it / STAGES) & 1, kWaitBudget)) {
                     set_error(16);
                     ok = false;
                     break;
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
         }
         // every MMA of this CTA completes before the TMEM is freed
         if (elected) tc::mma_commit(mma_done);
-        if (!tc::mbar_wait(mma_done, 0, kWaitBudget)) set_error(17);
+        if (!tc::mbar_wait_warp(mma_done, 0, kWaitBudget)) set_error(17);
     } else if (warp >= 2) {
         // ---- epilogue: 8 warps, two per TMEM lane group, each taking half of the channel groups ----
         const int lg = warp & 3;                 // TMEM lane group of this warp
@@ -835,16 +835,16 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
         const uint32_t idesc = tc::idesc_bf16(128, (uint32_t)p.n_tile);
         const uint32_t halo0 = tc::smem_u32(smem);
         const uint64_t bd0 = tc::smem_desc(tc::smem_u32(wst), 512u, 4u);
-        bool ok = (int)blockIdx.x >= p.num_tiles || tc::mbar_wait(wbar, 0, kWaitBudget);
+        bool ok = (int)blockIdx.x >= p.num_tiles || tc::mbar_wait_warp(wbar, 0, kWaitBudget);
         if (!ok) set_error(34);
         uint32_t it = 0;
         for (int t = blockIdx.x; t < p.num_tiles && ok; t += gridDim.x, ++it) {
             const uint32_t b = p.bufs == 2 ? (it & 1) : 0, use = p.bufs == 2 ? it >> 1 : it, a = it & 1;
-            if (it >= 2 && !tc::mbar_wait(&acc_empty[a], ((it / 2) - 1) & 1, kWaitBudget)) {
+            if (it >= 2 && !tc::mbar_wait_warp(&acc_empty[a], ((it / 2) - 1) & 1, kWaitBudget)) {
                 set_error(35);
                 break;
             }
-            if (!tc::mbar_wait(&full[b], use & 1, kWaitBudget)) {
+            if (!tc::mbar_wait_warp(&full[b], use & 1, kWaitBudget)) {
                 set_error(36);
                 break;
             }
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
         }
         // every MMA of this CTA completes before the TMEM is freed
         if (elected) tc::mma_commit(mma_done);
-        if (!tc::mbar_wait(mma_done, 0, kWaitBudget)) set_error(37);
+        if (!tc::mbar_wait_warp(mma_done, 0, kWaitBudget)) set_error(37);
     } else if (warp >= 2) {
         // ---- epilogue: lane = pixel (4 rows of 8 per lane group) ----
         const int lg = warp & 3, m = lg * 32 + lane;
@@ -1103,7 +1103,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(const __grid_constant__
         const uint32_t idesc = tc::idesc_bf16(128, 3u * (uint32_t)p.co_block) | tc::kIdescMnMajorAB;
         uint32_t it = 0, s = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
-            if (!tc::mbar_wait(&full[s], (it / p.stages) & 1, kWaitBudget)) {
+            if (!tc::mbar_wait_warp(&full[s], (it / p.stages) & 1, kWaitBudget)) {
                 set_error(23);
                 break;
             }

@@ -99,6 +99,11 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// The wait by a whole warp, which stays converged and goes on, or gives up, as one.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long budget) {
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, budget));
+}
+
 // One lane of a converged warp: 1 there, 0 in the others. The warp that issues MMAs runs its whole
 // sequence converged and only the MMA and commit instructions are predicated with this, which keeps
 // the descriptors in uniform registers. An M = 128, N = 32, K = 16 MMA then takes 40 cycles, the
