@@ -10,7 +10,10 @@
 //
 // In each, one thread issues TMA into mbarrier-guarded shared memory, another the MMAs, and
 // other warps drain TMEM. Every wait is bounded (~1 s of SM clock); on expiry the kernel records
-// an error code, drains its own copies and frees its TMEM.
+// an error code, drains its own copies and frees its TMEM. A warp that goes on to warp-wide
+// instructions (TMEM loads, shuffles, votes) waits and gives up as one (mbar_wait_warp): lanes
+// that decide for themselves could leave the others alone in them. Only single-lane roles
+// (the producers) wait by themselves.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -159,7 +162,8 @@ __global__ void __launch_bounds__(128, 1) k_tc(const __grid_constant__ CUtensorM
     }
 
     // ---- epilogue: all 4 warps, warp w owns TMEM lanes [32w, 32w + 32) ----
-    const bool ready = (nk == 0) ? true : tc::mbar_wait(done, 0, kWaitBudget);
+    __syncwarp(); // warp 0: its producer lane
+    const bool ready = nk == 0 || tc::mbar_wait_warp(done, 0, kWaitBudget);
     if (!ready) set_error(4);
     __syncwarp();
     tc::fence_after_sync();
@@ -593,7 +597,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(
                             p.base + (((size_t)n_img * p.H + y0 + r) * p.W + px) * 4));
             }
-            const bool ready = tc::mbar_wait(&acc_full[b], (j / 2) & 1, kWaitBudget);
+            const bool ready = tc::mbar_wait_warp(&acc_full[b], (j / 2) & 1, kWaitBudget);
             __syncwarp();
             if (!ready) {
                 set_error(18);
@@ -872,7 +876,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
         uint32_t it = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
             const uint32_t a = it & 1;
-            const bool ready = tc::mbar_wait(&acc_full[a], (it / 2) & 1, kWaitBudget);
+            const bool ready = tc::mbar_wait_warp(&acc_full[a], (it / 2) & 1, kWaitBudget);
             __syncwarp();
             if (!ready) {
                 set_error(38);
@@ -1040,7 +1044,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(const __grid_constant__
         for (int q = 0; q < 8; ++q) sum[q] = 0.0f;
         uint32_t it = 0, s = 0;
         for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++it) {
-            const bool ready = tc::mbar_wait(&full[s], (it / p.stages) & 1, kWaitBudget);
+            const bool ready = tc::mbar_wait_warp(&full[s], (it / p.stages) & 1, kWaitBudget);
             __syncwarp();
             if (!ready) {
                 set_error(25);
@@ -1123,7 +1127,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(const __grid_constant__
     }
 
     const bool any = (int)blockIdx.x < p.num_tiles;
-    const bool ready = any && tc::mbar_wait(done, 0, kWaitBudget);
+    __syncwarp(); // warp 0: its producer lane
+    const bool ready = any && tc::mbar_wait_warp(done, 0, kWaitBudget);
     if (any && !ready) set_error(24);
     __syncwarp();
     tc::fence_after_sync();

@@ -1,0 +1,73 @@
+"""Rules of the tensor-core and path kernels whose breach no run shows reliably (it would hang or
+race on some machine, some day), checked on their source: which lanes may wait or store where, and
+in which order a kernel takes resources. Comments are stripped before reading."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "kuafu_gb300" / "csrc"
+
+
+def _source(name):
+    s = (CSRC / name).read_text()
+    s = re.sub(r"/\*.*?\*/", "", s, flags=re.S)
+    return re.sub(r"//[^\n]*", "", s)
+
+
+def _body(s, at):
+    """The brace block that opens at or after position `at`, without its braces."""
+    i = s.index("{", at)
+    depth, j = 0, i
+    while True:
+        depth += {"{": 1, "}": -1}.get(s[j], 0)
+        if depth == 0:
+            return s[i + 1:j]
+        j += 1
+
+
+def _function(s, name):
+    """The body of the function defined as `name` (the match whose parameter list a block follows)."""
+    for m in re.finditer(r"\b" + name + r"\s*\(", s):
+        depth, j = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(s[j], 0)
+            j += 1
+        if re.match(r"\s*\{", s[j:]):
+            return _body(s, j)
+    raise AssertionError(f"no definition of {name}")
+
+
+def _kernels(s):
+    names = re.findall(r"__global__\s+void\s+(?:__launch_bounds__\s*\([^()]*(?:\([^()]*\)[^()]*)*\)\s*)?(\w+)\s*\(", s)
+    return {n: _function(s, n) for n in names}
+
+
+def _headers_at(body, at):
+    """What opens each block around position `at`: the text before its brace."""
+    stack, start = [], 0
+    for i, c in enumerate(body[:at]):
+        if c == "{":
+            stack.append(body[start:i])
+        elif c == "}":
+            stack.pop()
+        if c in "{};":
+            start = i + 1
+    return stack
+
+
+CONV = _kernels(_source("kf_conv.cu"))
+
+
+def test_the_kernels_are_found():
+    assert {"k_tc", "k_conv_halo", "k_conv_tile", "k_wgrad"} <= set(CONV)
+
+
+@pytest.mark.parametrize("kernel", sorted(CONV))
+def test_a_warp_waits_and_gives_up_as_one(kernel):
+    """A bounded wait that each lane decides for itself stands only where a single lane runs: a warp
+    whose lanes disagree would run TMEM loads and shuffles with a part of its lanes."""
+    body = CONV[kernel]
+    for m in re.finditer(r"\bmbar_wait\s*\(", body):
+        headers = _headers_at(body, m.start())
+        assert any("lane == 0" in h or "threadIdx.x == 0" in h for h in headers), body[m.start():m.start() + 80]
