@@ -9,7 +9,9 @@
 //   * K-major GEMM D += A * B^T (k_tc): 2D TMA, 128-byte swizzle, split-K with FP32 atomics.
 //
 // In each, one thread issues TMA into mbarrier-guarded shared memory, another the MMAs, and
-// other warps drain TMEM. Every wait is bounded (~1 s of SM clock); on expiry the kernel records
+// other warps drain TMEM. A kernel lets the next one of the stream start only when it holds its own
+// TMEM: the next one may take its columns before it waits for this one to end, and an allocation
+// waits without a bound. Every wait is bounded (~1 s of SM clock); on expiry the kernel records
 // an error code, drains its own copies and frees its TMEM. A warp that goes on to warp-wide
 // instructions (TMEM loads, shuffles, votes) waits and gives up as one (mbar_wait_warp): lanes
 // that decide for themselves could leave the others alone in them. Only single-lane roles
@@ -454,7 +456,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
         tc::prefetch_map(&tmX);
         tc::prefetch_map(&tmW);
     }
-    if (!p.settled) grid_dependency_wait();
+    if (!p.settled) grid_wait();
     if (warp == 0) tc::tmem_alloc(tmem_slot, p.tmem_cols);
     for (int i = threadIdx.x; i < p.n_tile; i += blockDim.x)
         sbias[i] = (p.bias && n0 + i < p.Cout) ? p.bias[n0 + i] : 0.0f;
@@ -475,6 +477,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) k_conv_halo(const __grid_cons
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    if (!p.settled) grid_launch_dependents();
 
     auto tile_origin = [&](int t, int& n_img, int& y0, int& x0) {
         const int per_img = p.tiles_x * p.tiles_y;
@@ -777,7 +780,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
         tc::prefetch_map(&tmX);
         tc::prefetch_map(&tmW);
     }
-    if (!p.settled) grid_dependency_wait();
+    if (!p.settled) grid_wait();
     if (warp == 0) tc::tmem_alloc(tmem_slot, p.tmem_cols);
     for (int i = threadIdx.x; i < p.n_tile; i += blockDim.x)
         sbias[i] = (p.bias && n0 + i < p.Cout) ? p.bias[n0 + i] : 0.0f;
@@ -796,6 +799,7 @@ __global__ void __launch_bounds__(kTileThreads) k_conv_tile(const __grid_constan
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    if (!p.settled) grid_launch_dependents();
 
     auto tile_origin = [&](int t, int& n_img, int& y0, int& x0) {
         const int per_img = p.tiles_x * p.tiles_y;

@@ -104,11 +104,16 @@ void launch_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
 
 #ifdef __CUDACC__
 // Waits until every kernel before this one in the stream is complete and its writes are visible
-// (returns at once in a kernel launched the usual way), then lets the next kernel's blocks start
-// their own prologue as this one's leave room.
-__device__ __forceinline__ void grid_dependency_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+// (returns at once in a kernel launched the usual way).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel's blocks start their own prologue as this one's leave room. What a block
+// takes and the next kernel's blocks might take as well (TMEM) it holds by then.
+__device__ __forceinline__ void grid_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency_wait() {
+    grid_wait();
+    grid_launch_dependents();
 }
 #endif
 

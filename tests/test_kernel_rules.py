@@ -71,3 +71,12 @@ def test_a_warp_waits_and_gives_up_as_one(kernel):
     for m in re.finditer(r"\bmbar_wait\s*\(", body):
         headers = _headers_at(body, m.start())
         assert any("lane == 0" in h or "threadIdx.x == 0" in h for h in headers), body[m.start():m.start() + 80]
+
+
+@pytest.mark.parametrize("kernel", sorted(k for k in CONV if "tmem_alloc" in CONV[k]))
+def test_tmem_is_held_before_the_next_kernel_may_start(kernel):
+    """A kernel that may start early takes TMEM before it waits for the one ahead: had that one not
+    allocated yet, both would wait for each other, and a TMEM allocation waits without a bound."""
+    body = CONV[kernel]
+    triggers = [m.start() for m in re.finditer(r"\bgrid_(dependency_wait|launch_dependents)\s*\(", body)]
+    assert all(t > body.index("tmem_alloc(") for t in triggers)
