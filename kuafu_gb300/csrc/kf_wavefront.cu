@@ -516,14 +516,15 @@ __device__ __forceinline__ uint32_t tiled_pixel(uint32_t idx, uint32_t width, ui
 }
 
 // Queue position j of a chunk: its path's view, pixel, sample and global number, with the pixels'
-// AOVs cleared (those of pixels that hit no material stay zero).
+// AOVs cleared where `clears` is set (those of pixels that hit no material stay zero). A path's AOVs
+// are cleared and written by one thread, whose own order puts the clearing first.
 // A pixel's samples are queued one after the other, so a warp's camera rays start in few
 // neighbouring pixels (+5 % over queuing each sample's pixels together); a band of kTileH rows
 // that lies in this chunk is queued in tile order.
 template <bool BATCH>
 __device__ __forceinline__ View<BATCH> camera_path(const FrameDev* __restrict__ fp, const BatchDev& b, const WaveDev& w,
-                                                   uint64_t chunk_start, uint32_t chunk_n, uint32_t j, uint32_t& item,
-                                                   uint32_t& pix, uint32_t& sample, uint64_t& G) {
+                                                   uint64_t chunk_start, uint32_t chunk_n, uint32_t j, bool clears,
+                                                   uint32_t& item, uint32_t& pix, uint32_t& sample, uint64_t& G) {
     uint64_t g = chunk_start + j;
     uint64_t view_start = 0; // global index of the view's first path
     View<BATCH> v;
@@ -545,7 +546,7 @@ __device__ __forceinline__ View<BATCH> camera_path(const FrameDev* __restrict__ 
     if (b0 >= chunk_start && b1 <= chunk_start + chunk_n) pix = tiled_pixel(pix, f.width, f.height);
     v.g = (uint64_t)pix * f.pc.spp + sample;
     G = view_start + v.g;
-    if (sample == 0) {
+    if (clears && sample == 0) {
         (BATCH ? v.it->albedo : w.albedo)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         (BATCH ? v.it->normal : w.normal)[pix] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
@@ -605,7 +606,7 @@ __global__ void k_raygen(const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
     if (j >= chunk_n) return;
     uint32_t item, pix, sample;
     uint64_t G;
-    const View<BATCH> v = camera_path<BATCH>(fp, b, w, chunk_start, chunk_n, j, item, pix, sample, G);
+    const View<BATCH> v = camera_path<BATCH>(fp, b, w, chunk_start, chunk_n, j, true, item, pix, sample, G);
     const FrameDev& f = *v.f;
     const uint32_t p = (uint32_t)(G - chunk_start);
     if (BATCH) w.path_item[p] = (uint16_t)item;
@@ -969,13 +970,14 @@ __device__ bool light_sample(const SceneDev& s, const LS& ls, uint32_t slot, uin
 // the path weight; the path ends. The rays that hit are listed in w.sel for k_shade, so
 // that its warps shade hits only.
 // ---------------------------------------------------------------------------
+// first: this thread writes the AOVs of a first bounce.
 template <bool BATCH>
-__device__ __forceinline__ v3 miss_emission(const SceneDev& s, const WaveDev& w, const View<BATCH>& vw, uint32_t depth,
+__device__ __forceinline__ v3 miss_emission(const SceneDev& s, const WaveDev& w, const View<BATCH>& vw, bool first,
                                             v3 dir) {
     const FrameDev& f = *vw.f;
     const float4* env = BATCH ? vw.it->env : s.env;
     const uint32_t env_size = BATCH ? vw.it->env_size : s.env_size;
-    if (depth == 0) { // AOVs of sample 0 of the first bounce
+    if (first) { // AOVs of sample 0
         uint32_t pix, sample;
         split_path(vw.g, f.pc.spp, pix, sample);
         if (sample == 0) {
@@ -1001,7 +1003,7 @@ __device__ __forceinline__ void miss_path(const SceneDev& s, const FrameDev* fp,
         wold = mk(qd.w, wyz.x, wyz.y);
         color = xyz(w.radiance[g]);
     }
-    color = color + miss_emission<BATCH>(s, w, vw, depth, mk(qd.x, qd.y, qd.z)) * wold;
+    color = color + miss_emission<BATCH>(s, w, vw, depth == 0, mk(qd.x, qd.y, qd.z)) * wold;
     w.radiance[g] = make_float4(color.x, color.y, color.z, 0.0f);
 }
 
@@ -1061,7 +1063,8 @@ __global__ void __launch_bounds__(kMissThreads) k_miss(SceneDev s, const FrameDe
 }
 
 // One hit shaded (rchit:322-468, rgen:109-138): emission, or the PrincipledBSDF's sample, the
-// throughput after it and whether the path goes on. Writes the AOVs of sample 0 of the first bounce.
+// throughput after it and whether the path goes on. aov: writes the pixel's AOVs (one thread does,
+// of sample 0 at the first bounce).
 struct HitShade {
     bool emissive, is_mat, cont;
     v3 worldPos, N, V, L;
@@ -1070,7 +1073,7 @@ struct HitShade {
 };
 template <bool BATCH>
 __device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, const View<BATCH>& vw, uint32_t depth,
-                                          const PathKey& pk, uint32_t pix, uint32_t sample, v3 rayO, v3 rayD, v3 wold,
+                                          const PathKey& pk, uint32_t pix, bool aov, v3 rayO, v3 rayD, v3 wold,
                                           float4 hv, uint32_t inst, HitShade& o) {
     const FrameDev& f = *vw.f;
     float4* aov_albedo = BATCH ? vw.it->albedo : w.albedo;
@@ -1204,8 +1207,7 @@ __device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, c
         o.sh.specularColor = specularColor;
         o.sh.transmissionColor = transmissionColor;
         o.sh.isInside = isInside;
-        // AOVs of sample 0, first bounce (rgen:114-117)
-        if (depth == 0 && sample == 0) {
+        if (aov) { // rgen:114-117
             aov_albedo[pix] = make_float4(baseColor.x, baseColor.y, baseColor.z, 1.0f);
             aov_normal[pix] = make_float4(o.N.x, o.N.y, o.N.z, 1.0f);
         }
@@ -1228,7 +1230,7 @@ __device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, c
             o.cont = alive && (depth + 1 <= f.pc.max_path_depth);
         }
     }
-    if (depth == 0 && sample == 0) {
+    if (aov) {
         aov_depth[pix] = hv.x;
         uint4* aov_seg = BATCH ? vw.it->seg : w.seg;
         if (aov_seg) {
@@ -1286,8 +1288,8 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const Fr
                 const float2 wyz = ld_once(w.q_w[cur] + i);
                 wold = mk(qd.w, wyz.x, wyz.y);
             }
-            shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, mk(qo.x, qo.y, qo.z), mk(qd.x, qd.y, qd.z), wold,
-                             ld_once(w.hit + i), ld_once(w.hit_inst + i), o);
+            shade_hit<BATCH>(s, w, vw, depth, pk, pix, depth == 0 && sample == 0, mk(qo.x, qo.y, qo.z),
+                             mk(qd.x, qd.y, qd.z), wold, ld_once(w.hit + i), ld_once(w.hit_inst + i), o);
             if (o.emissive) {
                 const uint64_t g = chunk_start + p; // radiance index (the batch's path space)
                 const v3 color = (depth > 0 ? xyz(w.radiance[g]) : splat(0.0f)) + o.wnew;
@@ -1409,7 +1411,7 @@ __global__ void __launch_bounds__(kThreadsTrace, kPathsBlocks)
                 pk = PathKey{make_uint2(vw.f->seed ^ pix, vw.f->camera_index), sample, vw.f->frame};
             } else {
                 uint32_t item;
-                vw = camera_path<BATCH>(fp, b, w, 0, n, j, item, pix, sample, G);
+                vw = camera_path<BATCH>(fp, b, w, 0, n, j, sub == 0, item, pix, sample, G);
                 pk = PathKey{make_uint2(vw.f->seed ^ pix, vw.f->camera_index), sample, vw.f->frame};
                 float origin[4], dir[4];
                 camera_ray(*vw.f, pix, pk, origin, dir);
@@ -1435,12 +1437,12 @@ __global__ void __launch_bounds__(kThreadsTrace, kPathsBlocks)
                     }
                 }
                 if (h.inst == kMiss) {
-                    color = color + miss_emission<BATCH>(s, w, vw, depth, D) * weight;
+                    color = color + miss_emission<BATCH>(s, w, vw, depth == 0 && sub == 0, D) * weight;
                     break;
                 }
                 HitShade o;
                 o.emissive = o.is_mat = o.cont = false;
-                shade_hit<BATCH>(s, w, vw, depth, pk, pix, sample, O, D, weight,
+                shade_hit<BATCH>(s, w, vw, depth, pk, pix, depth == 0 && sample == 0 && sub == 0, O, D, weight,
                                  make_float4(h.t, h.u, h.v, __uint_as_float(h.prim)), h.inst, o);
                 if (o.emissive) color = color + o.wnew;
                 if (LIT && o.is_mat) {

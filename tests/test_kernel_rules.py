@@ -80,3 +80,25 @@ def test_tmem_is_held_before_the_next_kernel_may_start(kernel):
     body = CONV[kernel]
     triggers = [m.start() for m in re.finditer(r"\bgrid_(dependency_wait|launch_dependents)\s*\(", body)]
     assert all(t > body.index("tmem_alloc(") for t in triggers)
+
+
+def _calls(body, name):
+    """The arguments of each call of `name` in a body, as one string without line breaks."""
+    for m in re.finditer(r"\b" + name + r"<\w+>\s*\(", body):
+        depth, j = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(body[j], 0)
+            j += 1
+        yield " ".join(body[m.end():j - 1].split())
+
+
+def test_one_lane_of_a_shared_path_writes_its_aovs():
+    """Several lanes may run one path: what clears a pixel's AOVs or writes them does it in the
+    path's first lane, so that no lane that falls behind clears what another has written."""
+    body = _kernels(_source("kf_wavefront.cu"))["k_paths"]
+    for name in ("camera_path", "miss_emission", "shade_hit"):
+        calls = list(_calls(body, name))
+        assert calls and all("sub == 0" in c for c in calls), name
+    for m in re.finditer(r"w\.(radiance|primary|albedo|normal|depth|seg)\[[^\]]*\]\s*=[^=]", body):
+        line = body[body.rindex("\n", 0, m.start()):m.start()]
+        assert any("sub == 0" in h for h in _headers_at(body, m.start()) + [line]), m.group(0)
