@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "kf_host.h"
 
@@ -212,7 +213,9 @@ void ensure_wave(kf_renderer_s* r, uint32_t chunk, uint32_t slots, uint64_t npat
     }
 }
 
-WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, bool lit) {
+// What the kernels of a launch get: slots = its light slots (the buffers may hold more from earlier
+// launches), c = the camera of a single view (a batch's kernels find the targets in its items).
+WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, uint32_t slots) {
     WaveBuffers& W = r->wave;
     WaveDev w{};
     w.q_o[0] = W.q_o0.ptr; w.q_o[1] = W.q_o1.ptr;
@@ -223,8 +226,8 @@ WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, bool lit
     w.hit_inst = W.hit_inst.ptr;
     w.sel = W.sel.ptr;
     w.scount = W.counters.ptr + ((size_t)max_depth + 2) * kCounterRow;
-    w.lit = lit ? 1u : 0u;
-    w.nslot = W.slot_cap;
+    w.lit = slots ? 1u : 0u;
+    w.nslot = slots;
     w.nee_w = W.nee_w.ptr;
     w.nee_in = W.nee_in.ptr;
     w.req = W.req.ptr;
@@ -234,10 +237,12 @@ WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, bool lit
     w.sq_d = W.sq_d.ptr;
     w.radiance = W.radiance.ptr;
     w.primary = r->cfg.debug_outputs ? W.primary.ptr : nullptr;
-    w.albedo = c->albedo.ptr;
-    w.normal = c->normal.ptr;
-    w.depth = c->depth.ptr;
-    w.seg = c->seg.ptr;
+    if (c) {
+        w.albedo = c->albedo.ptr;
+        w.normal = c->normal.ptr;
+        w.depth = c->depth.ptr;
+        w.seg = c->seg.ptr;
+    }
     w.stats = W.stats.ptr;
     w.chunk_cap = W.chunk_cap;
     return w;
@@ -394,6 +399,13 @@ static std::string scene_view_key(const SceneDev& v) {
     return k;
 }
 
+// The same for the launch's wavefront state, which is passed by value as well: all of it, so that a
+// replay never sees an address, a stride or a slot count of buffers that have moved or grown since.
+static std::string wave_key(const WaveDev& w) {
+    static_assert(std::has_unique_object_representations_v<WaveDev>, "no padding: the bytes are the key");
+    return std::string(reinterpret_cast<const char*>(&w), sizeof(w));
+}
+
 static uint32_t chunk_for(const kf_renderer_s* r, uint64_t npaths) {
     uint64_t cap = r->cfg.max_paths_in_flight ? r->cfg.max_paths_in_flight : (1ull << 24);
     cap = std::min<uint64_t>(cap, (1ull << 26) - 1);
@@ -420,7 +432,7 @@ void render_frame(kf_renderer_s* r, kf_scene_s* s, kf_camera_s* c, uint32_t spp)
     const FrameDev f = make_frame(r, s, c, spp, r->frame_count);
     if (r->frame_dev.count == 0) r->frame_dev.resize(1, st);
     KF_CUDA_CHECK(cudaMemcpyAsync(r->frame_dev.ptr, &f, sizeof(f), cudaMemcpyHostToDevice, st));
-    const WaveDev w = wave_view(r, c, r->cfg.path_depth, sv.num_slots > 0);
+    const WaveDev w = wave_view(r, c, r->cfg.path_depth, sv.num_slots);
     const bool profile = r->cfg.profile != 0;
     cudaEvent_t f0 = r->ev[4], f1 = r->ev[5];
     if (profile) KF_CUDA_CHECK(cudaEventRecord(f0, st));
@@ -429,12 +441,12 @@ void render_frame(kf_renderer_s* r, kf_scene_s* s, kf_camera_s* c, uint32_t spp)
         // The launch sequence depends only on buffer addresses and sizes; the
         // per-frame values live in frame_dev, so a captured graph replays as is.
         char head[512];
-        std::snprintf(head, sizeof(head), "%p|%p|%llu|%u|%u|%u|%llu|%u|%p|%p|%p|%p|%p|%p|%u|%s|", (void*)s, (void*)c,
+        std::snprintf(head, sizeof(head), "%p|%p|%llu|%u|%u|%u|%llu|%u|%p|%p|%p|%p|%u|%s|", (void*)s, (void*)c,
                       (unsigned long long)s->gpu.generation, npix, spp, r->cfg.path_depth,
-                      (unsigned long long)npaths, chunk, (void*)w.q_o[0], (void*)w.radiance, (void*)w.contrib,
-                      (void*)w.counters, (void*)c->accum.ptr, (void*)w.primary,
-                      r->cfg.russian_roulette | (r->cfg.traversal << 1), launch_shape_key(r).c_str());
-        const std::string key = std::string(head) + scene_view_key(sv);
+                      (unsigned long long)npaths, chunk, (void*)r->frame_dev.ptr, (void*)c->accum.ptr,
+                      (void*)c->sum64.ptr, (void*)c->bgra.ptr, r->cfg.russian_roulette | (r->cfg.traversal << 1),
+                      launch_shape_key(r).c_str());
+        const std::string key = head + wave_key(w) + scene_view_key(sv);
         if (!r->graph_exec || r->graph_key != key) {
             if (r->graph_exec) {
                 cudaGraphExecDestroy(r->graph_exec);
@@ -545,7 +557,7 @@ void render_batch(kf_renderer_s* r, const kf_batch_item* items, uint32_t count) 
     if (r->wave.hit_item.count < chunk) r->wave.hit_item.resize(chunk, st);
     B.items.resize(count, st);
     KF_CUDA_CHECK(cudaMemcpyAsync(B.items.ptr, hv.data(), sizeof(ItemDev) * count, cudaMemcpyHostToDevice, st));
-    WaveDev w = wave_view(r, items[0].camera, r->cfg.path_depth, max_slots > 0);
+    WaveDev w = wave_view(r, nullptr, r->cfg.path_depth, max_slots);
     w.path_item = r->wave.path_item.ptr;
     w.hit_item = r->wave.hit_item.ptr;
     const BatchDev bd{B.items.ptr, count, 0};
@@ -557,16 +569,14 @@ void render_batch(kf_renderer_s* r, const kf_batch_item* items, uint32_t count) 
     cudaEvent_t f0 = r->ev[4], f1 = r->ev[5];
     if (profile) KF_CUDA_CHECK(cudaEventRecord(f0, st));
     if (r->cfg.use_graph && !profile && !r->count_traversal) {
-        std::string key;
         // the items (sizes, samples, targets, lights) live in device memory; what a graph bakes
         // in are the wave buffers, the pools and the launch counts
-        char buf[256];
-        std::snprintf(buf, sizeof(buf), "%llu|%u|%llu|%u|%llu|%p|%p|%p|%p|%p|%p|%p|%p|%u|%u|%u|%u|",
-                      (unsigned long long)B.generation, count, (unsigned long long)total, chunk,
-                      (unsigned long long)resolve_blocks, (void*)w.q_o[0], (void*)w.radiance, (void*)w.contrib,
-                      (void*)w.counters, (void*)w.path_item, (void*)w.hit_item, (void*)w.primary, (void*)B.items.ptr,
-                      w.nslot, w.lit, r->cfg.path_depth, r->cfg.russian_roulette | (r->cfg.traversal << 1));
-        key = buf + launch_shape_key(r) + "|" + scene_view_key(B.view);
+        char head[512];
+        std::snprintf(head, sizeof(head), "%llu|%u|%llu|%u|%llu|%p|%u|%u|%s|", (unsigned long long)B.generation, count,
+                      (unsigned long long)total, chunk, (unsigned long long)resolve_blocks, (void*)B.items.ptr,
+                      r->cfg.path_depth, r->cfg.russian_roulette | (r->cfg.traversal << 1),
+                      launch_shape_key(r).c_str());
+        const std::string key = head + wave_key(w) + scene_view_key(B.view);
         if (!B.graph_exec || B.graph_key != key) {
             if (B.graph_exec) {
                 cudaGraphExecDestroy(B.graph_exec);

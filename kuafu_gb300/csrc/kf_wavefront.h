@@ -109,7 +109,7 @@ struct WaveDev {
     uint32_t* hit_inst;   // instance, or all ones on a miss (apart: k_miss reads this word of every ray only)
     uint32_t* sel;        // queue positions of this bounce's rays that hit
     uint32_t* scount;     // kSlotRow words per depth: slot j's shadow rays, at sq_o/sq_d[j * chunk_cap + k]
-    uint32_t nslot;       // light slots with a shadow queue (scount entries)
+    uint32_t nslot;       // light slots of the launch, each with a shadow queue (scount entries)
     uint32_t lit;         // some view of the launch has a light slot (else no NEE is recorded)
     float4* nee_w;        // per hit: throughput that scales this bounce's NEE + path id and flag bits
     float4* nee_in;       // per hit, 5 arrays of chunk_cap: what k_nee needs of k_shade's shading
@@ -128,6 +128,7 @@ struct WaveDev {
     uint16_t* path_item;       // batched launch: item of each path of the chunk
     uint16_t* hit_item;        // batched launch: item of each hit
     uint32_t chunk_cap;
+    uint32_t pad; // no padding bytes: a captured launch is known by this struct's
 };
 
 // Every launcher takes the batch description b: b.items == nullptr renders the single

@@ -200,3 +200,47 @@ def test_changed_lights_reach_the_next_frame():
 
     assert _same(render(1), render(0))
     assert not _same(render(1), render(2))
+
+
+def test_replayed_frames_follow_buffers_that_moved():
+    """Frames between which other launches grow the wavefront's buffers (more light slots, more
+    paths, deeper paths) and a camera is resized to and fro: captured launches against direct ones."""
+    light = lambda k: api.PointLight(position=(-10.0 + 3 * k, 5.0 - k, 4.0 + k), radius=0.2, strength=200.0)
+
+    def render(use_graph):
+        cfg = scenes.icosphere_config(spp=2, depth=4, count=64)
+        cfg.setUseGraph(use_graph)
+        out = []
+        with api.Kuafu(cfg) as r:
+            s, many = r.getScene(), r.createScene()
+            cam = scenes.icospheres(r, 150, 130, count=8, level=2, seed=3, scene=s)
+            wide = scenes.icospheres(r, 211, 190, count=8, level=2, seed=4, scene=many)
+            s.removeLights()
+            s.addPointLight(light(0))
+            for k in range(9):
+                many.addPointLight(light(k))
+
+            def frame():
+                r.resetFrame()
+                r.run()
+                out.append([_aov(r, cam, k) for k in AOVS[:6]])
+
+            frame()
+            r.runBatch([(many, wide, 3)])
+            out.append([_aov(r, wide, AOVS[0])])
+            frame()
+            cam.setSize(170, 140)
+            r.runBatch([(s, cam, 1), (many, wide, 2)])
+            cam.setSize(150, 130)
+            frame()
+            r.config.setPathDepth(7)
+            r.applyConfig()
+            r.runBatch([(many, wide, 3)])
+            r.config.setPathDepth(4)
+            r.applyConfig()
+            frame()
+        return out
+
+    for n, (a, b) in enumerate(zip(render(True), render(False))):
+        for k, (x, y) in enumerate(zip(a, b)):
+            assert _same(x, y), (n, k)

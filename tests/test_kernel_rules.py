@@ -102,3 +102,14 @@ def test_one_lane_of_a_shared_path_writes_its_aovs():
     for m in re.finditer(r"w\.(radiance|primary|albedo|normal|depth|seg)\[[^\]]*\]\s*=[^=]", body):
         line = body[body.rindex("\n", 0, m.start()):m.start()]
         assert any("sub == 0" in h for h in _headers_at(body, m.start()) + [line]), m.group(0)
+
+
+def test_captured_launches_are_known_by_all_of_the_wavefront_state():
+    """A captured launch sequence bakes in the wavefront state by value. Its key takes every byte of
+    it: with a few addresses only, a replay could read buffers that were freed since (an allocator
+    may return one of them to its old place and not the others)."""
+    s = _source("kf_render.cu")
+    assert "sizeof(w)" in _function(s, "wave_key")
+    for f in ("render_frame", "render_batch"):
+        (key,) = re.findall(r"std::string key = ([^;]*);", _function(s, f))
+        assert "wave_key(w)" in key
