@@ -470,14 +470,20 @@ KF_API int kf_renderer_download_aov(kf_renderer r, kf_camera cam, int kind, void
             default: throw KfError(KF_ERR_INVALID_ARGUMENT, "unknown AOV kind");
         }
         KF_REQUIRE(bytes >= need, KF_ERR_OUT_OF_RANGE, "output buffer too small for the AOV");
-        if (path_words) {
-            DeviceBuffer<float4> slice; // one sample's image at a time
-            slice.resize(npix * path_words, r->stream);
-            for (uint32_t k = 0; k < c->last_spp; ++k) {
-                launch_sample_slice(static_cast<const float4*>(src), (uint32_t)npix, c->last_spp, k, path_words,
-                                    slice.ptr, r->stream);
-                KF_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t*>(out) + k * slice.bytes(), slice.ptr, slice.bytes(),
-                                              cudaMemcpyDeviceToHost, r->stream));
+        if (path_words && c->last_spp > 1) {
+            // reordered in the largest buffer of the bounce loop, which is idle between frames and holds
+            // five float4 per path in flight: one kernel and one copy for all paths, or as many as the
+            // frame was cut into chunks (a copy per sample took 13.6 ms for 64 x 64 pixels at 1024
+            // samples, 67 MB, of which the copy itself is 0.4)
+            const DeviceBuffer<float4>& scratch = r->wave.nee_in;
+            const uint64_t paths = (uint64_t)c->last_spp * npix, part = scratch.count / path_words;
+            const size_t path_bytes = (size_t)path_words * sizeof(float4);
+            for (uint64_t first = 0; first < paths; first += part) {
+                const uint32_t n = (uint32_t)std::min<uint64_t>(part, paths - first);
+                launch_sample_major(static_cast<const float4*>(src), (uint32_t)npix, c->last_spp, path_words, first, n,
+                                    scratch.ptr, r->stream);
+                KF_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t*>(out) + first * path_bytes, scratch.ptr,
+                                              n * path_bytes, cudaMemcpyDeviceToHost, r->stream));
             }
             sync_stream(r);
             return;

@@ -59,8 +59,8 @@ struct AnyHitCtx {
     Stream st;
 };
 
-// Pixel and sample of path g of a view (pixel-major): a 32-bit division whenever g fits
-// in 32 bits (a view below 2^32 paths), the 64-bit one otherwise.
+// Pixel and sample of path g of a view (pixel-major; quotient and remainder): a 32-bit division
+// whenever g fits in 32 bits (a view below 2^32 paths), the 64-bit one otherwise.
 __device__ __forceinline__ void split_path(uint64_t g, uint32_t spp, uint32_t& pix, uint32_t& sample) {
     if ((g >> 32) == 0) {
         const uint32_t g32 = (uint32_t)g;
@@ -1930,13 +1930,15 @@ __global__ void __launch_bounds__(kResolvePix) k_resolve(const FrameDev* __restr
     bgra[pix] = make_uchar4(srgb8(s_thresh, out.z), srgb8(s_thresh, out.y), srgb8(s_thresh, out.x), 255);
 }
 
-// One sample of a per-path buffer as an image (downloads of path data are sample-major).
-__global__ void k_sample_slice(const float4* __restrict__ src, uint32_t npix, uint32_t spp, uint32_t sample,
-                               uint32_t words, float4* dst) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npix) return;
+// Part of a per-path buffer in sample-major order (downloads of path data).
+__global__ void k_sample_major(const float4* __restrict__ src, uint32_t npix, uint32_t spp, uint32_t words,
+                               uint64_t first, uint32_t n, float4* dst) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    uint32_t sample, pix;
+    split_path(first + k, npix, sample, pix);
     for (uint32_t q = 0; q < words; ++q)
-        dst[(size_t)i * words + q] = src[((size_t)i * spp + sample) * words + q];
+        dst[(size_t)k * words + q] = src[((size_t)pix * spp + sample) * words + q];
 }
 
 // Linear RGBA32F -> B8G8R8A8 sRGB.
@@ -2130,9 +2132,9 @@ void launch_resolve_batch(const BatchDev& b, const float4* radiance, uint32_t bl
     k_resolve<true><<<blocks, kResolvePix, 0, st>>>(nullptr, b, radiance, 0, 0, nullptr, nullptr, nullptr);
     KF_CUDA_CHECK(cudaGetLastError());
 }
-void launch_sample_slice(const float4* src, uint32_t npix, uint32_t spp, uint32_t sample, uint32_t words, float4* dst,
-                         cudaStream_t st) {
-    k_sample_slice<<<(npix + 255) / 256, 256, 0, st>>>(src, npix, spp, sample, words, dst);
+void launch_sample_major(const float4* src, uint32_t npix, uint32_t spp, uint32_t words, uint64_t first, uint32_t n,
+                         float4* dst, cudaStream_t st) {
+    k_sample_major<<<(n + 255) / 256, 256, 0, st>>>(src, npix, spp, words, first, n, dst);
     KF_CUDA_CHECK(cudaGetLastError());
 }
 void launch_srgb(const float4* img, uint32_t npix, uchar4* out, cudaStream_t st) {

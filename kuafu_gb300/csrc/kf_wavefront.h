@@ -177,10 +177,10 @@ void launch_resolve(const FrameDev* f, const float4* radiance, uint32_t npix, ui
                     dbl4* sum64, uchar4* bgra, cudaStream_t st);
 // The same for every view of a batch in one launch (blocks: the items' resolve blocks in all).
 void launch_resolve_batch(const BatchDev& b, const float4* radiance, uint32_t blocks, cudaStream_t st);
-// dst[pix] = src[pix * spp + sample] of `words` float4 per path: one sample of a per-path buffer
-// as an image (downloads are sample-major).
-void launch_sample_slice(const float4* src, uint32_t npix, uint32_t spp, uint32_t sample, uint32_t words, float4* dst,
-                         cudaStream_t st);
+// Paths first .. first + n - 1 of a per-path buffer (`words` float4 each) in sample-major order, as
+// downloads have them: dst[k] = src[pix * spp + sample] with sample * npix + pix = first + k.
+void launch_sample_major(const float4* src, uint32_t npix, uint32_t spp, uint32_t words, uint64_t first, uint32_t n,
+                         float4* dst, cudaStream_t st);
 void launch_srgb(const float4* img, uint32_t npix, uchar4* out, cudaStream_t st);
 void upload_srgb_thresholds(const float* thresh256);
 void launch_relmse(const float4* x, const float4* ref, uint64_t n, double eps, double* partial, uint32_t blocks,

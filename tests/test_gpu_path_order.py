@@ -244,3 +244,36 @@ def test_replayed_frames_follow_buffers_that_moved():
     for n, (a, b) in enumerate(zip(render(True), render(False))):
         for k, (x, y) in enumerate(zip(a, b)):
             assert _same(x, y), (n, k)
+
+
+@pytest.mark.parametrize("kind,words", [(N.KF_AOV_PATH_RADIANCE, 1), (N.KF_AOV_PRIMARY_HITS, 2)])
+def test_path_data_comes_in_one_copy(kind, words):
+    """A download of per-path data costs about what its bytes cost: at 64 x 64 pixels and 1024
+    samples at most three times a plain copy of as many bytes to ordinary memory (a copy per sample
+    takes 37 times as long). Best of several, both sides."""
+    import time
+
+    import torch
+
+    w, h, spp = 64, 64, 1024
+    cfg = scenes.cornell_config(spp=spp, depth=2)
+    cfg.setDebugOutputs(True)
+    out = np.zeros(w * h * spp * 4 * words, np.float32)
+    plain, host = torch.zeros(out.size, device="cuda"), torch.from_numpy(out)
+    with api.Kuafu(cfg) as r:
+        cam = scenes.cornell(r, w, h)
+        r.run()
+
+        def best(f):
+            times = []
+            for _ in range(9):
+                torch.cuda.synchronize()
+                t = time.perf_counter()
+                f()
+                torch.cuda.synchronize()
+                times.append(time.perf_counter() - t)
+            return min(times)
+
+        copy = best(lambda: host.copy_(plain))
+        got = best(lambda: N.check(N.load().kf_renderer_download_aov(r._h, cam._h, kind, out.ctypes.data, out.nbytes)))
+    assert got <= 3.0 * copy, (got, copy)
