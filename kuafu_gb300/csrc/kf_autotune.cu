@@ -4,7 +4,9 @@
 // scheduling (refill threshold, steps between refills) and the BLAS leaf size (the BVH
 // shape), one knob at a time (coordinate descent), each candidate timed with CUDA events
 // on the renderer's stream over `reps` batches after one warm-up batch (which also
-// captures the batch graph and, for a new leaf size, rebuilds every BLAS).
+// captures the batch graph and, for a new leaf size, rebuilds every BLAS). A candidate that leaves
+// the launch as it is (small batches run whole paths in one kernel) is not taken however its time
+// came out.
 //
 // It also holds the L2 read-bandwidth probe that the traversal's roofline is stated
 // against: the achievable rate at which this GPU's SMs read data that sits in L2.
@@ -76,13 +78,22 @@ void autotune_batch(kf_renderer_s* r, const kf_batch_item* items, uint32_t count
     float best_ms = time_batch(r, items, count, reps);
     const float start_ms = best_ms;
     uint32_t tried = 1;
+    auto runs_whole = [&] {
+        bool lit = false;
+        for (const kf_scene_s* s : scenes) lit = lit || s->gpu.view.num_slots > 0;
+        return runs_whole_paths(r, lit, total);
+    };
+    bool best_whole = runs_whole();
     auto consider = [&](Knobs k) {
         apply(r, scenes, k);
         const float ms = time_batch(r, items, count, reps);
         ++tried;
+        const bool whole = runs_whole();
+        if (whole && best_whole && k.leaf == best.leaf) return; // the same launch
         if (ms < best_ms) {
             best_ms = ms;
             best = k;
+            best_whole = whole;
         }
     };
     // 1. traversal kernel

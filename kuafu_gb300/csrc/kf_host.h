@@ -237,6 +237,9 @@ void render_frame(kf_renderer_s* r, kf_scene_s* s, kf_camera_s* c, uint32_t spp)
 void batch_sync(kf_renderer_s* r, const std::vector<kf_scene_s*>& scenes);
 // One frame of every (scene, camera, spp) item in one wavefront (kf_renderer_run_batch).
 void render_batch(kf_renderer_s* r, const kf_batch_item* items, uint32_t count);
+// Whether a launch of npaths paths runs them whole in one kernel, into which neither the chunk size
+// nor the grids nor the persistent traversal's scheduling enter (lit: some view has lights to sample).
+bool runs_whole_paths(const kf_renderer_s* r, bool lit, uint64_t npaths);
 // kf_renderer_autotune (kf_autotune.cu)
 void autotune_batch(kf_renderer_s* r, const kf_batch_item* items, uint32_t count, uint32_t reps,
                     kf_autotune_result* out);

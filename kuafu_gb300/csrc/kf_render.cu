@@ -250,6 +250,21 @@ WaveDev wave_view(kf_renderer_s* r, kf_camera_s* c, uint32_t max_depth, uint32_t
 
 } // namespace
 
+static uint32_t chunk_for(const kf_renderer_s* r, uint64_t npaths) {
+    uint64_t cap = r->cfg.max_paths_in_flight ? r->cfg.max_paths_in_flight : (1ull << 24);
+    cap = std::min<uint64_t>(cap, (1ull << 26) - 1);
+    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(npaths, cap));
+}
+
+// A small launch: whole paths in one kernel, and one for the last of a lit wavefront's paths (the
+// thread-per-ray setting, profiling and counting ask for the wavefront's kernels).
+static bool may_run_whole_paths(const kf_renderer_s* r) {
+    return r->cfg.traversal == 1 && !r->cfg.profile && !r->count_traversal;
+}
+bool runs_whole_paths(const kf_renderer_s* r, bool lit, uint64_t npaths) {
+    return may_run_whole_paths(r) && npaths <= chunk_for(r, npaths) && npaths <= (lit ? kPathsMaxLit : kPathsMax);
+}
+
 // The bounce loop on two streams. Bounce d's shadow traversal and NEE gather (stream2)
 // overlap bounce d+1's closest-hit traversal (stream): they share no buffer — the closest-hit
 // kernel reads the next ray queue and writes hit records, the shadow kernel reads the shadow
@@ -264,10 +279,8 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
                           const WaveDev& w, uint32_t max_depth, uint64_t npaths, uint32_t chunk, bool profile) {
     cudaStream_t st = r->stream, st2 = profile ? r->stream : r->stream2;
     const bool dyn = r->cfg.traversal == 1, lit = w.lit != 0, fork = lit && !profile;
-    // a small launch: whole paths in one kernel, and one for the last of a lit wavefront's paths (the
-    // thread-per-ray setting, profiling and counting ask for the wavefront's kernels)
-    const bool whole = dyn && !profile && !r->count_traversal;
-    if (whole && npaths <= chunk && npaths <= (lit ? kPathsMaxLit : kPathsMax)) {
+    const bool whole = may_run_whole_paths(r);
+    if (runs_whole_paths(r, lit, npaths)) {
         launch_paths(sv, fd, b, w, (uint32_t)npaths, max_depth, (uint32_t)r->num_sms, st);
         return;
     }
@@ -404,12 +417,6 @@ static std::string scene_view_key(const SceneDev& v) {
 static std::string wave_key(const WaveDev& w) {
     static_assert(std::has_unique_object_representations_v<WaveDev>, "no padding: the bytes are the key");
     return std::string(reinterpret_cast<const char*>(&w), sizeof(w));
-}
-
-static uint32_t chunk_for(const kf_renderer_s* r, uint64_t npaths) {
-    uint64_t cap = r->cfg.max_paths_in_flight ? r->cfg.max_paths_in_flight : (1ull << 24);
-    cap = std::min<uint64_t>(cap, (1ull << 26) - 1);
-    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(npaths, cap));
 }
 
 void render_frame(kf_renderer_s* r, kf_scene_s* s, kf_camera_s* c, uint32_t spp) {

@@ -134,3 +134,18 @@ def test_batch_replay_and_scene_change():
         assert np.isfinite(hits).all()
         with pytest.raises(N.KfError):
             r.runBatch([(s0, c0, 1), (s0, c0, 1)])  # a camera twice
+
+
+def test_autotune_keeps_settings_that_do_not_enter_the_launch():
+    """A batch small enough for whole paths in one kernel has no chunks, shading grids or ray fetches:
+    the tuner leaves those settings alone (whichever of them happened to be timed fastest)."""
+    cfg = scenes.batch_config(depth=3)
+    with api.Kuafu(cfg) as r:
+        items = scenes.batch_views(r, n_scenes=2, cams_per_scene=2, seed=3, min_side=32, max_side=64,
+                                   spp_range=(1, 3), inst_range=(3, 12), level=2, variants=2)
+        refill, steps = r.config._c.dyn_refill_below, r.config._c.dyn_steps
+        res = r.autotune(items, reps=1)
+        assert res.traversal == 1  # one kernel against a wavefront of a dozen launches a bounce
+        assert (res.dyn_refill_below, res.dyn_steps) == (refill, steps)
+        assert res.max_paths_in_flight == res.start_max_paths_in_flight
+        assert res.grid_shade == res.grid_extend  # both 16 blocks per SM from the start
