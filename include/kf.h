@@ -336,6 +336,12 @@ KF_API int kf_renderer_measure_l2_read(kf_renderer r, uint64_t bytes, uint32_t p
  * 32 (or 16 for images at least 96 wide); x, weight and y 16-byte aligned. */
 KF_API int kf_conv3x3_bf16(const void* x, int n, int h, int w, int cin, const void* weight, int w_rows,
                            const float* bias, int cout, int relu, void* y, int y_cstride, int y_coff, void* stream);
+/* Weight and bias gradients of that convolution, added to dw and db: dw[tap][co][ci] += sum over
+ * pixels of dz[n,y,x,co] * x[n,y+dy,x+dx,ci], db[co] += sum of dz[n,y,x,co], for co < cout. x: NHWC
+ * BF16 with a channel stride x_cstride >= cin (a multiple of 8), dz: dense [n][h][w][dz_channels]
+ * BF16; cin and dz_channels multiples of 32; x and dz 16-byte aligned; FP32 accumulation. */
+KF_API int kf_conv3x3_wgrad_bf16(const void* x, int x_cstride, int n, int h, int w, int cin, const void* dz,
+                                 int dz_channels, int cout, float* dw, float* db, void* stream);
 /* d[m][n] += sum_k a[m][k] * b[n][k], BF16 K-major operands (16-byte aligned, k % 8 == 0),
  * FP32 accumulation into d (row stride ldd >= n) by split-K atomics: d is added to, not
  * overwritten. */

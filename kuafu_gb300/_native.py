@@ -232,6 +232,7 @@ PROTOTYPES = {
     "kf_relmse_noalloc": (I, [VP, VP, C.c_uint64, C.c_double, VP, C.POINTER(C.c_double)]),
     "kf_renderer_measure_l2_read": (I, [VP, C.c_uint64, C.c_uint32, C.c_uint32, C.POINTER(C.c_double)]),
     "kf_conv3x3_bf16": (I, [VP, I, I, I, I, VP, I, VP, I, I, VP, I, I, VP]),
+    "kf_conv3x3_wgrad_bf16": (I, [VP, I, I, I, I, I, VP, I, I, VP, VP, VP]),
     "kf_gemm_bf16_tn": (I, [VP, I, VP, I, I, VP, I, I, VP]),
     "kf_tc_error": (I, [C.POINTER(U32)]),
     "kf_tc_wait_probe": (I, [C.c_uint64, VP]),

@@ -1293,6 +1293,15 @@ KF_API int kf_conv3x3_bf16(const void* x, int n, int h, int w, int cin, const vo
                      static_cast<cudaStream_t>(stream));
     });
 }
+KF_API int kf_conv3x3_wgrad_bf16(const void* x, int x_cstride, int n, int h, int w, int cin, const void* dz,
+                                 int dz_channels, int cout, float* dw, float* db, void* stream) {
+    return guarded([&] {
+        REQ(x && dz && dw && db, "null tensor");
+        conv3x3_wgrad_bf16(static_cast<const __nv_bfloat16*>(x), x_cstride, n, h, w, cin,
+                           static_cast<const __nv_bfloat16*>(dz), dz_channels, cout, dw, db,
+                           static_cast<cudaStream_t>(stream));
+    });
+}
 KF_API int kf_gemm_bf16_tn(const void* a, int m, const void* b, int n, int k, float* d, int ldd, int splits,
                            void* stream) {
     return guarded([&] {

@@ -1596,6 +1596,11 @@ void conv3x3_wgrad_bf16(const __nv_bfloat16* x, int x_cstride, int N, int H, int
                KF_ERR_INVALID_ARGUMENT, "wgrad: channels must be multiples of 32");
     KF_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)dz & 15) == 0 && x_cstride % 8 == 0, KF_ERR_INVALID_ARGUMENT,
                "wgrad: tensors must be 16-byte aligned");
+    KF_REQUIRE(x_cstride >= Cin, KF_ERR_INVALID_ARGUMENT, "wgrad: channel stride below the input channels");
+    KF_REQUIRE(((uintptr_t)dw & 3) == 0 && ((uintptr_t)db & 3) == 0, KF_ERR_INVALID_ARGUMENT,
+               "wgrad: gradients must be 4-byte aligned");
+    KF_REQUIRE((int64_t)((W + 7) / 8) * ((H + kWgRows - 1) / kWgRows) * N <= (1 << 30), KF_ERR_LIMIT,
+               "wgrad: too many pixels in one call");
     WgradParams p{};
     // K steps are 16 pixels of a row, or two rows of 8 where the image is that narrow; 32-pixel
     // tiles halve the halo columns where they leave no more padding than 16-pixel ones

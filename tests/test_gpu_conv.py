@@ -86,6 +86,70 @@ def test_conv3x3_tiles_of_narrow_images(n, h, w, cin, cout, rows, relu, cstride,
     test_conv3x3_matches_torch(n, h, w, cin, cout, rows, relu, cstride, coff)
 
 
+# The weight-gradient kernel by itself: pixel tiles of 8 rows by 8, 16 or 32 pixels with remainders of
+# 1 and all but 1 in both directions, images smaller than a tile, more tiles than CTAs, one and
+# several blocks of 32 input and of 32 or 64 output channels, channel slices, a head of 3 channels.
+# Operands are small integers, so every product and every sum stays an integer below 2^24: whatever
+# the order of the sums, FP32 holds them exactly, and the result has to be equal.
+@pytest.mark.parametrize("n,h,w,cin,cstride,coff,dzc,cout", [
+    (1, 1, 1, 32, 32, 0, 32, 32),
+    (2, 3, 7, 32, 64, 32, 64, 64),
+    (1, 9, 8, 64, 64, 0, 32, 3),
+    (3, 17, 9, 32, 40, 8, 96, 96),
+    (1, 8, 15, 96, 96, 0, 64, 40),
+    (2, 7, 16, 32, 32, 0, 160, 160),
+    (1, 20, 17, 160, 288, 128, 64, 64),
+    (2, 33, 24, 64, 64, 0, 96, 80),
+    (1, 5, 31, 32, 96, 64, 32, 32),
+    (1, 16, 33, 32, 32, 0, 64, 64),
+    (2, 12, 40, 96, 160, 64, 32, 32),
+    (1, 10, 63, 32, 32, 0, 160, 130),
+    (1, 24, 64, 288, 288, 0, 128, 128),
+    (5, 130, 150, 32, 32, 0, 32, 32),
+    (16, 64, 97, 64, 96, 32, 64, 64),
+])
+def test_weight_gradients_are_exact_on_integers(n, h, w, cin, cstride, coff, dzc, cout):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(n * 1000 + 10 * h + w)
+
+    def ints(*shape):
+        return torch.randint(-3, 4, shape, device="cuda", generator=g)
+
+    x, dz = ints(n, h, w, cstride), ints(n, h, w, dzc)
+    dw, db = ints(9, cout, cin).float(), ints(cout).float()  # gradients are added to what is there
+    xs = x[..., coff:coff + cin].double()
+    z = dz[..., :cout].double().reshape(-1, cout)
+    pad = torch.nn.functional.pad(xs, (0, 0, 1, 1, 1, 1))
+    want_w = dw.double() + torch.stack([z.T @ pad[:, t // 3:t // 3 + h, t % 3:t % 3 + w].reshape(-1, cin)
+                                        for t in range(9)])
+    want_b = db.double() + z.sum(0)
+    xb, zb = x.to(torch.bfloat16), dz.to(torch.bfloat16)
+    torch.cuda.synchronize()
+    N.check(N.load().kf_conv3x3_wgrad_bf16(xb.data_ptr() + 2 * coff, cstride, n, h, w, cin, zb.data_ptr(), dzc, cout,
+                                           dw.data_ptr(), db.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert _tc_error() == 0
+    assert torch.equal(dw.double(), want_w)
+    assert torch.equal(db.double(), want_b)
+
+
+def test_weight_gradients_refuse_what_the_kernel_cannot_read():
+    """Refused on the host: channels that are not multiples of 32, a stride below the channels, null
+    and misaligned tensors, empty images."""
+    import torch
+
+    x = torch.zeros((1, 8, 8, 64), device="cuda", dtype=torch.bfloat16)
+    out = torch.zeros(9 * 64 * 64, device="cuda")
+    good = dict(x=x.data_ptr(), xs=64, n=1, h=8, w=8, cin=64, dz=x.data_ptr(), dzc=64, cout=64, dw=out.data_ptr(),
+                db=out.data_ptr())
+    for bad in (dict(cin=48), dict(dzc=48), dict(xs=32), dict(cout=65), dict(cout=0), dict(n=0), dict(w=0),
+                dict(x=x.data_ptr() + 2), dict(dz=x.data_ptr() + 8), dict(dw=None), dict(db=out.data_ptr() + 2)):
+        a = {**good, **bad}
+        with pytest.raises(N.KfError):
+            N.check(N.load().kf_conv3x3_wgrad_bf16(*a.values(), None))
+
+
 @pytest.mark.parametrize("m,n,k,splits", [(200, 96, 4096, 4), (128, 32, 64, 1), (77, 160, 1000, 3)])
 def test_gemm_tn_matches_torch(m, n, k, splits):
     import torch
