@@ -8,7 +8,11 @@ issued; BVH build is outside the timed region.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-The line also carries "time_to_relmse": the Cornell box at 1920x1080, the learned
+The line is one JSON object of at most 2800 characters (a reader that keeps the end of the output
+gets it whole): the measured value with its configuration, and the main figures of what else ran.
+Everything measured goes to stderr, a line "detail NAME: JSON" for each part.
+
+"time_to_relmse": the Cornell box at 1920x1080, the learned
 denoiser (trained first on this renderer's own low/high-spp pairs) against plain
 accumulation, both measured until relMSE <= 1e-3 against a 40960-spp FP64
 reference (kuafu_gb300/denoise_eval.py; --no-denoise skips it; N = 1 only). The
@@ -483,6 +487,61 @@ def run_denoiser_profile(reps: int) -> int:
     return 0
 
 
+LINE_LIMIT = 2800  # characters of the result line
+CONTRACT = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "e2e", "clocks", "gpu_launches")
+
+
+def _short(x):
+    """x with its floats at six significant digits."""
+    if isinstance(x, float):
+        return float(f"{x:.6g}")
+    if isinstance(x, dict):
+        return {k: _short(v) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [_short(v) for v in x]
+    return x
+
+
+def _pick(d, *keys):
+    """The entries of d under keys that are there (d may be None or an error record)."""
+    d = d if isinstance(d, dict) else {}
+    return {k: d[k] for k in keys + ("error",) if d.get(k) is not None}
+
+
+def result_line(full: dict) -> str:
+    """The printed line of a full result: the contract's entries as they are, then the main figures of
+    each further part, as many as LINE_LIMIT leaves room for."""
+    line = {k: full[k] for k in CONTRACT if k in full}
+    ttr = full.get("time_to_relmse") or {}
+    heads = {"in_run": ttr.get("headline"), "shipped": (ttr.get("shipped_network") or {}).get("headline"),
+             "mixed": (ttr.get("mixed_network") or {}).get("headline"),
+             "icospheres_mixed": (ttr.get("icosphere_headline") or {}).get("mixed")}
+    batched = full.get("batched") or {}
+    parts = {
+        "roofline": _pick(full.get("roofline"), "bound", "kernel", "achieved", "peak", "unit", "frac", "traffic"),
+        "time_to_relmse": {**_pick(ttr, "headline_tau"), **{k: _pick(h, "plain_ms", "denoised_ms", "speedup")
+                                                           for k, h in heads.items() if h}},
+        "denoiser_roofline": _pick(ttr.get("denoiser_roofline"), "bound", "achieved", "peak", "unit", "frac"),
+        "batched": {**_pick(batched), **{k: _pick(batched.get(k), "ms_per_batch", "mrays_s")
+                                         for k in ("default", "autotuned") if batched.get(k)}},
+        "active_light": _pick(full.get("active_light"), "ms_per_batch", "mrays_s", "rgb_denoise_ms"),
+        "cpu_baseline": _pick(full.get("cpu_baseline"), "value", "unit", "cores", "kind", "sample"),
+        "bvh_build_ms": {k: v for k, v in (full.get("bvh_build_ms") or {}).items() if k != "note"},
+    }
+    for name, part in parts.items():
+        if part and len(json.dumps({**line, name: _short(part)})) <= LINE_LIMIT:
+            line[name] = _short(part)
+    return json.dumps(line)
+
+
+def print_result(full: dict) -> None:
+    for name, part in full.items():
+        if isinstance(part, dict):
+            print(f"detail {name}: {json.dumps(part)}", file=sys.stderr, flush=True)
+    print(result_line(full), flush=True)
+
+
 def run_reference(args):
     ws, rank, local = _dist()
     if rank != 0:
@@ -687,7 +746,7 @@ def run_ours(args):
             result["batched"] = batched
         if active is not None:
             result["active_light"] = active
-        print(json.dumps(result), flush=True)
+        print_result(result)
     else:
         r.close()
     _finish_ranks(ws)
