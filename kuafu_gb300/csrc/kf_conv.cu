@@ -345,7 +345,7 @@ __device__ __forceinline__ void mask16(const __nv_bfloat16* m, uint32_t (&w)[8])
         }
     }
 }
-// ((a + b) + c) + d, quartered, of packed BF16 pairs: the order of the separate pooling pass
+// ((a + b) + c) + d in FP32, quartered, of packed BF16 pairs: the order the pooled values are defined by
 __device__ __forceinline__ uint32_t pool_pair(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     const float lo = 0.25f * (((__uint_as_float(a << 16) + __uint_as_float(b << 16)) + __uint_as_float(c << 16)) +
                               __uint_as_float(d << 16));

@@ -8,9 +8,8 @@
 
 namespace kf {
 
-// Work a convolution can take over from the pass that follows it: 2x2 average pooling of
-// its BF16 output into a dense [N][H/2][W/2][Cout] tensor. The values equal those of the
-// separate pass (both read the BF16-rounded outputs).
+// Work a convolution can take over from what follows it: 2x2 average pooling of its BF16 output into
+// a dense [N][H/2][W/2][Cout] tensor (FP32 averages of the rounded outputs, rounded to BF16).
 // And a ReLU's backward mask: outputs whose place in `mask` (NHWC, channel stride mask_cs, slice
 // starting at mask_co, both multiples of 8) is not positive become zero.
 // And nearest 2x upsampling of the BF16 output into the channel slice up_co of an NHWC tensor
@@ -38,8 +37,8 @@ struct ConvFuse {
 // Cout_rows a multiple of 16 (rows >= Cout are computed and dropped); Cin % 32 == 0, or
 // Cin == 16 for images at least 96 wide.
 // With y_f32 set, the output is written there in FP32 (same strides) and y is unused.
-// Returns true when it also did the pooling asked for in `fuse` (the persistent kernels do it for
-// suitable shapes; otherwise the caller runs the separate pass). A mask is always applied (at
+// Returns true when it also did the pooling asked for in `fuse` (the persistent kernels do it for even
+// sizes and, from 96 pixels wide on, up to 128 output channels). A mask is always applied (at
 // most 288 input channels then).
 bool conv3x3_bf16(const __nv_bfloat16* x, int N, int H, int W, int Cin, const __nv_bfloat16* w, int Cout_rows,
                   const float* bias, int Cout, bool relu, __nv_bfloat16* y, int y_cstride, int y_coff,

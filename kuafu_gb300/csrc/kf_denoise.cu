@@ -56,25 +56,6 @@ __device__ __forceinline__ void st8(bf16* p, const F8& f) {
     *reinterpret_cast<uint4*>(p) = q;
 }
 
-// y (dense, H/2 x W/2) = 2x2 average of x[slice] (H x W)
-__global__ void k_pool_fwd(const bf16* __restrict__ x, int xs, int xo, int C, int N, int H, int W, bf16* y) {
-    grid_dependency_wait();
-    const int Ho = H / 2, Wo = W / 2, G = C / 8;
-    const size_t total = (size_t)N * Ho * Wo * G;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int g = (int)(i % G);
-        const size_t pix = i / G; // (n, yh, xw) of the output
-        const int xw = (int)(pix % Wo);
-        const size_t ny = pix / Wo; // n * Ho + yh
-        const size_t row0 = (2 * ny) * W + 2 * xw; // n * H + 2 yh == 2 * (n * Ho + yh)
-        F8 a = ld8(x + row0 * xs + xo + 8 * g), b = ld8(x + (row0 + 1) * xs + xo + 8 * g);
-        const F8 c = ld8(x + (row0 + W) * xs + xo + 8 * g), d = ld8(x + (row0 + W + 1) * xs + xo + 8 * g);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) a.v[k] = 0.25f * (((a.v[k] + b.v[k]) + c.v[k]) + d.v[k]);
-        st8(y + pix * C + 8 * g, a);
-    }
-}
-
 // ReLU's backward mask on the BF16-rounded gradient: zero where the forward output y is not positive
 __device__ __forceinline__ void mask8(F8& v, const bf16* y) {
     const F8 m = ld8(y);
@@ -547,8 +528,7 @@ struct Ctx {
     size_t P(int level) const { return (size_t)n * H(level) * W(level); }
 };
 
-// The convolution, and (when `fuse` is given) the pooling / upsampling pass after it: the
-// persistent conv kernel does that work in its epilogue where it can, else the pass runs here.
+// The convolution, with what `f` asks its epilogue to do besides; true: it pooled as well.
 bool conv_fwd(Ctx& c, int li, int level, TRef x, TRef y, ConvFuse f = ConvFuse()) {
     const Layer& l = c.d.L[li];
     f.settled = li > 0; // behind the first convolution, whatever wrote the weights is complete
@@ -586,15 +566,12 @@ void conv_bwd(Ctx& c, int li, int level, TRef x, TRef dz, TRef gx, bool mask) {
 TRef T(Acts& a, int k) { return TRef{a.at(k), kT[k].c, 0, kT[k].c}; }
 TRef S(Acts& a, int k, int off, int cnt) { return TRef{a.at(k), kT[k].c, off, cnt}; }
 
-void pool_fwd(Ctx& c, TRef x, int level, TRef y) {
-    const size_t n = c.P(level + 1) * x.c / 8;
-    launch_overlapped(k_pool_fwd, dim3(grid_for(n)), dim3(256), 0, c.st, x.p, x.cs, x.co, x.c, c.n, c.H(level), c.W(level), y.p);
-}
-// conv into y, then 2x2 pooling of y into `pooled` (at level + 1)
+// conv into y, and 2x2 pooling of y into `pooled` (at level + 1) in the convolution's epilogue: for the
+// network's layers (at most 128 channels at even sizes) both convolution kernels do it
 void conv_pool(Ctx& c, int li, int level, TRef x, TRef y, TRef pooled) {
     ConvFuse f;
     f.pool_out = pooled.p;
-    if (!conv_fwd(c, li, level, x, y, f)) pool_fwd(c, y, level, pooled);
+    KF_REQUIRE(conv_fwd(c, li, level, x, y, f), KF_ERR_INTERNAL, "a convolution did not pool its output");
 }
 // conv, then nearest 2x upsampling of its output into the channel slice `up` (at level - 1), both
 // in the convolution's epilogue; the output itself goes to y where a backward pass will read it.
@@ -654,13 +631,13 @@ void forward(Ctx& c, const float* base, float* out, bool in16 = false) {
 
 void pool_bwd_add(Ctx& c, TRef gy_low, TRef gskip, int level_hi, TRef y, TRef gx) {
     const size_t n = c.P(level_hi) * gx.c / 8;
-    launch_overlapped(k_pool_bwd_add, dim3(grid_for(n)), dim3(256), 0, c.st, gy_low.p, gskip.p, gskip.cs, gskip.co, gx.c, c.n, c.H(level_hi),
-                                                   c.W(level_hi), y.p, y.cs, y.co, gx.p);
+    launch_overlapped(k_pool_bwd_add, dim3(grid_for(n)), dim3(256), 0, c.st, gy_low.p, gskip.p, gskip.cs, gskip.co,
+                      gx.c, c.n, c.H(level_hi), c.W(level_hi), y.p, y.cs, y.co, gx.p);
 }
 void up_bwd(Ctx& c, TRef gy_slice, int level_hi, TRef y, TRef gx_low) {
     const size_t n = c.P(level_hi + 1) * gx_low.c / 8;
-    launch_overlapped(k_up_bwd, dim3(grid_for(n)), dim3(256), 0, c.st, gy_slice.p, gy_slice.cs, gy_slice.co, gx_low.c, c.n, c.H(level_hi),
-                                             c.W(level_hi), y.p, gx_low.p);
+    launch_overlapped(k_up_bwd, dim3(grid_for(n)), dim3(256), 0, c.st, gy_slice.p, gy_slice.cs, gy_slice.co, gx_low.c,
+                      c.n, c.H(level_hi), c.W(level_hi), y.p, gx_low.p);
 }
 
 // Every gradient tensor G_* of a ReLU layer's output holds dL/dz: the ReLU's mask is applied by

@@ -364,6 +364,4 @@ KF_DEV bool closer(float t, uint32_t inst, uint32_t prim, float bt, uint32_t bin
     return false;
 }
 
-KF_DEV float4 ldg4(const float4* p) { return __ldg(p); }
-
 } // namespace kf

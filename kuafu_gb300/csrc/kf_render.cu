@@ -272,9 +272,9 @@ bool runs_whole_paths(const kf_renderer_s* r, bool lit, uint64_t npaths) {
 // the radiance. What bounce d+1 writes of that (the NEE records, requests, contributions and
 // the radiance of the paths) is written by k_miss / k_shade, which wait for the gather (the
 // join). The tail (k_paths), which finishes the paths when few are left, reads and writes what
-// the gather does and sits behind the join, too. Counters are per bounce and cleared once per chunk, after the last gather of the
-// chunk before it. A launch without lights has no NEE: one stream, three kernels per bounce.
-// With `profile` everything runs on one stream with events around the kernel groups.
+// the gather does and sits behind the join, too. Counters are per bounce and cleared once per
+// chunk, after the last gather of the chunk before it. A launch without lights has no NEE: one
+// stream, three kernels per bounce. With `profile` everything runs on one stream with events around the kernel groups.
 static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* fd, const BatchDev& b,
                           const WaveDev& w, uint32_t max_depth, uint64_t npaths, uint32_t chunk, bool profile) {
     cudaStream_t st = r->stream, st2 = profile ? r->stream : r->stream2;
@@ -301,7 +301,8 @@ static void enqueue_paths(kf_renderer_s* r, const SceneDev& sv, const FrameDev* 
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[0], st));
             if (dyn)
                 launch_trace_dyn(sv, fd, b, w, cur, depth, start, false,
-                                 trace_grid(depth ? r->grid_dyn : r->grid_dyn_camera, rays), r->count_traversal, r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
+                                 trace_grid(depth ? r->grid_dyn : r->grid_dyn_camera, rays), r->count_traversal,
+                                 r->cfg.dyn_refill_below, r->cfg.dyn_steps, st);
             else
                 launch_extend(sv, fd, b, w, cur, depth, start, r->grid_extend, r->count_traversal, st);
             if (profile) KF_CUDA_CHECK(cudaEventRecord(r->ev[1], st));

@@ -11,7 +11,9 @@
 //   nee      light samples -> one shadow queue per light   (rchit:204-316)
 //   shadow   any-hit occlusion of the shadow queues        (rchit:175-200)
 //   gather   ordered NEE sum into the path radiance        (rchit:457-460, rgen:111)
-// then a per-pixel resolve (rgen:140-166) and the sRGB frame (PostProcessing.frag).
+// then a per-pixel resolve (rgen:140-166) with the sRGB frame (PostProcessing.frag). Small frames, and
+// the last paths of a lit wavefront, run path by path instead: paths, one kernel from the camera
+// ray (or a bounce's hits) to the end, same steps and streams.
 // Queues are compacted in order: a block scan per tile with one atomic per tile (warp
 // ballots + one atomic per warp where the warps of a block differ). A launch whose views have
 // no lights to sample skips nee, shadow and gather.
@@ -394,7 +396,7 @@ template <bool SHADOW, bool COUNT, bool VOTE> struct Tracer {
     }
 };
 
-// smem: the block's shared stack area (kSmemStack * kThreadsTrace words).
+// smem: the block's shared area, kSmemTrace words (the stacks, and the world rays behind them).
 template <bool SHADOW, bool COUNT>
 __device__ bool trace(const SceneDev& s, uint32_t root, uint32_t* smem, float ox, float oy, float oz, float dx,
                       float dy, float dz, float tmin, float tmax, HitOut& h, TraceCounters& cnt,
@@ -963,9 +965,6 @@ __device__ bool light_sample(const SceneDev& s, const LS& ls, uint32_t slot, uin
 }
 
 // ---------------------------------------------------------------------------
-// Shade: miss / emission / PrincipledBSDF (rchit:322-468), light samples, RR.
-// ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // Rays that missed (PathTrace.rmiss:12-31): environment map, else clear colour, added with
 // the path weight; the path ends. The rays that hit are listed in w.sel for k_shade, so
 // that its warps shade hits only.
@@ -1109,7 +1108,7 @@ __device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, c
         const v3 wn = mk(ln.x * m0.x + ln.y * m1.x + ln.z * m2.x, ln.x * m0.y + ln.y * m1.y + ln.z * m2.y,
                          ln.x * m0.z + ln.y * m1.z + ln.z * m2.z);
         o.N = normalize(wn);
-                            o.worldPos = rayO + rayD * hv.x;
+        o.worldPos = rayO + rayD * hv.x;
         const float uvx = a2v.y * bx + b2.y * by + c2.y * bz;
         const float uvy = a2v.z * bx + b2.z * by + c2.z * bz;
         // facing in object space: front when dir opposes (v1-v0)x(v2-v0)
@@ -1235,7 +1234,7 @@ __device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, c
         uint4* aov_seg = BATCH ? vw.it->seg : w.seg;
         if (aov_seg) {
             const uint32_t gidx = __ldg(&s.inst[inst].geometry);
-                const uint32_t midx = __ldg(s.matidx + __ldg(s.geom + gidx).y + prim);
+            const uint32_t midx = __ldg(s.matidx + __ldg(s.geom + gidx).y + prim);
             aov_seg[pix] = BATCH ? make_uint4(inst - vw.it->inst_base, gidx - vw.it->geom_base, midx, prim)
                                  : make_uint4(inst, gidx, midx, prim);
         }
@@ -1245,7 +1244,7 @@ __device__ __forceinline__ void shade_hit(const SceneDev& s, const WaveDev& w, c
 // Blocks of the shading kernels (k_shade, k_nee).
 constexpr uint32_t kShadeThreads = 128, kShadeWarps = kShadeThreads / 32;
 
-template <bool BATCH>
+// Hits shaded (rchit:322-468, rgen:109-138): emission, the PrincipledBSDF's sample, Russian roulette.
 // Bound by the latency of its five dependent levels of loads (list, hit, instance, indices,
 // vertices): 8 resident blocks per SM (64 registers, 44 bytes spilled) hide more of it than 4 to 6
 // without a spill. A Cornell room of 256 x 256 at 64 spp takes 3.03 ms with 4 or 5 blocks, 2.85 with 6,
@@ -1253,6 +1252,7 @@ template <bool BATCH>
 // The next rays of a block's 128 hits are sorted by direction octant, so that a warp's rays, whose
 // origins are near each other already, also meet nodes in a similar order: the room 2.59 -> 2.53 ms,
 // the batch 46.5 -> 46.2, 256 icospheres 17.11 -> 17.06 (tiles of 256 the same, 512 slower by 1 %).
+template <bool BATCH>
 __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(SceneDev s, const FrameDev* __restrict__ fp, BatchDev b, WaveDev w,
                                                int cur, uint32_t depth, uint64_t chunk_start) {
     const uint32_t count = w.counters[depth * kCounterRow + 1]; // rays that hit (k_miss takes the others)
